@@ -191,6 +191,91 @@ def run(state):
     raise ValueError(f"unknown kind {kind!r}")
 
 
+def _int4_rows64(A, packed, scale, group, tok, ids, E, N):
+    """[slots, N] float64: A[tok] @ W[ids]^T; the weight is what the format says, code x scale rounded to bf16"""
+    shifts = 4 * torch.arange(8, device=A.device, dtype=torch.int32)
+    out = torch.zeros(ids.numel(), N, dtype=torch.float64, device=A.device)
+    for e in range(E):
+        at = (ids == e).nonzero(as_tuple=True)[0]
+        if at.numel() == 0:
+            continue
+        codes = ((packed[e].unsqueeze(-1) >> shifts) & 15).reshape(N, -1) - 8
+        W = (codes.float() * scale[e].float().repeat_interleave(group, dim=1)).to(torch.bfloat16).double()
+        out[at] = A[tok[at]].double() @ W.t()
+    return out
+
+
+def _silu_up64(gate, up, limit):
+    if limit:
+        gate, up = gate.clamp(max=limit), up.clamp(-limit, limit)
+    return gate * torch.sigmoid(gate) * up
+
+
+def _mx64(w, scale, e):
+    """[rows, K] float64 weights of expert e: E2M1 codes (low nibble = even k) x 2^(byte - 127)"""
+    table = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, -0.0, -0.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64,
+                         device=w.device)
+    codes = torch.stack([w[e] & 15, w[e] >> 4], dim=-1).reshape(w.shape[1], -1)
+    return table[codes.long()] * torch.exp2(scale[e].double() - 127).repeat_interleave(32, dim=1)
+
+
+def _combine64(rows, w, M, top_k):
+    return (rows * w.reshape(-1, 1).double()).reshape(M, top_k, -1).sum(dim=1)
+
+
+def exact(case, seed):
+    """``run``'s outputs in 64 bits from plain torch.  Weights are what their formats say; no other rounding."""
+    st = prepare(case, seed)
+    kind = case["kind"]
+    if kind == "align":
+        return None
+    if kind == "router":
+        p = torch.softmax(st["x"].double(), dim=-1)
+        w = torch.topk(p, st["topk"], dim=-1).values
+        return (w / w.sum(dim=-1, keepdim=True) if st["renorm"] else w), None
+    if kind == "reduce":
+        return torch.cat([(y.double() * w.double().unsqueeze(-1)).sum(dim=1)
+                          for y, w in zip(st["y"].split(1024), st["w"].split(1024))])
+    if kind == "ep":
+        R, k = case["R"], case["top_k"]
+        ids, w = st["routing"][:, :k].reshape(-1), st["routing"][:, k:].contiguous().view(torch.float32)
+        tok = torch.arange(R, device=ids.device).repeat_interleave(k)
+        rows = _combine64(_int4_rows64(st["A"], st["packed"], st["scale"], 32, tok, ids, case["E"], case["N"]), w, R, k)
+        at = st["index"].long()
+        return rows, (rows[at.clamp(min=0)] * (at >= 0).unsqueeze(-1)).sum(dim=1)
+    ids, w, M, k = st["ids"].reshape(-1), st["w"], case["M"], case["top_k"]
+    tok = torch.arange(M, device=ids.device).repeat_interleave(k)
+    if kind == "int4":
+        out = torch.zeros(M, case["N"], dtype=torch.float64, device=ids.device)
+        step = max(1, 65536 // k)
+        for lo in range(0, M, step):
+            hi = min(M, lo + step)
+            s = slice(lo * k, hi * k)
+            rows = _int4_rows64(st["A"], st["packed"], st["scale"], st["group"], tok[s], ids[s], case["E"], case["N"])
+            out[lo:hi] = _combine64(rows, w[lo:hi], hi - lo, k)
+        return out
+    if kind == "ffn":
+        I = case["inter"]
+        gu = _int4_rows64(st["A"], st["w13"], st["s13"], 32, tok, ids, case["E"], 2 * I)
+        act = _silu_up64(gu[:, :I], gu[:, I:], 0.0)
+        slot = torch.arange(M * k, device=ids.device)
+        return _combine64(_int4_rows64(act, st["w2"], st["s2"], 32, slot, ids, case["E"], case["hidden"]), w, M, k)
+    if kind == "mxfp4":
+        t, I = st["wts"], case["ispp"]
+        rows = torch.zeros(M * k, case["hidden"], dtype=torch.float64, device=ids.device)
+        for e in range(case["E"]):
+            at = (ids == e).nonzero(as_tuple=True)[0]
+            if at.numel() == 0:
+                continue
+            gu = st["A"][tok[at]].double() @ _mx64(t["w13"], t["w13_scale"], e).t()
+            if t["b13"] is not None:
+                gu = gu + t["b13"][e].double()
+            down = _silu_up64(gu[:, :I], gu[:, I:], 10.0) @ _mx64(t["w2"], t["w2_scale"], e).t()
+            rows[at] = down if t["b2"] is None else down + t["b2"][e].double()
+        return _combine64(rows, w, M, k)
+    raise ValueError(f"unknown kind {kind!r}")
+
+
 def _active(E, slots):
     """experts hit by `slots` slots, each token's distinct"""
     return min(E, E * (1.0 - (1.0 - 1.0 / E) ** slots))
