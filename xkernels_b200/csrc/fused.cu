@@ -112,6 +112,10 @@ Routing make_routing(const RoutingBuffers& b, int64_t numel, int E, int block) {
   return r;
 }
 
+bool tma_base_ok(const void* a, const void* b) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+}
+
 }  // namespace
 }  // namespace xkb
 
@@ -167,8 +171,10 @@ static int int4_impl(const void* A, int a_dtype, const int32_t* packed, const vo
   if (rows_out != nullptr) scratch = rows_out;
   void* tc_ws = carve.take<char>(int4_tc_workspace_bytes(numel, N, K, E));
 
-  const bool tc_fit = int4_tc_supported(a_dtype, M, N, K, E, top_k, group_size);
-  if (path == XKB_PATH_TC && !tc_fit)
+  // (the other groups came to the tcgen05 path later: weights that TMA cannot read keep the generic kernel there)
+  const bool tc_fit = int4_tc_supported(a_dtype, M, N, K, E, top_k, group_size) &&
+                      (group_size == 32 || tma_base_ok(packed, scale));
+  if (path == XKB_PATH_TC && !(tc_fit && group_size == 32))
     return fail(XKB_ERR_ARG,
                 "fused_moe_int4_w4a16: shape not supported by the tcgen05 path (needs bf16 A, "
                 "N %% 128 == 0, K %% 256 == 0, group_size 32)");
@@ -181,8 +187,8 @@ static int int4_impl(const void* A, int a_dtype, const int32_t* packed, const vo
                         rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream);
   if (rc != XKB_OK) return rc;
   if (use_tc)
-    rc = launch_int4_tc(A, packed, scale, r, topk_w, scratch, N, K, E, top_k, mul_routed_weight,
-                        tc_ws, rb.status, stream);
+    rc = launch_int4_tc(A, packed, scale, r, topk_w, scratch, N, K, E, top_k, group_size,
+                        mul_routed_weight, tc_ws, rb.status, stream);
   else
     rc = launch_int4_simt(A, a_dtype, packed, scale, r, topk_w, scratch, N, K, top_k, group_size,
                           mul_routed_weight, stream);
@@ -313,8 +319,9 @@ extern "C" int xkb_fused_moe_int4_ffn(const void* A, int a_dtype, const int32_t*
   void* act = carve.take<float>(routing_max_pad(numel, E, kMaxBlock) * inter);
   void* tc_ws = carve.take<char>(int4_tc_workspace_bytes(numel, hidden, hidden, E));
 
-  const bool tc_fit = int4_ffn_tc_supported(a_dtype, M, hidden, inter, E, top_k, group_size);
-  if (path == XKB_PATH_TC && !tc_fit)
+  const bool tc_fit = int4_ffn_tc_supported(a_dtype, M, hidden, inter, E, top_k, group_size) &&
+                      (group_size == 32 || (tma_base_ok(w13_packed, w13_scale) && tma_base_ok(w2_packed, w2_scale)));
+  if (path == XKB_PATH_TC && !(tc_fit && group_size == 32))
     return fail(XKB_ERR_ARG, "fused_moe_int4_ffn: shape not supported by the tcgen05 path (needs bf16 A, "
                              "hidden %% 256 == 0, inter %% 256 == 0, group_size 32)");
   const bool use_tc = (path == XKB_PATH_TC) || (path == XKB_PATH_AUTO && tc_fit);
@@ -326,7 +333,7 @@ extern "C" int xkb_fused_moe_int4_ffn(const void* A, int a_dtype, const int32_t*
   if (rc != XKB_OK) return rc;
   if (use_tc)
     rc = launch_int4_ffn_tc(A, w13_packed, w13_scale, w2_packed, w2_scale, r, topk_w, static_cast<__nv_bfloat16*>(act),
-                            scratch, hidden, inter, E, top_k, swiglu_limit, tc_ws, rb.status, stream);
+                            scratch, hidden, inter, E, top_k, group_size, swiglu_limit, tc_ws, rb.status, stream);
   else
     rc = launch_int4_ffn_simt(A, a_dtype, w13_packed, w13_scale, w2_packed, w2_scale, r, topk_ids, expert_map, num_map,
                               E, topk_w, rows1, act, scratch, hidden, inter, top_k, group_size, swiglu_limit, stream);

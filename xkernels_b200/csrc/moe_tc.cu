@@ -215,6 +215,7 @@ struct TcParams {
   int64_t numel;
   int N, K;                     // tile rows are taken from N rows per expert; K = contraction length
   int mul_w;
+  int group_shift;              // INT4: log2 of the scale group (5 .. 8)
   int round_rows;               // INT4: round each weighted slot row to bf16 (the second GEMM of a two-GEMM layer,
                                 // whose per-slot results the reference composition holds in bf16)
   // MXFP4 only
@@ -436,7 +437,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           if (mode_is_int4(MODE)) {
             mbar_expect_tx(&w_full[st], kPackedStageBytes + kScaleStageBytes);
             tma_load_2d(s_packed + st * kPackedStageBytes, &tm_packed, &w_full[st], ks * (kStageK / 2), row0);
-            tma_load_2d(s_scale + st * kScaleStageBytes, &tm_scale, &w_full[st], ks * (kStageK / 32), row0);
+            // eight scales per row: the stage's own at group 32, those of 2 / 4 / 8 stages at groups 64 / 128 / 256
+            // (sixteen bytes are the smallest TMA row and x must be a multiple of them)
+            tma_load_2d(s_scale + st * kScaleStageBytes, &tm_scale, &w_full[st], ((ks * kStageK) >> p.group_shift) & ~7, row0);
           } else {  // e8m0 scales: 16 bytes per row = the scales of stages ks & ~1 and ks | 1
             mbar_expect_tx(&w_full[st], kPackedStageBytes + kScaleStageBytes);
             tma_load_2d(s_packed + st * kPackedStageBytes, &tm_packed, &w_full[st], ks * (kStageK / 2), row0);
@@ -741,8 +744,15 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         const uint32_t pk = s_packed_u32 + wst * kPackedStageBytes + row * 128;
         uint2 sw = make_uint2(0, 0);  // INT4: the kChunks bf16 group scales of this share; MXFP4: .x = its e8m0 bytes
         if (mode_is_int4(MODE)) {
-          if (kChunks == 4) sw = lds64(s_scale_u32 + wst * kScaleStageBytes + row * 16 + part * 8);
-          else sw.x = lds32(s_scale_u32 + wst * kScaleStageBytes + row * 16 + part * 4);
+          const uint32_t sa = s_scale_u32 + wst * kScaleStageBytes + row * 16;
+          if (p.group_shift == 5) {
+            if (kChunks == 4) sw = lds64(sa + part * 8);
+            else sw.x = lds32(sa + part * 4);
+          } else {  // two chunks or more share a scale: the first and the third chunk's, each twice
+            const uint32_t k0 = (uint32_t)(vs / kMats) * kStageK + (uint32_t)(part * kChunks) * 32u;
+            sw.x = lds16(sa + ((k0 >> p.group_shift) & 7u) * 2u) * 0x00010001u;
+            if (kChunks == 4) sw.y = lds16(sa + (((k0 + 64u) >> p.group_shift) & 7u) * 2u) * 0x00010001u;
+          }
         } else {  // the kChunks e8m0 bytes of this share: this stage's half of the row's sixteen
           const uint32_t sa = s_scale_u32 + wst * kScaleStageBytes + row * 16 + (((vs / kMats) & 1) << 3) + part * kChunks;
           if (kChunks == 4) sw.x = lds32(sa);
@@ -1026,8 +1036,17 @@ int launch_bt(const CUtensorMap& tmp, const CUtensorMap& tms, const CUtensorMap&
 
 }  // namespace
 
+// Scale groups the tcgen05 path takes: 32, and 64 / 128 / 256 where a row's bf16 scales are whole 16-byte
+// TMA rows (K a multiple of eight groups).  The generic kernel is the alternative and reads the weights
+// once per 16-token block with scalar arithmetic: 2530 us there against 206 us here for the whole call at
+// E=48, N=4096, K=7168, top_k=8, M=64, group 128 (0.73 GB of weights: 109 us at the copy rate).
+static bool int4_tc_group(int group, int64_t K) {
+  return group == 32 || ((group == 64 || group == 128 || group == 256) && K % (8 * (int64_t)group) == 0);
+}
+static int log2_of(int x) { int n = 0; while ((1 << (n + 1)) <= x) ++n; return n; }
+
 bool int4_tc_supported(int a_dtype, int64_t M, int64_t N, int64_t K, int E, int top_k, int group) {
-  return a_dtype == XKB_BF16 && group == 32 && N > 0 && N % kTileRows == 0 && K > 0 && K % kStageK == 0 &&
+  return a_dtype == XKB_BF16 && int4_tc_group(group, K) && N > 0 && N % kTileRows == 0 && K > 0 && K % kStageK == 0 &&
          M > 0 && E > 0 && top_k > 0 && (int64_t)E * N < (1ll << 31) && K < (1 << 30);
 }
 
@@ -1065,7 +1084,7 @@ static int launch_int4_by_block(const CUtensorMap& tm_packed, const CUtensorMap&
 }
 
 int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, const Routing& r,
-                   const float* topk_w, float* scratch, int64_t N, int64_t K, int E, int top_k, int mul_w,
+                   const float* topk_w, float* scratch, int64_t N, int64_t K, int E, int top_k, int group, int mul_w,
                    void* tc_ws, int* status, cudaStream_t stream) {
   Carver carve(tc_ws);
   __nv_bfloat16* Ag = carve.take<__nv_bfloat16>(r.max_pad * K);
@@ -1081,7 +1100,7 @@ int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, cons
   int rc = make_map_2d(&tm_packed, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, packed, (uint64_t)E * N, (uint64_t)K / 2,
                        kTileRows, kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "packed weights");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, scale, (uint64_t)E * N, (uint64_t)K / 32,
+  rc = make_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, scale, (uint64_t)E * N, (uint64_t)(K / group),
                    kTileRows, kStageK / 32, CU_TENSOR_MAP_SWIZZLE_NONE, "group scales");
   if (rc != XKB_OK) return rc;
   rc = make_map_2d(&tm_tokens, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Ag, (uint64_t)r.max_pad, (uint64_t)K,
@@ -1101,6 +1120,7 @@ int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, cons
   prm.N = (int)N;
   prm.K = (int)K;
   prm.mul_w = mul_w;
+  prm.group_shift = log2_of(group);
   prm.round_rows = 0;
   prm.bias = nullptr;
   prm.act = nullptr;
@@ -1118,14 +1138,16 @@ int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, cons
 // second fused_moe_int4_w4a16 call and moe_sum_reduce).
 // ---------------------------------------------------------------------------
 bool int4_ffn_tc_supported(int a_dtype, int64_t M, int64_t hidden, int64_t inter, int E, int top_k, int group) {
-  return a_dtype == XKB_BF16 && group == 32 && M > 0 && E > 0 && top_k > 0 && hidden > 0 && inter > 0 &&
+  return a_dtype == XKB_BF16 && int4_tc_group(group, hidden) && int4_tc_group(group, inter) && M > 0 && E > 0 &&
+         top_k > 0 && hidden > 0 && inter > 0 &&
          hidden % kStageK == 0 && inter % kStageK == 0 &&   // both are contraction lengths and tile-row counts
          (int64_t)E * 2 * inter < (1ll << 31) && (int64_t)E * hidden < (1ll << 31);
 }
 
 int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const int32_t* w2, const void* s2,
                        const Routing& r, const float* topk_w, __nv_bfloat16* act, float* scratch, int64_t hidden,
-                       int64_t inter, int E, int top_k, float limit, void* tc_ws, int* status, cudaStream_t stream) {
+                       int64_t inter, int E, int top_k, int group, float limit, void* tc_ws, int* status,
+                       cudaStream_t stream) {
   Carver carve(tc_ws);
   int32_t* done = r.block_counters != nullptr ? r.block_counters + r.counters_each : nullptr;   // block hand-over counters
   __nv_bfloat16* Ag = carve.take<__nv_bfloat16>(r.max_pad * hidden);
@@ -1138,13 +1160,13 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
   int rc = make_map_2d(&tm_w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w13, (uint64_t)E * 2 * inter, (uint64_t)hidden / 2,
                        kTileRows, kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "w13 packed weights");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_s13, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s13, (uint64_t)E * 2 * inter, (uint64_t)hidden / 32,
+  rc = make_map_2d(&tm_s13, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s13, (uint64_t)E * 2 * inter, (uint64_t)(hidden / group),
                    kTileRows, kStageK / 32, CU_TENSOR_MAP_SWIZZLE_NONE, "w13 group scales");
   if (rc != XKB_OK) return rc;
   rc = make_map_2d(&tm_w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w2, (uint64_t)E * hidden, (uint64_t)inter / 2, kTileRows,
                    kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "w2 packed weights");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_s2, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s2, (uint64_t)E * hidden, (uint64_t)inter / 32,
+  rc = make_map_2d(&tm_s2, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s2, (uint64_t)E * hidden, (uint64_t)(inter / group),
                    kTileRows, kStageK / 32, CU_TENSOR_MAP_SWIZZLE_NONE, "w2 group scales");
   if (rc != XKB_OK) return rc;
   rc = make_map_2d(&tm_tok0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Ag, (uint64_t)r.max_pad, (uint64_t)hidden,
@@ -1164,6 +1186,7 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
   prm.max_blocks = (int)r.max_blocks;
   prm.num_experts = E;
   prm.bias = nullptr;
+  prm.group_shift = log2_of(group);
   prm.limit = limit;
   // gate_up + SwiGLU -> act
   prm.scratch = nullptr;
@@ -1271,6 +1294,7 @@ int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   prm.max_blocks = (int)r.max_blocks;
   prm.num_experts = E;
   prm.mul_w = mul_w;
+  prm.group_shift = 5;
   prm.round_rows = 0;
   prm.limit = limit;
   // stage 0: gate_up + SwiGLU -> act
