@@ -6,9 +6,16 @@
 // selected weights are optionally divided by their sum.  Equal logits give equal probabilities
 // here as there, so the tie rule decides the same way.
 //
-// One warp per token row: lane l holds experts l, l + 32, ...; row maximum and sum by shuffles;
-// k rounds of "best of my lane, then best of the warp" on the key (probability, -id).
-
+// One warp per token row: lane l holds experts l, l + 32, ...; row maximum and sum by shuffles.
+//
+// Bound by the warp's instructions, not by memory (a row of 256 bf16 logits is 512 bytes).  k rounds of
+// "best of my lane, then best of the warp" over all experts cost about 900 instructions per row, so the
+// selection first cuts the row down to a handful of candidates: the k-th largest of the 32 lane maxima
+// bounds the k-th largest element from below, usually 8 to 16 of the experts reach it, and only those
+// are divided by the sum (one per lane), ranked against each other and written.  Rows that leave more
+// than 32 candidates (long runs of equal logits), a top-k above 32 or a sum that is not finite take the
+// rounds (select_by_rounds), which order every probability of the row.
+// M=16384, E=256, bf16, top 8, renormalised: 28.7 -> 11.8 us on the device (15.5 us a call, host-bound).
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -31,40 +38,10 @@ __device__ __forceinline__ bool better(float pa, int ia, float pb, int ib) {
   return pa > pb || (pa == pb && ia < ib);
 }
 
-template <typename T, int PER_LANE>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
-topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, int32_t* __restrict__ topk_ids,
-                    int64_t M, int E, int topk, int renormalize) {
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (row >= M) return;
-  const T* x = gating + row * E;
-
-  float p[PER_LANE];
-  float mx = -INFINITY;
-#pragma unroll
-  for (int t = 0; t < PER_LANE; ++t) {
-    const int e = lane + 32 * t;
-    p[t] = e < E ? load_logit<T>(x + e) : -INFINITY;
-    mx = fmaxf(mx, p[t]);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  float sum = 0.f;
-#pragma unroll
-  for (int t = 0; t < PER_LANE; ++t) {
-    const int e = lane + 32 * t;
-    p[t] = e < E ? expf(p[t] - mx) : 0.f;
-    sum += p[t];
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-#pragma unroll
-  for (int t = 0; t < PER_LANE; ++t) {
-    const int e = lane + 32 * t;
-    p[t] = e < E ? p[t] / sum : -1.f;   // -1 marks "not a candidate" (probabilities are >= 0)
-  }
-
+// k rounds over the whole row: p[t] = probability of expert lane + 32 t, or -1 where there is none.
+template <int PER_LANE>
+__device__ __noinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t row, int lane, int topk, int renormalize,
+                                              float* __restrict__ topk_w, int32_t* __restrict__ topk_ids) {
   float wsum = 0.f;
   float my_w = 0.f;     // lane j keeps the j-th selected weight (j < 32), further ones go out directly
   for (int j = 0; j < topk; ++j) {
@@ -100,6 +77,97 @@ topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, in
     if (lane < topk) topk_w[row * topk + lane] = my_w / wsum;
     if (lane == 0)
       for (int j = 32; j < topk; ++j) topk_w[row * topk + j] = topk_w[row * topk + j] / wsum;
+  }
+}
+
+template <typename T, int PER_LANE>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, int32_t* __restrict__ topk_ids,
+                    int64_t M, int E, int topk, int renormalize) {
+  __shared__ uint64_t s_cand[kWarpsPerBlock][32];   // candidates, then their sort keys
+  __shared__ float s_w[kWarpsPerBlock][32];         // the selected weights in order
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
+  if (row >= M) return;
+  const T* x = gating + row * E;
+
+  float p[PER_LANE];
+  float mx = -INFINITY;
+#pragma unroll
+  for (int t = 0; t < PER_LANE; ++t) {
+    const int e = lane + 32 * t;
+    p[t] = e < E ? load_logit<T>(x + e) : -INFINITY;
+    mx = fmaxf(mx, p[t]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  float sum = 0.f;
+  float lane_max = -1.f;
+#pragma unroll
+  for (int t = 0; t < PER_LANE; ++t) {
+    const int e = lane + 32 * t;
+    p[t] = e < E ? expf(p[t] - mx) : 0.f;
+    sum += p[t];
+    p[t] = e < E ? p[t] : -1.f;    // -1 marks "not a candidate" (exponentials are >= 0)
+    lane_max = fmaxf(lane_max, p[t]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+
+  // The k-th largest lane maximum (equal ones leave together, so it may be a smaller one: still a bound).
+  // The floats are >= 0 or -1, and as signed integers they order the same way.
+  int tau = -1, lm = __float_as_int(lane_max);
+  const bool short_way = topk <= 32 && sum < INFINITY;   // (a NaN sum fails the comparison)
+  if (short_way) {
+    for (int j = 0; j < topk; ++j) {
+      tau = __reduce_max_sync(0xffffffffu, lm);
+      if (lm == tau) lm = __float_as_int(-1.f);
+    }
+  }
+  // Division by the sum is monotone but may round neighbours to one probability, and then the smaller id
+  // wins: exponentials a few units in the last place below the bound are candidates as well.
+  const float bound = (short_way && tau >= 0) ? __int_as_float(tau) * (1.f - 9.5367431640625e-7f) : -1.f;
+  int n = 0;
+  uint64_t* cand = s_cand[warp];
+#pragma unroll
+  for (int t = 0; t < PER_LANE; ++t) {
+    const bool c = p[t] >= bound && p[t] >= 0.f;
+    const unsigned who = __ballot_sync(0xffffffffu, c);
+    const int at = n + __popc(who & ((1u << lane) - 1u));
+    if (c && at < 32) cand[at] = ((uint64_t)__float_as_uint(p[t]) << 32) | (uint32_t)(lane + 32 * t);
+    n += __popc(who);
+  }
+  if (!short_way || n > 32) {
+#pragma unroll
+    for (int t = 0; t < PER_LANE; ++t) p[t] = lane + 32 * t < E ? p[t] / sum : -1.f;
+    select_by_rounds<PER_LANE>(p, row, lane, topk, renormalize, topk_w, topk_ids);
+    return;
+  }
+  // one candidate per lane: probability, then a key whose larger value is the better one
+  __syncwarp();
+  float prob = -1.f;
+  uint64_t key = 0;
+  if (lane < n) {
+    const uint64_t v = cand[lane];
+    prob = __uint_as_float((uint32_t)(v >> 32)) / sum;
+    key = ((uint64_t)__float_as_uint(prob) << 32) | (uint32_t)~(uint32_t)v;
+  }
+  __syncwarp();
+  cand[lane] = key;
+  __syncwarp();
+  int rank = 0;
+  for (int j = 0; j < n; ++j) rank += cand[j] > key ? 1 : 0;
+  const bool selected = lane < n && rank < topk;   // keys differ in the id: ranks 0 .. topk - 1 are all taken
+  float wsum = 1.f;
+  if (renormalize) {
+    if (selected) s_w[warp][rank] = prob;
+    __syncwarp();
+    wsum = 0.f;
+    for (int j = 0; j < topk; ++j) wsum += s_w[warp][j];
+  }
+  if (selected) {
+    topk_ids[row * topk + rank] = (int32_t)~(uint32_t)key;
+    topk_w[row * topk + rank] = renormalize ? prob / wsum : prob;
   }
 }
 
