@@ -9,8 +9,14 @@
 // + (# same-expert lanes below it in its warp)             -> __match_any_sync ballot
 // Counters only ever count, so atomics never decide an output position.
 //
-// numel <= kSmallMax runs as ONE single-CTA kernel; larger inputs use three
-// launches (count -> offsets -> scatter) over 1024-slot chunks.
+// Latency-bound: a call moves about a megabyte at most, so what counts is the number of dependent steps.
+// numel <= kSmallMax (a decode batch) runs as ONE single-CTA kernel with one pass over the ids: the ranks
+// of the slots and the expert counts come out of the same warp x expert matrix.  Larger inputs use two
+// launches over at most kMaxChunks chunks of whole 1024-slot rounds: count, then place.  Every CTA of the
+// second adds up the chunk x expert matrix for itself (a few hundred KB from L2 at most) instead of waiting
+// for a single-CTA scan between the two, and is launched while the first still runs.
+// M=16384, top_k=8, E=48, block 16: 10.5 us on the device for the two launches (7.5 of it the second), 29.4 ->
+// 24.7 us a call (host-bound); the fused calls lose a memset launch besides, 49.1 -> 45.7 us at M=1.
 #include "common.cuh"
 
 namespace xkb {
@@ -18,8 +24,9 @@ namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
-constexpr int kChunk = kThreads;       // slots per chunk (one per thread)
-constexpr int64_t kSmallMax = 8192;    // single-CTA path up to this many slots
+constexpr int kChunk = kThreads;       // slots per round (one per thread)
+constexpr int64_t kSmallMax = kChunk;  // single-CTA path up to this many slots
+constexpr int kMaxChunks = 148;        // CTAs of the two-launch path: one wave
 constexpr int kMaxExperts = 1024;
 
 __device__ __forceinline__ int map_expert(int id, int E, const int32_t* expert_map, int num_map) {
@@ -84,14 +91,13 @@ __device__ void write_expert_ids(const int* off, int E, int block, int32_t* expe
   }
 }
 
-// One 1024-slot round of the stable scatter.  `base[e]` = position of the first
-// slot of expert e that belongs to this round.  wcnt: [kWarps][E+1] uint16.
-// tot[e] receives the number of slots of expert e in this round.
-__device__ void scatter_round(int my_e, bool active, int64_t slot, const int* base, int E,
-                              uint16_t* wcnt, int* tot, int32_t* sorted_ids) {
+// Rank of this thread's slot among the slots of its expert in one 1024-slot round (0 if inactive), and the
+// round's slots per expert in tot[0 .. E].  wcnt: [kWarps][E+1] uint16.
+__device__ int round_rank(int my_e, bool active, int E, uint16_t* wcnt, int* tot) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int EP = E + 1;
-  for (int i = tid; i < kWarps * EP; i += kThreads) wcnt[i] = 0;
+  uint32_t* wcnt2 = reinterpret_cast<uint32_t*>(wcnt);
+  for (int i = tid; i < kWarps * EP / 2; i += kThreads) wcnt2[i] = 0;   // kWarps is even
   __syncthreads();
   // inactive lanes vote with a key no expert uses so they never match
   const int key = active ? my_e : (EP + lane);
@@ -112,144 +118,141 @@ __device__ void scatter_round(int my_e, bool active, int64_t slot, const int* ba
     if (lane == 31) tot[e] = incl;
   }
   __syncthreads();
-  if (active && my_e < E) {
-    const int pos = base[my_e] + (int)wcnt[warp * EP + my_e] + rank;
-    sorted_ids[pos] = (int32_t)slot;
-  }
+  return active ? (int)wcnt[warp * EP + my_e] + rank : 0;
 }
 
 // ---------------------------------------------------------------------------
-// Single-CTA path
+// Single-CTA path: numel <= 1024.  zero / zero_n: ints the caller wants cleared (nullptr, 0: none).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads)
 align_small_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int E, int block,
                    const int32_t* __restrict__ expert_map, int num_map,
                    int32_t* __restrict__ sorted_ids, int64_t max_pad,
                    int32_t* __restrict__ expert_ids, int64_t max_blocks,
-                   int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out) {
+                   int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out,
+                   int32_t* __restrict__ zero, int64_t zero_n) {
   chain_trigger();   // a kernel chained behind this one may be launched; it waits for completion itself
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int EP = E + 1;
-  int* hist = reinterpret_cast<int*>(smem_raw);   // [EP]
-  int* off = hist + EP;                            // [EP]   off[E] = total
-  int* run = off + EP;                             // [EP]   running base per expert
-  int* tot = run + EP;                             // [EP]
-  int* warp_tot = tot + EP;                        // [kWarps]
-  uint16_t* wcnt = reinterpret_cast<uint16_t*>(warp_tot + kWarps);  // [kWarps][EP]
+  uint16_t* wcnt = reinterpret_cast<uint16_t*>(smem_raw);                 // [kWarps][EP]
+  int* off = reinterpret_cast<int*>(smem_raw + kWarps * EP * sizeof(uint16_t));   // [EP]   off[E] = total
+  int* tot = off + EP;                                                    // [EP]
+  int* warp_tot = tot + EP;                                               // [kWarps]
   const int tid = threadIdx.x;
-
-  for (int i = tid; i < EP; i += kThreads) hist[i] = 0;
-  __syncthreads();
-  for (int64_t s = tid; s < numel; s += kThreads)
-    atomicAdd(&hist[map_expert(topk_ids[s], E, expert_map, num_map)], 1);
-  __syncthreads();
-  padded_offsets(hist, off, warp_tot, E, block);
-  for (int i = tid; i < EP; i += kThreads) run[i] = (i < E) ? off[i] : 0;
+  const bool active = tid < numel;
+  const int e = active ? map_expert(topk_ids[tid], E, expert_map, num_map) : E;
+  for (int64_t i = tid; i < zero_n; i += kThreads) zero[i] = 0;
+  for (int64_t i = tid; i < max_pad; i += kThreads) sorted_ids[i] = (int32_t)numel;
+  const int rank = round_rank(e, active, E, wcnt, tot);
+  padded_offsets(tot, off, warp_tot, E, block);
+  // (the barriers in between order the fill above before these stores of other threads)
+  if (active && e < E) sorted_ids[off[e] + rank] = tid;
   if (tid == 0) num_post[0] = off[E];
   if (expert_off_out != nullptr)
     for (int i = tid; i < EP; i += kThreads) expert_off_out[i] = off[i];
-  for (int64_t i = tid; i < max_pad; i += kThreads) sorted_ids[i] = (int32_t)numel;
   write_expert_ids(off, E, block, expert_ids, max_blocks, tid, kThreads);
-  __syncthreads();
-  const int64_t rounds = (numel + kChunk - 1) / kChunk;
-  for (int64_t r = 0; r < rounds; ++r) {
-    const int64_t slot = r * kChunk + tid;
-    const bool active = slot < numel;
-    const int e = active ? map_expert(topk_ids[slot], E, expert_map, num_map) : E;
-    scatter_round(e, active, slot, run, E, wcnt, tot, sorted_ids);
-    __syncthreads();
-    for (int i = tid; i < E; i += kThreads) run[i] += tot[i];
-    __syncthreads();
-  }
 }
 
 // ---------------------------------------------------------------------------
-// Multi-CTA path: count -> offsets -> scatter over 1024-slot chunks
+// Two-launch path: count -> place, chunk c = slots [c * span, (c + 1) * span), span a multiple of 1024
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads)
-align_count_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int E,
+align_count_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t span, int E,
                    const int32_t* __restrict__ expert_map, int num_map,
                    int32_t* __restrict__ chunk_cnt /*[C][E+1]*/,
-                   int32_t* __restrict__ sorted_ids, int64_t max_pad) {
+                   int32_t* __restrict__ sorted_ids, int64_t max_pad, int32_t* __restrict__ zero, int64_t zero_n) {
+  chain_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int* hist = reinterpret_cast<int*>(smem_raw);
   const int EP = E + 1, tid = threadIdx.x;
   for (int i = tid; i < EP; i += kThreads) hist[i] = 0;
   __syncthreads();
-  const int64_t slot = (int64_t)blockIdx.x * kChunk + tid;
-  if (slot < numel) atomicAdd(&hist[map_expert(topk_ids[slot], E, expert_map, num_map)], 1);
+  const int64_t first = (int64_t)blockIdx.x * span;
+  const int64_t last = first + span < numel ? first + span : numel;
+  for (int64_t slot = first + tid; slot < last; slot += kThreads)
+    atomicAdd(&hist[map_expert(topk_ids[slot], E, expert_map, num_map)], 1);
   // pre-fill this CTA's slice of sorted_ids with the padding id
   const int64_t per = (max_pad + gridDim.x - 1) / gridDim.x;
   const int64_t lo = (int64_t)blockIdx.x * per;
   const int64_t hi = (lo + per < max_pad) ? lo + per : max_pad;
   for (int64_t i = lo + tid; i < hi; i += kThreads) sorted_ids[i] = (int32_t)numel;
+  for (int64_t i = (int64_t)blockIdx.x * kThreads + tid; i < zero_n; i += (int64_t)gridDim.x * kThreads) zero[i] = 0;
   __syncthreads();
   for (int i = tid; i < EP; i += kThreads) chunk_cnt[(int64_t)blockIdx.x * EP + i] = hist[i];
 }
 
 __global__ void __launch_bounds__(kThreads)
-align_offsets_kernel(int32_t* __restrict__ chunk_cnt /*in: counts, out: exclusive bases*/,
-                     int C, int E, int block, int32_t* __restrict__ expert_ids,
-                     int64_t max_blocks, int32_t* __restrict__ num_post,
-                     int32_t* __restrict__ expert_off_g /*[E+1], always written*/) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int EP = E + 1;
-  int* hist = reinterpret_cast<int*>(smem_raw);  // [EP]
-  int* off = hist + EP;                           // [EP]
-  int* warp_tot = off + EP;                       // [kWarps]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // per expert: exclusive scan of its counts over the chunks (warp per expert)
-  for (int e = warp; e < EP; e += kWarps) {
-    int carry = 0;
-    for (int c0 = 0; c0 < C; c0 += 32) {
-      const int c = c0 + lane;
-      int v = (c < C) ? chunk_cnt[(int64_t)c * EP + e] : 0;
-      int incl = v;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        int u = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += u;
-      }
-      if (c < C) chunk_cnt[(int64_t)c * EP + e] = carry + incl - v;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) hist[e] = carry;
-  }
-  __syncthreads();
-  padded_offsets(hist, off, warp_tot, E, block);
-  if (tid == 0) num_post[0] = off[E];
-  for (int i = tid; i < EP; i += kThreads) expert_off_g[i] = off[i];
-  write_expert_ids(off, E, block, expert_ids, max_blocks, tid, kThreads);
-}
-
-__global__ void __launch_bounds__(kThreads)
-align_scatter_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int E,
-                     const int32_t* __restrict__ expert_map, int num_map,
-                     const int32_t* __restrict__ chunk_base /*[C][E+1]*/,
-                     const int32_t* __restrict__ expert_off_g, int32_t* __restrict__ sorted_ids) {
+align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t span, int E, int block,
+                   const int32_t* __restrict__ expert_map, int num_map,
+                   const int32_t* chunk_cnt /*[C][E+1]: written by the kernel this one overlaps*/,
+                   int32_t* sorted_ids, int32_t* __restrict__ expert_ids, int64_t max_blocks,
+                   int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out) {
   chain_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int EP = E + 1;
-  int* base = reinterpret_cast<int*>(smem_raw);   // [EP]
-  int* tot = base + EP;                            // [EP]
-  uint16_t* wcnt = reinterpret_cast<uint16_t*>(tot + EP);
-  const int tid = threadIdx.x;
-  for (int i = tid; i < EP; i += kThreads)
-    base[i] = (i < E) ? expert_off_g[i] + chunk_base[(int64_t)blockIdx.x * EP + i] : 0;
-  const int64_t slot = (int64_t)blockIdx.x * kChunk + tid;
-  const bool active = slot < numel;
-  const int e = active ? map_expert(topk_ids[slot], E, expert_map, num_map) : E;
+  const int EP = E + 1, tid = threadIdx.x, C = (int)gridDim.x;
+  uint16_t* wcnt = reinterpret_cast<uint16_t*>(smem_raw);                 // [kWarps][EP]
+  int* off = reinterpret_cast<int*>(smem_raw + kWarps * EP * sizeof(uint16_t));   // [EP]   off[E] = total
+  int* base = off + EP;                                                   // [EP]   next position per expert
+  int* tot = base + EP;                                                   // [EP]
+  int* warp_tot = tot + EP;                                               // [kWarps]
+  for (int i = tid; i < EP; i += kThreads) base[i] = tot[i] = 0;
   __syncthreads();
-  scatter_round(e, active, slot, base, E, wcnt, tot, sorted_ids);
+  const int64_t first = (int64_t)blockIdx.x * span;
+  const int64_t last = first + span < numel ? first + span : numel;
+  int64_t slot = first + tid;
+  bool active = slot < last;
+  int e = active ? map_expert(topk_ids[slot], E, expert_map, num_map) : E;   // an input of the call, not of the kernel before
+  chain_wait();
+  // slots per expert in all chunks (tot) and in the chunks before this one (base): threads side by side
+  // take neighbouring experts, the groups of threads share the chunks out
+  const int width = E < kThreads ? (E > 0 ? E : 1) : kThreads;
+  const int groups = kThreads / width, grp = tid / width;
+  if (grp < groups) {
+    for (int x = tid - grp * width; x < E; x += width) {
+      int all = 0, before = 0;
+#pragma unroll 8
+      for (int c = grp; c < C; c += groups) {
+        const int v = __ldcg(chunk_cnt + (int64_t)c * EP + x);
+        all += v;
+        if (c < (int)blockIdx.x) before += v;
+      }
+      if (all != 0) atomicAdd(&tot[x], all);
+      if (before != 0) atomicAdd(&base[x], before);
+    }
+  }
+  __syncthreads();
+  padded_offsets(tot, off, warp_tot, E, block);
+  for (int i = tid; i < E; i += kThreads) base[i] += off[i];
+  if (blockIdx.x == 0) {
+    if (tid == 0) num_post[0] = off[E];
+    if (expert_off_out != nullptr)
+      for (int i = tid; i < EP; i += kThreads) expert_off_out[i] = off[i];
+  }
+  write_expert_ids(off, E, block, expert_ids, max_blocks, (int)blockIdx.x * kThreads + tid, C * kThreads);
+  __syncthreads();
+  for (int64_t s0 = first; s0 < last; s0 += kThreads) {
+    if (s0 != first) {
+      slot = s0 + tid;
+      active = slot < last;
+      e = active ? map_expert(topk_ids[slot], E, expert_map, num_map) : E;
+    }
+    const int rank = round_rank(e, active, E, wcnt, tot);
+    if (active && e < E) sorted_ids[base[e] + rank] = (int32_t)slot;
+    if (s0 + kThreads < last) {
+      __syncthreads();
+      for (int i = tid; i < E; i += kThreads) base[i] += tot[i];
+      __syncthreads();
+    }
+  }
 }
 
 size_t small_smem(int E) {
   const size_t EP = E + 1;
-  return 4 * EP * sizeof(int) + kWarps * sizeof(int) + kWarps * EP * sizeof(uint16_t) + 16;
+  return kWarps * EP * sizeof(uint16_t) + 2 * EP * sizeof(int) + kWarps * sizeof(int);
 }
-size_t scatter_smem(int E) {
+size_t place_smem(int E) {
   const size_t EP = E + 1;
-  return 2 * EP * sizeof(int) + kWarps * EP * sizeof(uint16_t) + 16;
+  return kWarps * EP * sizeof(uint16_t) + 3 * EP * sizeof(int) + kWarps * sizeof(int);
 }
 
 template <typename K>
@@ -262,14 +265,14 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
 
 int64_t align_workspace_bytes(int64_t numel, int num_experts) {
   const int64_t C = ceil_div(numel > 0 ? numel : 1, kChunk);
-  // chunk x expert matrix + a private expert_off copy
+  // at least the chunk x expert matrix (callers size buffers by this formula: it stays as it is)
   return align_up(C * (num_experts + 1) * 4, 256) + align_up((int64_t)(num_experts + 1) * 4, 256);
 }
 
 int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
                  const int32_t* expert_map, int num_map, int32_t* sorted_ids,
                  int32_t* expert_ids, int32_t* num_post, int32_t* expert_off,
-                 void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
+                 void* workspace, int64_t workspace_bytes, cudaStream_t stream, int32_t* zero, int64_t zero_n) {
   XKB_REQUIRE(numel >= 0 && numel < (1ll << 30), "moe_align: numel=%lld out of range", (long long)numel);
   XKB_REQUIRE(block > 0, "moe_align: block_size must be > 0 (got %d)", block);
   XKB_REQUIRE(E >= 0 && E <= kMaxExperts, "moe_align: num_experts=%d outside [0,%d]", E, kMaxExperts);
@@ -282,7 +285,7 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
     XKB_CHECK_CUDA(allow_smem(align_small_kernel, smem));
     align_small_kernel<<<1, kThreads, smem, stream>>>(topk_ids, numel, E, block, expert_map, num_map,
                                                       sorted_ids, max_pad, expert_ids, max_blocks,
-                                                      num_post, expert_off);
+                                                      num_post, expert_off, zero, zero_n);
     XKB_CHECK_LAUNCH("align_small_kernel");
     return XKB_OK;
   }
@@ -290,24 +293,19 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
   if (workspace == nullptr || workspace_bytes < need)
     return fail(XKB_ERR_WORKSPACE, "moe_align: workspace of %lld bytes needed, %lld given",
                 (long long)need, (long long)workspace_bytes);
-  const int C = (int)ceil_div(numel, kChunk);
-  Carver carve(workspace);
-  int32_t* chunk_cnt = carve.take<int32_t>((int64_t)C * (E + 1));
-  int32_t* off_priv = carve.take<int32_t>(E + 1);
-  int32_t* off_g = expert_off ? expert_off : off_priv;
-  const size_t smem1 = (size_t)(E + 1) * sizeof(int) + 16;
-  const size_t smem2 = (size_t)(2 * (E + 1) + kWarps) * sizeof(int) + 16;
-  const size_t smem3 = scatter_smem(E);
-  XKB_CHECK_CUDA(allow_smem(align_scatter_kernel, smem3));
-  align_count_kernel<<<C, kThreads, smem1, stream>>>(topk_ids, numel, E, expert_map, num_map,
-                                                     chunk_cnt, sorted_ids, max_pad);
+  const int64_t span = ceil_div(numel, (int64_t)kMaxChunks * kChunk) * kChunk;
+  const int C = (int)ceil_div(numel, span);
+  int32_t* chunk_cnt = static_cast<int32_t*>(workspace);
+  const size_t smem1 = (size_t)(E + 1) * sizeof(int);
+  const size_t smem2 = place_smem(E);
+  XKB_CHECK_CUDA(allow_smem(align_place_kernel, smem2));
+  align_count_kernel<<<C, kThreads, smem1, stream>>>(topk_ids, numel, span, E, expert_map, num_map,
+                                                     chunk_cnt, sorted_ids, max_pad, zero, zero_n);
   XKB_CHECK_LAUNCH("align_count_kernel");
-  align_offsets_kernel<<<1, kThreads, smem2, stream>>>(chunk_cnt, C, E, block, expert_ids, max_blocks,
-                                                       num_post, off_g);
-  XKB_CHECK_LAUNCH("align_offsets_kernel");
-  align_scatter_kernel<<<C, kThreads, smem3, stream>>>(topk_ids, numel, E, expert_map, num_map,
-                                                       chunk_cnt, off_g, sorted_ids);
-  XKB_CHECK_LAUNCH("align_scatter_kernel");
+  XKB_CHECK_CUDA(launch_chained(align_place_kernel, dim3((unsigned)C), dim3(kThreads), smem2, stream, topk_ids, numel,
+                                span, E, block, expert_map, num_map, chunk_cnt, sorted_ids, expert_ids, max_blocks,
+                                num_post, expert_off));
+  XKB_CHECK_LAUNCH("align_place_kernel");
   return XKB_OK;
 }
 
@@ -390,7 +388,7 @@ extern "C" int xkb_moe_align_block_size_static(const int32_t* topk_ids, int64_t 
   const int rc = static_scratch_address(&scratch);
   if (rc != XKB_OK) return rc;
   // Nothing in the scratch has to start at zero: the count kernel writes every entry of the
-  // chunk x expert matrix that the later kernels read, and the offsets slice is fully rewritten.
+  // chunk x expert matrix that the place kernel reads.
   return launch_align(topk_ids, numel, num_experts, block_size, expert_map, num_map, sorted_ids,
                       expert_ids, num_post_pad, expert_offsets, scratch,
                       kStaticInts * (int64_t)sizeof(int32_t), static_cast<cudaStream_t>(stream));

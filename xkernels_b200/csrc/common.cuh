@@ -82,7 +82,8 @@ struct Routing {
 int launch_align(const int32_t* topk_ids, int64_t numel, int num_experts, int block_size,
                  const int32_t* expert_map, int num_map, int32_t* sorted_ids,
                  int32_t* expert_ids, int32_t* num_post, int32_t* expert_off,
-                 void* workspace, int64_t workspace_bytes, cudaStream_t stream);
+                 void* workspace, int64_t workspace_bytes, cudaStream_t stream,
+                 int32_t* zero = nullptr, int64_t zero_n = 0);   // zero_n ints at `zero` are cleared on the way
 int64_t align_workspace_bytes(int64_t numel, int num_experts);
 
 // out[m,n] = sum_j scratch[m*top_k+j, n] over the slots whose (mapped) expert id lies in [0, E)

@@ -52,7 +52,7 @@ namespace {
 
 struct RoutingBuffers {
   int* status;
-  int32_t* counters;        // directly behind the status header: one memset clears both
+  int32_t* counters;        // directly behind the status header: cleared as one span
   int64_t counters_each;
   int32_t* sorted_ids;
   int32_t* expert_ids;
@@ -87,9 +87,7 @@ RoutingBuffers carve_routing(Carver& c, int64_t numel, int E) {
 }
 
 // status header and the block counters behind it, as one span
-size_t header_bytes(const RoutingBuffers& r) {
-  return (size_t)(reinterpret_cast<const char*>(r.counters + 2 * r.counters_each) - reinterpret_cast<const char*>(r.status));
-}
+int64_t header_ints(const RoutingBuffers& r) { return r.counters + 2 * r.counters_each - r.status; }
 
 int64_t routing_bytes(int64_t numel, int E) {
   Carver c(nullptr);
@@ -182,9 +180,9 @@ static int int4_impl(const void* A, int a_dtype, const int32_t* packed, const vo
   const int block = use_tc ? int4_tc_block(numel, E) : kSimtBlock;
 
   Routing r = make_routing(rb, numel, E, block);
-  XKB_CHECK_CUDA(cudaMemsetAsync(rb.status, 0, header_bytes(rb), stream));   // status word + block counters
+  // (the align stage clears the status word and the block counters on its way)
   int rc = launch_align(topk_ids, numel, E, block, expert_map, num_map, rb.sorted_ids, rb.expert_ids,
-                        rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream);
+                        rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb));
   if (rc != XKB_OK) return rc;
   if (use_tc)
     rc = launch_int4_tc(A, packed, scale, r, topk_w, scratch, N, K, E, top_k, group_size,
@@ -327,9 +325,9 @@ extern "C" int xkb_fused_moe_int4_ffn(const void* A, int a_dtype, const int32_t*
   const bool use_tc = (path == XKB_PATH_TC) || (path == XKB_PATH_AUTO && tc_fit);
   const int block = use_tc ? int4_tc_block(numel, E) : kSimtBlock;
   Routing r = make_routing(rb, numel, E, block);
-  XKB_CHECK_CUDA(cudaMemsetAsync(rb.status, 0, header_bytes(rb), stream));   // status word + block counters
+  // (the align stage clears the status word and the block counters on its way)
   int rc = launch_align(topk_ids, numel, E, block, expert_map, num_map, rb.sorted_ids, rb.expert_ids, rb.num_post,
-                        rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream);
+                        rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb));
   if (rc != XKB_OK) return rc;
   if (use_tc)
     rc = launch_int4_ffn_tc(A, w13_packed, w13_scale, w2_packed, w2_scale, r, topk_w, static_cast<__nv_bfloat16*>(act),
@@ -397,9 +395,9 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
   const int block = use_tc ? mxfp4_tc_block(numel, E) : kSimtBlock;
 
   Routing r = make_routing(rb, numel, E, block);
-  XKB_CHECK_CUDA(cudaMemsetAsync(rb.status, 0, header_bytes(rb), stream));   // status word + block counters
+  // (the align stage clears the status word and the block counters on its way)
   int rc = launch_align(topk_ids, numel, E, block, expert_map, num_map, rb.sorted_ids, rb.expert_ids,
-                        rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream);
+                        rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb));
   if (rc != XKB_OK) return rc;
   if (use_tc)
     rc = launch_mxfp4_tc(A, w13, w13_scale, w2, w2_scale, b13, b2, r, topk_w, act, scratch, hidden,
