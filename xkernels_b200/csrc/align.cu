@@ -130,7 +130,7 @@ align_small_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int E, i
                    int32_t* __restrict__ sorted_ids, int64_t max_pad,
                    int32_t* __restrict__ expert_ids, int64_t max_blocks,
                    int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out,
-                   int32_t* __restrict__ zero, int64_t zero_n) {
+                   int32_t* __restrict__ slot_pos, int32_t* __restrict__ zero, int64_t zero_n) {
   chain_trigger();   // a kernel chained behind this one may be launched; it waits for completion itself
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int EP = E + 1;
@@ -147,6 +147,7 @@ align_small_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int E, i
   padded_offsets(tot, off, warp_tot, E, block);
   // (the barriers in between order the fill above before these stores of other threads)
   if (active && e < E) sorted_ids[off[e] + rank] = tid;
+  if (active && slot_pos != nullptr) slot_pos[tid] = e < E ? off[e] + rank : -1;
   if (tid == 0) num_post[0] = off[E];
   if (expert_off_out != nullptr)
     for (int i = tid; i < EP; i += kThreads) expert_off_out[i] = off[i];
@@ -186,7 +187,8 @@ align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t 
                    const int32_t* __restrict__ expert_map, int num_map,
                    const int32_t* chunk_cnt /*[C][E+1]: written by the kernel this one overlaps*/,
                    int32_t* sorted_ids, int32_t* __restrict__ expert_ids, int64_t max_blocks,
-                   int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out) {
+                   int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out,
+                   int32_t* __restrict__ slot_pos) {
   chain_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int EP = E + 1, tid = threadIdx.x, C = (int)gridDim.x;
@@ -238,6 +240,7 @@ align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t 
     }
     const int rank = round_rank(e, active, E, wcnt, tot);
     if (active && e < E) sorted_ids[base[e] + rank] = (int32_t)slot;
+    if (active && slot_pos != nullptr) slot_pos[slot] = e < E ? base[e] + rank : -1;
     if (s0 + kThreads < last) {
       __syncthreads();
       for (int i = tid; i < E; i += kThreads) base[i] += tot[i];
@@ -272,7 +275,8 @@ int64_t align_workspace_bytes(int64_t numel, int num_experts) {
 int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
                  const int32_t* expert_map, int num_map, int32_t* sorted_ids,
                  int32_t* expert_ids, int32_t* num_post, int32_t* expert_off,
-                 void* workspace, int64_t workspace_bytes, cudaStream_t stream, int32_t* zero, int64_t zero_n) {
+                 void* workspace, int64_t workspace_bytes, cudaStream_t stream, int32_t* zero, int64_t zero_n,
+                 int32_t* slot_pos) {
   XKB_REQUIRE(numel >= 0 && numel < (1ll << 30), "moe_align: numel=%lld out of range", (long long)numel);
   XKB_REQUIRE(block > 0, "moe_align: block_size must be > 0 (got %d)", block);
   XKB_REQUIRE(E >= 0 && E <= kMaxExperts, "moe_align: num_experts=%d outside [0,%d]", E, kMaxExperts);
@@ -285,7 +289,7 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
     XKB_CHECK_CUDA(allow_smem(align_small_kernel, smem));
     align_small_kernel<<<1, kThreads, smem, stream>>>(topk_ids, numel, E, block, expert_map, num_map,
                                                       sorted_ids, max_pad, expert_ids, max_blocks,
-                                                      num_post, expert_off, zero, zero_n);
+                                                      num_post, expert_off, slot_pos, zero, zero_n);
     XKB_CHECK_LAUNCH("align_small_kernel");
     return XKB_OK;
   }
@@ -304,7 +308,7 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
   XKB_CHECK_LAUNCH("align_count_kernel");
   XKB_CHECK_CUDA(launch_chained(align_place_kernel, dim3((unsigned)C), dim3(kThreads), smem2, stream, topk_ids, numel,
                                 span, E, block, expert_map, num_map, chunk_cnt, sorted_ids, expert_ids, max_blocks,
-                                num_post, expert_off));
+                                num_post, expert_off, slot_pos));
   XKB_CHECK_LAUNCH("align_place_kernel");
   return XKB_OK;
 }

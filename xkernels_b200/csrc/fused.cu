@@ -58,6 +58,7 @@ struct RoutingBuffers {
   int32_t* expert_ids;
   int32_t* num_post;
   int32_t* expert_off;
+  int32_t* slot_pos;
   void* align_ws;
   int64_t align_ws_bytes;
 };
@@ -81,6 +82,7 @@ RoutingBuffers carve_routing(Carver& c, int64_t numel, int E) {
   r.expert_ids = c.take<int32_t>(ceil_div(routing_max_pad(numel, E, kMinBlock), kMinBlock) + 1);
   r.num_post = c.take<int32_t>(1);
   r.expert_off = c.take<int32_t>(E + 1);
+  r.slot_pos = c.take<int32_t>(numel);
   r.align_ws_bytes = align_workspace_bytes(numel, E);
   r.align_ws = c.take<char>(r.align_ws_bytes);
   return r;
@@ -101,6 +103,7 @@ Routing make_routing(const RoutingBuffers& b, int64_t numel, int E, int block) {
   r.expert_ids = b.expert_ids;
   r.num_post = b.num_post;
   r.expert_off = b.expert_off;
+  r.slot_pos = b.slot_pos;
   r.numel = numel;
   r.block = block;
   r.max_pad = routing_max_pad(numel, E, block);
@@ -182,7 +185,8 @@ static int int4_impl(const void* A, int a_dtype, const int32_t* packed, const vo
   Routing r = make_routing(rb, numel, E, block);
   // (the align stage clears the status word and the block counters on its way)
   int rc = launch_align(topk_ids, numel, E, block, expert_map, num_map, rb.sorted_ids, rb.expert_ids,
-                        rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb));
+                        rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb),
+                        rb.slot_pos);
   if (rc != XKB_OK) return rc;
   if (use_tc)
     rc = launch_int4_tc(A, packed, scale, r, topk_w, scratch, N, K, E, top_k, group_size,
@@ -327,7 +331,8 @@ extern "C" int xkb_fused_moe_int4_ffn(const void* A, int a_dtype, const int32_t*
   Routing r = make_routing(rb, numel, E, block);
   // (the align stage clears the status word and the block counters on its way)
   int rc = launch_align(topk_ids, numel, E, block, expert_map, num_map, rb.sorted_ids, rb.expert_ids, rb.num_post,
-                        rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb));
+                        rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb),
+                        rb.slot_pos);
   if (rc != XKB_OK) return rc;
   if (use_tc)
     rc = launch_int4_ffn_tc(A, w13_packed, w13_scale, w2_packed, w2_scale, r, topk_w, static_cast<__nv_bfloat16*>(act),
@@ -397,7 +402,8 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
   Routing r = make_routing(rb, numel, E, block);
   // (the align stage clears the status word and the block counters on its way)
   int rc = launch_align(topk_ids, numel, E, block, expert_map, num_map, rb.sorted_ids, rb.expert_ids,
-                        rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb));
+                        rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb),
+                        rb.slot_pos);
   if (rc != XKB_OK) return rc;
   if (use_tc)
     rc = launch_mxfp4_tc(A, w13, w13_scale, w2, w2_scale, b13, b2, r, topk_w, act, scratch, hidden,

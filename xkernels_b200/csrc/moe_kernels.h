@@ -6,6 +6,17 @@ namespace xkb {
 
 constexpr int kSimtBlock = 16;  // align block the SIMT kernels consume
 
+// ---- activation gathers: one thread per 8 elements, blocks of one token or a piece of one ----
+constexpr int kGatherThreads = 256;
+inline int gather_grid(int64_t M, int64_t units, unsigned* pieces, unsigned* threads, unsigned* blocks) {
+  const int64_t p = ceil_div(units, kGatherThreads);
+  XKB_REQUIRE(p * M <= 0x7fffffff, "activation gather: %lld blocks do not fit a grid", (long long)(p * M));
+  *pieces = (unsigned)p;
+  *threads = (unsigned)align_up(ceil_div(units, p), 32);
+  *blocks = (unsigned)(p * M);
+  return XKB_OK;
+}
+
 // ---- generic SIMT path (moe_simt.cu) ---------------------------------------
 int launch_int4_simt(const void* A, int a_dtype, const int32_t* packed, const void* scale,
                      const Routing& r, const float* topk_w, float* scratch, int64_t N, int64_t K,
@@ -15,6 +26,8 @@ int launch_mxfp4_simt(const void* A, int a_dtype, const uint8_t* w13, const uint
                       const Routing& r, const float* topk_w, __nv_bfloat16* act, float* scratch,
                       int64_t hidden, int64_t ispp, int top_k, float limit, int mul_w,
                       cudaStream_t stream);
+
+constexpr int kErrBadRouting = 3;   // status code: a routing value read by a kernel was outside what the buffers can hold
 
 // ---- tcgen05 path (moe_tc.cu) ----------------------------------------------
 bool int4_tc_supported(int a_dtype, int64_t M, int64_t N, int64_t K, int E, int top_k, int group);

@@ -293,7 +293,6 @@ constexpr int kMxShift = 62;
 constexpr float kMxUnscale = 4611686018427387904.f;   // 2^62
 constexpr uint32_t kMxMaxScale = 190;
 constexpr int kErrMxScaleRange = 2;                  // status code: an e8m0 scale byte in 191..254
-constexpr int kErrBadRouting = 3;    // status code: a routing value read by a kernel was outside what the buffers can hold
 __device__ __forceinline__ uint32_t mx_scale_factor(uint32_t s) {
   // exponent field of 2^(s - 1 - kMxShift), twice; 0 for the NaN code
   const uint32_t f = (s + (uint32_t)(126 - kMxShift)) * 0x00800080u;
@@ -390,7 +389,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
   // the second, so the wait cannot deadlock; it is bounded all the same.  The first GEMM lets its
   // dependents go only after its own wait for the kernels before it, so that what those wrote (the
   // routing) is visible to the second GEMM although it skips its wait; the counters are cleared
-  // together with the status word by the memset that opens the fused call.
+  // together with the status word by the align stage.
   const bool hand_over_first = mode_is_gate_up(MODE) && p.done_signal != nullptr;
   const bool hand_over_second = p.done_wait != nullptr;
   if (!hand_over_first) chain_trigger();   // the next kernel may be launched; it waits for this one's completion itself
@@ -885,14 +884,32 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
 }
 
 // ---------------------------------------------------------------------------
-// Activation gather: Ag[p, :] = A[sorted_ids[p] / top_k, :] with the nibble-order
-// permutation (0,4,1,5,2,6,3,7) applied inside every group of 8 K elements.
-// Padding positions are left untouched: their accumulator columns are never read.
+// Activation gather: Ag[slot_pos[s], :] = A[s / top_k, :] with the nibble-order permutation
+// (0,4,1,5,2,6,3,7) applied inside every group of 8 K elements.  Padding positions are left untouched:
+// their accumulator columns are never read.
+//
+// HBM-bound at prefill.  A block takes one token (a piece of its columns when there are few tokens), reads
+// the row once and writes it to the positions of all its slots: going through the positions instead reads
+// A once per slot, and at prefill A is larger than L2
+// (M=16384, K=7168, top_k=8, E=48: 612 -> 355 us).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-gather_permute_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* sorted_ids,
-                      const int32_t* num_post, __nv_bfloat16* __restrict__ Ag, int64_t numel,
-                      int K, int top_k, int permute, int64_t max_pad, int* __restrict__ status) {
+__global__ void __launch_bounds__(kGatherThreads)
+gather_permute_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos, __nv_bfloat16* __restrict__ Ag,
+                      int K, int top_k, int permute, int64_t max_pad, unsigned pieces, int* __restrict__ status) {
+  const unsigned m = blockIdx.x / pieces;
+  const int i = (int)((blockIdx.x - m * pieces) * blockDim.x + threadIdx.x);
+  const bool mine = i < K / 8;
+  uint4 o = make_uint4(0, 0, 0, 0);
+  if (mine) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(A + (int64_t)m * K) + i);  // elements (e1:e0, e3:e2, e5:e4, e7:e6); an input of the call
+    o = v;                                  // consumers that convert in natural K order
+    if (permute) {
+      o.x = __byte_perm(v.x, v.z, 0x5410);  // (e4 : e0)
+      o.y = __byte_perm(v.x, v.z, 0x7632);  // (e5 : e1)
+      o.z = __byte_perm(v.y, v.w, 0x5410);  // (e6 : e2)
+      o.w = __byte_perm(v.y, v.w, 0x7632);  // (e7 : e3)
+    }
+  }
   // The routing comes from the align kernel before this one, which may still be running when this
   // kernel starts.  It is read with L2 loads after the wait and through pointers that are NOT
   // `const __restrict__`: loads the compiler may treat as invariant (ld.global.nc) were seen to
@@ -900,25 +917,14 @@ gather_permute_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* sorted
   // the non-coherent cache).
   chain_wait();
   chain_trigger();
-  int total = __ldcg(num_post);
-  if (total < 0 || total > max_pad) {   // never with a routing the align stage wrote: recorded, nothing gathered
-    if (threadIdx.x == 0 && blockIdx.x == 0) atomicCAS(status, 0, kErrBadRouting + (3 << 8));
-    total = 0;
-  }
-  for (int64_t pos = blockIdx.x; pos < total; pos += gridDim.x) {
-    const int32_t slot = __ldcg(sorted_ids + pos);
-    if (slot < 0 || slot >= numel) continue;
-    const uint4* src = reinterpret_cast<const uint4*>(A + (int64_t)(slot / top_k) * K);
-    uint4* dst = reinterpret_cast<uint4*>(Ag + pos * K);
-    for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
-      const uint4 v = __ldg(src + i);  // elements e0..e7 as (e1:e0, e3:e2, e5:e4, e7:e6)
-      if (!permute) { dst[i] = v; continue; }   // consumers that convert in natural K order
-      uint4 o;
-      o.x = __byte_perm(v.x, v.z, 0x5410);  // (e4 : e0)
-      o.y = __byte_perm(v.x, v.z, 0x7632);  // (e5 : e1)
-      o.z = __byte_perm(v.y, v.w, 0x5410);  // (e6 : e2)
-      o.w = __byte_perm(v.y, v.w, 0x7632);  // (e7 : e3)
-      dst[i] = o;
+  const int lane = threadIdx.x & 31;
+  for (int j0 = 0; j0 < top_k; j0 += 32) {   // the positions of up to 32 slots in one load
+    const int32_t mine_pos = j0 + lane < top_k ? __ldcg(slot_pos + (int64_t)m * top_k + j0 + lane) : -1;
+    if (mine_pos >= max_pad) atomicCAS(status, 0, kErrBadRouting + (3 << 8));   // never with a routing the align stage wrote
+    unsigned live = __ballot_sync(0xffffffffu, mine_pos >= 0 && mine_pos < max_pad);
+    for (; live != 0; live &= live - 1) {
+      const int32_t pos = __shfl_sync(0xffffffffu, mine_pos, __ffs(live) - 1);
+      if (mine) reinterpret_cast<uint4*>(Ag + (int64_t)pos * K)[i] = o;
     }
   }
 }
@@ -992,6 +998,18 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const 
     g_map_cache.keys[slot] = key;
     g_map_cache.maps[slot] = *map;
   }
+  return XKB_OK;
+}
+
+int launch_gather(const void* A, const Routing& r, __nv_bfloat16* Ag, int64_t K, int top_k, int permute, int* status,
+                  cudaStream_t stream) {
+  unsigned pieces, threads, blocks;
+  const int rc = gather_grid(r.numel / top_k, K / 8, &pieces, &threads, &blocks);
+  if (rc != XKB_OK) return rc;
+  XKB_CHECK_CUDA(launch_chained(gather_permute_kernel, dim3(blocks), dim3(threads), 0, stream,
+                                static_cast<const __nv_bfloat16*>(A), r.slot_pos, Ag, (int)K, top_k, permute, r.max_pad,
+                                pieces, status));
+  XKB_CHECK_LAUNCH("gather_permute_kernel");
   return XKB_OK;
 }
 
@@ -1089,15 +1107,11 @@ int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, cons
   Carver carve(tc_ws);
   __nv_bfloat16* Ag = carve.take<__nv_bfloat16>(r.max_pad * K);
 
-  int64_t gblocks = r.max_pad < 148 * 16 ? r.max_pad : 148 * 16;
-  if (gblocks < 1) gblocks = 1;
-  XKB_CHECK_CUDA(launch_chained(gather_permute_kernel, dim3((unsigned)gblocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(A),
-                                                               r.sorted_ids, r.num_post, Ag, r.numel, (int)K,
-                                                               top_k, 1, r.max_pad, status));
-  XKB_CHECK_LAUNCH("gather_permute_kernel");
+  int rc = launch_gather(A, r, Ag, K, top_k, 1, status, stream);
+  if (rc != XKB_OK) return rc;
 
   CUtensorMap tm_packed, tm_scale, tm_tokens;
-  int rc = make_map_2d(&tm_packed, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, packed, (uint64_t)E * N, (uint64_t)K / 2,
+  rc = make_map_2d(&tm_packed, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, packed, (uint64_t)E * N, (uint64_t)K / 2,
                        kTileRows, kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "packed weights");
   if (rc != XKB_OK) return rc;
   rc = make_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, scale, (uint64_t)E * N, (uint64_t)(K / group),
@@ -1151,13 +1165,10 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
   Carver carve(tc_ws);
   int32_t* done = r.block_counters != nullptr ? r.block_counters + r.counters_each : nullptr;   // block hand-over counters
   __nv_bfloat16* Ag = carve.take<__nv_bfloat16>(r.max_pad * hidden);
-  int64_t gblocks = r.max_pad < 148 * 16 ? r.max_pad : 148 * 16;
-  if (gblocks < 1) gblocks = 1;
-  XKB_CHECK_CUDA(launch_chained(gather_permute_kernel, dim3((unsigned)gblocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(A), r.sorted_ids,
-                                                               r.num_post, Ag, r.numel, (int)hidden, top_k, 1, r.max_pad, status));
-  XKB_CHECK_LAUNCH("gather_permute_kernel");
+  int rc = launch_gather(A, r, Ag, hidden, top_k, 1, status, stream);
+  if (rc != XKB_OK) return rc;
   CUtensorMap tm_w13, tm_s13, tm_w2, tm_s2, tm_tok0, tm_tok1;
-  int rc = make_map_2d(&tm_w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w13, (uint64_t)E * 2 * inter, (uint64_t)hidden / 2,
+  rc = make_map_2d(&tm_w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w13, (uint64_t)E * 2 * inter, (uint64_t)hidden / 2,
                        kTileRows, kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "w13 packed weights");
   if (rc != XKB_OK) return rc;
   rc = make_map_2d(&tm_s13, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s13, (uint64_t)E * 2 * inter, (uint64_t)(hidden / group),
@@ -1255,17 +1266,11 @@ int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   Carver carve(tc_ws);
   int32_t* done = r.block_counters != nullptr ? r.block_counters + r.counters_each : nullptr;   // block hand-over counters
   __nv_bfloat16* Ag = carve.take<__nv_bfloat16>(r.max_pad * hidden);
-  int64_t gblocks = r.max_pad < 148 * 16 ? r.max_pad : 148 * 16;
-  if (gblocks < 1) gblocks = 1;
-  XKB_CHECK_CUDA(launch_chained(gather_permute_kernel, dim3((unsigned)gblocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(A),
-                                                               r.sorted_ids, r.num_post, Ag, r.numel,
-                                                               (int)hidden, top_k,
-                                                               r.block == 16 ? 0 : 1,   // 16-token tiles convert through the table: natural K order
-                                                               r.max_pad, status));
-  XKB_CHECK_LAUNCH("gather_permute_kernel");
+  int rc = launch_gather(A, r, Ag, hidden, top_k, r.block == 16 ? 0 : 1, status, stream);   // 16-token tiles convert through the table: natural K order
+  if (rc != XKB_OK) return rc;
 
   CUtensorMap tm_w13, tm_w2, tm_tok0, tm_tok1, tm_s13, tm_s2;
-  int rc = make_map_2d(&tm_w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w13, (uint64_t)E * 2 * ispp, (uint64_t)hidden / 2,
+  rc = make_map_2d(&tm_w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w13, (uint64_t)E * 2 * ispp, (uint64_t)hidden / 2,
                        kTileRows, kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "w13");
   if (rc != XKB_OK) return rc;
   rc = make_map_2d(&tm_w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w2, (uint64_t)E * hidden, (uint64_t)ispp / 2,
