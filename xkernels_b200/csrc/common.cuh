@@ -95,6 +95,11 @@ int launch_combine(const float* scratch, const int32_t* topk_ids, const int32_t*
                    int num_map, int E, void* out, int out_dtype, int64_t M, int top_k, int64_t N,
                    cudaStream_t stream);
 
+// The same over bf16 rows: out[m,n] = sum_j fl32(rows[m*top_k+j, n] * w[m,j]) (w == nullptr: the rows themselves).
+int launch_combine_bf16(const __nv_bfloat16* rows, const float* w, const int32_t* topk_ids, const int32_t* expert_map,
+                        int num_map, int E, void* out, int out_dtype, int64_t M, int top_k, int64_t N,
+                        cudaStream_t stream);
+
 // Records one event pair of the optional GEMM timer (xkb_gemm_timer_enable) around
 // the launches made while it is alive; does nothing when the timer is not armed.
 struct GemmTimerScope {

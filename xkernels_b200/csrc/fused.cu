@@ -352,10 +352,11 @@ extern "C" int64_t xkb_fused_moe_mxfp4_workspace_bytes(int64_t M, int64_t hidden
   if (M < 0 || hidden < 0 || ispp < 0 || E < 0 || top_k < 0) return -1;
   const int64_t numel = M * top_k;
   int64_t total = routing_bytes(numel, E);
-  total += align_up(numel * hidden * 4, 256);                                 // fp32 partial rows
-  total += align_up(routing_max_pad(numel, E, kMaxBlock) * ispp * 2, 256);    // bf16 activations
-  total += mxfp4_tc_workspace_bytes(numel, hidden, ispp, E);
-  return total + 256;
+  int64_t own = align_up(numel * hidden * 4, 256);                          // fp32 partial rows
+  own += align_up(routing_max_pad(numel, E, kMaxBlock) * ispp * 2, 256);    // bf16 activations
+  own += mxfp4_tc_workspace_bytes(numel, hidden, ispp, E);
+  const int64_t bs = mxfp4_bs_workspace_bytes(numel, hidden, ispp, E);      // the block-scaled path's, in the same place
+  return total + (own > bs ? own : bs) + 256;
 }
 
 extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w13,
@@ -387,6 +388,7 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
   const int64_t numel = M * top_k;
   Carver carve(workspace);
   RoutingBuffers rb = carve_routing(carve, numel, E);
+  void* bs_ws = carve.take<char>(0);
   float* scratch = carve.take<float>(numel * hidden);
   __nv_bfloat16* act = carve.take<__nv_bfloat16>(routing_max_pad(numel, E, kMaxBlock) * ispp);
   void* tc_ws = carve.take<char>(mxfp4_tc_workspace_bytes(numel, hidden, ispp, E));
@@ -397,7 +399,8 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
                 "fused_moe_mxfp4: shape not supported by the tcgen05 path (needs bf16 A, "
                 "hidden %% 512 == 0, ispp %% 512 == 0)");
   const bool use_tc = (path == XKB_PATH_TC) || (path == XKB_PATH_AUTO && tc_fit);
-  const int block = use_tc ? mxfp4_tc_block(numel, E) : kSimtBlock;
+  const bool use_bs = use_tc && mxfp4_bs_supported(w13, w2, w13_scale, w2_scale);
+  const int block = use_bs ? mxfp4_bs_block(numel, E) : use_tc ? mxfp4_tc_block(numel, E) : kSimtBlock;
 
   Routing r = make_routing(rb, numel, E, block);
   // (the align stage clears the status word and the block counters on its way)
@@ -405,6 +408,15 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
                         rb.num_post, rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb),
                         rb.slot_pos);
   if (rc != XKB_OK) return rc;
+  if (use_bs) {
+    const __nv_bfloat16* rows = nullptr;
+    // prefill-sized batches report scale bytes 191..254, as they always have
+    rc = launch_mxfp4_bs(A, w13, w13_scale, w2, w2_scale, b13, b2, r, hidden, ispp, E, top_k, swiglu_limit,
+                         mxfp4_tc_block(numel, E) == 128, bs_ws, rb.status, &rows, stream);
+    if (rc != XKB_OK) return rc;
+    return launch_combine_bf16(rows, mul_routed_weight ? topk_w : nullptr, topk_ids, expert_map, num_map, E, out,
+                               a_dtype, M, top_k, hidden, stream);
+  }
   if (use_tc)
     rc = launch_mxfp4_tc(A, w13, w13_scale, w2, w2_scale, b13, b2, r, topk_w, act, scratch, hidden,
                          ispp, E, top_k, swiglu_limit, mul_routed_weight, tc_ws, rb.status, stream);

@@ -48,6 +48,16 @@ int launch_int4_ffn_simt(const void* A, int a_dtype, const int32_t* w13, const v
                          int num_map, int E, const float* topk_w, float* rows1, void* act, float* scratch,
                          int64_t hidden, int64_t inter, int top_k, int group, float limit, cudaStream_t stream);
 
+// MXFP4 on the block-scaled instructions (moe_mx.cu): the shapes of mxfp4_tc_supported, 32-byte aligned weights.
+// Leaves the bf16 rows of the slots, before the routing weight, in the workspace (*rows).
+bool mxfp4_bs_supported(const void* w13, const void* w2, const void* s13, const void* s2);
+int mxfp4_bs_block(int64_t numel, int E);
+int64_t mxfp4_bs_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, int E);
+int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale, const uint8_t* w2,
+                    const uint8_t* w2_scale, const void* b13, const void* b2, const Routing& r, int64_t hidden,
+                    int64_t ispp, int E, int top_k, float limit, int check_scale, void* ws, int* status,
+                    const __nv_bfloat16** rows, cudaStream_t stream);
+
 bool mxfp4_tc_supported(int a_dtype, int64_t M, int64_t hidden, int64_t ispp, int E, int top_k);
 int mxfp4_tc_block(int64_t numel, int E);
 int64_t mxfp4_tc_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, int E);

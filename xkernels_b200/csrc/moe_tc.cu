@@ -45,6 +45,7 @@
 #include <mutex>
 #include "moe_kernels.h"
 #include "tc_common.cuh"
+#include "tensor_map.h"
 
 namespace xkb {
 std::atomic<int> g_sm_margin{0};
@@ -950,16 +951,15 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// 2-D row-major tensor [rows, cols] of `elem_bytes` elements, box [box_rows, box_cols].
 // Encoded maps are kept per (base, shape, box, type, swizzle): a serving loop calls with the same
 // weights and workspace addresses every step, and an encode costs about as much host time as a launch.
 // A map holds no device state, so a stale entry (memory freed and reused with another layout) is
 // harmless: the key is everything the encoding depends on.
 struct MapKey {
-  const void* base; uint64_t rows, cols; uint32_t box_rows, box_cols; int dt, elem_bytes, swz;
+  const void* base; uint64_t rows, cols; uint32_t box_rows, box_cols; int dt, elem_bits, swz;
   bool operator==(const MapKey& o) const {
     return base == o.base && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols &&
-           dt == o.dt && elem_bytes == o.elem_bytes && swz == o.swz;
+           dt == o.dt && elem_bits == o.elem_bits && swz == o.swz;
   }
 };
 constexpr int kMapCacheSize = 64;
@@ -971,9 +971,11 @@ struct MapCache {
 };
 MapCache g_map_cache;
 
-int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t rows,
+}  // namespace
+
+int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bits, const void* base, uint64_t rows,
                 uint64_t cols, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swz, const char* what) {
-  const MapKey key{base, rows, cols, box_rows, box_cols, (int)dt, elem_bytes, (int)swz};
+  const MapKey key{base, rows, cols, box_rows, box_cols, (int)dt, elem_bits, (int)swz};
   {
     std::lock_guard<std::mutex> lock(g_map_cache.mu);
     for (int i = 0; i < g_map_cache.used; ++i)
@@ -982,11 +984,11 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const 
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return fail(XKB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   XKB_REQUIRE(reinterpret_cast<uintptr_t>(base) % 16 == 0, "%s: base pointer must be 16-byte aligned", what);
-  XKB_REQUIRE((cols * elem_bytes) % 16 == 0, "%s: row pitch %llu B is not a multiple of 16", what,
-              (unsigned long long)(cols * elem_bytes));
-  XKB_REQUIRE(box_rows <= 256 && box_cols <= 256 && (box_cols * elem_bytes) % 16 == 0, "%s: bad box", what);
+  XKB_REQUIRE((cols * elem_bits) % 128 == 0, "%s: row pitch %llu B is not a multiple of 16", what,
+              (unsigned long long)(cols * elem_bits / 8));
+  XKB_REQUIRE(box_rows <= 256 && box_cols <= 256 && (box_cols * elem_bits) % 128 == 0, "%s: bad box", what);
   const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * (uint64_t)elem_bytes};
+  const cuuint64_t strides[1] = {cols * (uint64_t)elem_bits / 8};
   const cuuint32_t box[2] = {box_cols, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
@@ -1000,6 +1002,8 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const 
   }
   return XKB_OK;
 }
+
+namespace {
 
 int launch_gather(const void* A, const Routing& r, __nv_bfloat16* Ag, int64_t K, int top_k, int permute, int* status,
                   cudaStream_t stream) {
@@ -1111,13 +1115,13 @@ int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, cons
   if (rc != XKB_OK) return rc;
 
   CUtensorMap tm_packed, tm_scale, tm_tokens;
-  rc = make_map_2d(&tm_packed, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, packed, (uint64_t)E * N, (uint64_t)K / 2,
+  rc = make_map_2d(&tm_packed, CU_TENSOR_MAP_DATA_TYPE_UINT8, 8, packed, (uint64_t)E * N, (uint64_t)K / 2,
                        kTileRows, kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "packed weights");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, scale, (uint64_t)E * N, (uint64_t)(K / group),
+  rc = make_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, scale, (uint64_t)E * N, (uint64_t)(K / group),
                    kTileRows, kStageK / 32, CU_TENSOR_MAP_SWIZZLE_NONE, "group scales");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tokens, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Ag, (uint64_t)r.max_pad, (uint64_t)K,
+  rc = make_map_2d(&tm_tokens, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, Ag, (uint64_t)r.max_pad, (uint64_t)K,
                    (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "gathered activations");
   if (rc != XKB_OK) return rc;
 
@@ -1168,22 +1172,22 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
   int rc = launch_gather(A, r, Ag, hidden, top_k, 1, status, stream);
   if (rc != XKB_OK) return rc;
   CUtensorMap tm_w13, tm_s13, tm_w2, tm_s2, tm_tok0, tm_tok1;
-  rc = make_map_2d(&tm_w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w13, (uint64_t)E * 2 * inter, (uint64_t)hidden / 2,
+  rc = make_map_2d(&tm_w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 8, w13, (uint64_t)E * 2 * inter, (uint64_t)hidden / 2,
                        kTileRows, kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "w13 packed weights");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_s13, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s13, (uint64_t)E * 2 * inter, (uint64_t)(hidden / group),
+  rc = make_map_2d(&tm_s13, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, s13, (uint64_t)E * 2 * inter, (uint64_t)(hidden / group),
                    kTileRows, kStageK / 32, CU_TENSOR_MAP_SWIZZLE_NONE, "w13 group scales");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w2, (uint64_t)E * hidden, (uint64_t)inter / 2, kTileRows,
+  rc = make_map_2d(&tm_w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 8, w2, (uint64_t)E * hidden, (uint64_t)inter / 2, kTileRows,
                    kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "w2 packed weights");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_s2, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s2, (uint64_t)E * hidden, (uint64_t)(inter / group),
+  rc = make_map_2d(&tm_s2, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, s2, (uint64_t)E * hidden, (uint64_t)(inter / group),
                    kTileRows, kStageK / 32, CU_TENSOR_MAP_SWIZZLE_NONE, "w2 group scales");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tok0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Ag, (uint64_t)r.max_pad, (uint64_t)hidden,
+  rc = make_map_2d(&tm_tok0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, Ag, (uint64_t)r.max_pad, (uint64_t)hidden,
                    (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "gathered activations");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tok1, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, act, (uint64_t)r.max_pad, (uint64_t)inter,
+  rc = make_map_2d(&tm_tok1, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, act, (uint64_t)r.max_pad, (uint64_t)inter,
                    (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "SwiGLU activations");
   if (rc != XKB_OK) return rc;
 
@@ -1270,22 +1274,22 @@ int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   if (rc != XKB_OK) return rc;
 
   CUtensorMap tm_w13, tm_w2, tm_tok0, tm_tok1, tm_s13, tm_s2;
-  rc = make_map_2d(&tm_w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w13, (uint64_t)E * 2 * ispp, (uint64_t)hidden / 2,
+  rc = make_map_2d(&tm_w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 8, w13, (uint64_t)E * 2 * ispp, (uint64_t)hidden / 2,
                        kTileRows, kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "w13");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w2, (uint64_t)E * hidden, (uint64_t)ispp / 2,
+  rc = make_map_2d(&tm_w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 8, w2, (uint64_t)E * hidden, (uint64_t)ispp / 2,
                    kTileRows, kStageK / 2, CU_TENSOR_MAP_SWIZZLE_128B, "w2");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_s13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w13_scale, (uint64_t)E * 2 * ispp, (uint64_t)hidden / 32,
+  rc = make_map_2d(&tm_s13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 8, w13_scale, (uint64_t)E * 2 * ispp, (uint64_t)hidden / 32,
                    kTileRows, 16, CU_TENSOR_MAP_SWIZZLE_NONE, "w13 scales");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_s2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w2_scale, (uint64_t)E * hidden, (uint64_t)ispp / 32,
+  rc = make_map_2d(&tm_s2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 8, w2_scale, (uint64_t)E * hidden, (uint64_t)ispp / 32,
                    kTileRows, 16, CU_TENSOR_MAP_SWIZZLE_NONE, "w2 scales");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tok0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Ag, (uint64_t)r.max_pad, (uint64_t)hidden,
+  rc = make_map_2d(&tm_tok0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, Ag, (uint64_t)r.max_pad, (uint64_t)hidden,
                    (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "gathered activations");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tok1, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, act, (uint64_t)r.max_pad, (uint64_t)ispp,
+  rc = make_map_2d(&tm_tok1, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, act, (uint64_t)r.max_pad, (uint64_t)ispp,
                    (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "SwiGLU activations");
   if (rc != XKB_OK) return rc;
 

@@ -109,7 +109,11 @@ sum_reduce_vec8_kernel(const TY* y, const TW* __restrict__ w, TO* __restrict__ o
       if (w != nullptr) {
         const float wk = to_f(w[slot0 + k0 + j]);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] += v[j].get(i) * wk;
+        for (int i = 0; i < 8; ++i) {
+          // the combine's rows count as fp32 products: rounded before they are added, not fused
+          if (ROWS == kSlots) acc[i] = __fadd_rn(acc[i], __fmul_rn(v[j].get(i), wk));
+          else acc[i] += v[j].get(i) * wk;
+        }
       } else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] += v[j].get(i);
@@ -149,7 +153,8 @@ sum_reduce_scalar_kernel(const TY* __restrict__ y, const TW* __restrict__ w, TO*
     for (int k = 0; k < top_k; ++k) {
       if (!slot_valid(ids, emap, num_map, E, m * top_k + k)) continue;
       const float v = to_f(y[(m * top_k + k) * H + h]);
-      acc += (w != nullptr) ? v * to_f(w[m * top_k + k]) : v;
+      if (w != nullptr && ids != nullptr) acc = __fadd_rn(acc, __fmul_rn(v, to_f(w[m * top_k + k])));   // as above
+      else acc += (w != nullptr) ? v * to_f(w[m * top_k + k]) : v;
     }
     from_f(out[idx], acc * rsf);
   }
@@ -222,6 +227,13 @@ int launch_combine(const float* scratch, const int32_t* topk_ids, const int32_t*
                    cudaStream_t stream) {
   return dispatch_out<float, float>(out_dtype, scratch, nullptr, out, M, top_k, N, 1.0f, topk_ids,
                                     expert_map, num_map, E, stream);
+}
+
+int launch_combine_bf16(const __nv_bfloat16* rows, const float* w, const int32_t* topk_ids, const int32_t* expert_map,
+                        int num_map, int E, void* out, int out_dtype, int64_t M, int top_k, int64_t N,
+                        cudaStream_t stream) {
+  return dispatch_out<__nv_bfloat16, float>(out_dtype, rows, w, out, M, top_k, N, 1.0f, topk_ids, expert_map, num_map, E,
+                                            stream);
 }
 
 }  // namespace xkb
