@@ -10,6 +10,9 @@ device memory and the current stream only; all arithmetic happens in
 
 from __future__ import annotations
 
+import contextlib
+import functools
+
 import torch
 
 from . import _lib
@@ -41,8 +44,26 @@ def _ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+# The small ops take less time on the device than a call spends in Python, so a call asks for the raw
+# stream (0.1 us; a Stream object 1 us) and enters a device only if another one is current (2 us).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_CURRENT = contextlib.nullcontext()
+
+
 def _stream(dev: torch.device) -> int:
+    if _raw_stream is not None and dev.index is not None:
+        return _raw_stream(dev.index)
     return torch.cuda.current_stream(dev).cuda_stream
+
+
+def _on(dev: torch.device):
+    return _CURRENT if dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
+
+
+@functools.lru_cache(maxsize=512)
+def _bytes(query: str, *dims) -> int:
+    """A workspace size query of the library (arithmetic on the dimensions only)."""
+    return int(getattr(_lib.load(), query)(*dims))
 
 
 _retired: list[torch.Tensor] = []
@@ -166,36 +187,38 @@ def moe_align_block_size(topk_ids, block_size, num_experts, truncate=True, works
     use_ws = False
     if workspace is not None and hasattr(workspace, "matches") and topk_ids.dim() == 2:
         use_ws = bool(workspace.matches(topk_ids.shape[0], topk_ids.shape[1], num_experts, block_size, device=dev))
-    with torch.cuda.device(dev):
-        ws_bytes = int(lib.xkb_moe_align_workspace_bytes(numel, num_experts))
+    with _on(dev):
+        ws_bytes = _bytes("xkb_moe_align_workspace_bytes", numel, num_experts)
         if use_ws:
             sorted_ids, expert_ids, num_post = workspace.sorted_ids, workspace.expert_ids, workspace.num_post
             if max_blocks == 0:
                 expert_ids[:1].zero_()
             ws = getattr(workspace, "_xkb200_scratch", None)
             if ws is None or ws.numel() < ws_bytes:
-                cap = int(lib.xkb_moe_align_workspace_bytes(max(workspace.sorted_ids.numel(), numel), num_experts))
+                cap = _bytes("xkb_moe_align_workspace_bytes", max(workspace.sorted_ids.numel(), numel), num_experts)
                 ws = torch.empty(max(cap, ws_bytes, 256), dtype=torch.uint8, device=dev)
                 workspace._xkb200_scratch = ws
         else:
-            sorted_ids = torch.empty(max_pad, dtype=torch.int32, device=dev)
+            # the kernels' scratch lies behind the sorted ids: one allocation less
+            sorted_ids = torch.empty(max_pad + -(-ws_bytes // 4), dtype=torch.int32, device=dev)
             expert_ids = torch.empty(max(max_blocks, 1), dtype=torch.int32, device=dev)
             num_post = torch.empty(1, dtype=torch.int32, device=dev)
             if max_blocks == 0:
                 expert_ids.zero_()
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+            ws = None
         _lib.check(
             lib.xkb_moe_align_block_size(
                 _ptr(ids), numel, num_experts, block_size, _ptr(emap),
                 0 if emap is None else emap.numel(), _ptr(sorted_ids), _ptr(expert_ids),
-                _ptr(num_post), 0, _ptr(ws), ws.numel(), _stream(dev)),
+                _ptr(num_post), 0, sorted_ids.data_ptr() + 4 * max_pad if ws is None else _ptr(ws),
+                ws_bytes if ws is None else ws.numel(), _stream(dev)),
             "xkb_moe_align_block_size")
     sorted_ids = sorted_ids[:max_pad]
     if truncate:
         used = int(num_post.item()) // block_size
         expert_ids = expert_ids[: max(used, 1)]
-    else:
-        expert_ids = expert_ids[: max(max_blocks, 1)] if max_blocks == 0 else expert_ids[:max_blocks]
+    elif expert_ids.numel() != max(max_blocks, 1):
+        expert_ids = expert_ids[: max(max_blocks, 1)]
     return sorted_ids, expert_ids, num_post
 
 
@@ -220,7 +243,7 @@ def topk_softmax(gating_output, topk, renormalize=True):
     if not (1 <= int(topk) <= E):
         raise ValueError(f"topk must satisfy 1 <= topk <= E (got topk={topk}, E={E})")
     g = gating_output.contiguous()
-    with torch.cuda.device(dev):
+    with _on(dev):
         w = torch.empty((M, int(topk)), dtype=torch.float32, device=dev)
         ids = torch.empty((M, int(topk)), dtype=torch.int32, device=dev)
         _lib.check(
@@ -252,7 +275,7 @@ def moe_sum_reduce(y, w=None, routed_scaling_factor=1.0):
         if tuple(w.shape) != (M, top_k):
             raise ValueError(f"w must be [M, top_k] = [{M}, {top_k}], got {tuple(w.shape)}")
         w = w.contiguous()
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty((M, H), dtype=y.dtype, device=dev)
         _lib.check(
             lib.xkb_moe_sum_reduce(_ptr(y), _DT[y.dtype], _ptr(w),
@@ -337,15 +360,15 @@ def fused_moe_int4_w4a16(A, packed, scale, topk_ids, topk_w, group_size=32, mul_
     pcode = {"auto": _lib.PATH_AUTO, "simt": _lib.PATH_SIMT, "tc": _lib.PATH_TC}[path]
     if path != "simt":
         _check_int4_scales(scale)
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty((M, N), dtype=A.dtype, device=dev)
-        ws_bytes = int(lib.xkb_fused_moe_int4_w4a16_workspace_bytes(M, N, K, E, top_k, _DT[A.dtype]))
+        ws_bytes = _bytes("xkb_fused_moe_int4_w4a16_workspace_bytes", M, N, K, E, top_k, _DT[A.dtype])
         fits, cap_bytes = False, ws_bytes
         if workspace is not None and hasattr(workspace, "matches"):
             fits = bool(workspace.matches(M, top_k, N, dtype=A.dtype, device=dev))
             if fits:   # capacity of the object = rows of its combine buffer (workspace.py:199-213)
-                cap_bytes = int(lib.xkb_fused_moe_int4_w4a16_workspace_bytes(int(workspace.combine_out.shape[0]), N, K, E,
-                                                                             top_k, _DT[A.dtype]))
+                cap_bytes = _bytes("xkb_fused_moe_int4_w4a16_workspace_bytes", int(workspace.combine_out.shape[0]), N, K, E,
+                                                                             top_k, _DT[A.dtype])
         ws = _caller_workspace(workspace, fits, cap_bytes, dev, ws_bytes)
         _lib.check(
             lib.xkb_fused_moe_int4_w4a16(
@@ -398,9 +421,9 @@ def fused_moe_mxfp4(A, w13, w13_scale, w2, w2_scale, topk_ids, topk_w, b13=None,
     top_k = ids.shape[1]
     limit = 0.0 if swiglu_limit is None else float(swiglu_limit)
     pcode = {"auto": _lib.PATH_AUTO, "simt": _lib.PATH_SIMT, "tc": _lib.PATH_TC}[path]
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty((M, hidden), dtype=A.dtype, device=dev)
-        ws_bytes = int(lib.xkb_fused_moe_mxfp4_workspace_bytes(M, hidden, ispp, E, top_k))
+        ws_bytes = _bytes("xkb_fused_moe_mxfp4_workspace_bytes", M, hidden, ispp, E, top_k)
         fits, cap_bytes = False, ws_bytes
         if workspace is not None and hasattr(workspace, "out") and hasattr(workspace, "act"):
             # matches() of MoeMxfp4Workspace wants the align block of ITS kernel; what matters here is
@@ -408,7 +431,7 @@ def fused_moe_mxfp4(A, w13, w13_scale, w2, w2_scale, topk_ids, topk_w, b13=None,
             fits = (workspace.act.shape[1] == ispp and workspace.out.shape[1] == hidden and workspace.out.shape[0] >= M
                     and workspace.act.dtype == A.dtype and workspace.act.device == dev)
             if fits:
-                cap_bytes = int(lib.xkb_fused_moe_mxfp4_workspace_bytes(int(workspace.out.shape[0]), hidden, ispp, E, top_k))
+                cap_bytes = _bytes("xkb_fused_moe_mxfp4_workspace_bytes", int(workspace.out.shape[0]), hidden, ispp, E, top_k)
         ws = _caller_workspace(workspace, fits, cap_bytes, dev, ws_bytes)
         _lib.check(
             lib.xkb_fused_moe_mxfp4(
@@ -459,9 +482,9 @@ def fused_moe_int4_ffn(A, w13_packed, w13_scale, w2_packed, w2_scale, topk_ids, 
     if path != "simt":
         _check_int4_scales(w13_scale)
         _check_int4_scales(w2_scale)
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty((M, hidden), dtype=A.dtype, device=dev)
-        ws_bytes = int(lib.xkb_fused_moe_int4_ffn_workspace_bytes(M, hidden, inter, E, top_k, _DT[A.dtype]))
+        ws_bytes = _bytes("xkb_fused_moe_int4_ffn_workspace_bytes", M, hidden, inter, E, top_k, _DT[A.dtype])
         ws = _caller_workspace(workspace if isinstance(workspace, torch.Tensor) else None, False, ws_bytes, dev, ws_bytes)
         _lib.check(
             lib.xkb_fused_moe_int4_ffn(
@@ -492,11 +515,11 @@ def moe_int4_w4a16_rows(A, packed, scale, topk_ids, topk_w=None, group_size=32, 
     pcode = {"auto": _lib.PATH_AUTO, "simt": _lib.PATH_SIMT, "tc": _lib.PATH_TC}[path]
     if path != "simt":
         _check_int4_scales(scale)
-    with torch.cuda.device(dev):
+    with _on(dev):
         rows = torch.empty((M * top_k, N), dtype=torch.float32, device=dev)
         if M == 0:
             return rows
-        ws_bytes = int(lib.xkb_fused_moe_int4_w4a16_workspace_bytes(M, N, K, E, top_k, _DT[A.dtype]))
+        ws_bytes = _bytes("xkb_fused_moe_int4_w4a16_workspace_bytes", M, N, K, E, top_k, _DT[A.dtype])
         ws = get_workspace(dev, ws_bytes)
         _lib.check(
             lib.xkb_moe_int4_w4a16_rows(_ptr(A), _DT[A.dtype], _ptr(packed), _ptr(scale), _ptr(ids),
@@ -529,14 +552,14 @@ def moe_int4_w4a16_partial(A, packed, scale, routing, group_size=32, *, out=None
     pcode = {"auto": _lib.PATH_AUTO, "simt": _lib.PATH_SIMT, "tc": _lib.PATH_TC}[path]
     if path != "simt":
         _check_int4_scales(scale)
-    with torch.cuda.device(dev):
+    with _on(dev):
         if out is None:
             out = torch.empty((R, N), dtype=torch.float32, device=dev)
         if out.dtype != torch.float32 or tuple(out.shape) != (R, N) or not out.is_contiguous():
             raise ValueError("moe_int4_w4a16_partial: out must be a contiguous fp32 [R, N] tensor")
         if R == 0:
             return out
-        ws_bytes = int(lib.xkb_moe_int4_w4a16_partial_workspace_bytes(R, N, K, E, top_k, _DT[A.dtype]))
+        ws_bytes = _bytes("xkb_moe_int4_w4a16_partial_workspace_bytes", R, N, K, E, top_k, _DT[A.dtype])
         ws = get_workspace(dev, ws_bytes, tag=int(workspace_tag))
         _lib.check(
             lib.xkb_moe_int4_w4a16_partial(_ptr(A), _DT[A.dtype], _ptr(packed), _ptr(scale), _ptr(routing), _ptr(out),
@@ -557,7 +580,7 @@ def moe_gather_sum_reduce(rows, row_index, w, out_dtype=torch.bfloat16):
     M, top_k = idx.shape
     H = rows.shape[1]
     w = None if w is None else w.to(torch.float32).contiguous()
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty((M, H), dtype=out_dtype, device=dev)
         _lib.check(
             lib.xkb_moe_gather_sum_reduce(_ptr(rows), _ptr(idx), _ptr(w), _ptr(out), _DT[out_dtype], M, top_k,
@@ -577,7 +600,7 @@ def gather_rows(src, index, count=None, out=None):
     idx = idx.contiguous()
     row_bytes = src.shape[1] * src.element_size()
     n = idx.numel()
-    with torch.cuda.device(dev):
+    with _on(dev):
         if out is None:
             out = torch.empty((n, src.shape[1]), dtype=src.dtype, device=dev)
         if out.dtype != src.dtype or out.shape[1] != src.shape[1] or out.shape[0] < n or not out.is_contiguous():
@@ -608,14 +631,14 @@ def ep_plan(topk_ids, topk_w, experts_per_rank, world, placement="contiguous", c
         if table.dtype != torch.int32 or tuple(table.shape) != (int(experts_per_rank) * int(world), 2) or not table.is_cuda:
             raise ValueError("ep_plan: table must be a CUDA int32 tensor of shape [experts_per_rank * world, 2]")
         table = table.contiguous()
-    with torch.cuda.device(dev):
+    with _on(dev):
         pair_token = torch.empty((numel,), dtype=torch.int32, device=dev)
         pair_dest = torch.empty((numel,), dtype=torch.int32, device=dev)
         routing = torch.empty((numel, 2 * top_k), dtype=torch.int32, device=dev)
         pair_of = torch.empty((M, world), dtype=torch.int32, device=dev)
         counts = torch.empty((chunks, world), dtype=torch.int32, device=dev)
         info = torch.empty((2,), dtype=torch.int32, device=dev)
-        ws_bytes = int(lib.xkb_ep_plan_workspace_bytes(M, top_k, world, chunks))
+        ws_bytes = _bytes("xkb_ep_plan_workspace_bytes", M, top_k, world, chunks)
         ws = get_workspace(dev, ws_bytes, tag=1)     # not the fused ops' buffer: that one starts with their status words
         _lib.check(
             lib.xkb_ep_plan(_ptr(ids), _ptr(w), M, top_k, int(experts_per_rank), int(world),
