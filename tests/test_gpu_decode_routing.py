@@ -1,0 +1,47 @@
+"""Decode batches, whose routing the activation gather sorts itself (up to 1024 slots and a top-k of 32):
+both sides of those limits, few and many experts, dropped slots, an expert map.  The generic path, which
+takes the sort's own kernels, is the check: same bf16 weights, fp32 sums in another order."""
+
+import pytest
+import torch
+
+import xkernels_b200 as xkb
+from tests.gpu_util import assert_within
+from xkernels_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,top_k,E", [
+    (1, 1, 1), (1, 8, 48), (3, 32, 40), (3, 33, 40), (127, 8, 48), (128, 8, 48), (129, 8, 48), (1024, 1, 7),
+    (1025, 1, 7), (20, 8, 1024),
+])
+@pytest.mark.parametrize("dropped", [False, True])
+def test_int4(M, top_k, E, dropped, cuda_device):
+    K, N = 256, 128
+    A = synth.activations(M, K, seed=M, device=cuda_device)
+    packed, scale = synth.int4_weights(E, N, K, 32, seed=E, device=cuda_device)
+    ids, w = synth.routing(M, E, top_k, seed=7, device=cuda_device)
+    emap = None
+    if dropped:
+        g = torch.Generator(device=cuda_device).manual_seed(1)
+        ids[torch.rand(ids.shape, generator=g, device=cuda_device) < 0.3] = -1
+        emap = torch.arange(E, dtype=torch.int32, device=cuda_device).flip(0).contiguous()
+        emap[::5] = -1
+    args = (A, packed, scale, ids, w)
+    got = xkb.fused_moe_int4_w4a16(*args, expert_map=emap, path="tc")
+    ops.check_status(cuda_device)
+    assert_within(got, xkb.fused_moe_int4_w4a16(*args, expert_map=emap, path="simt"), 1e-2, 1e-2, what="tc vs simt")
+    assert torch.equal(got, xkb.fused_moe_int4_w4a16(*args, expert_map=emap, path="tc"))
+
+
+@pytest.mark.parametrize("M,top_k,E", [(1, 6, 256), (5, 32, 64), (5, 33, 64), (170, 6, 256), (171, 6, 256)])
+def test_mxfp4(M, top_k, E, cuda_device):
+    A = synth.activations(M, 512, seed=M, device=cuda_device)
+    t = synth.mxfp4_weights(E, 512, 512, seed=E, device=cuda_device, scale_lo=117, scale_hi=121)
+    ids, w = synth.routing(M, E, top_k, seed=7, device=cuda_device)
+    args = (A, t["w13"], t["w13_scale"], t["w2"], t["w2_scale"], ids, w)
+    got = xkb.fused_moe_mxfp4(*args)
+    ops.check_status(cuda_device)
+    simt = xkb.fused_moe_mxfp4(*args, path="simt")
+    assert_within(got, simt, 2e-2, 1e-2, what="auto vs simt", allowed=max(1, simt.numel() // 2000))

@@ -17,109 +17,15 @@
 // for a single-CTA scan between the two, and is launched while the first still runs.
 // M=16384, top_k=8, E=48, block 16: 10.5 us on the device for the two launches (7.5 of it the second), 29.4 ->
 // 24.7 us a call (host-bound); the fused calls lose a memset launch besides, 49.1 -> 45.7 us at M=1.
+#include "align_dev.cuh"
 #include "common.cuh"
 
 namespace xkb {
 namespace {
 
-constexpr int kThreads = 1024;
-constexpr int kWarps = kThreads / 32;
-constexpr int kChunk = kThreads;       // slots per round (one per thread)
-constexpr int64_t kSmallMax = kChunk;  // single-CTA path up to this many slots
+using namespace align;
+
 constexpr int kMaxChunks = 148;        // CTAs of the two-launch path: one wave
-constexpr int kMaxExperts = 1024;
-
-__device__ __forceinline__ int map_expert(int id, int E, const int32_t* expert_map, int num_map) {
-  if (expert_map != nullptr) {
-    if (id < 0 || id >= num_map) return E;
-    id = expert_map[id];
-  }
-  return (id < 0 || id >= E) ? E : id;  // E = ghost expert (dropped)
-}
-
-// Exclusive scan of padded per-expert counts; one CTA, any E <= kMaxExperts.
-// hist[e] (e < E) -> off[e], off[E] = total.  scratch: kWarps ints.
-__device__ void padded_offsets(const int* hist, int* off, int* warp_tot, int E, int block) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // E <= 1024 = kThreads: one expert per thread.
-  int padded = 0;
-  if (tid < E) padded = (hist[tid] + block - 1) / block * block;
-  int incl = padded;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    int v = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += v;
-  }
-  if (lane == 31) warp_tot[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    int t = warp_tot[lane];
-    int ti = t;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      int v = __shfl_up_sync(0xffffffffu, ti, d);
-      if (lane >= d) ti += v;
-    }
-    warp_tot[lane] = ti - t;  // exclusive
-  }
-  __syncthreads();
-  const int excl = incl - padded + warp_tot[warp];
-  if (tid < E) off[tid] = excl;
-  if (tid == E - 1) off[E] = excl + padded;
-  if (E == 0 && tid == 0) off[0] = 0;
-  __syncthreads();
-}
-
-// expert_ids[b] for every block b < max_blocks: the expert whose padded run
-// holds position b*block, 0 past the used blocks.
-__device__ void write_expert_ids(const int* off, int E, int block, int32_t* expert_ids,
-                                 int64_t max_blocks, int tid0, int stride) {
-  const int total = off[E];
-  for (int64_t b = tid0; b < max_blocks; b += stride) {
-    const int64_t pos = b * block;
-    int e = 0;
-    if (pos < total) {
-      // largest e with off[e] <= pos and off[e+1] > pos (runs of zero length skipped)
-      int lo = 0, hi = E;  // invariant: off[lo] <= pos < off[hi]
-      while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (off[mid] <= pos) lo = mid; else hi = mid;
-      }
-      e = lo;
-    }
-    expert_ids[b] = e;
-  }
-}
-
-// Rank of this thread's slot among the slots of its expert in one 1024-slot round (0 if inactive), and the
-// round's slots per expert in tot[0 .. E].  wcnt: [kWarps][E+1] uint16.
-__device__ int round_rank(int my_e, bool active, int E, uint16_t* wcnt, int* tot) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int EP = E + 1;
-  uint32_t* wcnt2 = reinterpret_cast<uint32_t*>(wcnt);
-  for (int i = tid; i < kWarps * EP / 2; i += kThreads) wcnt2[i] = 0;   // kWarps is even
-  __syncthreads();
-  // inactive lanes vote with a key no expert uses so they never match
-  const int key = active ? my_e : (EP + lane);
-  const unsigned peers = __match_any_sync(0xffffffffu, key);
-  const int rank = __popc(peers & ((1u << lane) - 1u));
-  if (active && rank == 0) wcnt[warp * EP + my_e] = (uint16_t)__popc(peers);
-  __syncthreads();
-  // exclusive scan over warps, one expert per scanning warp per step
-  for (int e = warp; e < EP; e += kWarps) {
-    int v = wcnt[lane * EP + e];
-    int incl = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      int u = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += u;
-    }
-    wcnt[lane * EP + e] = (uint16_t)(incl - v);
-    if (lane == 31) tot[e] = incl;
-  }
-  __syncthreads();
-  return active ? (int)wcnt[warp * EP + my_e] + rank : 0;
-}
 
 // ---------------------------------------------------------------------------
 // Single-CTA path: numel <= 1024.  zero / zero_n: ints the caller wants cleared (nullptr, 0: none).
@@ -133,25 +39,10 @@ align_small_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int E, i
                    int32_t* __restrict__ slot_pos, int32_t* __restrict__ zero, int64_t zero_n) {
   chain_trigger();   // a kernel chained behind this one may be launched; it waits for completion itself
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int EP = E + 1;
-  uint16_t* wcnt = reinterpret_cast<uint16_t*>(smem_raw);                 // [kWarps][EP]
-  int* off = reinterpret_cast<int*>(smem_raw + kWarps * EP * sizeof(uint16_t));   // [EP]   off[E] = total
-  int* tot = off + EP;                                                    // [EP]
-  int* warp_tot = tot + EP;                                               // [kWarps]
-  const int tid = threadIdx.x;
-  const bool active = tid < numel;
-  const int e = active ? map_expert(topk_ids[tid], E, expert_map, num_map) : E;
-  for (int64_t i = tid; i < zero_n; i += kThreads) zero[i] = 0;
-  for (int64_t i = tid; i < max_pad; i += kThreads) sorted_ids[i] = (int32_t)numel;
-  const int rank = round_rank(e, active, E, wcnt, tot);
-  padded_offsets(tot, off, warp_tot, E, block);
-  // (the barriers in between order the fill above before these stores of other threads)
-  if (active && e < E) sorted_ids[off[e] + rank] = tid;
-  if (active && slot_pos != nullptr) slot_pos[tid] = e < E ? off[e] + rank : -1;
-  if (tid == 0) num_post[0] = off[E];
-  if (expert_off_out != nullptr)
-    for (int i = tid; i < EP; i += kThreads) expert_off_out[i] = off[i];
-  write_expert_ids(off, E, block, expert_ids, max_blocks, tid, kThreads);
+  const Job j{topk_ids, expert_map, sorted_ids, expert_ids, num_post, expert_off_out, zero, zero_n, numel, max_pad,
+              max_blocks, num_map, E, block};
+  const int pos = align_in_block(j, smem_raw, true);
+  if (threadIdx.x < numel && slot_pos != nullptr) slot_pos[threadIdx.x] = pos;
 }
 
 // ---------------------------------------------------------------------------
@@ -249,10 +140,6 @@ align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t 
   }
 }
 
-size_t small_smem(int E) {
-  const size_t EP = E + 1;
-  return kWarps * EP * sizeof(uint16_t) + 2 * EP * sizeof(int) + kWarps * sizeof(int);
-}
 size_t place_smem(int E) {
   const size_t EP = E + 1;
   return kWarps * EP * sizeof(uint16_t) + 3 * EP * sizeof(int) + kWarps * sizeof(int);

@@ -57,6 +57,8 @@ struct Carver {
   }
 };
 
+namespace align { struct Job; }
+
 // ---- layout of the routing produced by the align stage ---------------------
 // sorted_ids[p]  slot id (token*top_k + j) at sorted position p, or `numel`
 //                for a padding position.
@@ -78,6 +80,8 @@ struct Routing {
   // GEMM of a two-GEMM layer per token block (nullptr: the kernels do not overlap that way)
   int32_t* block_counters;
   int64_t counters_each;
+  // not nullptr: the routing is not sorted yet, the activation gather does it on its way (decode batches)
+  const align::Job* job;
 };
 
 // Internal launchers shared between translation units --------------------------

@@ -8,12 +8,16 @@ constexpr int kSimtBlock = 16;  // align block the SIMT kernels consume
 
 // ---- activation gathers: one thread per 8 elements, blocks of one token or a piece of one ----
 constexpr int kGatherThreads = 256;
-inline int gather_grid(int64_t M, int64_t units, unsigned* pieces, unsigned* threads, unsigned* blocks) {
-  const int64_t p = ceil_div(units, kGatherThreads);
+struct GatherGrid { unsigned pieces, units, threads, blocks; };   // pieces of `units` 8-element units per token
+// sorting: blocks of 1024 threads that sort the routing first; few tokens are cut finer, over sixteen SMs
+inline int gather_grid(int64_t M, int64_t units, bool sorting, GatherGrid* g) {
+  int64_t p = ceil_div(units, sorting ? 1024 : kGatherThreads);
+  if (sorting && p * M < 16) p = ceil_div(16, M) < ceil_div(units, 32) ? ceil_div(16, M) : ceil_div(units, 32);
   XKB_REQUIRE(p * M <= 0x7fffffff, "activation gather: %lld blocks do not fit a grid", (long long)(p * M));
-  *pieces = (unsigned)p;
-  *threads = (unsigned)align_up(ceil_div(units, p), 32);
-  *blocks = (unsigned)(p * M);
+  g->pieces = (unsigned)p;
+  g->units = (unsigned)align_up(ceil_div(units, p), 32);
+  g->threads = sorting ? 1024u : g->units;
+  g->blocks = (unsigned)(p * M);
   return XKB_OK;
 }
 

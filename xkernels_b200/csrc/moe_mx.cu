@@ -27,6 +27,7 @@
 // Scale byte 0xFF means weight 0 here (it is NaN to the instruction): a mover that meets one clears the
 // group's weights in shared memory and puts byte 0 in its place.
 #include <cuda_fp16.h>
+#include "align_dev.cuh"
 #include "moe_kernels.h"
 #include "mx_split.cuh"
 #include "tc_common.cuh"
@@ -472,13 +473,15 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 
 // Rows of A, split into the two terms, at the positions of all their slots (token by token, as
 // gather_permute_kernel): 32 elements = one scale block = four threads.
-__global__ void __launch_bounds__(kGatherThreads)
+template <bool SORT>
+__global__ void __launch_bounds__(SORT ? 1024 : kGatherThreads)
 gather_split_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos, uint8_t* __restrict__ hi,
                     uint8_t* __restrict__ lo, uint8_t* __restrict__ shi, uint8_t* __restrict__ slo, int K, int top_k,
-                    int64_t max_pad, unsigned pieces, int* __restrict__ status) {
+                    int64_t max_pad, unsigned pieces, unsigned units, int* __restrict__ status, const align::Job job) {
+  if (SORT) chain_trigger();   // the first kernel of the call; the next one waits for its completion
   const unsigned m = blockIdx.x / pieces;
-  const int i = (int)((blockIdx.x - m * pieces) * blockDim.x + threadIdx.x);
-  const bool mine = i < K / 8;              // K / 8 is a multiple of 32: whole warps
+  const int i = (int)((blockIdx.x - m * pieces) * units + threadIdx.x);
+  const bool mine = threadIdx.x < units && i < K / 8;   // both are multiples of 32: whole warps
   uint32_t h[4] = {0, 0, 0, 0}, l[4] = {0, 0, 0, 0}, sh = 0;
   if (mine) {
     const uint4 v = __ldg(reinterpret_cast<const uint4*>(A + (int64_t)m * K) + i);
@@ -495,11 +498,19 @@ gather_split_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos
     for (int q = 0; q < 4; ++q)
       mx::split_pair(__uint_as_float(u[q] << 16), __uint_as_float(u[q] & 0xFFFF0000u), f, f, h[q], l[q]);
   }
-  chain_wait();     // the routing is read with L2 loads after the wait (see gather_permute_kernel)
-  chain_trigger();
+  if (!SORT) {
+    chain_wait();     // the routing is read with L2 loads after the wait (see gather_permute_kernel)
+    chain_trigger();
+  }
   const int lane = threadIdx.x & 31;
   for (int j0 = 0; j0 < top_k; j0 += 32) {   // the positions of up to 32 slots in one load
-    const int32_t mine_pos = j0 + lane < top_k ? __ldcg(slot_pos + (int64_t)m * top_k + j0 + lane) : -1;
+    int32_t mine_pos;
+    if (SORT) {
+      extern __shared__ __align__(16) unsigned char smem_raw[];
+      mine_pos = align::positions_of_token(job, smem_raw, m, top_k, blockIdx.x == 0);   // top_k <= 32: one round
+    } else {
+      mine_pos = j0 + lane < top_k ? __ldcg(slot_pos + (int64_t)m * top_k + j0 + lane) : -1;
+    }
     if (mine_pos >= max_pad) atomicCAS(status, 0, kErrBadRouting + (3 << 8));   // never with a routing the align stage wrote
     unsigned live = __ballot_sync(0xffffffffu, mine_pos >= 0 && mine_pos < max_pad);
     for (; live != 0; live &= live - 1) {
@@ -610,12 +621,22 @@ int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   Carver carve(ws);
   const MxBuffers buf = carve_mx(carve, r.numel, r.max_pad, hidden, ispp);
   *rows_out = buf.rows;
-  unsigned pieces, threads, blocks;
-  int rc = gather_grid(r.numel / top_k, hidden / 8, &pieces, &threads, &blocks);
+  GatherGrid g;
+  int rc = gather_grid(r.numel / top_k, hidden / 8, r.job != nullptr, &g);
   if (rc != XKB_OK) return rc;
-  XKB_CHECK_CUDA(launch_chained(gather_split_kernel, dim3(blocks), dim3(threads), 0, stream,
-                                static_cast<const __nv_bfloat16*>(A), r.slot_pos, buf.x[0], buf.x[1], buf.x[2], buf.x[3],
-                                (int)hidden, top_k, r.max_pad, pieces, status));
+  const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(A);
+  if (r.job != nullptr) {
+    const size_t smem = align::small_smem(r.job->E);
+    if (smem > 48 * 1024)
+      XKB_CHECK_CUDA(cudaFuncSetAttribute(gather_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    gather_split_kernel<true><<<g.blocks, g.threads, smem, stream>>>(a, nullptr, buf.x[0], buf.x[1], buf.x[2], buf.x[3],
+                                                                     (int)hidden, top_k, r.max_pad, g.pieces, g.units, status,
+                                                                     *r.job);
+  } else {
+    XKB_CHECK_CUDA(launch_chained(gather_split_kernel<false>, dim3(g.blocks), dim3(g.threads), 0, stream, a, r.slot_pos,
+                                  buf.x[0], buf.x[1], buf.x[2], buf.x[3], (int)hidden, top_k, r.max_pad, g.pieces, g.units,
+                                  status, align::Job{}));
+  }
   XKB_CHECK_LAUNCH("gather_split_kernel");
 
   CUtensorMap up[6], down[6];

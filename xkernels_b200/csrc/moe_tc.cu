@@ -43,6 +43,7 @@
 
 #include <atomic>
 #include <mutex>
+#include "align_dev.cuh"
 #include "moe_kernels.h"
 #include "tc_common.cuh"
 #include "tensor_map.h"
@@ -894,9 +895,12 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
 // A once per slot, and at prefill A is larger than L2
 // (M=16384, K=7168, top_k=8, E=48: 612 -> 355 us).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kGatherThreads)
+template <bool SORT>
+__global__ void __launch_bounds__(SORT ? 1024 : kGatherThreads)
 gather_permute_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos, __nv_bfloat16* __restrict__ Ag,
-                      int K, int top_k, int permute, int64_t max_pad, unsigned pieces, int* __restrict__ status) {
+                      int K, int top_k, int permute, int64_t max_pad, unsigned pieces, unsigned units,
+                      int* __restrict__ status, const align::Job job) {
+  if (SORT) chain_trigger();   // the first kernel of the call; the next one waits for its completion
   const unsigned m = blockIdx.x / pieces;
   const int i = (int)((blockIdx.x - m * pieces) * blockDim.x + threadIdx.x);
   const bool mine = i < K / 8;
@@ -916,11 +920,19 @@ gather_permute_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_p
   // `const __restrict__`: loads the compiler may treat as invariant (ld.global.nc) were seen to
   // deliver the value from before the align kernel's write (hoisted above the wait, or served from
   // the non-coherent cache).
-  chain_wait();
-  chain_trigger();
+  if (!SORT) {
+    chain_wait();
+    chain_trigger();
+  }
   const int lane = threadIdx.x & 31;
   for (int j0 = 0; j0 < top_k; j0 += 32) {   // the positions of up to 32 slots in one load
-    const int32_t mine_pos = j0 + lane < top_k ? __ldcg(slot_pos + (int64_t)m * top_k + j0 + lane) : -1;
+    int32_t mine_pos;
+    if (SORT) {
+      extern __shared__ __align__(16) unsigned char smem_raw[];
+      mine_pos = align::positions_of_token(job, smem_raw, m, top_k, blockIdx.x == 0);   // top_k <= 32: one round
+    } else {
+      mine_pos = j0 + lane < top_k ? __ldcg(slot_pos + (int64_t)m * top_k + j0 + lane) : -1;
+    }
     if (mine_pos >= max_pad) atomicCAS(status, 0, kErrBadRouting + (3 << 8));   // never with a routing the align stage wrote
     unsigned live = __ballot_sync(0xffffffffu, mine_pos >= 0 && mine_pos < max_pad);
     for (; live != 0; live &= live - 1) {
@@ -1007,12 +1019,20 @@ namespace {
 
 int launch_gather(const void* A, const Routing& r, __nv_bfloat16* Ag, int64_t K, int top_k, int permute, int* status,
                   cudaStream_t stream) {
-  unsigned pieces, threads, blocks;
-  const int rc = gather_grid(r.numel / top_k, K / 8, &pieces, &threads, &blocks);
+  GatherGrid g;
+  const int rc = gather_grid(r.numel / top_k, K / 8, r.job != nullptr, &g);
   if (rc != XKB_OK) return rc;
-  XKB_CHECK_CUDA(launch_chained(gather_permute_kernel, dim3(blocks), dim3(threads), 0, stream,
-                                static_cast<const __nv_bfloat16*>(A), r.slot_pos, Ag, (int)K, top_k, permute, r.max_pad,
-                                pieces, status));
+  const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(A);
+  if (r.job != nullptr) {
+    const size_t smem = align::small_smem(r.job->E);
+    if (smem > 48 * 1024)
+      XKB_CHECK_CUDA(cudaFuncSetAttribute(gather_permute_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    gather_permute_kernel<true><<<g.blocks, g.threads, smem, stream>>>(a, nullptr, Ag, (int)K, top_k, permute, r.max_pad,
+                                                                       g.pieces, g.units, status, *r.job);
+  } else {
+    XKB_CHECK_CUDA(launch_chained(gather_permute_kernel<false>, dim3(g.blocks), dim3(g.threads), 0, stream, a, r.slot_pos, Ag,
+                                  (int)K, top_k, permute, r.max_pad, g.pieces, g.units, status, align::Job{}));
+  }
   XKB_CHECK_LAUNCH("gather_permute_kernel");
   return XKB_OK;
 }
