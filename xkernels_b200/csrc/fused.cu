@@ -349,12 +349,15 @@ extern "C" int xkb_fused_moe_int4_ffn(const void* A, int a_dtype, const int32_t*
   align::Job job;
   int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc, &r, &job, stream);
   if (rc != XKB_OK) return rc;
-  if (use_tc)
+  if (use_tc) {
+    __nv_bfloat16* rows16 = reinterpret_cast<__nv_bfloat16*>(scratch);
     rc = launch_int4_ffn_tc(A, w13_packed, w13_scale, w2_packed, w2_scale, r, topk_w, static_cast<__nv_bfloat16*>(act),
-                            scratch, hidden, inter, E, top_k, group_size, swiglu_limit, tc_ws, rb.status, stream);
-  else
-    rc = launch_int4_ffn_simt(A, a_dtype, w13_packed, w13_scale, w2_packed, w2_scale, r, topk_ids, expert_map, num_map,
-                              E, topk_w, rows1, act, scratch, hidden, inter, top_k, group_size, swiglu_limit, stream);
+                            rows16, hidden, inter, E, top_k, group_size, swiglu_limit, tc_ws, rb.status, stream);
+    if (rc != XKB_OK) return rc;
+    return launch_combine_bf16(rows16, nullptr, topk_ids, expert_map, num_map, E, out, a_dtype, M, top_k, hidden, stream);
+  }
+  rc = launch_int4_ffn_simt(A, a_dtype, w13_packed, w13_scale, w2_packed, w2_scale, r, topk_ids, expert_map, num_map,
+                            E, topk_w, rows1, act, scratch, hidden, inter, top_k, group_size, swiglu_limit, stream);
   if (rc != XKB_OK) return rc;
   return launch_combine(scratch, topk_ids, expert_map, num_map, E, out, a_dtype, M, top_k, hidden, stream);
 }

@@ -44,7 +44,7 @@ int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, cons
 // INT4 two-GEMM expert layer (gate_up + SwiGLU, then down with bf16-rounded weighted slot rows)
 bool int4_ffn_tc_supported(int a_dtype, int64_t M, int64_t hidden, int64_t inter, int E, int top_k, int group);
 int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const int32_t* w2, const void* s2,
-                       const Routing& r, const float* topk_w, __nv_bfloat16* act, float* scratch, int64_t hidden,
+                       const Routing& r, const float* topk_w, __nv_bfloat16* act, __nv_bfloat16* rows16, int64_t hidden,
                        int64_t inter, int E, int top_k, int group, float limit, void* tc_ws, int* status,
                        cudaStream_t stream);
 int launch_int4_ffn_simt(const void* A, int a_dtype, const int32_t* w13, const void* s13, const int32_t* w2,

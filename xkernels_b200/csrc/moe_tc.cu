@@ -218,8 +218,9 @@ struct TcParams {
   int N, K;                     // tile rows are taken from N rows per expert; K = contraction length
   int mul_w;
   int group_shift;              // INT4: log2 of the scale group (5 .. 8)
-  int round_rows;               // INT4: round each weighted slot row to bf16 (the second GEMM of a two-GEMM layer,
-                                // whose per-slot results the reference composition holds in bf16)
+  __nv_bfloat16* rows16;        // INT4: not nullptr = the weighted slot rows go here rounded to bf16 instead of to scratch
+                                // (the second GEMM of a two-GEMM layer, whose per-slot results the reference
+                                // composition holds in bf16)
   // MXFP4 only
   const __nv_bfloat16* bias;    // b13 [E, 2*ispp] or b2 [E, hidden] or nullptr
   __nv_bfloat16* act;           // gate_up mode output: [positions, N] bf16 in the K-permuted order
@@ -679,21 +680,23 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
               if (p.mul_w) v = v * w;
             } else {
               if (p.mul_w) v = w * v;
-              if (p.round_rows) v = round_to_bf16(v);
             }
-            p.scratch[(int64_t)slot * p.N + n_glob] = v;
+            const int64_t at = (int64_t)slot * p.N + n_glob;
+            const bool narrow = mode_is_int4(MODE) && p.rows16 != nullptr;
+            if (narrow) p.rows16[at] = __float2bfloat16_rn(v);
+            else p.scratch[at] = v;
             if (mode_is_pair(MODE)) {  // the second weight tile: rows 128 further down
               float v2 = __uint_as_float(more[j]);
               if (MODE == kModeInt4Pair) {
                 if (kInt4NoSubtract) v2 *= kInt4Unscale;
                 if (p.mul_w) v2 = w * v2;
-                if (p.round_rows) v2 = round_to_bf16(v2);
               } else {
                 v2 = round_to_bf16(Cfg::kLut ? v2 : v2 * kMxUnscale);
                 if (p.bias != nullptr) v2 = round_to_bf16(v2 + bias1);
                 if (p.mul_w) v2 = v2 * w;
               }
-              p.scratch[(int64_t)slot * p.N + n_glob + kTileRows] = v2;
+              if (narrow) p.rows16[at + kTileRows] = __float2bfloat16_rn(v2);
+              else p.scratch[at + kTileRows] = v2;
             }
           }
         }
@@ -902,8 +905,8 @@ gather_permute_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_p
                       int* __restrict__ status, const align::Job job) {
   if (SORT) chain_trigger();   // the first kernel of the call; the next one waits for its completion
   const unsigned m = blockIdx.x / pieces;
-  const int i = (int)((blockIdx.x - m * pieces) * blockDim.x + threadIdx.x);
-  const bool mine = i < K / 8;
+  const int i = (int)((blockIdx.x - m * pieces) * units + threadIdx.x);
+  const bool mine = threadIdx.x < units && i < K / 8;
   uint4 o = make_uint4(0, 0, 0, 0);
   if (mine) {
     const uint4 v = __ldg(reinterpret_cast<const uint4*>(A + (int64_t)m * K) + i);  // elements (e1:e0, e3:e2, e5:e4, e7:e6); an input of the call
@@ -1159,7 +1162,7 @@ int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, cons
   prm.K = (int)K;
   prm.mul_w = mul_w;
   prm.group_shift = log2_of(group);
-  prm.round_rows = 0;
+  prm.rows16 = nullptr;
   prm.bias = nullptr;
   prm.act = nullptr;
   prm.rows_per_expert = (int)N;
@@ -1183,7 +1186,7 @@ bool int4_ffn_tc_supported(int a_dtype, int64_t M, int64_t hidden, int64_t inter
 }
 
 int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const int32_t* w2, const void* s2,
-                       const Routing& r, const float* topk_w, __nv_bfloat16* act, float* scratch, int64_t hidden,
+                       const Routing& r, const float* topk_w, __nv_bfloat16* act, __nv_bfloat16* rows16, int64_t hidden,
                        int64_t inter, int E, int top_k, int group, float limit, void* tc_ws, int* status,
                        cudaStream_t stream) {
   Carver carve(tc_ws);
@@ -1230,7 +1233,7 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
   prm.K = (int)hidden;
   prm.rows_per_expert = (int)(2 * inter);
   prm.mul_w = 0;
-  prm.round_rows = 0;
+  prm.rows16 = nullptr;
   prm.done_signal = done;
   prm.done_wait = nullptr;
   prm.done_target = (int)(inter / kTileRows) * hand_over_per_tile(r.block);
@@ -1244,14 +1247,14 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
     default: return fail(XKB_ERR_ARG, "int4 tcgen05 path: unsupported token tile %d", r.block);
   }
   if (rc != XKB_OK) return rc;
-  // down: weighted slot rows, rounded to bf16
-  prm.scratch = scratch;
+  // down: weighted slot rows, rounded to bf16 (kept as bf16: half the traffic of the rows, the same values)
+  prm.scratch = nullptr;
   prm.act = nullptr;
   prm.N = (int)hidden;
   prm.K = (int)inter;
   prm.rows_per_expert = (int)hidden;
   prm.mul_w = 1;
-  prm.round_rows = 1;
+  prm.rows16 = rows16;
   prm.limit = 0.f;
   prm.done_signal = nullptr;
   prm.done_wait = done;
@@ -1324,7 +1327,7 @@ int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   prm.num_experts = E;
   prm.mul_w = mul_w;
   prm.group_shift = 5;
-  prm.round_rows = 0;
+  prm.rows16 = nullptr;
   prm.limit = limit;
   // stage 0: gate_up + SwiGLU -> act
   prm.scratch = nullptr;
