@@ -69,6 +69,8 @@ template <int BT> struct MxCfg {
   static constexpr int kDFit = (kTmemCols - kScCols) / kSetCols;
   static constexpr int kDBuf = kDFit > 4 ? 4 : kDFit;
   static_assert(kDBuf >= 2, "the read-out must overlap the next tile");
+  // (with one column group the two warpgroups take alternate tiles: each must meet every use of its accumulator sets)
+  static_assert(BT > 16 || kDBuf % 2 == 0, "accumulator sets alternate with the warpgroups");
   static constexpr int kScCol0 = kDBuf * kSetCols;
   static constexpr int kColGroups = BT / 16;
   static constexpr int kEpiWGs = kColGroups < 2 ? 1 : 2;              // read-out warpgroups per tile
@@ -602,10 +604,12 @@ bool mxfp4_bs_supported(const void* w13, const void* w2, const void* s13, const 
 
 // The widest tile is the widest that leaves tensor memory for two accumulator sets beside the scales; a
 // narrower one is taken while a block still holds nearly every expert's slots (an expert that needs a second
-// block streams its weights twice).
+// block streams its weights twice).  E=256, hidden 4096, ispp 512, whole call: 16 against 32 tokens 220 / 229 us at 8 slots
+// per expert, 248 / 234 at 10; 32 against 64 253 / 291 at 21, 283 / 295 at 23, 360 / 312 at 33; 64 against 112
+// 335 / 392 at 47, 432 / 429 at 61, 653 / 459 at 80.
 int mxfp4_bs_block(int64_t numel, int E) {
   const double avg = (double)numel / (E > 0 ? E : 1);
-  return avg <= 10 ? 16 : avg <= 22 ? 32 : avg <= 48 ? 64 : 112;
+  return avg <= 9 ? 16 : avg <= 26 ? 32 : avg <= 56 ? 64 : 112;
 }
 
 int64_t mxfp4_bs_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, int E) {
