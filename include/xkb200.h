@@ -138,7 +138,9 @@ int xkb_moe_sum_reduce(const void* y, int y_dtype, const void* w, int w_dtype,
  *           src/xkernels/ops/moe/triton/moe_int4_kernel.py:438-577 (Triton
  *           entry: align + grouped GEMM + top-k combine).
  * A [M,K] (a_dtype), packed [E,N,K/8] int32 (low nibble = lowest k, zero
- * point 8), scale [E,N,K/group] bf16, topk_ids [M,top_k] int32, topk_w
+ * point 8), scale [E,N,K/group] bf16 (finite and below 2^24 in magnitude
+ * wherever the tcgen05 path may run: group 32, and groups 64 / 128 / 256 with K
+ * a multiple of eight groups), topk_ids [M,top_k] int32, topk_w
  * [M,top_k] fp32, expert_map NULL or [num_map] int32, out [M,N] (a_dtype).
  * ---------------------------------------------------------------------- */
 int64_t xkb_fused_moe_int4_w4a16_workspace_bytes(int64_t M, int64_t N,
@@ -289,8 +291,8 @@ int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w13,
  * `stream`, reads the status word in the workspace header and returns
  * XKB_ERR_DEVICE if the word is not zero.  Low byte of the word: 1 = a
  * tcgen05 kernel gave up one of its bounded waits (the wait site in the upper
- * bits), 2 = an MXFP4 scale byte outside the range the 128-token instance of
- * the tcgen05 path converts, 3 = a kernel read a routing value (token-block
+ * bits), 2 = an MXFP4 scale byte in 191..254 in a prefill-sized batch (more
+ * than 48 slots per expert on average), 3 = a kernel read a routing value (token-block
  * count, expert id) outside what the routing buffers can hold and skipped the
  * work instead of using it as an index.
  * The reference reports kernel failures as Python exceptions raised by the
