@@ -42,6 +42,7 @@
 // a status code, all roles leave their loops, and tensor memory is released.
 
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include "align_dev.cuh"
 #include "moe_kernels.h"
@@ -133,7 +134,7 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   // Token ring.  A token stage is released by the commit of the MMAs that read it and re-filled by
   // TMA from L2 about a microsecond later; narrow tiles are small, so their ring is made deep
   // enough that the issuers never wait for tokens.
-  static constexpr int kBStages = (BT <= 16) ? kBStages16 : (BT <= 32) ? 6 : (BT <= 64) ? (kGroups == 3 ? 3 : 4) : 2;
+  static constexpr int kBStages = (BT <= 16) ? kBStages16 : (BT <= 32) ? 6 : (BT <= 64) ? (kGroups == 3 ? 3 : 4) : (BT <= 96) ? 3 : 2;
   static constexpr int kBSubBytes = BT * kSubK * 2;
   static constexpr int kBStageBytes = kSubs * kBSubBytes;   // [4][BT x 64] bf16
   static constexpr int kWStages = (BT <= 16) ? kWStagesNarrow : (BT <= 32 || kGroups == 3) ? 6 : 4;
@@ -163,7 +164,7 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   static constexpr int kACol0 = kDCols;                     // the A slots follow the accumulators
   // A slots, counted in units (three stages' worth at most)
   static constexpr int kASlotsFit = (kTmemCols - kDCols) / kUnitCols;
-  static constexpr int kASlots = kASlotsFit > 3 * kUnits ? 3 * kUnits : kASlotsFit;
+  static constexpr int kASlots = kASlotsFit > 3 * kUnits ? 3 * kUnits : kASlotsFit / kUnits * kUnits;
   static_assert(kASlots >= 2 * kUnits, "need two stages of A slots so that conversion and MMA overlap");
   // mbarrier parity waits only tell "the phase with this parity is over", so a waiter must see every
   // phase of a barrier it waits on.  Unit u = g * kUnits + h (stage g, numbered across the tiles of
@@ -1095,11 +1096,19 @@ bool int4_tc_supported(int a_dtype, int64_t M, int64_t N, int64_t K, int E, int 
          M > 0 && E > 0 && top_k > 0 && (int64_t)E * N < (1ll << 31) && K < (1 << 30);
 }
 
-int int4_tc_block(int64_t numel, int E) {
+int int4_tc_block(int64_t numel, int E, int64_t N) {
   const double avg = (double)numel / (E > 0 ? E : 1);
   if (avg <= 12) return 16;
   if (avg <= 24) return 32;
   if (avg <= 48) return 64;
+  // 80, 96 or 112 tokens x two row tiles, while nearly every expert fits one block (its slots spread by about their
+  // square root): the tile's token bytes through shared memory, which bound it, shrink with the tile.
+  // E=48, top_k=8, whole call, 128-token tiles against these: K=2048, N=7168 184 -> 169 us at 50 slots per expert, 194 -> 185
+  // at 67, 200 -> 194 at 75, 206 -> 198 at 85, 212 -> 211 at 93 (96 tokens there: 241); K=7168, N=4096 333 -> 294 at
+  // 53, 344 -> 320 at 70, 353 -> 335 at 85, with a routing bias of 0.5 353 -> 353 at 58 and 408 -> 400 at 83.
+  if (N % (2 * kTileRows) == 0)
+    for (int block = 80; block < 128; block += 16)
+      if (avg + 2.0 * std::sqrt(avg) <= block) return block;
   return 128;  // wide: 128 tokens x two 128-row weight tiles per CTA (one tile if N % 256 != 0)
 }
 
@@ -1120,6 +1129,9 @@ static int launch_int4_by_block(const CUtensorMap& tm_packed, const CUtensorMap&
     case 16: return launch_bt<16, kModeInt4>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
     case 32: return launch_bt<32, kModeInt4>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
     case 64: return launch_bt<64, kModeInt4>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
+    case 80: return launch_bt<80, kModeInt4Pair>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
+    case 96: return launch_bt<96, kModeInt4Pair>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
+    case 112: return launch_bt<112, kModeInt4Pair>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
     case 128:
       if (N % (2 * kTileRows) == 0)
         return launch_bt<128, kModeInt4Pair>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
@@ -1243,6 +1255,9 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
     case 16: rc = launch_bt<16, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
     case 32: rc = launch_bt<32, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
     case 64: rc = launch_bt<64, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
+    case 80: rc = launch_bt<80, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
+    case 96: rc = launch_bt<96, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
+    case 112: rc = launch_bt<112, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
     case 128: rc = launch_bt<128, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
     default: return fail(XKB_ERR_ARG, "int4 tcgen05 path: unsupported token tile %d", r.block);
   }
