@@ -117,12 +117,15 @@ Routing make_routing(const RoutingBuffers& b, int64_t numel, int E, int block) {
 
 // The align stage of a fused call: clears the status word and the block counters on its way.  A decode batch on
 // a tensor-core path is sorted by the activation gather itself (r->job = *job): one launch less, and the gather
-// does not wait for another kernel's completion.  Larger batches need the sort's own kernels.
-// Whole calls: K=2048, N=7168, E=48, top_k=8 at M=1 39.8 -> 32.7 us, M=64 110.0 -> 108.1, M=128 (1024 slots) 132.4 -> 132.0;
-// K=7168, N=4096 at M=1 46.0 -> 44.0 us, M=64 177.5 -> 175.4.
+// does not wait for another kernel's completion.  Larger batches take the sort's own kernels.
+// Whole calls: K=2048, N=7168, E=48, top_k=8 at M=1 39.8 -> 32.7 us, M=64 110.0 -> 108.1; K=7168, N=4096 at M=1 46.0 -> 44.0 us,
+// M=64 177.5 -> 175.4.  At M=128 (1024 slots: nearly every SM sorts) nothing is left of it: 132.4 / 132.0 us, and the
+// two-GEMM layer 448 / 451, so the line lies at M=64's 512 slots.
+constexpr int64_t kSortInGatherMax = 512;
+static_assert(kSortInGatherMax <= align::kSmallMax, "the sort takes one slot per thread");
 int route(const RoutingBuffers& rb, const int32_t* topk_ids, const int32_t* expert_map, int num_map, int E, int top_k,
           bool gathers, Routing* r, align::Job* job, cudaStream_t stream) {
-  if (gathers && r->numel >= 1 && r->numel <= align::kSmallMax && top_k <= 32 && E >= 1 && E <= align::kMaxExperts) {
+  if (gathers && r->numel >= 1 && r->numel <= kSortInGatherMax && top_k <= 32 && E >= 1 && E <= align::kMaxExperts) {
     *job = align::Job{topk_ids, expert_map, rb.sorted_ids, rb.expert_ids, rb.num_post, rb.expert_off, rb.status,
                       header_ints(rb), r->numel, r->max_pad, r->max_blocks, num_map, E, r->block};
     r->job = job;
