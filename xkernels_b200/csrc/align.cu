@@ -15,8 +15,9 @@
 // launches over at most kMaxChunks chunks of whole 1024-slot rounds: count, then place.  Every CTA of the
 // second adds up the chunk x expert matrix for itself (a few hundred KB from L2 at most) instead of waiting
 // for a single-CTA scan between the two, and is launched while the first still runs.
-// M=16384, top_k=8, E=48, block 16: 10.5 us on the device for the two launches (7.5 of it the second), 29.4 ->
-// 24.7 us a call (host-bound); the fused calls lose a memset launch besides, 49.1 -> 45.7 us at M=1.
+// M=16384, top_k=8, E=48, block 16: 10.5 us on the device for the two launches (7.5 of it the second), a call 29.4 ->
+// 24.7 us, 18.0 with the shorter host path (which still bounds it); the fused calls lose a memset launch besides,
+// 49.1 -> 45.7 us at M=1.
 #include "align_dev.cuh"
 #include "common.cuh"
 

@@ -22,7 +22,7 @@
 //
 // Measured at E=256, hidden 4096, ispp 512, top_k 6, whole call, against the kernel that converts to bf16:
 // M=48 209 -> 158 us (0.58 GB of weights: 87 us at the copy rate; the same loads without any products 131 us),
-// M=4096 749 -> 616 us (without products and read-out 373: 2.4 GB pass from L2 to the SMs, tokens included).
+// M=4096 749 -> 597 us (without products and read-out 373: 2.4 GB pass from L2 to the SMs, tokens included).
 //
 // Scale byte 0xFF means weight 0 here (it is NaN to the instruction): a mover that meets one clears the
 // group's weights in shared memory and puts byte 0 in its place.
