@@ -13,8 +13,8 @@
 // selection first cuts the row down to a handful of candidates: the k-th largest of the 32 lane maxima
 // bounds the k-th largest element from below, usually 8 to 16 of the experts reach it, and only those
 // are divided by the sum (one per lane), ranked against each other and written.  Rows that leave more
-// than 32 candidates (long runs of equal logits), a top-k above 32 or a sum that is not finite take the
-// rounds (select_by_rounds), which order every probability of the row.
+// than 32 candidates (long runs of equal logits, a k-th probability near the subnormals), a top-k above 32
+// or a sum that is not finite take the rounds (select_by_rounds), which order every probability of the row.
 // M=16384, E=256, bf16, top 8, renormalised: 28.7 -> 11.8 us on the device, 12.3 us a call.
 #include <cuda_fp16.h>
 
@@ -125,8 +125,13 @@ topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, in
     }
   }
   // Division by the sum is monotone but may round neighbours to one probability, and then the smaller id
-  // wins: exponentials a few units in the last place below the bound are candidates as well.
-  const float bound = (short_way && tau >= 0) ? __int_as_float(tau) * (1.f - 9.5367431640625e-7f) : -1.f;
+  // wins: exponentials a few units in the last place below the bound are candidates as well.  That slack
+  // covers the rounding of normal quotients only.  Subnormal ones merge exponentials that lie far apart (at
+  // 27 and 28 * 2^-149 and a sum of 2 both are 14 * 2^-149, and below half a unit everything is 0), so with
+  // a bound whose quotient comes near the subnormals every expert is a candidate.
+  float bound = -1.f;
+  if (short_way && tau >= 0 && __int_as_float(tau) >= sum * 7.8886090522101181e-31f)   // 2^-100
+    bound = __int_as_float(tau) * (1.f - 9.5367431640625e-7f);
   int n = 0;
   uint64_t* cand = s_cand[warp];
 #pragma unroll
