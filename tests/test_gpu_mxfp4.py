@@ -37,10 +37,10 @@ def test_golden(name, path, cuda_device):
 @pytest.mark.parametrize("M,hidden,ispp,E,top_k,bias", [
     (1, 64, 32, 4, 2, False), (37, 96, 64, 8, 3, True), (16, 256, 128, 5, 4, False),
     (48, 512, 256, 16, 6, True),
-    (48, 512, 512, 16, 6, True),      # multiples of 512: the tcgen05 kernels, 16-token tiles
+    (48, 512, 512, 16, 6, True),      # multiples of 512: the tcgen05 kernels, decode batches
     (40, 1024, 512, 8, 4, False),     # four 256-K stages in gate_up, two in down
-    (640, 512, 512, 4, 2, True),      # more than 48 slots per expert: the 128-token tiles
-    (300, 512, 1024, 3, 2, False),    # ragged last blocks in the wide mode
+    (640, 512, 512, 4, 2, True),      # more than 48 slots per expert: prefill batches
+    (300, 512, 1024, 3, 2, False),    # ragged last blocks of a prefill batch
 ])
 def test_against_oracle_with_repeated_ids(M, hidden, ispp, E, top_k, bias, cuda_device):
     g = torch.Generator().manual_seed(M + hidden)

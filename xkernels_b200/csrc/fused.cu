@@ -420,8 +420,9 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
                 "fused_moe_mxfp4: shape not supported by the tcgen05 path (needs bf16 A, "
                 "hidden %% 512 == 0, ispp %% 512 == 0)");
   const bool use_tc = (path == XKB_PATH_TC) || (path == XKB_PATH_AUTO && tc_fit);
-  const bool use_bs = use_tc && mxfp4_bs_supported(w13, w2, w13_scale, w2_scale);
-  const int block = use_bs ? mxfp4_bs_block(numel, E) : use_tc ? mxfp4_tc_block(numel, E) : kSimtBlock;
+  const int bs_block = use_tc && mxfp4_bs_supported(w13, w2, w13_scale, w2_scale) ? mxfp4_bs_block(numel, E) : 0;
+  const bool use_bs = bs_block > 0;
+  const int block = use_bs ? bs_block : use_tc ? mxfp4_tc_block(numel, E) : kSimtBlock;
 
   Routing r = make_routing(rb, numel, E, block);
   align::Job job;
@@ -429,7 +430,7 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
   if (rc != XKB_OK) return rc;
   if (use_bs) {
     const __nv_bfloat16* rows = nullptr;
-    // prefill-sized batches report scale bytes 191..254, as they always have
+    // batches of more than 48 slots per expert report scale bytes 191..254, as they always have
     rc = launch_mxfp4_bs(A, w13, w13_scale, w2, w2_scale, b13, b2, r, hidden, ispp, E, top_k, swiglu_limit,
                          mxfp4_tc_block(numel, E) == 128, bs_ws, rb.status, &rows, stream);
     if (rc != XKB_OK) return rc;
@@ -454,8 +455,8 @@ extern "C" int xkb_workspace_status(const void* workspace, void* stream_) {
   XKB_CHECK_CUDA(cudaMemcpyAsync(&host, workspace, sizeof(int), cudaMemcpyDeviceToHost, stream));
   XKB_CHECK_CUDA(cudaStreamSynchronize(stream));
   if (host == 2)
-    return fail(XKB_ERR_DEVICE, "an MXFP4 scale byte in 191..254 (weights of 2^64 and more) is outside the range "
-                                "the tcgen05 dequantiser converts: status 0x2");
+    return fail(XKB_ERR_DEVICE, "an MXFP4 scale byte in 191..254 (weights of 2^64 and more), which batches of more than 48 "
+                                "slots per expert do not take: status 0x2");
   if ((host & 0xFF) == 3)
     return fail(XKB_ERR_DEVICE, "a kernel read a routing value outside what the routing buffers hold and skipped the "
                                 "work: status 0x%x (site %d)", host, host >> 8);

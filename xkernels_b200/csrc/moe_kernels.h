@@ -52,7 +52,8 @@ int launch_int4_ffn_simt(const void* A, int a_dtype, const int32_t* w13, const v
                          int num_map, int E, const float* topk_w, float* rows1, void* act, float* scratch,
                          int64_t hidden, int64_t inter, int top_k, int group, float limit, cudaStream_t stream);
 
-// MXFP4 on the block-scaled instructions (moe_mx.cu): the shapes of mxfp4_tc_supported, 32-byte aligned weights.
+// MXFP4 on the block-scaled instructions (moe_mx.cu): the shapes of mxfp4_tc_supported, 32-byte aligned weights, and
+// batches for which mxfp4_bs_block gives a token tile (0: too many slots per expert).
 // Leaves the bf16 rows of the slots, before the routing weight, in the workspace (*rows).
 bool mxfp4_bs_supported(const void* w13, const void* w2, const void* s13, const void* s2);
 int mxfp4_bs_block(int64_t numel, int E);

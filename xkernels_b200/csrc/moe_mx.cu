@@ -1,28 +1,27 @@
-// MXFP4 expert layer on the block-scaled tensor-core instructions (sm_100a).
+// MXFP4 expert layer on the block-scaled tensor-core instructions (sm_100a), decode-sized batches.
 //
 // tcgen05.mma kind::mxf8f6f4 takes the E2M1 weights and their e8m0 scales as they are: TMA unpacks the
 // nibbles into the byte containers the instruction reads, and nothing converts them.  The activations are
-// bf16 and stay exact as two block-scaled 8-bit terms (mx_split.cuh), so a 32-K step is two instructions
-// into one fp32 accumulator, which costs the tensor pipe what the bf16 product costs it (the 8-bit rate is
-// twice the bf16 rate).  What bounds the kernel is the weight stream at decode and the tensor pipe at
-// prefill; there is no conversion between the two.
+// bf16 and go in as three block-scaled 8-bit terms that hold every element down to 2^-31 of the largest of its
+// 32 exactly (mx_split.cuh).  What bounds the kernel is the weight stream; there is no conversion beside it.
+// Prefill-sized batches stay on the kernel that converts to bf16 (moe_tc.cu): three terms are half as many token
+// bytes again as bf16 activations, and from L2 they bound wide tiles (mxfp4_bs_block has the line).
 //
 // Swap-AB like the bf16 kernel: a tile is BT tokens of one expert block x two 128-row weight tiles (gate and
 // up rows, or two neighbouring row tiles of the down projection).  One persistent CTA per SM, sixteen warps:
 //   warp 0      weight producer: per 128-K stage two [128 x 128] tiles, per four stages their scales
-//   warps 1, 2  MMA issuers, one per weight matrix (eight MMAs a stage each).  One thread issues an MMA per 45
-//               cycles at best, whatever its width, so token tiles up to 32 have two issuers per matrix, one for
-//               each term with an accumulator of its own (warps 16, 17 are the second ones).
-//   warp 3      token producer (both terms of the stage, per four stages their scales)
+//   warps 1, 2  MMA issuers, one per weight matrix.  One thread issues a narrow MMA per 45 cycles at best, so token
+//               tiles up to 32 multiply the three terms in one instruction of 3 BT tokens (four a stage): M=48 below
+//               184 us with the terms on two issuers, 168 on three, 144 in one instruction.
+//   warp 3      token producer (the terms of the stage, per four stages their scales)
 //   warps 4-7   scale movers: the scale tiles are row-major, the instruction wants row r of a 128-row tile in
 //               lane r % 32, column r / 32 of tensor memory, the same in all four lane quarters.  Sixteen
 //               bytes of a row are four stages' scales: every warp reads them once and writes one column
 //               word per 32 rows and stage.
 //   warps 8-15  read-out, a tile behind the MMAs (two to four accumulator sets)
 //
-// Measured at E=256, hidden 4096, ispp 512, top_k 6, whole call, against the kernel that converts to bf16:
-// M=48 209 -> 158 us (0.58 GB of weights: 87 us at the copy rate; the same loads without any products 131 us),
-// M=4096 749 -> 597 us (without products and read-out 373: 2.4 GB pass from L2 to the SMs, tokens included).
+// Measured at E=256, hidden 4096, ispp 512, top_k 6, whole call in a graph, against the kernel that converts to
+// bf16: M=48 189 -> 144 us (0.58 GB of weights: 89 us at the copy rate), M=768 466 -> 259, M=2048 955 -> 425.
 //
 // Scale byte 0xFF means weight 0 here (it is NaN to the instruction): a mover that meets one clears the
 // group's weights in shared memory and puts byte 0 in its place.
@@ -43,29 +42,35 @@ constexpr int kRows = 128;          // weight rows per matrix and tile (UMMA M)
 constexpr int kStageK = 128;        // K per stage: one 128-byte swizzled row of byte containers
 constexpr int kChunkStages = 4;     // stages per 16-byte scale row
 constexpr int kWBytes = kRows * kStageK;
+constexpr int kTerms = 3;             // of an activation: hi, mid, lo
+constexpr int kThreads = 512;
 constexpr int kTmemCols = 512;
 constexpr uint32_t kProdSleepNs = 200;
 constexpr int kErrMxScaleRange = 2;
 constexpr uint32_t kMxMaxScale = 190;
 
 template <int BT> struct MxCfg {
-  static_assert(BT % 16 == 0 && BT <= 112, "token tile");
-  static constexpr int kTokRowGroups = (BT + 31) / 32;
+  static_assert(BT % 16 == 0 && BT <= 64, "token tile");
+  // Narrow tiles multiply all three terms in ONE instruction: the terms' tiles lie behind one another in shared
+  // memory, which is a tile of 3 BT tokens, each term with accumulators of its own that the read-out adds up.  An
+  // instruction costs its issuer 45 cycles up to 32 tokens or so, whatever its width.  Wider tiles have no room for the
+  // accumulators and issue three instructions into one.
+  static constexpr bool kMerged = BT <= 32;
+  static constexpr int kMmaTokens = kMerged ? kTerms * BT : BT;       // UMMA N
+  static constexpr int kTokRowGroups = (kMmaTokens + 31) / 32;
   static constexpr int kTokBytes = BT * kStageK;                      // one term
   static_assert(kTokBytes % 1024 == 0, "swizzle atoms");
-  static constexpr int kStageBytes = 2 * kWBytes + 2 * kTokBytes;
-  static constexpr int kStages = BT <= 32 ? 5 : BT <= 64 ? 4 : 3;
+  static constexpr int kStageBytes = 2 * kWBytes + kTerms * kTokBytes;
+  static constexpr int kStages = BT <= 16 ? 5 : BT <= 32 ? 4 : 3;
   // Scale tiles are loaded with the first stage of their four and read with all four: a slot is free again
   // when the MMAs kStages before that first stage are done, if kStages <= 4 * slots - 3.
   static constexpr int kScSlots = 2;
   static_assert(kStages <= 4 * kScSlots - 3, "scale slots");
-  static constexpr int kScBytes = 2 * kRows * 16 + 2 * BT * 16;
-  // columns: accumulator sets of two matrices, then per stage 4 gate + 4 up + 4 hi + 4 lo scale columns
-  static constexpr int kScCols = 16 * kStages;
-  static constexpr int kIssuersPerMat = BT <= 32 ? 2 : 1;
-  static constexpr int kIssuers = 2 * kIssuersPerMat;
-  static constexpr int kThreads = 512 + (kIssuersPerMat - 1) * 64;
-  static constexpr int kSetCols = 2 * kIssuersPerMat * BT;            // accumulator (matrix, issuer) at (matrix * kIssuersPerMat + issuer) * BT
+  static constexpr int kScBytes = 2 * kRows * 16 + BT * 16;
+  // columns: accumulator sets of two matrices, then per stage 4 gate + 4 up + 4 scale columns a token operand
+  static constexpr int kScStageCols = 8 + 4 * (kMerged ? 1 : kTerms);
+  static constexpr int kScCols = kScStageCols * kStages;
+  static constexpr int kSetCols = 2 * kMmaTokens;                     // accumulators of matrix 1 behind those of matrix 0
   static constexpr int kDFit = (kTmemCols - kScCols) / kSetCols;
   static constexpr int kDBuf = kDFit > 4 ? 4 : kDFit;
   static_assert(kDBuf >= 2, "the read-out must overlap the next tile");
@@ -84,10 +89,8 @@ struct MxParams {
   const int32_t* expert_ids;
   const int32_t* num_post;
   const __nv_bfloat16* bias;    // [E, rows_per_expert] or nullptr
-  uint8_t* act_hi;              // gate_up: the two terms [positions, N] and their scales [positions, N / 32]
-  uint8_t* act_lo;
-  uint8_t* act_shi;
-  uint8_t* act_slo;
+  uint8_t* act[kTerms];         // gate_up: the terms [positions, N] and hi's scales [positions, N / 32]
+  uint8_t* act_scale;
   __nv_bfloat16* rows;          // down: [slots, N], the bf16-rounded rows before the routing weight
   int* status;
   int64_t numel;
@@ -103,11 +106,11 @@ struct MxParams {
   int done_target;
 };
 
-// Instruction descriptor, kind::mxf8f6f4: b_sf_id [4,6), a type [7,10) (5 = e2m1), b type [10,13) (0 = e4m3,
-// 1 = e5m2), N >> 3 [17,23), scale type 23 (1 = ue8m0), M >> 7 [27,29), a_sf_id [29,31); fp32 accumulators,
+// Instruction descriptor, kind::mxf8f6f4: b_sf_id [4,6), a type [7,10) (5 = e2m1), b type [10,13) (1 = e5m2),
+// N >> 3 [17,23), scale type 23 (1 = ue8m0), M >> 7 [27,29), a_sf_id [29,31); fp32 accumulators,
 // both operands K-major.
-constexpr uint32_t mx_idesc(int n, int b_type, int sf) {
-  return ((uint32_t)sf << 4) | (5u << 7) | ((uint32_t)b_type << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | (1u << 27) |
+constexpr uint32_t mx_idesc(int n, int sf) {
+  return ((uint32_t)sf << 4) | (5u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | (1u << 27) |
          ((uint32_t)sf << 29);
 }
 __device__ __forceinline__ void umma_mx(uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa,
@@ -128,15 +131,15 @@ __device__ __forceinline__ void sts128_zero(uint32_t addr) {
 __device__ __forceinline__ uint32_t word_of(const uint4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
 
 template <int BT, bool GATE_UP>
-__global__ void __launch_bounds__(MxCfg<BT>::kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_ws,
-              const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo,
-              const __grid_constant__ CUtensorMap tm_shi, const __grid_constant__ CUtensorMap tm_slo, const MxParams p) {
+              const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_mid,
+              const __grid_constant__ CUtensorMap tm_lo, const __grid_constant__ CUtensorMap tm_xs, const MxParams p) {
   using Cfg = MxCfg<BT>;
   constexpr int kStages = Cfg::kStages, kDBuf = Cfg::kDBuf;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* s_sc = smem + kStages * Cfg::kStageBytes;     // kScSlots x { gate, up [128 x 16], hi, lo [BT x 16] }
+  unsigned char* s_sc = smem + kStages * Cfg::kStageBytes;     // kScSlots x { gate, up [128 x 16], tokens [BT x 16] }
   uint64_t* full = reinterpret_cast<uint64_t*>(s_sc + Cfg::kScSlots * Cfg::kScBytes);
   uint64_t* sf_full = full + kStages;
   uint64_t* empty = sf_full + kStages;
@@ -148,15 +151,15 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   Guard guard{abort_word, p.status};
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kStages; ++i) { mbar_init(&full[i], 2); mbar_init(&sf_full[i], 4); mbar_init(&empty[i], Cfg::kIssuers); }
-    for (int i = 0; i < kDBuf; ++i) { mbar_init(&d_full[i], Cfg::kIssuers); mbar_init(&d_empty[i], 4 * Cfg::kEpiWGs); }
+    for (int i = 0; i < kStages; ++i) { mbar_init(&full[i], 2); mbar_init(&sf_full[i], 4); mbar_init(&empty[i], 2); }
+    for (int i = 0; i < kDBuf; ++i) { mbar_init(&d_full[i], 2); mbar_init(&d_empty[i], 4 * Cfg::kEpiWGs); }
     *abort_word = 0;
     mbar_fence_init();
   }
   if (warp == 3) tmem_alloc(tmem_slot, kTmemCols);
   if (warp == 0 && lane == 0) { prefetch_tensormap(&tm_w); prefetch_tensormap(&tm_ws); }
   if (warp == 3 && lane == 0) {
-    prefetch_tensormap(&tm_hi); prefetch_tensormap(&tm_lo); prefetch_tensormap(&tm_shi); prefetch_tensormap(&tm_slo);
+    prefetch_tensormap(&tm_hi); prefetch_tensormap(&tm_mid); prefetch_tensormap(&tm_lo); prefetch_tensormap(&tm_xs);
   }
   // Block hand-over between the two GEMMs: as in the bf16 kernel (moe_tc.cu).  The first lets its dependents
   // go after its own wait; the second does not wait for the first grid but per token block, on a counter.
@@ -234,49 +237,45 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           if (!mbar_wait(&empty[st], ph, guard, 2, kProdSleepNs)) { ok = false; break; }
           unsigned char* s = smem + st * Cfg::kStageBytes + 2 * kWBytes;
           const bool head = (ks & (kChunkStages - 1)) == 0;
-          mbar_expect_tx(&full[st], 2 * Cfg::kTokBytes + (head ? 2 * BT * 16 : 0));
+          mbar_expect_tx(&full[st], kTerms * Cfg::kTokBytes + (head ? BT * 16 : 0));
           tma_load_2d(s, &tm_hi, &full[st], ks * kStageK, pos0);
-          tma_load_2d(s + Cfg::kTokBytes, &tm_lo, &full[st], ks * kStageK, pos0);
+          tma_load_2d(s + Cfg::kTokBytes, &tm_mid, &full[st], ks * kStageK, pos0);
+          tma_load_2d(s + 2 * Cfg::kTokBytes, &tm_lo, &full[st], ks * kStageK, pos0);
           if (head) {
             unsigned char* sc = s_sc + (chunk % Cfg::kScSlots) * Cfg::kScBytes + 2 * kRows * 16;
-            tma_load_2d(sc, &tm_shi, &full[st], ks * (kStageK / 32), pos0);
-            tma_load_2d(sc + BT * 16, &tm_slo, &full[st], ks * (kStageK / 32), pos0);
+            tma_load_2d(sc, &tm_xs, &full[st], ks * (kStageK / 32), pos0);
             ++chunk;
           }
           if (++st == kStages) { st = 0; ph ^= 1; }
         }
       }
     }
-  } else if (warp < 3 || warp >= 16) {
-    // ---------------- MMA issuers: warp 1 + matrix, 16 + matrix ----------------
+  } else if (warp < 3) {
+    // ---------------- MMA issuers: warp 1 + matrix ----------------
     if (lane == 0) {
-      const uint32_t mat = warp < 3 ? (uint32_t)warp - 1 : (uint32_t)warp - 16, term = warp < 3 ? 0u : 1u;
+      const uint32_t mat = (uint32_t)warp - 1;
       uint32_t st = 0, ph = 0, dbuf = 0, dph = 1;
       bool ok = true;
       for (int t = (int)blockIdx.x; t < total_tiles && ok && !guard.aborted(); t += (int)gridDim.x) {
         if (!mbar_wait(&d_empty[dbuf], dph, guard, 8)) break;
         tc_fence_after();
-        const uint32_t d = tmem_base + dbuf * Cfg::kSetCols + (mat * Cfg::kIssuersPerMat + term) * BT;
+        const uint32_t d = tmem_base + dbuf * Cfg::kSetCols + mat * Cfg::kMmaTokens;
         for (int ks = 0; ks < k_stages; ++ks) {
           if (!mbar_wait(&full[st], ph, guard, 3) || !mbar_wait(&sf_full[st], ph, guard, 4)) { ok = false; break; }
           tc_fence_after();
           const uint32_t s = smem_u32(smem + st * Cfg::kStageBytes);
           const uint64_t a = umma_desc_k_sw128(s + mat * kWBytes);
-          const uint64_t bh = umma_desc_k_sw128(s + 2 * kWBytes), bl = umma_desc_k_sw128(s + 2 * kWBytes + Cfg::kTokBytes);
-          const uint32_t sc = tmem_base + Cfg::kScCol0 + st * 16;
+          const uint64_t bh = umma_desc_k_sw128(s + 2 * kWBytes), bm = umma_desc_k_sw128(s + 2 * kWBytes + Cfg::kTokBytes),
+                         bl = umma_desc_k_sw128(s + 2 * kWBytes + 2 * Cfg::kTokBytes);
+          const uint32_t sc = tmem_base + Cfg::kScCol0 + st * Cfg::kScStageCols, sw = sc + mat * 4;
           // 32 K each: 32 bytes on in the swizzled rows, the next scale byte
-          if (Cfg::kIssuersPerMat == 1) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              umma_mx(d, a + k * 2, bh + k * 2, mx_idesc(BT, 1, k), sc + mat * 4, sc + 8, (ks | k) != 0);
-              umma_mx(d, a + k * 2, bl + k * 2, mx_idesc(BT, 0, k), sc + mat * 4, sc + 12, 1u);
+          for (int k = 0; k < 4; ++k) {
+            umma_mx(d, a + k * 2, bh + k * 2, mx_idesc(Cfg::kMmaTokens, k), sw, sc + 8, (ks | k) != 0);
+            if (!Cfg::kMerged) {
+              umma_mx(d, a + k * 2, bm + k * 2, mx_idesc(BT, k), sw, sc + 12, 1u);
+              umma_mx(d, a + k * 2, bl + k * 2, mx_idesc(BT, k), sw, sc + 16, 1u);
             }
-          } else if (term == 0) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) umma_mx(d, a + k * 2, bh + k * 2, mx_idesc(BT, 1, k), sc + mat * 4, sc + 8, (ks | k) != 0);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) umma_mx(d, a + k * 2, bl + k * 2, mx_idesc(BT, 0, k), sc + mat * 4, sc + 12, (ks | k) != 0);
           }
           tc_commit(&empty[st]);
           if (++st == kStages) { st = 0; ph ^= 1; }
@@ -295,7 +294,7 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     for (int t = (int)blockIdx.x; t < total_tiles && ok && !guard.aborted(); t += (int)gridDim.x) {
       for (int kc = 0; kc < k_stages && ok; kc += kChunkStages, ++chunk) {
         const uint32_t sc = smem_u32(s_sc + (chunk % Cfg::kScSlots) * Cfg::kScBytes);
-        uint4 w[2][4], x[2][Cfg::kTokRowGroups];
+        uint4 w[2][4], x[Cfg::kTokRowGroups];
 #pragma unroll
         for (int j = 0; j < kChunkStages; ++j) {
           if (!mbar_wait(&full[st], ph, guard, 5)) { ok = false; break; }
@@ -305,13 +304,11 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 #pragma unroll
               for (int c = 0; c < 4; ++c) w[m][c] = lds128(sc + (uint32_t)((m * kRows + c * 32 + lane) * 16));
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-              for (int c = 0; c < Cfg::kTokRowGroups; ++c)
-                x[m][c] = (c * 32 + lane < BT) ? lds128(sc + 2 * kRows * 16 + (uint32_t)((m * BT + c * 32 + lane) * 16))
-                                               : make_uint4(0, 0, 0, 0);
+            for (int c = 0; c < Cfg::kTokRowGroups; ++c)
+              x[c] = (c * 32 + lane < Cfg::kMmaTokens) ? lds128(sc + 2 * kRows * 16 + (uint32_t)((c * 32 + lane) % BT * 16))
+                                                       : make_uint4(0, 0, 0, 0);
           }
-          const uint32_t dst = tmem_base + lane_base + Cfg::kScCol0 + st * 16;
+          const uint32_t dst = tmem_base + lane_base + Cfg::kScCol0 + st * Cfg::kScStageCols;
 #pragma unroll
           for (int m = 0; m < 2; ++m) {
             uint32_t v[4], nan = 0;
@@ -344,12 +341,22 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
             }
             tmem_st_32x4(dst + m * 4, v[0], v[1], v[2], v[3]);
           }
+          uint32_t v[4] = {0, 0, 0, 0};
 #pragma unroll
-          for (int m = 0; m < 2; ++m) {
-            uint32_t v[4] = {0, 0, 0, 0};
+          for (int c = 0; c < Cfg::kTokRowGroups; ++c) v[c] = word_of(x[c], j);
+          // hi's bytes are kLoShift at least (padding positions hold anything: their columns are never read)
+          constexpr uint32_t kMid4 = mx::kMidShift * 0x01010101u, kLo4 = mx::kLoShift * 0x01010101u;
+          if (Cfg::kMerged) {
 #pragma unroll
-            for (int c = 0; c < Cfg::kTokRowGroups; ++c) v[c] = word_of(x[m][c], j);
-            tmem_st_32x4(dst + 8 + m * 4, v[0], v[1], v[2], v[3]);
+            for (int c = 0; c < Cfg::kTokRowGroups; ++c) {
+              const int term = (c * 32 + lane) / BT;
+              v[c] = __vsub4(v[c], term == 0 ? 0u : term == 1 ? kMid4 : kLo4);
+            }
+            tmem_st_32x4(dst + 8, v[0], v[1], v[2], v[3]);
+          } else {
+            tmem_st_32x4(dst + 8, v[0], v[1], v[2], v[3]);
+            tmem_st_32x4(dst + 12, __vsub4(v[0], kMid4), __vsub4(v[1], kMid4), __vsub4(v[2], kMid4), __vsub4(v[3], kMid4));
+            tmem_st_32x4(dst + 16, __vsub4(v[0], kLo4), __vsub4(v[1], kLo4), __vsub4(v[2], kLo4), __vsub4(v[3], kLo4));
           }
           tmem_wait_st();
           tc_fence_before();
@@ -390,19 +397,19 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           uint32_t a0[16], a1[16];
           const uint32_t d = tmem_base + lane_base + dbuf * Cfg::kSetCols + cg * 16;
           tmem_ld_32x16(d, a0);
-          tmem_ld_32x16(d + Cfg::kIssuersPerMat * BT, a1);
-          if (Cfg::kIssuersPerMat == 2) {
+          tmem_ld_32x16(d + Cfg::kMmaTokens, a1);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 1; i < (Cfg::kMerged ? kTerms : 1); ++i) {
             uint32_t b0[16], b1[16];
-            tmem_ld_32x16(d + BT, b0);
-            tmem_ld_32x16(d + 3 * BT, b1);
+            tmem_ld_32x16(d + i * BT, b0);
+            tmem_ld_32x16(d + Cfg::kMmaTokens + i * BT, b1);
             tmem_wait_ld();
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               a0[j] = __float_as_uint(__uint_as_float(a0[j]) + __uint_as_float(b0[j]));
               a1[j] = __float_as_uint(__uint_as_float(a1[j]) + __uint_as_float(b1[j]));
             }
-          } else {
-            tmem_wait_ld();
           }
           // The sixteen columns are computed side by side whether they are live or padding (whose values are
           // never stored): their chains overlap, which branches between them would not allow.
@@ -421,25 +428,25 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 #pragma unroll
             for (int j = 0; j < 16; ++j) top[j] = __reduce_max_sync(0xffffffffu, mx::finite_abs_bits(a0[j] >> 16));
             const int64_t pos = (int64_t)b * BT + cg * 16;
-            uint8_t* hi8 = p.act_hi + pos * p.N + n_glob;
-            uint8_t* lo8 = p.act_lo + pos * p.N + n_glob;
+            const int64_t at = pos * p.N + n_glob;
 #pragma unroll
             for (int j = 0; j < 16; j += 2) {
               const float x0 = __uint_as_float(a0[j]), x1 = __uint_as_float(a0[j + 1]);
               const uint32_t s0 = mx::hi_scale(top[j]), s1 = mx::hi_scale(top[j + 1]);
-              uint32_t hi, lo;
-              mx::split_pair(x0, x1, mx::hi_factor(s0), mx::hi_factor(s1), hi, lo);
-              if ((live >> j) & 1u) { hi8[(int64_t)j * p.N] = (uint8_t)hi; lo8[(int64_t)j * p.N] = (uint8_t)lo; }
-              if ((live >> (j + 1)) & 1u) { hi8[(int64_t)(j + 1) * p.N] = (uint8_t)(hi >> 8); lo8[(int64_t)(j + 1) * p.N] = (uint8_t)(lo >> 8); }
+              uint32_t term[kTerms];
+              mx::split_pair(x0, x1, mx::hi_factor(s0), mx::hi_factor(s1), term[0], term[1], term[2]);
+#pragma unroll
+              for (int i = 0; i < kTerms; ++i) {
+                if ((live >> j) & 1u) p.act[i][at + (int64_t)j * p.N] = (uint8_t)term[i];
+                if ((live >> (j + 1)) & 1u) p.act[i][at + (int64_t)(j + 1) * p.N] = (uint8_t)(term[i] >> 8);
+              }
             }
-            // lane j stores the scale bytes of position j
+            // lane j stores the scale byte of position j
             uint32_t sh = 0;
 #pragma unroll
             for (int j = 0; j < 16; ++j) sh = lane == j ? mx::hi_scale(top[j]) : sh;
-            if ((live >> lane) & 1u) {   // (live has sixteen bits)
-              p.act_shi[(pos + lane) * (p.N / 32) + (n_glob >> 5)] = (uint8_t)sh;
-              p.act_slo[(pos + lane) * (p.N / 32) + (n_glob >> 5)] = (uint8_t)(sh + mx::kLoShift);
-            }
+            if ((live >> lane) & 1u)   // (live has sixteen bits)
+              p.act_scale[(pos + lane) * (p.N / 32) + (n_glob >> 5)] = (uint8_t)sh;
           } else {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -473,20 +480,14 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   }
 }
 
-// Rows of A, split into the two terms, at the positions of all their slots (token by token, as
+// Rows of A, split into the three terms, at the positions of all their slots (token by token, as
 // gather_permute_kernel): 32 elements = one scale block = four threads.
-template <bool SORT>
-__global__ void __launch_bounds__(SORT ? 1024 : kGatherThreads)
-gather_split_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos, uint8_t* __restrict__ hi,
-                    uint8_t* __restrict__ lo, uint8_t* __restrict__ shi, uint8_t* __restrict__ slo, int K, int top_k,
-                    int64_t max_pad, unsigned pieces, unsigned units, int* __restrict__ status, const align::Job job) {
-  if (SORT) chain_trigger();   // the first kernel of the call; the next one waits for its completion
-  const unsigned m = blockIdx.x / pieces;
-  const int i = (int)((blockIdx.x - m * pieces) * units + threadIdx.x);
-  const bool mine = threadIdx.x < units && i < K / 8;   // both are multiples of 32: whole warps
-  uint32_t h[4] = {0, 0, 0, 0}, l[4] = {0, 0, 0, 0}, sh = 0;
-  if (mine) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(A + (int64_t)m * K) + i);
+struct SplitRows { uint8_t *hi, *mid, *lo, *scale; };   // [positions, K], scales of hi [positions, K / 32]
+struct SplitUnit {
+  uint32_t h[4], d[4], l[4], scale;
+  // eight elements; the four threads of a scale block are neighbours
+  __device__ __forceinline__ void load(const uint4* src) {
+    const uint4 v = __ldg(src);   // an input of the call
     const uint32_t u[4] = {v.x, v.y, v.z, v.w};
     uint32_t top = 0;
 #pragma unroll
@@ -494,12 +495,30 @@ gather_split_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos
       top = max(top, max(mx::finite_abs_bits(u[q] & 0xFFFFu), mx::finite_abs_bits(u[q] >> 16)));
     top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
     top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
-    sh = mx::hi_scale(top);
-    const float f = mx::hi_factor(sh);
+    scale = mx::hi_scale(top);
+    const float f = mx::hi_factor(scale);
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      mx::split_pair(__uint_as_float(u[q] << 16), __uint_as_float(u[q] & 0xFFFF0000u), f, f, h[q], l[q]);
+      mx::split_pair(__uint_as_float(u[q] << 16), __uint_as_float(u[q] & 0xFFFF0000u), f, f, h[q], d[q], l[q]);
   }
+  __device__ __forceinline__ void store(const SplitRows& x, int64_t pos, int K, int i) const {
+    reinterpret_cast<uint2*>(x.hi + pos * K)[i] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+    reinterpret_cast<uint2*>(x.mid + pos * K)[i] = make_uint2(d[0] | (d[1] << 16), d[2] | (d[3] << 16));
+    reinterpret_cast<uint2*>(x.lo + pos * K)[i] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+    if ((i & 3) == 0) x.scale[pos * (K / 32) + (i >> 2)] = (uint8_t)scale;
+  }
+};
+
+template <bool SORT>
+__global__ void __launch_bounds__(SORT ? 1024 : kGatherThreads)
+gather_split_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos, const SplitRows x, int K, int top_k,
+                    int64_t max_pad, unsigned pieces, unsigned units, int* __restrict__ status, const align::Job job) {
+  if (SORT) chain_trigger();   // the first kernel of the call; the next one waits for its completion
+  const unsigned m = blockIdx.x / pieces;
+  const int i = (int)((blockIdx.x - m * pieces) * units + threadIdx.x);
+  const bool mine = threadIdx.x < units && i < K / 8;   // both are multiples of 32: whole warps
+  SplitUnit o = {};
+  if (mine) o.load(reinterpret_cast<const uint4*>(A + (int64_t)m * K) + i);
   if (!SORT) {
     chain_wait();     // the routing is read with L2 loads after the wait (see gather_permute_kernel)
     chain_trigger();
@@ -517,13 +536,7 @@ gather_split_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos
     unsigned live = __ballot_sync(0xffffffffu, mine_pos >= 0 && mine_pos < max_pad);
     for (; live != 0; live &= live - 1) {
       const int64_t pos = __shfl_sync(0xffffffffu, mine_pos, __ffs(live) - 1);
-      if (!mine) continue;
-      reinterpret_cast<uint2*>(hi + pos * K)[i] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-      reinterpret_cast<uint2*>(lo + pos * K)[i] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
-      if ((i & 3) == 0) {
-        shi[pos * (K / 32) + (i >> 2)] = (uint8_t)sh;
-        slo[pos * (K / 32) + (i >> 2)] = (uint8_t)(sh + mx::kLoShift);
-      }
+      if (mine) o.store(x, pos, K, i);
     }
   }
 }
@@ -545,7 +558,7 @@ int launch_mx(const CUtensorMap (&tm)[6], const MxParams& prm, int64_t max_tiles
   if (grid < 8) grid = 8;
   if (grid > max_tiles) grid = max_tiles;
   if (grid < 1) grid = 1;
-  XKB_CHECK_CUDA(launch_chained(moe_mx_kernel<BT, GATE_UP>, dim3((unsigned)grid), dim3(MxCfg<BT>::kThreads), MxCfg<BT>::kSmemBytes,
+  XKB_CHECK_CUDA(launch_chained(moe_mx_kernel<BT, GATE_UP>, dim3((unsigned)grid), dim3(kThreads), MxCfg<BT>::kSmemBytes,
                                 stream, tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], prm));
   XKB_CHECK_LAUNCH("moe_mx_kernel");
   return XKB_OK;
@@ -557,26 +570,25 @@ int launch_mx_by_block(int block, const CUtensorMap (&tm)[6], const MxParams& pr
     case 16: return launch_mx<16, GATE_UP>(tm, prm, max_tiles, stream);
     case 32: return launch_mx<32, GATE_UP>(tm, prm, max_tiles, stream);
     case 64: return launch_mx<64, GATE_UP>(tm, prm, max_tiles, stream);
-    case 112: return launch_mx<112, GATE_UP>(tm, prm, max_tiles, stream);
     default: return fail(XKB_ERR_ARG, "mxfp4 block-scaled path: unsupported token tile %d", block);
   }
 }
 
 struct MxBuffers {
   __nv_bfloat16* rows;
-  uint8_t *x[4], *act[4];   // hi, lo, scales of hi, scales of lo
+  uint8_t *x[kTerms + 1], *act[kTerms + 1];   // hi, mid, lo, scales of hi
 };
 MxBuffers carve_mx(Carver& c, int64_t numel, int64_t max_pad, int64_t hidden, int64_t ispp) {
   MxBuffers b;
   b.rows = c.take<__nv_bfloat16>(numel * hidden);
-  for (int i = 0; i < 4; ++i) b.x[i] = c.take<uint8_t>(max_pad * (i < 2 ? hidden : hidden / 32));
-  for (int i = 0; i < 4; ++i) b.act[i] = c.take<uint8_t>(max_pad * (i < 2 ? ispp : ispp / 32));
+  for (int i = 0; i <= kTerms; ++i) b.x[i] = c.take<uint8_t>(max_pad * (i < kTerms ? hidden : hidden / 32));
+  for (int i = 0; i <= kTerms; ++i) b.act[i] = c.take<uint8_t>(max_pad * (i < kTerms ? ispp : ispp / 32));
   return b;
 }
 
-int token_maps(CUtensorMap* tm, uint8_t* const (&x)[4], int64_t max_pad, int64_t K, int block) {
-  for (int i = 0; i < 4; ++i) {
-    const bool sc = i >= 2;
+int token_maps(CUtensorMap* tm, uint8_t* const (&x)[kTerms + 1], int64_t max_pad, int64_t K, int block) {
+  for (int i = 0; i <= kTerms; ++i) {
+    const bool sc = i == kTerms;
     const int rc = make_map_2d(&tm[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 8, x[i], (uint64_t)max_pad, (uint64_t)(sc ? K / 32 : K),
                                (uint32_t)block, sc ? 16 : kStageK, sc ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
                                sc ? "activation scales" : "activation terms");
@@ -602,19 +614,23 @@ bool mxfp4_bs_supported(const void* w13, const void* w2, const void* s13, const 
          ((reinterpret_cast<uintptr_t>(s13) | reinterpret_cast<uintptr_t>(s2)) & 15) == 0;
 }
 
-// The widest tile is the widest that leaves tensor memory for two accumulator sets beside the scales; a
-// narrower one is taken while a block still holds nearly every expert's slots (an expert that needs a second
-// block streams its weights twice).  E=256, hidden 4096, ispp 512, whole call: 16 against 32 tokens 220 / 229 us at 8 slots
-// per expert, 248 / 234 at 10; 32 against 64 253 / 291 at 21, 283 / 295 at 23, 360 / 312 at 33; 64 against 112
-// 335 / 392 at 47, 432 / 429 at 61, 653 / 459 at 80.
+// A narrower tile is taken while a block still holds nearly every expert's slots (an expert that needs a second block
+// streams its weights twice); 0 = the bf16 kernel's 128-token tiles, whose tokens are 2 bytes and not 3.  Whole
+// calls in a graph, E=256, hidden 4096, ispp 512 / E=128, 4096, 1024 / E=64, 2048, 1024:
+//   16 against 32 tokens  241 / 241 us at 11 slots per expert, 259 / 247 at 14; 222 / 227 at 12; 73 / 80 at 12
+//   32 against 64         323 / 362 at 30, 398 / 374 at 36; 282 / 348 at 28, 403 / 355 at 40; 95 / 111 at 28, 123 / 115 at 40
+//   64 against bf16       484 / 500 at 54, 525 / 526 at 60; 422 / 451 at 56, 527 / 459 at 64; 126 / 133 at 56, 158 / 138 at 64
+// (96-token tiles, the widest that fit: 537 / 565 at 66, but 495 / 459 and 138 / 138 at 64; left out.)
 int mxfp4_bs_block(int64_t numel, int E) {
   const double avg = (double)numel / (E > 0 ? E : 1);
-  return avg <= 9 ? 16 : avg <= 26 ? 32 : avg <= 56 ? 64 : 112;
+  return avg <= 12 ? 16 : avg <= 32 ? 32 : avg <= 56 ? 64 : 0;
 }
 
 int64_t mxfp4_bs_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, int E) {
+  const int block = mxfp4_bs_block(numel, E);
+  if (block == 0) return 0;
   Carver c(nullptr);
-  carve_mx(c, numel, numel + (int64_t)(E + 1) * 111, hidden, ispp);
+  carve_mx(c, numel, numel + (int64_t)(E + 1) * (block - 1), hidden, ispp);
   return c.off;
 }
 
@@ -625,21 +641,20 @@ int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   Carver carve(ws);
   const MxBuffers buf = carve_mx(carve, r.numel, r.max_pad, hidden, ispp);
   *rows_out = buf.rows;
+  const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(A);
+  const SplitRows x{buf.x[0], buf.x[1], buf.x[2], buf.x[kTerms]};
   GatherGrid g;
   int rc = gather_grid(r.numel / top_k, hidden / 8, r.job != nullptr, &g);
   if (rc != XKB_OK) return rc;
-  const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(A);
   if (r.job != nullptr) {
     const size_t smem = align::small_smem(r.job->E);
     if (smem > 48 * 1024)
       XKB_CHECK_CUDA(cudaFuncSetAttribute(gather_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    gather_split_kernel<true><<<g.blocks, g.threads, smem, stream>>>(a, nullptr, buf.x[0], buf.x[1], buf.x[2], buf.x[3],
-                                                                     (int)hidden, top_k, r.max_pad, g.pieces, g.units, status,
-                                                                     *r.job);
+    gather_split_kernel<true><<<g.blocks, g.threads, smem, stream>>>(a, nullptr, x, (int)hidden, top_k, r.max_pad, g.pieces,
+                                                                     g.units, status, *r.job);
   } else {
-    XKB_CHECK_CUDA(launch_chained(gather_split_kernel<false>, dim3(g.blocks), dim3(g.threads), 0, stream, a, r.slot_pos,
-                                  buf.x[0], buf.x[1], buf.x[2], buf.x[3], (int)hidden, top_k, r.max_pad, g.pieces, g.units,
-                                  status, align::Job{}));
+    XKB_CHECK_CUDA(launch_chained(gather_split_kernel<false>, dim3(g.blocks), dim3(g.threads), 0, stream, a, r.slot_pos, x,
+                                  (int)hidden, top_k, r.max_pad, g.pieces, g.units, status, align::Job{}));
   }
   XKB_CHECK_LAUNCH("gather_split_kernel");
 
@@ -661,10 +676,8 @@ int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   prm.max_blocks = (int)r.max_blocks;
   prm.num_experts = E;
   prm.bias = static_cast<const __nv_bfloat16*>(b13);
-  prm.act_hi = buf.act[0];
-  prm.act_lo = buf.act[1];
-  prm.act_shi = buf.act[2];
-  prm.act_slo = buf.act[3];
+  for (int i = 0; i < kTerms; ++i) prm.act[i] = buf.act[i];
+  prm.act_scale = buf.act[kTerms];
   prm.rows = nullptr;
   prm.N = (int)ispp;
   prm.K = (int)hidden;
