@@ -39,3 +39,21 @@ def test_gather_sum_reduce(H, k, dtype, cuda_device):
     got = ops.moe_gather_sum_reduce(rows, index, None, out_dtype=dtype).double()
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -24
     assert bool(((got - picked.sum(1)).abs() <= k * 2.0 ** -24 * picked.abs().sum(1) + eps * picked.sum(1).abs() * 1.01).all())
+
+
+@pytest.mark.parametrize("H", [8, 24, 64, 128, 136, 1024])
+@pytest.mark.parametrize("M", [1183, 1184, 1185, 151553])
+def test_narrow_rows_share_a_block(M, H, cuda_device):
+    """Many tokens of narrow rows: several per block from twice 592 tokens on, up to a whole block of them."""
+    if M * H > 2 ** 25:
+        M = 20001
+    g = torch.Generator(device=cuda_device).manual_seed(M + H)
+    y = torch.randn(M, 3, H, generator=g, device=cuda_device)
+    w = torch.randn(M, 3, generator=g, device=cuda_device)
+    term = y.double() * w.double().unsqueeze(-1)
+    bound = 4 * 2.0 ** -24 * term.abs().sum(1) + 2.0 ** -24 * 1.01 * term.sum(1).abs()
+    assert bool(((xkb.moe_sum_reduce(y, w).double() - term.sum(1)).abs() <= bound).all())
+    rows, index = y.reshape(-1, H), torch.randint(-2, 3 * M, (M, 3), generator=g, device=cuda_device, dtype=torch.int32)
+    picked = rows[index.long().clamp(min=0)].double() * (index >= 0).unsqueeze(-1)
+    got = ops.moe_gather_sum_reduce(rows, index, None, out_dtype=torch.float32).double()
+    assert bool(((got - picked.sum(1)).abs() <= 4 * 2.0 ** -24 * picked.abs().sum(1)).all())

@@ -3,8 +3,8 @@
 //   out[m, h] = rsf * sum_k (w[m,k] or 1) * y[m,k,h]        fp32, ascending k
 //
 // HBM-bound.  A thread owns 8 consecutive columns of one token and requests up to kBatch of its top_k
-// rows with 128-bit loads before it adds the first; a block is a piece of one token's columns, so that
-// the token is found with one 32-bit division per block and not one 64-bit division per thread.
+// rows with 128-bit loads before it adds the first; a block is a piece of one token's columns, or several
+// tokens of narrow rows, so that the token is found with one 32-bit division and not a 64-bit one.
 // No atomics, fixed summation order: the result is bit-reproducible run to run.  Reference semantics:
 // src/xkernels/ops/moe/sum_reduce.py:20-39.
 // M=8192, top_k=8, H=7168, bf16 (1.06 GB): 232 -> 153 us, 6.9 TB/s.
@@ -76,21 +76,28 @@ __device__ __forceinline__ bool slot_valid(const int32_t* ids, const int32_t* em
 //   kIndexed: row ids[m * top_k + k], none where that is negative.
 enum Rows { kAll, kSlots, kIndexed };
 
-template <typename TY, typename TW, typename TO, Rows ROWS>
+// NARROW: a block is `per` tokens instead of a piece of one.
+template <typename TY, typename TW, typename TO, Rows ROWS, bool NARROW>
 __global__ void __launch_bounds__(256)
 sum_reduce_vec8_kernel(const TY* y, const TW* __restrict__ w, TO* __restrict__ out,
-                       unsigned pieces, int top_k, int64_t H, float rsf, const int32_t* __restrict__ ids,
-                       const int32_t* __restrict__ emap, int num_map, int E) {
+                       int64_t M, unsigned pieces, unsigned per, int top_k, int64_t H, float rsf,
+                       const int32_t* __restrict__ ids, const int32_t* __restrict__ emap, int num_map, int E) {
   // As the combine of a fused call the slot rows come from the GEMM kernel before this one, which is
   // still running when this kernel starts: `y` is therefore not `const __restrict__` (no invariant /
   // non-coherent loads, which may deliver what was there before the wait).
   chain_wait();
-  const unsigned m = blockIdx.x / pieces;
-  const int64_t h = ((int64_t)(blockIdx.x - m * pieces) * blockDim.x + threadIdx.x) << 3;
+  unsigned m = blockIdx.x / pieces;
+  int64_t h = ((int64_t)(blockIdx.x - m * pieces) * blockDim.x + threadIdx.x) << 3;
+  if (NARROW) {
+    const unsigned hv = (unsigned)(H >> 3), t = threadIdx.x / hv;
+    m = blockIdx.x * per + t;
+    h = (int64_t)(threadIdx.x - t * hv) << 3;
+    if (t >= per || m >= M) return;
+  }
   if (h >= H) return;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const int64_t slot0 = (int64_t)m * top_k;
-  constexpr int kBatch = Vec8<TY>::kBatch;
+  constexpr int kBatch = NARROW ? 4 : Vec8<TY>::kBatch;   // (there are enough tokens)
   for (int k0 = 0; k0 < top_k; k0 += kBatch) {
     Vec8<TY> v[kBatch];
     bool take[kBatch];
@@ -125,16 +132,24 @@ sum_reduce_vec8_kernel(const TY* y, const TW* __restrict__ w, TO* __restrict__ o
   Vec8<TO>::store(out + (int64_t)m * H + h, acc);
 }
 
-// Pieces per token and threads per block: as few pieces of at most `most` threads as cover H / 8 columns,
-// in whole warps.  False if the grid would not fit.  The combine of a fused call takes 128: blocks of 256
-// threads need more registers than a GEMM block leaves free, so that they could not be resident yet when
-// the GEMM ends (2 us a call).
-bool vec8_grid(int64_t M, int64_t H, int64_t most, unsigned* pieces, unsigned* threads, unsigned* blocks) {
+// The grid: as few pieces of a token of at most `most` threads as cover H / 8 columns, in whole warps; or, where
+// a row fills half a block or less and the tokens are many, `per` tokens per block (a block of a few live threads
+// per token costs more in launches than in loads: M=262144, H=8, top_k=2, bf16 137 us with a token per block,
+// 3.3 with as many as fit; M=65536, H=64, top_k=8 36.3 and 8.2; M=16384, H=128, top_k=8 10.7 and 4.7).  At least kFullGrid blocks are left, below which the
+// tokens are spread over the chip instead.  False if the grid would not fit.  The combine of a fused call takes
+// 128: blocks of 256 threads need more registers than a GEMM block leaves free, so that they could not be resident
+// yet when the GEMM ends (2 us a call).
+struct Vec8Grid { unsigned pieces, per, threads, blocks; };
+constexpr int64_t kFullGrid = 4 * 148;
+bool vec8_grid(int64_t M, int64_t H, int64_t most, Vec8Grid* g) {
   const int64_t hv = H / 8, p = ceil_div(hv, most);
-  if (p * M > 0x7fffffff) return false;
-  *pieces = (unsigned)p;
-  *threads = (unsigned)align_up(ceil_div(hv, p), 32);
-  *blocks = (unsigned)(p * M);
+  int64_t per = most / hv < M / kFullGrid ? most / hv : M / kFullGrid;
+  if (per < 1) per = 1;
+  if (p * ceil_div(M, per) > 0x7fffffff || M > 0x7fffffff) return false;
+  g->pieces = (unsigned)p;
+  g->per = (unsigned)per;
+  g->threads = (unsigned)align_up(per > 1 ? per * hv : ceil_div(hv, p), 32);
+  g->blocks = (unsigned)(p * ceil_div(M, per));
   return true;
 }
 
@@ -164,14 +179,16 @@ template <typename TY, typename TW, typename TO>
 int launch_typed(const void* y, const void* w, void* out, int64_t M, int top_k, int64_t H, float rsf,
                  const int32_t* ids, const int32_t* emap, int num_map, int E, cudaStream_t stream) {
   if (M == 0 || H == 0) return XKB_OK;
-  unsigned pieces = 1, threads = 32, vblocks = 1;
+  Vec8Grid g{};
   const bool vec_ok = (H % 8 == 0) && (reinterpret_cast<uintptr_t>(y) % 16 == 0) &&
-                      (reinterpret_cast<uintptr_t>(out) % 16 == 0) && vec8_grid(M, H, ids != nullptr ? 128 : 256, &pieces, &threads, &vblocks);
+                      (reinterpret_cast<uintptr_t>(out) % 16 == 0) && vec8_grid(M, H, ids != nullptr ? 128 : 256, &g);
   if (vec_ok) {
-    auto kernel = ids != nullptr ? sum_reduce_vec8_kernel<TY, TW, TO, kSlots> : sum_reduce_vec8_kernel<TY, TW, TO, kAll>;
-    XKB_CHECK_CUDA(launch_chained(kernel, dim3(vblocks), dim3(threads), 0, stream,
-                                  static_cast<const TY*>(y), static_cast<const TW*>(w), static_cast<TO*>(out), pieces,
-                                  top_k, H, rsf, ids, emap, num_map, E));
+    const bool narrow = g.per > 1;
+    auto kernel = ids != nullptr ? (narrow ? sum_reduce_vec8_kernel<TY, TW, TO, kSlots, true> : sum_reduce_vec8_kernel<TY, TW, TO, kSlots, false>)
+                                 : (narrow ? sum_reduce_vec8_kernel<TY, TW, TO, kAll, true> : sum_reduce_vec8_kernel<TY, TW, TO, kAll, false>);
+    XKB_CHECK_CUDA(launch_chained(kernel, dim3(g.blocks), dim3(g.threads), 0, stream,
+                                  static_cast<const TY*>(y), static_cast<const TW*>(w), static_cast<TO*>(out), M, g.pieces,
+                                  g.per, top_k, H, rsf, ids, emap, num_map, E));
     XKB_CHECK_LAUNCH("sum_reduce_vec8_kernel");
   } else {
     // 148 SMs x 8 resident 256-thread CTAs; grid-stride covers the rest
@@ -218,6 +235,17 @@ gather_reduce_kernel(const float* __restrict__ rows, const int32_t* __restrict__
     TO* o = out + m * H + h;
     from_f(o[0], acc.x); from_f(o[1], acc.y); from_f(o[2], acc.z); from_f(o[3], acc.w);
   }
+}
+
+template <bool NARROW>
+void launch_indexed_as(const Vec8Grid& g, const float* rows, const int32_t* row_index, const float* w, void* out, int out_dtype,
+                       int64_t M, int top_k, int64_t H, cudaStream_t s) {
+  if (out_dtype == XKB_BF16)
+    sum_reduce_vec8_kernel<float, float, __nv_bfloat16, kIndexed, NARROW><<<g.blocks, g.threads, 0, s>>>(
+        rows, w, static_cast<__nv_bfloat16*>(out), M, g.pieces, g.per, top_k, H, 1.f, row_index, nullptr, 0, 0);
+  else
+    sum_reduce_vec8_kernel<float, float, float, kIndexed, NARROW><<<g.blocks, g.threads, 0, s>>>(
+        rows, w, static_cast<float*>(out), M, g.pieces, g.per, top_k, H, 1.f, row_index, nullptr, 0, 0);
 }
 
 }  // namespace
@@ -272,14 +300,9 @@ extern "C" int xkb_moe_gather_sum_reduce(const float* rows, const int32_t* row_i
   XKB_REQUIRE(rows && row_index && out, "moe_gather_sum_reduce: null pointer");
   XKB_REQUIRE(reinterpret_cast<uintptr_t>(rows) % 16 == 0, "moe_gather_sum_reduce: rows must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  unsigned pieces = 1, threads = 32, vblocks = 1;
-  if (H % 8 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 && vec8_grid(M, H, 256, &pieces, &threads, &vblocks)) {
-    if (out_dtype == XKB_BF16)
-      sum_reduce_vec8_kernel<float, float, __nv_bfloat16, kIndexed><<<vblocks, threads, 0, s>>>(
-          rows, w, static_cast<__nv_bfloat16*>(out), pieces, top_k, H, 1.f, row_index, nullptr, 0, 0);
-    else
-      sum_reduce_vec8_kernel<float, float, float, kIndexed><<<vblocks, threads, 0, s>>>(
-          rows, w, static_cast<float*>(out), pieces, top_k, H, 1.f, row_index, nullptr, 0, 0);
+  Vec8Grid g{};
+  if (H % 8 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 && vec8_grid(M, H, 256, &g)) {
+    (g.per > 1 ? launch_indexed_as<true> : launch_indexed_as<false>)(g, rows, row_index, w, out, out_dtype, M, top_k, H, s);
     XKB_CHECK_LAUNCH("sum_reduce_vec8_kernel");
     return XKB_OK;
   }
