@@ -27,7 +27,7 @@ def _rows(kind, M, E, g):
 
 
 @pytest.mark.parametrize("kind", ["random", "levels", "underflow", "minus_inf", "neighbours"])
-@pytest.mark.parametrize("E,topk", [(1, 1), (31, 8), (32, 8), (33, 32), (64, 6), (256, 8), (257, 33), (1024, 32)])
+@pytest.mark.parametrize("E,topk", [(1, 1), (31, 8), (32, 8), (32, 32), (33, 32), (64, 6), (64, 20), (64, 21), (256, 8), (257, 33), (1024, 32)])
 def test_edges_against_oracle(kind, E, topk, cuda_device):
     x = _rows(kind, 65, E, torch.Generator().manual_seed(E + topk))
     want_w, want_ids = oracle.topk_softmax(x, topk, True)

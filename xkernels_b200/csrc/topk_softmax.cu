@@ -14,7 +14,9 @@
 // bounds the k-th largest element from below, usually 8 to 16 of the experts reach it, and only those
 // are divided by the sum (one per lane), ranked against each other and written.  Rows that leave more
 // than 32 candidates (long runs of equal logits, a k-th probability near the subnormals), a top-k above 32
-// or a sum that is not finite take the rounds (select_by_rounds), which order every probability of the row.
+// or a sum that is not finite take the rounds (select_by_rounds), which order every probability of the row.  They
+// pay for the candidates first, and make that good with two warp reductions a round instead of ten shuffles (all
+// logits equal, E=256, top 8, fp32, M=16384: 28.1 us before there were candidates, 32.1 with shuffles, 25.9 now).
 // M=16384, E=256, bf16, top 8, renormalised: 28.7 -> 11.8 us on the device, 12.3 us a call.
 #include <cuda_fp16.h>
 
@@ -25,6 +27,10 @@ namespace {
 
 constexpr int kMaxPerLane = 32;               // experts per lane -> at most 1024 experts
 constexpr int kWarpsPerBlock = 8;
+// Up to this top-k the candidates of rows of independent logits fit 32 lanes (74-100 % of the rows at 20, E = 48 to
+// 1024; 31-99 % at 22; 5-85 % at 24); above, looking for them mostly comes on top of the rounds (top 32 of 1024
+// experts, M=16384: 227 us without, 231 with).  Up to 32 experts they fit in any case.
+constexpr int kShortTopk = 20;
 
 template <typename T> __device__ __forceinline__ float load_logit(const T* p);
 template <> __device__ __forceinline__ float load_logit<float>(const float* p) { return *p; }
@@ -40,7 +46,7 @@ __device__ __forceinline__ bool better(float pa, int ia, float pb, int ib) {
 
 // k rounds over the whole row: p[t] = probability of expert lane + 32 t, or -1 where there is none.
 template <int PER_LANE>
-__device__ __noinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t row, int lane, int topk, int renormalize,
+__device__ __forceinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t row, int lane, int topk, int renormalize,
                                               float* __restrict__ topk_w, int32_t* __restrict__ topk_ids) {
   float wsum = 0.f;
   float my_w = 0.f;     // lane j keeps the j-th selected weight (j < 32), further ones go out directly
@@ -52,12 +58,10 @@ __device__ __noinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t row,
       const int e = lane + 32 * t;
       if (better(p[t], e, bp, bi)) { bp = p[t]; bi = e; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float op = __shfl_xor_sync(0xffffffffu, bp, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (better(op, oi, bp, bi)) { bp = op; bi = oi; }
-    }
+    // best of the warp: bp is -1 or >= 0 and never NaN (better() is false for one), so its bits order as signed integers
+    const int top = __reduce_max_sync(0xffffffffu, __float_as_int(bp));
+    bi = __reduce_min_sync(0xffffffffu, __float_as_int(bp) == top ? bi : 0x7fffffff);
+    bp = __int_as_float(top);
     // every lane now holds the same winner; its owner retires it
     if ((bi & 31) == lane) {
 #pragma unroll
@@ -117,7 +121,7 @@ topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, in
   // The k-th largest lane maximum (equal ones leave together, so it may be a smaller one: still a bound).
   // The floats are >= 0 or -1, and as signed integers they order the same way.
   int tau = -1, lm = __float_as_int(lane_max);
-  const bool short_way = topk <= 32 && sum < INFINITY;   // (a NaN sum fails the comparison)
+  const bool short_way = topk <= (PER_LANE == 1 ? 32 : kShortTopk) && sum < INFINITY;   // (a NaN sum fails the comparison)
   if (short_way) {
     for (int j = 0; j < topk; ++j) {
       tau = __reduce_max_sync(0xffffffffu, lm);
