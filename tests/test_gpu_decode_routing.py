@@ -1,4 +1,4 @@
-"""Decode batches, whose routing the activation gather sorts itself (up to 512 slots and a top-k of 32):
+"""Decode batches, whose routing the activation gather sorts itself (up to 512 slots, 148 blocks and a top-k of 32):
 both sides of those limits, few and many experts, dropped slots, an expert map.  The generic path, which
 takes the sort's own kernels, is the check: same bf16 weights, fp32 sums in another order."""
 
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("M,top_k,E", [
     (1, 1, 1), (1, 8, 48), (3, 32, 40), (3, 33, 40), (63, 8, 48), (64, 8, 48), (65, 8, 48), (128, 8, 48),
-    (129, 8, 48), (512, 1, 7), (513, 1, 7), (1025, 1, 7), (20, 8, 1024),
+    (129, 8, 48), (148, 2, 7), (149, 2, 7), (512, 1, 7), (513, 1, 7), (1025, 1, 7), (20, 8, 1024),
 ])
 @pytest.mark.parametrize("dropped", [False, True])
 def test_int4(M, top_k, E, dropped, cuda_device):

@@ -118,14 +118,20 @@ Routing make_routing(const RoutingBuffers& b, int64_t numel, int E, int block) {
 // The align stage of a fused call: clears the status word and the block counters on its way.  A decode batch on
 // a tensor-core path is sorted by the activation gather itself (r->job = *job): one launch less, and the gather
 // does not wait for another kernel's completion.  Larger batches take the sort's own kernels.
-// Whole calls: K=2048, N=7168, E=48, top_k=8 at M=1 39.8 -> 32.7 us, M=64 110.0 -> 108.1; K=7168, N=4096 at M=1 46.0 -> 44.0 us,
-// M=64 177.5 -> 175.4.  At M=128 (1024 slots: nearly every SM sorts) nothing is left of it: 132.4 / 132.0 us, and the
-// two-GEMM layer 448 / 451, so the line lies at M=64's 512 slots.
+// Whole calls: K=2048, N=7168, E=48, top_k=8 at M=1 39.8 -> 32.7 us, M=64 110.0 -> 108.1; K=7168, N=4096 at M=1 46.0 -> 44.0 us
+// (M=64: 1 %, within its runs' spread).  At M=128 (1024 slots: nearly every SM sorts) nothing is left of it: 132.4 / 132.0
+// us, and the two-GEMM layer 448 / 451, so the line lies at M=64's 512 slots.  Every block of the gather sorts, so they
+// have to fit the SMs side by side as well: K=2048, N=512, E=48, the sort's own kernels against this, 128 blocks 20.5 /
+// 19.1 us (top_k 1) and 21.4 / 20.0 (2), 256 blocks 21.1 / 22.7 and 22.4 / 23.9, 512 blocks 21.9 / 29.6; E=1024, N=256
+// 27.9 / 26.6, 36.9 / 43.1 and 49.4 / 73.3.
 constexpr int64_t kSortInGatherMax = 512;
+constexpr unsigned kSortInGatherBlocks = 148;
 static_assert(kSortInGatherMax <= align::kSmallMax, "the sort takes one slot per thread");
 int route(const RoutingBuffers& rb, const int32_t* topk_ids, const int32_t* expert_map, int num_map, int E, int top_k,
-          bool gathers, Routing* r, align::Job* job, cudaStream_t stream) {
-  if (gathers && r->numel >= 1 && r->numel <= kSortInGatherMax && top_k <= 32 && E >= 1 && E <= align::kMaxExperts) {
+          int64_t gather_units, Routing* r, align::Job* job, cudaStream_t stream) {   // gather_units: of a row, 0 = no gather
+  GatherGrid g{};
+  if (gather_units > 0 && r->numel >= 1 && r->numel <= kSortInGatherMax && top_k <= 32 && E >= 1 && E <= align::kMaxExperts &&
+      gather_grid(r->numel / top_k, gather_units, true, &g) == XKB_OK && g.blocks <= kSortInGatherBlocks) {
     *job = align::Job{topk_ids, expert_map, rb.sorted_ids, rb.expert_ids, rb.num_post, rb.expert_off, rb.status,
                       header_ints(rb), r->numel, r->max_pad, r->max_blocks, num_map, E, r->block};
     r->job = job;
@@ -206,7 +212,7 @@ static int int4_impl(const void* A, int a_dtype, const int32_t* packed, const vo
 
   Routing r = make_routing(rb, numel, E, block);
   align::Job job;
-  int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc, &r, &job, stream);
+  int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? K / 8 : 0, &r, &job, stream);
   if (rc != XKB_OK) return rc;
   if (use_tc)
     rc = launch_int4_tc(A, packed, scale, r, topk_w, scratch, N, K, E, top_k, group_size,
@@ -350,7 +356,7 @@ extern "C" int xkb_fused_moe_int4_ffn(const void* A, int a_dtype, const int32_t*
   const int block = use_tc ? int4_tc_block(numel, E, hidden) : kSimtBlock;
   Routing r = make_routing(rb, numel, E, block);
   align::Job job;
-  int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc, &r, &job, stream);
+  int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? hidden / 8 : 0, &r, &job, stream);
   if (rc != XKB_OK) return rc;
   if (use_tc) {
     __nv_bfloat16* rows16 = reinterpret_cast<__nv_bfloat16*>(scratch);
@@ -426,7 +432,7 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
 
   Routing r = make_routing(rb, numel, E, block);
   align::Job job;
-  int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc, &r, &job, stream);
+  int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? hidden / 8 : 0, &r, &job, stream);
   if (rc != XKB_OK) return rc;
   if (use_bs) {
     const __nv_bfloat16* rows = nullptr;
