@@ -45,3 +45,24 @@ def test_mxfp4(M, top_k, E, cuda_device):
     ops.check_status(cuda_device)
     simt = xkb.fused_moe_mxfp4(*args, path="simt")
     assert_within(got, simt, 2e-2, 1e-2, what="auto vs simt", allowed=max(1, simt.numel() // 2000))
+
+
+@pytest.mark.parametrize("M,top_k", [(65, 8), (300, 33), (700, 1), (4736, 8), (4737, 8), (5001, 33)])
+def test_most_tokens_without_a_slot_here(M, top_k, cuda_device):
+    """A rank that holds 2 of 64 experts (expert_map).  From 4737 blocks on the gather goes through the kept slots'
+    positions instead of the tokens; outputs of tokens without a local expert are zero."""
+    A = synth.activations(M, 512, seed=M, device=cuda_device)
+    ids, w = synth.routing(M, 64, top_k, seed=7, device=cuda_device)
+    emap = torch.full((64,), -1, dtype=torch.int32, device=cuda_device)
+    emap[5], emap[60] = 1, 0
+    none = (emap[ids.long()] < 0).all(dim=1)
+    packed, scale = synth.int4_weights(2, 256, 512, 32, seed=3, device=cuda_device)
+    t = synth.mxfp4_weights(2, 512, 512, seed=4, device=cuda_device, scale_lo=117, scale_hi=121)
+    calls = ((xkb.fused_moe_int4_w4a16, (A, packed, scale, ids, w)),
+             (xkb.fused_moe_mxfp4, (A, t["w13"], t["w13_scale"], t["w2"], t["w2_scale"], ids, w)))
+    for call, args in calls:
+        got = call(*args, expert_map=emap)
+        ops.check_status(cuda_device)
+        simt = call(*args, expert_map=emap, path="simt")
+        assert_within(got, simt, 2e-2, 1e-2, what="auto vs simt", allowed=max(1, simt.numel() // 2000))
+        assert bool((got[none] == 0).all())

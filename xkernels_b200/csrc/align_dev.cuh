@@ -117,6 +117,15 @@ struct Job {
   int num_map, E, block;
 };
 
+// Sorted positions that a gather may go through, read after its wait (0 if the count is none the sort wrote: recorded).
+constexpr int kErrGatherPositions = 3 + (3 << 8);   // kErrBadRouting, site 3
+__device__ __forceinline__ int positions_to_gather(const int32_t* num_post, int64_t max_pad, int* status) {
+  const int total = __ldcg(num_post);
+  if (total >= 0 && total <= max_pad) return total;
+  if (threadIdx.x == 0 && blockIdx.x == 0) atomicCAS(status, 0, kErrGatherPositions);
+  return 0;
+}
+
 // shared memory of align_in_block; the first kThreads ints are free again when it returns
 inline size_t small_smem(int E) {
   const size_t EP = E + 1;

@@ -80,6 +80,7 @@ struct Routing {
   // GEMM of a two-GEMM layer per token block (nullptr: the kernels do not overlap that way)
   int32_t* block_counters;
   int64_t counters_each;
+  bool by_position;   // the activation gather goes through the sorted positions instead of the tokens
   // not nullptr: the routing is not sorted yet, the activation gather does it on its way (decode batches)
   const align::Job* job;
 };

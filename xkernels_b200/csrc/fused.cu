@@ -127,9 +127,18 @@ Routing make_routing(const RoutingBuffers& b, int64_t numel, int E, int block) {
 constexpr int64_t kSortInGatherMax = 512;
 constexpr unsigned kSortInGatherBlocks = 148;
 static_assert(kSortInGatherMax <= align::kSmallMax, "the sort takes one slot per thread");
+// A map that leaves a token two kept slots or fewer on average (top_k * local experts / all experts: a rank's share)
+// has the gather of a large batch go through the kept slots' positions: going through the tokens starts a block for each
+// of them, most of which only find out that they have nothing to do.  K=2048, N=2048, top_k=8, whole calls, tokens against
+// positions: M=16384 with 1 of 256 experts 104 / 84 us, 8 of 256 130 / 115, 32 of 256 248 / 242; M=2048 (2048 blocks)
+// 36.0 / 36.4, 38.3 / 39.5 and 58.7 / 60.7, so the line lies at two rounds of sixteen blocks per SM.
+constexpr int64_t kPositionsPerToken = 2;
+constexpr unsigned kPositionsMinBlocks = 2 * 16 * 148;
 int route(const RoutingBuffers& rb, const int32_t* topk_ids, const int32_t* expert_map, int num_map, int E, int top_k,
           int64_t gather_units, Routing* r, align::Job* job, cudaStream_t stream) {   // gather_units: of a row, 0 = no gather
   GatherGrid g{};
+  r->by_position = gather_units > 0 && expert_map != nullptr && (int64_t)top_k * E <= kPositionsPerToken * num_map &&
+                   gather_grid(r->numel / top_k, gather_units, false, &g) == XKB_OK && g.blocks > kPositionsMinBlocks;
   if (gather_units > 0 && r->numel >= 1 && r->numel <= kSortInGatherMax && top_k <= 32 && E >= 1 && E <= align::kMaxExperts &&
       gather_grid(r->numel / top_k, gather_units, true, &g) == XKB_OK && g.blocks <= kSortInGatherBlocks) {
     *job = align::Job{topk_ids, expert_map, rb.sorted_ids, rb.expert_ids, rb.num_post, rb.expert_off, rb.status,

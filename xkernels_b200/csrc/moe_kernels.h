@@ -21,6 +21,9 @@ inline int gather_grid(int64_t M, int64_t units, bool sorting, GatherGrid* g) {
   return XKB_OK;
 }
 
+// going through the sorted positions instead: sixteen blocks per SM at most, each takes positions in turn
+inline unsigned position_blocks(int64_t max_pad) { return (unsigned)(max_pad < 148 * 16 ? max_pad : 148 * 16); }
+
 // ---- generic SIMT path (moe_simt.cu) ---------------------------------------
 int launch_int4_simt(const void* A, int a_dtype, const int32_t* packed, const void* scale,
                      const Routing& r, const float* topk_w, float* scratch, int64_t N, int64_t K,

@@ -541,6 +541,25 @@ gather_split_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos
   }
 }
 
+// The same through the sorted positions, for calls whose tokens mostly have no slot here.
+__global__ void __launch_bounds__(kGatherThreads)
+gather_split_positions_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* sorted_ids, const int32_t* num_post,
+                              const SplitRows x, int64_t numel, int K, int top_k, int64_t max_pad, int* __restrict__ status) {
+  chain_wait();
+  chain_trigger();
+  const int total = align::positions_to_gather(num_post, max_pad, status);
+  for (int64_t pos = blockIdx.x; pos < total; pos += gridDim.x) {
+    const int32_t slot = __ldcg(sorted_ids + pos);
+    if (slot < 0 || slot >= numel) continue;
+    const uint4* src = reinterpret_cast<const uint4*>(A + (int64_t)(slot / top_k) * K);
+    for (int i = threadIdx.x; i < K / 8; i += kGatherThreads) {   // K / 8 is a multiple of 32: whole warps
+      SplitUnit o;
+      o.load(src + i);
+      o.store(x, pos, K, i);
+    }
+  }
+}
+
 template <int BT, bool GATE_UP>
 int launch_mx(const CUtensorMap (&tm)[6], const MxParams& prm, int64_t max_tiles, cudaStream_t stream) {
   int dev = 0;
@@ -652,6 +671,9 @@ int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
       XKB_CHECK_CUDA(cudaFuncSetAttribute(gather_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     gather_split_kernel<true><<<g.blocks, g.threads, smem, stream>>>(a, nullptr, x, (int)hidden, top_k, r.max_pad, g.pieces,
                                                                      g.units, status, *r.job);
+  } else if (r.by_position) {
+    XKB_CHECK_CUDA(launch_chained(gather_split_positions_kernel, dim3(position_blocks(r.max_pad)), dim3(kGatherThreads), 0, stream,
+                                  a, r.sorted_ids, r.num_post, x, r.numel, (int)hidden, top_k, r.max_pad, status));
   } else {
     XKB_CHECK_CUDA(launch_chained(gather_split_kernel<false>, dim3(g.blocks), dim3(g.threads), 0, stream, a, r.slot_pos, x,
                                   (int)hidden, top_k, r.max_pad, g.pieces, g.units, status, align::Job{}));

@@ -899,6 +899,14 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
 // A once per slot, and at prefill A is larger than L2
 // (M=16384, K=7168, top_k=8, E=48: 612 -> 355 us).
 // ---------------------------------------------------------------------------
+// elements (e1:e0, e3:e2, e5:e4, e7:e6) of an input of the call -> (e4:e0, e5:e1, e6:e2, e7:e3)
+__device__ __forceinline__ uint4 load_permuted(const uint4* src, int permute) {
+  const uint4 v = __ldg(src);
+  if (!permute) return v;                 // consumers that convert in natural K order
+  return make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410),
+                    __byte_perm(v.y, v.w, 0x7632));
+}
+
 template <bool SORT>
 __global__ void __launch_bounds__(SORT ? 1024 : kGatherThreads)
 gather_permute_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_pos, __nv_bfloat16* __restrict__ Ag,
@@ -909,16 +917,7 @@ gather_permute_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_p
   const int i = (int)((blockIdx.x - m * pieces) * units + threadIdx.x);
   const bool mine = threadIdx.x < units && i < K / 8;
   uint4 o = make_uint4(0, 0, 0, 0);
-  if (mine) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(A + (int64_t)m * K) + i);  // elements (e1:e0, e3:e2, e5:e4, e7:e6); an input of the call
-    o = v;                                  // consumers that convert in natural K order
-    if (permute) {
-      o.x = __byte_perm(v.x, v.z, 0x5410);  // (e4 : e0)
-      o.y = __byte_perm(v.x, v.z, 0x7632);  // (e5 : e1)
-      o.z = __byte_perm(v.y, v.w, 0x5410);  // (e6 : e2)
-      o.w = __byte_perm(v.y, v.w, 0x7632);  // (e7 : e3)
-    }
-  }
+  if (mine) o = load_permuted(reinterpret_cast<const uint4*>(A + (int64_t)m * K) + i, permute);
   // The routing comes from the align kernel before this one, which may still be running when this
   // kernel starts.  It is read with L2 loads after the wait and through pointers that are NOT
   // `const __restrict__`: loads the compiler may treat as invariant (ld.global.nc) were seen to
@@ -946,6 +945,22 @@ gather_permute_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* slot_p
   }
 }
 
+// The same through the sorted positions, for calls whose tokens mostly have no slot here.
+__global__ void __launch_bounds__(kGatherThreads)
+gather_permute_positions_kernel(const __nv_bfloat16* __restrict__ A, const int32_t* sorted_ids, const int32_t* num_post,
+                                __nv_bfloat16* __restrict__ Ag, int64_t numel, int K, int top_k, int permute,
+                                int64_t max_pad, int* __restrict__ status) {
+  chain_wait();
+  chain_trigger();
+  const int total = align::positions_to_gather(num_post, max_pad, status);
+  for (int64_t pos = blockIdx.x; pos < total; pos += gridDim.x) {
+    const int32_t slot = __ldcg(sorted_ids + pos);
+    if (slot < 0 || slot >= numel) continue;
+    const uint4* src = reinterpret_cast<const uint4*>(A + (int64_t)(slot / top_k) * K);
+    for (int i = threadIdx.x; i < K / 8; i += kGatherThreads) reinterpret_cast<uint4*>(Ag + pos * K)[i] = load_permuted(src + i, permute);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -968,7 +983,8 @@ EncodeTiledFn get_encode_fn() {
 }
 
 // Encoded maps are kept per (base, shape, box, type, swizzle): a serving loop calls with the same
-// weights and workspace addresses every step, and an encode costs about as much host time as a launch.
+// weights and workspace addresses every step.  (A miss costs little: calls of 24 layers in turn, whose maps do not fit,
+// take the same host time as calls of one, 24.3 and 24.7 us for the twelve maps of an MXFP4 layer.)
 // A map holds no device state, so a stale entry (memory freed and reused with another layout) is
 // harmless: the key is everything the encoding depends on.
 struct MapKey {
@@ -1023,10 +1039,16 @@ namespace {
 
 int launch_gather(const void* A, const Routing& r, __nv_bfloat16* Ag, int64_t K, int top_k, int permute, int* status,
                   cudaStream_t stream) {
+  const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(A);
+  if (r.by_position && r.job == nullptr) {
+    XKB_CHECK_CUDA(launch_chained(gather_permute_positions_kernel, dim3(position_blocks(r.max_pad)), dim3(kGatherThreads), 0, stream, a,
+                                  r.sorted_ids, r.num_post, Ag, r.numel, (int)K, top_k, permute, r.max_pad, status));
+    XKB_CHECK_LAUNCH("gather_permute_positions_kernel");
+    return XKB_OK;
+  }
   GatherGrid g;
   const int rc = gather_grid(r.numel / top_k, K / 8, r.job != nullptr, &g);
   if (rc != XKB_OK) return rc;
-  const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(A);
   if (r.job != nullptr) {
     const size_t smem = align::small_smem(r.job->E);
     if (smem > 48 * 1024)
