@@ -208,6 +208,14 @@ constexpr bool mode_is_gate_up(int mode) { return mode == kModeMxGateUp || mode 
 constexpr int mode_mats(int mode) { return (mode_is_gate_up(mode) || mode_is_pair(mode)) ? 2 : 1; }
 constexpr bool mode_is_int4(int mode) { return mode == kModeInt4 || mode == kModeInt4Pair || mode == kModeInt4GateUp; }
 
+// Variants of the INT4 modes.  Instances of their own and not run-time switches: the narrow tiles run at their
+// register cap of 80, and with the switches inside <16, kModeInt4> spilled 16 bytes, <32, kModeInt4> 4 and
+// <32, kModeInt4GateUp> 60 (now 8, none and 52; the weights' shuffle sits under its branch for the same reason).
+constexpr int kWideGroups = 1;    // scale groups of 64, 128 or 256 (TcParams::group_shift) instead of 32
+constexpr int kRows16 = 2;        // the weighted slot rows go to TcParams::rows16, rounded to bf16, instead of to scratch (the
+                                  // second GEMM of a two-GEMM layer, whose per-slot results the reference composition
+                                  // holds in bf16)
+
 struct TcParams {
   const int32_t* sorted_ids;
   const int32_t* expert_ids;
@@ -218,10 +226,8 @@ struct TcParams {
   int64_t numel;
   int N, K;                     // tile rows are taken from N rows per expert; K = contraction length
   int mul_w;
-  int group_shift;              // INT4: log2 of the scale group (5 .. 8)
-  __nv_bfloat16* rows16;        // INT4: not nullptr = the weighted slot rows go here rounded to bf16 instead of to scratch
-                                // (the second GEMM of a two-GEMM layer, whose per-slot results the reference
-                                // composition holds in bf16)
+  int group_shift;              // kWideGroups: log2 of the scale group (6 .. 8)
+  __nv_bfloat16* rows16;        // kRows16
   // MXFP4 only
   const __nv_bfloat16* bias;    // b13 [E, 2*ispp] or b2 [E, hidden] or nullptr
   __nv_bfloat16* act;           // gate_up mode output: [positions, N] bf16 in the K-permuted order
@@ -331,11 +337,13 @@ __device__ __forceinline__ void mx_word(uint32_t x, uint32_t c, uint32_t& r0, ui
   r3 = mx_pair(x >> 6, x, c);
 }
 
-template <int BT, int MODE>
+template <int BT, int MODE, int VAR>
 __global__ void __launch_bounds__((TcCfg<BT, mode_mats(MODE), mode_is_int4(MODE)>::kThreads), 1)
 moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_constant__ CUtensorMap tm_scale,
                const __grid_constant__ CUtensorMap tm_tokens, const TcParams p) {
   using Cfg = TcCfg<BT, mode_mats(MODE), mode_is_int4(MODE)>;
+  constexpr bool kWide = (VAR & kWideGroups) != 0, kNarrowRows = (VAR & kRows16) != 0;
+  static_assert(VAR == 0 || mode_is_int4(MODE), "variants of the INT4 modes");
   constexpr int kWStages = Cfg::kWStages;
   constexpr int kMatsC = mode_mats(MODE);
   extern __shared__ unsigned char smem_raw[];
@@ -442,7 +450,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
             tma_load_2d(s_packed + st * kPackedStageBytes, &tm_packed, &w_full[st], ks * (kStageK / 2), row0);
             // eight scales per row: the stage's own at group 32, those of 2 / 4 / 8 stages at groups 64 / 128 / 256
             // (sixteen bytes are the smallest TMA row and x must be a multiple of them)
-            tma_load_2d(s_scale + st * kScaleStageBytes, &tm_scale, &w_full[st], ((ks * kStageK) >> p.group_shift) & ~7, row0);
+            tma_load_2d(s_scale + st * kScaleStageBytes, &tm_scale, &w_full[st],
+                        kWide ? ((ks * kStageK) >> p.group_shift) & ~7 : ks * (kStageK / 32), row0);
           } else {  // e8m0 scales: 16 bytes per row = the scales of stages ks & ~1 and ks | 1
             mbar_expect_tx(&w_full[st], kPackedStageBytes + kScaleStageBytes);
             tma_load_2d(s_packed + st * kPackedStageBytes, &tm_packed, &w_full[st], ks * (kStageK / 2), row0);
@@ -672,20 +681,21 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           for (int j = 0; j < 16; ++j) {
             if (!((live >> j) & 1u)) continue;          // warp-uniform
             const int32_t slot = __shfl_sync(0xffffffffu, cur_slot, j);
-            const float w = __shfl_sync(0xffffffffu, cur_w, j);
-            float v = __uint_as_float(acc[j]);
+            float v = __uint_as_float(acc[j]), w = 1.f;
             if (mode_is_int4(MODE) && kInt4NoSubtract) v *= kInt4Unscale;   // exact: a power of two
             if (MODE == kModeMxDown) {  // reference rounds `down` to bf16, adds the bf16 bias, then x w
               v = round_to_bf16(Cfg::kLut ? v : v * kMxUnscale);
               if (p.bias != nullptr) v = round_to_bf16(v + bias0);
+              w = __shfl_sync(0xffffffffu, cur_w, j);
               if (p.mul_w) v = v * w;
             } else {
-              if (p.mul_w) v = w * v;
+              if (p.mul_w) {
+                w = __shfl_sync(0xffffffffu, cur_w, j);
+                v = w * v;
+              }
             }
-            const int64_t at = (int64_t)slot * p.N + n_glob;
-            const bool narrow = mode_is_int4(MODE) && p.rows16 != nullptr;
-            if (narrow) p.rows16[at] = __float2bfloat16_rn(v);
-            else p.scratch[at] = v;
+            if (kNarrowRows) p.rows16[(int64_t)slot * p.N + n_glob] = __float2bfloat16_rn(v);
+            else p.scratch[(int64_t)slot * p.N + n_glob] = v;
             if (mode_is_pair(MODE)) {  // the second weight tile: rows 128 further down
               float v2 = __uint_as_float(more[j]);
               if (MODE == kModeInt4Pair) {
@@ -696,8 +706,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
                 if (p.bias != nullptr) v2 = round_to_bf16(v2 + bias1);
                 if (p.mul_w) v2 = v2 * w;
               }
-              if (narrow) p.rows16[at + kTileRows] = __float2bfloat16_rn(v2);
-              else p.scratch[at + kTileRows] = v2;
+              if (kNarrowRows) p.rows16[(int64_t)slot * p.N + n_glob + kTileRows] = __float2bfloat16_rn(v2);
+              else p.scratch[(int64_t)slot * p.N + n_glob + kTileRows] = v2;
             }
           }
         }
@@ -750,7 +760,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         uint2 sw = make_uint2(0, 0);  // INT4: the kChunks bf16 group scales of this share; MXFP4: .x = its e8m0 bytes
         if (mode_is_int4(MODE)) {
           const uint32_t sa = s_scale_u32 + wst * kScaleStageBytes + row * 16;
-          if (p.group_shift == 5) {
+          if (!kWide) {
             if (kChunks == 4) sw = lds64(sa + part * 8);
             else sw.x = lds32(sa + part * 4);
           } else {  // two chunks or more share a scale: the first and the third chunk's, each twice
@@ -1063,7 +1073,7 @@ int launch_gather(const void* A, const Routing& r, __nv_bfloat16* Ag, int64_t K,
   return XKB_OK;
 }
 
-template <int BT, int MODE>
+template <int BT, int MODE, int VAR = 0>
 int launch_bt(const CUtensorMap& tmp, const CUtensorMap& tms, const CUtensorMap& tmt, const TcParams& prm,
               int64_t max_tiles, cudaStream_t stream) {
   using Cfg = TcCfg<BT, mode_mats(MODE), mode_is_int4(MODE)>;
@@ -1074,7 +1084,7 @@ int launch_bt(const CUtensorMap& tmp, const CUtensorMap& tms, const CUtensorMap&
   static std::atomic<int> sm_count[64];
   const uint64_t bit = dev < 64 ? (1ull << dev) : 0ull;
   if (bit == 0 || (smem_set.load(std::memory_order_acquire) & bit) == 0) {
-    XKB_CHECK_CUDA(cudaFuncSetAttribute(moe_tc_kernel<BT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    XKB_CHECK_CUDA(cudaFuncSetAttribute(moe_tc_kernel<BT, MODE, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)Cfg::kSmemBytes));
     int n = 148;
     XKB_CHECK_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
@@ -1095,7 +1105,7 @@ int launch_bt(const CUtensorMap& tmp, const CUtensorMap& tms, const CUtensorMap&
   if (grid < 1) grid = 1;
   {
     GemmTimerScope timed(stream);
-    XKB_CHECK_CUDA(launch_chained(moe_tc_kernel<BT, MODE>, dim3((unsigned)grid), dim3(Cfg::kThreads), Cfg::kSmemBytes,
+    XKB_CHECK_CUDA(launch_chained(moe_tc_kernel<BT, MODE, VAR>, dim3((unsigned)grid), dim3(Cfg::kThreads), Cfg::kSmemBytes,
                                   stream, tmp, tms, tmt, prm));
   }
   XKB_CHECK_LAUNCH("moe_tc_kernel");
@@ -1144,20 +1154,46 @@ int64_t int4_tc_workspace_bytes(int64_t numel, int64_t N, int64_t K, int E) {
 }
 
 // one INT4 GEMM (tokens through `tm_tokens`) at the token tile the routing was aligned for
-static int launch_int4_by_block(const CUtensorMap& tm_packed, const CUtensorMap& tm_scale, const CUtensorMap& tm_tokens,
-                                const TcParams& prm, const Routing& r, int64_t N, cudaStream_t stream) {
+template <int VAR>
+static int launch_int4_variant(const CUtensorMap& tm_packed, const CUtensorMap& tm_scale, const CUtensorMap& tm_tokens,
+                               const TcParams& prm, const Routing& r, int64_t N, cudaStream_t stream) {
   const int64_t max_tiles = r.max_blocks * (N / kTileRows);
   switch (r.block) {
-    case 16: return launch_bt<16, kModeInt4>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
-    case 32: return launch_bt<32, kModeInt4>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
-    case 64: return launch_bt<64, kModeInt4>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
-    case 80: return launch_bt<80, kModeInt4Pair>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
-    case 96: return launch_bt<96, kModeInt4Pair>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
-    case 112: return launch_bt<112, kModeInt4Pair>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
+    case 16: return launch_bt<16, kModeInt4, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
+    case 32: return launch_bt<32, kModeInt4, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
+    case 64: return launch_bt<64, kModeInt4, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
+    case 80: return launch_bt<80, kModeInt4Pair, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
+    case 96: return launch_bt<96, kModeInt4Pair, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
+    case 112: return launch_bt<112, kModeInt4Pair, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
     case 128:
-      if (N % (2 * kTileRows) == 0)
-        return launch_bt<128, kModeInt4Pair>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
-      return launch_bt<128, kModeInt4>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
+      if constexpr ((VAR & kRows16) == 0) {   // (a two-GEMM layer's N is a multiple of 256)
+        if (N % (2 * kTileRows) != 0)
+          return launch_bt<128, kModeInt4, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
+      }
+      return launch_bt<128, kModeInt4Pair, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
+    default: return fail(XKB_ERR_ARG, "int4 tcgen05 path: unsupported token tile %d", r.block);
+  }
+}
+static int launch_int4_by_block(const CUtensorMap& tm_packed, const CUtensorMap& tm_scale, const CUtensorMap& tm_tokens,
+                                const TcParams& prm, const Routing& r, int64_t N, cudaStream_t stream) {
+  switch ((prm.group_shift > 5 ? kWideGroups : 0) | (prm.rows16 != nullptr ? kRows16 : 0)) {
+    case 0: return launch_int4_variant<0>(tm_packed, tm_scale, tm_tokens, prm, r, N, stream);
+    case kWideGroups: return launch_int4_variant<kWideGroups>(tm_packed, tm_scale, tm_tokens, prm, r, N, stream);
+    case kRows16: return launch_int4_variant<kRows16>(tm_packed, tm_scale, tm_tokens, prm, r, N, stream);
+    default: return launch_int4_variant<kWideGroups | kRows16>(tm_packed, tm_scale, tm_tokens, prm, r, N, stream);
+  }
+}
+template <int VAR>
+static int launch_int4_gate_up(const CUtensorMap& tm_packed, const CUtensorMap& tm_scale, const CUtensorMap& tm_tokens,
+                               const TcParams& prm, const Routing& r, int64_t tiles, cudaStream_t stream) {
+  switch (r.block) {
+    case 16: return launch_bt<16, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
+    case 32: return launch_bt<32, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
+    case 64: return launch_bt<64, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
+    case 80: return launch_bt<80, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
+    case 96: return launch_bt<96, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
+    case 112: return launch_bt<112, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
+    case 128: return launch_bt<128, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
     default: return fail(XKB_ERR_ARG, "int4 tcgen05 path: unsupported token tile %d", r.block);
   }
 }
@@ -1273,16 +1309,8 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
   prm.done_target = (int)(inter / kTileRows) * hand_over_per_tile(r.block);
   GemmTimerScope timed(stream);   // both GEMMs in one scope: they overlap
   const int64_t tiles0 = r.max_blocks * (inter / kTileRows);
-  switch (r.block) {
-    case 16: rc = launch_bt<16, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
-    case 32: rc = launch_bt<32, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
-    case 64: rc = launch_bt<64, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
-    case 80: rc = launch_bt<80, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
-    case 96: rc = launch_bt<96, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
-    case 112: rc = launch_bt<112, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
-    case 128: rc = launch_bt<128, kModeInt4GateUp>(tm_w13, tm_s13, tm_tok0, prm, tiles0, stream); break;
-    default: return fail(XKB_ERR_ARG, "int4 tcgen05 path: unsupported token tile %d", r.block);
-  }
+  rc = group > 32 ? launch_int4_gate_up<kWideGroups>(tm_w13, tm_s13, tm_tok0, prm, r, tiles0, stream)
+                  : launch_int4_gate_up<0>(tm_w13, tm_s13, tm_tok0, prm, r, tiles0, stream);
   if (rc != XKB_OK) return rc;
   // down: weighted slot rows, rounded to bf16 (kept as bf16: half the traffic of the rows, the same values)
   prm.scratch = nullptr;
