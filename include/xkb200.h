@@ -138,9 +138,8 @@ int xkb_moe_sum_reduce(const void* y, int y_dtype, const void* w, int w_dtype,
  *           src/xkernels/ops/moe/triton/moe_int4_kernel.py:438-577 (Triton
  *           entry: align + grouped GEMM + top-k combine).
  * A [M,K] (a_dtype), packed [E,N,K/8] int32 (low nibble = lowest k, zero
- * point 8), scale [E,N,K/group] bf16 (finite and below 2^24 in magnitude
- * wherever the tcgen05 path may run: group 32, and groups 64 / 128 / 256 with K
- * a multiple of eight groups), topk_ids [M,top_k] int32, topk_w
+ * point 8), scale [E,N,K/group] bf16 (at group 32 finite and below 2^24 in
+ * magnitude wherever the tcgen05 path may run; any value at other groups), topk_ids [M,top_k] int32, topk_w
  * [M,top_k] fp32, expert_map NULL or [num_map] int32, out [M,N] (a_dtype).
  * ---------------------------------------------------------------------- */
 int64_t xkb_fused_moe_int4_w4a16_workspace_bytes(int64_t M, int64_t N,

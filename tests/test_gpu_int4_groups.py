@@ -65,3 +65,31 @@ def test_two_gemm_layer_at_group_128(cuda_device):
     got = xkb.fused_moe_int4_ffn(*t, group_size=group)
     ops.check_status(cuda_device)
     assert_within(got, xkb.fused_moe_int4_ffn(*t, group_size=group, path="simt"), 2e-2, 1e-2, what="auto vs simt")
+
+
+@pytest.mark.parametrize("M,group", [(8, 128), (100, 64), (200, 256)])
+def test_scales_of_any_magnitude(M, group, cuda_device, monkeypatch):
+    """A C caller may pass any bf16 scale at these groups: the generic path answered them, so the tensor-core path
+    gives the same (weights rounded once; infinities and NaN where the generic path has them).  Below 2^-118 its
+    weights are off by 2^-126 at most."""
+    monkeypatch.setattr(ops, "_check_int4_scales", lambda scale: None)   # Python refuses them before the library sees them
+    K, N, E, top_k = 2048, 256, 4, 2
+    A = synth.activations(M, K, seed=1, device=cuda_device)
+    packed, scale = synth.int4_weights(E, N, K, group, seed=2, device=cuda_device)
+    ids, w = synth.routing(M, E, top_k, seed=3, device=cuda_device)
+    scale[:, 0:32] *= 2.0 ** 100                       # rows of their own magnitude
+    scale[:, 32:64] *= 2.0 ** -100
+    scale[:, 64:96] = torch.finfo(torch.bfloat16).tiny / 8   # subnormal
+    scale[:, 112:128, ::2] = 100.0                     # in and out of the fast conversion's range inside a row
+    scale[:, 96, 0], scale[:, 97, 1], scale[:, 98, 2] = float("inf"), float("nan"), 3.0e38
+    got = xkb.fused_moe_int4_w4a16(A, packed, scale, ids, w, group_size=group)
+    want = xkb.fused_moe_int4_w4a16(A, packed, scale, ids, w, group_size=group, path="simt")
+    ops.check_status(cuda_device)
+    off = 2.0 ** -126 * A.double().abs().sum(dim=1, keepdim=True)
+    assert bool(((got - want)[:, 64:96].double().abs() <= 1.01 * off).all())
+    for rows in (slice(0, 32), slice(32, 64), slice(96, 112), slice(112, 256)):
+        a, b = got[:, rows].double(), want[:, rows].double()
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+        ok = b.isfinite()
+        # sums in another order, then one bf16 rounding; relative to the rows' own magnitude
+        assert bool(((a - b).abs()[ok] <= 1e-2 * b[ok].abs() + 1e-2 * b[ok].abs().median()).all())

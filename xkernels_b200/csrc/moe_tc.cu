@@ -273,11 +273,21 @@ __device__ __forceinline__ uint32_t dequant_pair(uint32_t biased, uint32_t scale
 // s * 2^99, addend -s * 2^-27, and the epilogue multiplies the fp32 accumulators by 2^30, which
 // is exact.  Exact for scales with 2^-96 <= |s| < 2^24 (and for s = 0); the host side refuses
 // scale tensors outside that range.
-constexpr bool kInt4NoSubtract = true;
-constexpr uint32_t kMulLo = 0x73007300u;    // 2^103, twice: multiplier for nibbles at bits 3..0
-constexpr uint32_t kMulHi = 0x71007100u;    // 2^99: nibbles at bits 7..4
-constexpr uint32_t kMulAdd = 0xB200B200u;   // -2^-27 = -8 * 2^-30
-constexpr float kInt4Unscale = 1073741824.f;  // 2^30
+//
+// Calls with groups of 64 and more were answered by the generic kernel for any scale before this kernel took them, so
+// kWideGroups keeps its weights 2^-8 smaller only (multipliers s * 2^125 and s * 2^121, finite for |s| < 8), and a warp
+// that meets a larger, infinite or NaN scale converts that stage with a subtraction instead (dequant_pair): the
+// reference's one rounding, then times 2^-8, which is exact down to |s| = 2^-118.  (Smaller scales lose bits below
+// 2^-126, bf16's smallest normal number.)  The check is a vote per stage; subtracting always cost 9 to 29 % of a decode
+// call at group 128 (M=1 55 -> 61 us, M=37 232 -> 254, M=64 201 -> 260).
+template <bool WIDE> struct Int4Scaling {
+  static constexpr uint32_t kMulLo = WIDE ? 0x7E007E00u : 0x73007300u;    // 2^125, 2^103, twice: multiplier for nibbles at bits 3..0
+  static constexpr uint32_t kMulHi = WIDE ? 0x7C007C00u : 0x71007100u;    // 2^121, 2^99: nibbles at bits 7..4
+  static constexpr uint32_t kMulAdd = WIDE ? 0xBD00BD00u : 0xB200B200u;   // -8 * 2^-8, -8 * 2^-30
+  static constexpr float kUnscale = WIDE ? 256.f : 1073741824.f;
+};
+constexpr uint32_t kWideLimit = 0x4100u;    // 8.0: the first |scale| (bf16 bits) whose multiplier overflows
+constexpr uint32_t kWideShift = 0x3B803B80u;   // 2^-8, twice
 __device__ __forceinline__ uint32_t bf2_mul(uint32_t a, uint32_t b) {
   const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
   return *reinterpret_cast<const uint32_t*>(&r);
@@ -287,6 +297,8 @@ __device__ __forceinline__ uint32_t bf2_fma(uint32_t a, uint32_t b, uint32_t c) 
                                    *reinterpret_cast<const __nv_bfloat162*>(&c));
   return *reinterpret_cast<const uint32_t*>(&r);
 }
+
+__device__ __forceinline__ uint32_t wide_pair(uint32_t x, uint32_t scale2) { return bf2_mul(dequant_pair(nib_pair(x), scale2), kWideShift); }
 
 // ---- MXFP4: E2M1 code -> bf16 -------------------------------------------------------------
 // The three magnitude bits (e1 e0 m) placed at bf16 bits 8..6 read as  e2m1 * 2^-126  (the code
@@ -668,7 +680,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             if (!((live >> j) & 1u)) continue;          // warp-uniform
-            constexpr float kUnscale = (MODE == kModeInt4GateUp) ? kInt4Unscale : (Cfg::kLut ? 1.f : kMxUnscale);
+            constexpr float kUnscale = (MODE == kModeInt4GateUp) ? Int4Scaling<kWide>::kUnscale : (Cfg::kLut ? 1.f : kMxUnscale);
             float g = round_to_bf16(__uint_as_float(acc[j]) * kUnscale);   // exact: a power of two
             float u = round_to_bf16(__uint_as_float(more[j]) * kUnscale);
             if (p.bias != nullptr) { g = round_to_bf16(g + bias0); u = round_to_bf16(u + bias1); }
@@ -682,7 +694,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
             if (!((live >> j) & 1u)) continue;          // warp-uniform
             const int32_t slot = __shfl_sync(0xffffffffu, cur_slot, j);
             float v = __uint_as_float(acc[j]), w = 1.f;
-            if (mode_is_int4(MODE) && kInt4NoSubtract) v *= kInt4Unscale;   // exact: a power of two
+            if (mode_is_int4(MODE)) v *= Int4Scaling<kWide>::kUnscale;   // exact: a power of two
             if (MODE == kModeMxDown) {  // reference rounds `down` to bf16, adds the bf16 bias, then x w
               v = round_to_bf16(Cfg::kLut ? v : v * kMxUnscale);
               if (p.bias != nullptr) v = round_to_bf16(v + bias0);
@@ -699,7 +711,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
             if (mode_is_pair(MODE)) {  // the second weight tile: rows 128 further down
               float v2 = __uint_as_float(more[j]);
               if (MODE == kModeInt4Pair) {
-                if (kInt4NoSubtract) v2 *= kInt4Unscale;
+                v2 *= Int4Scaling<kWide>::kUnscale;
                 if (p.mul_w) v2 = w * v2;
               } else {
                 v2 = round_to_bf16(Cfg::kLut ? v2 : v2 * kMxUnscale);
@@ -773,6 +785,10 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           if (kChunks == 4) sw.x = lds32(sa);
           else sw.x = lds16(sa);
         }
+        bool subtract = false;   // kWideGroups: a scale of this warp is out of the multipliers' range (never for sane weights)
+        if (kWide)
+          subtract = __any_sync(0xffffffffu, __vcmpgeu2(sw.x & 0x7FFF7FFFu, kWideLimit * 0x00010001u) != 0 ||
+                                                 __vcmpgeu2(sw.y & 0x7FFF7FFFu, kWideLimit * 0x00010001u) != 0);
         // 16-byte chunk = 32 weights = one scale group; this share is chunks kChunks * part ...
         uint4 w4[kChunks];
 #pragma unroll
@@ -797,8 +813,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           if (mode_is_int4(MODE)) {
             const uint32_t s01 = (c < 2) ? sw.x : sw.y;
             const uint32_t s2 = (c & 1) ? __byte_perm(s01, s01, 0x3232) : __byte_perm(s01, s01, 0x1010);
-            if (kInt4NoSubtract) {
-              const uint32_t m_lo = bf2_mul(s2, kMulLo), m_hi = bf2_mul(s2, kMulHi), add = bf2_mul(s2, kMulAdd);
+            if (!kWide || !subtract) {
+              using S = Int4Scaling<kWide>;
+              const uint32_t m_lo = bf2_mul(s2, S::kMulLo), m_hi = bf2_mul(s2, S::kMulHi), add = bf2_mul(s2, S::kMulAdd);
 #pragma unroll
               for (int wp = 0; wp < 2; ++wp) {  // two words = 16 weights = 8 columns
                 const uint32_t x0 = words[2 * wp], x1 = words[2 * wp + 1];
@@ -814,10 +831,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
               for (int wp = 0; wp < 2; ++wp) {  // two words = 16 weights = 8 columns
                 const uint32_t x0 = words[2 * wp], x1 = words[2 * wp + 1];
                 tmem_st_32x8(dst + c * 16 + wp * 8,
-                             dequant_pair(nib_pair(x0), s2), dequant_pair(nib_pair(x0 >> 4), s2),
-                             dequant_pair(nib_pair(x0 >> 8), s2), dequant_pair(nib_pair(x0 >> 12), s2),
-                             dequant_pair(nib_pair(x1), s2), dequant_pair(nib_pair(x1 >> 4), s2),
-                             dequant_pair(nib_pair(x1 >> 8), s2), dequant_pair(nib_pair(x1 >> 12), s2));
+                             wide_pair(x0, s2), wide_pair(x0 >> 4, s2), wide_pair(x0 >> 8, s2), wide_pair(x0 >> 12, s2),
+                             wide_pair(x1, s2), wide_pair(x1 >> 4, s2), wide_pair(x1 >> 8, s2), wide_pair(x1 >> 12, s2));
               }
             }
           } else {
@@ -1136,8 +1151,10 @@ int int4_tc_block(int64_t numel, int E, int64_t N) {
   // 80, 96 or 112 tokens x two row tiles, while nearly every expert fits one block (its slots spread by about their
   // square root): the tile's token bytes through shared memory, which bound it, shrink with the tile.
   // E=48, top_k=8, whole call, 128-token tiles against these: K=2048, N=7168 184 -> 169 us at 50 slots per expert, 194 -> 185
-  // at 67, 200 -> 194 at 75, 206 -> 198 at 85, 212 -> 211 at 93 (96 tokens there: 241); K=7168, N=4096 333 -> 294 at
-  // 53, 344 -> 320 at 70, 353 -> 335 at 85, with a routing bias of 0.5 353 -> 353 at 58 and 408 -> 400 at 83.
+  // at 67, 200 -> 194 at 75, 206 -> 198 at 85, 212 -> 211 at 93 (96 tokens there: 241); K=7168, N=4096 (means of two
+  // runs) 328 -> 288 at 53, 364 -> 312 at 67, 365 -> 334 at 83, 380 -> 361 at 100.  A skewed routing spreads the slots
+  // further: with a bias of 0.5 334 -> 333, 365 -> 364, 414 -> 391 and 433 -> 418, with 1.0 331 -> 337, 363 -> 370,
+  // 416 -> 435 and 481 -> 454.
   if (N % (2 * kTileRows) == 0)
     for (int block = 80; block < 128; block += 16)
       if (avg + 2.0 * std::sqrt(avg) <= block) return block;

@@ -292,9 +292,9 @@ _INT4_SCALE_LIMIT = float(2 ** 24)
 
 
 def _check_int4_scales(scale: torch.Tensor) -> None:
-    """The tcgen05 INT4 dequantiser is exact for group scales below 2^24 in magnitude (it multiplies
+    """The tcgen05 INT4 dequantiser of groups of 32 is exact for scales below 2^24 in magnitude (it multiplies
     by s * 2^103 in bf16); a larger or non-finite scale would come out as inf/NaN, so such a tensor
-    is refused.  Checked once per tensor (keyed by storage address, size and version counter): one
+    is refused (at every group size: the wider groups' kernels would take it).  Checked once per tensor (keyed by storage address, size and version counter): one
     reduction and one host read on the first call with it, so make that call before a stream capture."""
     key = (scale.data_ptr(), scale.numel())
     if _checked_scales.get(key) == scale._version:
