@@ -27,6 +27,7 @@ namespace {
 using namespace align;
 
 constexpr int kMaxChunks = 148;        // CTAs of the two-launch path: one wave
+constexpr int64_t kNoWorkspaceMax = 8192;   // slots that need no workspace (callers may pass none)
 
 // ---------------------------------------------------------------------------
 // Single-CTA path: numel <= 1024.  zero / zero_n: ints the caller wants cleared (nullptr, 0: none).
@@ -77,8 +78,8 @@ align_count_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t 
 __global__ void __launch_bounds__(kThreads)
 align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t span, int E, int block,
                    const int32_t* __restrict__ expert_map, int num_map,
-                   const int32_t* chunk_cnt /*[C][E+1]: written by the kernel this one overlaps*/,
-                   int32_t* sorted_ids, int32_t* __restrict__ expert_ids, int64_t max_blocks,
+                   const int32_t* chunk_cnt /*[C][E+1]: written by the kernel this one overlaps; nullptr: one chunk*/,
+                   int32_t* sorted_ids, int64_t max_pad, int32_t* __restrict__ expert_ids, int64_t max_blocks,
                    int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out,
                    int32_t* __restrict__ slot_pos) {
   chain_trigger();
@@ -97,11 +98,16 @@ align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t 
   bool active = slot < last;
   int e = active ? map_expert(topk_ids[slot], E, expert_map, num_map) : E;   // an input of the call, not of the kernel before
   chain_wait();
+  if (chunk_cnt == nullptr) {   // one CTA without a workspace: counts and fills for itself
+    for (int64_t s = tid; s < numel; s += kThreads)
+      atomicAdd(&tot[map_expert(topk_ids[s], E, expert_map, num_map)], 1);
+    for (int64_t i = tid; i < max_pad; i += kThreads) sorted_ids[i] = (int32_t)numel;
+  }
   // slots per expert in all chunks (tot) and in the chunks before this one (base): threads side by side
   // take neighbouring experts, the groups of threads share the chunks out
   const int width = E < kThreads ? (E > 0 ? E : 1) : kThreads;
   const int groups = kThreads / width, grp = tid / width;
-  if (grp < groups) {
+  if (chunk_cnt != nullptr && grp < groups) {
     for (int x = tid - grp * width; x < E; x += width) {
       int all = 0, before = 0;
 #pragma unroll 8
@@ -182,6 +188,14 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
     return XKB_OK;
   }
   const int64_t need = align_workspace_bytes(numel, E);
+  if ((workspace == nullptr || workspace_bytes < need) && numel <= kNoWorkspaceMax && zero_n == 0) {
+    const size_t smem = place_smem(E);
+    XKB_CHECK_CUDA(allow_smem(align_place_kernel, smem));
+    align_place_kernel<<<1, kThreads, smem, stream>>>(topk_ids, numel, numel, E, block, expert_map, num_map, nullptr, sorted_ids,
+                                                      max_pad, expert_ids, max_blocks, num_post, expert_off, slot_pos);
+    XKB_CHECK_LAUNCH("align_place_kernel");
+    return XKB_OK;
+  }
   if (workspace == nullptr || workspace_bytes < need)
     return fail(XKB_ERR_WORKSPACE, "moe_align: workspace of %lld bytes needed, %lld given",
                 (long long)need, (long long)workspace_bytes);
@@ -195,7 +209,7 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
                                                      chunk_cnt, sorted_ids, max_pad, zero, zero_n);
   XKB_CHECK_LAUNCH("align_count_kernel");
   XKB_CHECK_CUDA(launch_chained(align_place_kernel, dim3((unsigned)C), dim3(kThreads), smem2, stream, topk_ids, numel,
-                                span, E, block, expert_map, num_map, chunk_cnt, sorted_ids, expert_ids, max_blocks,
+                                span, E, block, expert_map, num_map, chunk_cnt, sorted_ids, max_pad, expert_ids, max_blocks,
                                 num_post, expert_off, slot_pos));
   XKB_CHECK_LAUNCH("align_place_kernel");
   return XKB_OK;
