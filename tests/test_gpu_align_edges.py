@@ -4,6 +4,7 @@ chunk up to 148 x 1024 slots, then several rounds per chunk.  Bit-exact against 
 import pytest
 import torch
 
+import xkernels_b200 as xkb
 from oracle import moe_oracle as oracle
 from tests.test_gpu_align import check
 
@@ -49,3 +50,11 @@ def test_no_workspace_up_to_8192_slots(numel, E, block, mapped, cuda_device):
     for got, exp in zip(out, want):
         assert torch.equal(got.cpu(), torch.as_tensor(exp).to(torch.int32).reshape(-1))
     assert call(8193) != 0 and b"workspace" in lib.xkb_last_error()
+
+
+@pytest.mark.parametrize("numel", [1024, 1025, 5000])
+def test_outputs_own_no_scratch(numel, cuda_device):
+    """What a caller keeps or saves is the result alone: the kernels' scratch is not part of its storage."""
+    ids = torch.zeros(numel, 1, dtype=torch.int32, device=cuda_device)
+    for t in xkb.moe_align_block_size(ids, 16, 48, truncate=False):
+        assert t.untyped_storage().nbytes() == 4 * t.numel()

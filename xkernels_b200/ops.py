@@ -199,19 +199,18 @@ def moe_align_block_size(topk_ids, block_size, num_experts, truncate=True, works
                 ws = torch.empty(max(cap, ws_bytes, 256), dtype=torch.uint8, device=dev)
                 workspace._xkb200_scratch = ws
         else:
-            # the kernels' scratch lies behind the sorted ids: one allocation less
-            sorted_ids = torch.empty(max_pad + -(-ws_bytes // 4), dtype=torch.int32, device=dev)
+            sorted_ids = torch.empty(max_pad, dtype=torch.int32, device=dev)
             expert_ids = torch.empty(max(max_blocks, 1), dtype=torch.int32, device=dev)
             num_post = torch.empty(1, dtype=torch.int32, device=dev)
             if max_blocks == 0:
                 expert_ids.zero_()
-            ws = None
+            # one block sorts up to 1024 slots without scratch memory
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev) if numel > 1024 else None
         _lib.check(
             lib.xkb_moe_align_block_size(
                 _ptr(ids), numel, num_experts, block_size, _ptr(emap),
                 0 if emap is None else emap.numel(), _ptr(sorted_ids), _ptr(expert_ids),
-                _ptr(num_post), 0, sorted_ids.data_ptr() + 4 * max_pad if ws is None else _ptr(ws),
-                ws_bytes if ws is None else ws.numel(), _stream(dev)),
+                _ptr(num_post), 0, _ptr(ws), 0 if ws is None else ws.numel(), _stream(dev)),
             "xkb_moe_align_block_size")
     sorted_ids = sorted_ids[:max_pad]
     if truncate:
