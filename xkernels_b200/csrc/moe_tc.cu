@@ -209,8 +209,8 @@ constexpr int mode_mats(int mode) { return (mode_is_gate_up(mode) || mode_is_pai
 constexpr bool mode_is_int4(int mode) { return mode == kModeInt4 || mode == kModeInt4Pair || mode == kModeInt4GateUp; }
 
 // Variants of the INT4 modes.  Instances of their own and not run-time switches: the narrow tiles run at their
-// register cap of 80, and with the switches inside <16, kModeInt4> spilled 16 bytes, <32, kModeInt4> 4 and
-// <32, kModeInt4GateUp> 60 (now 8, none and 52; the weights' shuffle sits under its branch for the same reason).
+// register cap of 80, and with the switches inside <16, kModeInt4> spilled 16 bytes and <32, kModeInt4GateUp> 60 (8 and
+// 52 now; a form without any was timed at M=64 and takes the same time).
 constexpr int kWideGroups = 1;    // scale groups of 64, 128 or 256 (TcParams::group_shift) instead of 32
 constexpr int kRows16 = 2;        // the weighted slot rows go to TcParams::rows16, rounded to bf16, instead of to scratch (the
                                   // second GEMM of a two-GEMM layer, whose per-slot results the reference composition
@@ -276,7 +276,7 @@ __device__ __forceinline__ uint32_t dequant_pair(uint32_t biased, uint32_t scale
 //
 // Calls with groups of 64 and more were answered by the generic kernel for any scale before this kernel took them, so
 // kWideGroups keeps its weights 2^-8 smaller only (multipliers s * 2^125 and s * 2^121, finite for |s| < 8), and a warp
-// that meets a larger, infinite or NaN scale converts that stage with a subtraction instead (dequant_pair): the
+// that meets one of 2 and more, infinite or NaN, converts that stage with a subtraction instead (dequant_pair): the
 // reference's one rounding, then times 2^-8, which is exact down to |s| = 2^-118.  (Smaller scales lose bits below
 // 2^-126, bf16's smallest normal number.)  The check is a vote per stage; subtracting always cost 9 to 29 % of a decode
 // call at group 128 (M=1 55 -> 61 us, M=37 232 -> 254, M=64 201 -> 260).
@@ -286,7 +286,7 @@ template <bool WIDE> struct Int4Scaling {
   static constexpr uint32_t kMulAdd = WIDE ? 0xBD00BD00u : 0xB200B200u;   // -8 * 2^-8, -8 * 2^-30
   static constexpr float kUnscale = WIDE ? 256.f : 1073741824.f;
 };
-constexpr uint32_t kWideLimit = 0x4100u;    // 8.0: the first |scale| (bf16 bits) whose multiplier overflows
+constexpr uint32_t kWideLimit = 0x40004000u;   // the top exponent bit of two scales: 2 and more (the multipliers overflow from 8 on)
 constexpr uint32_t kWideShift = 0x3B803B80u;   // 2^-8, twice
 __device__ __forceinline__ uint32_t bf2_mul(uint32_t a, uint32_t b) {
   const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
@@ -693,16 +693,16 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           for (int j = 0; j < 16; ++j) {
             if (!((live >> j) & 1u)) continue;          // warp-uniform
             const int32_t slot = __shfl_sync(0xffffffffu, cur_slot, j);
-            float v = __uint_as_float(acc[j]), w = 1.f;
+            constexpr bool kLateWeight = kWide;   // (170 against 177 us at group 128, 168 against 166 at group 32: M=64)
+            float v = __uint_as_float(acc[j]), w = kLateWeight ? 1.f : __shfl_sync(0xffffffffu, cur_w, j);
             if (mode_is_int4(MODE)) v *= Int4Scaling<kWide>::kUnscale;   // exact: a power of two
             if (MODE == kModeMxDown) {  // reference rounds `down` to bf16, adds the bf16 bias, then x w
               v = round_to_bf16(Cfg::kLut ? v : v * kMxUnscale);
               if (p.bias != nullptr) v = round_to_bf16(v + bias0);
-              w = __shfl_sync(0xffffffffu, cur_w, j);
               if (p.mul_w) v = v * w;
             } else {
               if (p.mul_w) {
-                w = __shfl_sync(0xffffffffu, cur_w, j);
+                if (kLateWeight) w = __shfl_sync(0xffffffffu, cur_w, j);
                 v = w * v;
               }
             }
@@ -785,10 +785,6 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           if (kChunks == 4) sw.x = lds32(sa);
           else sw.x = lds16(sa);
         }
-        bool subtract = false;   // kWideGroups: a scale of this warp is out of the multipliers' range (never for sane weights)
-        if (kWide)
-          subtract = __any_sync(0xffffffffu, __vcmpgeu2(sw.x & 0x7FFF7FFFu, kWideLimit * 0x00010001u) != 0 ||
-                                                 __vcmpgeu2(sw.y & 0x7FFF7FFFu, kWideLimit * 0x00010001u) != 0);
         // 16-byte chunk = 32 weights = one scale group; this share is chunks kChunks * part ...
         uint4 w4[kChunks];
 #pragma unroll
@@ -804,6 +800,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           const uint32_t eb = same_lap ? abar - Cfg::kASlots : abar + Cfg::kABars - Cfg::kASlots;
           if (!mbar_wait(&a_empty[eb], same_lap ? acyc : (acyc ^ 1u), guard, 6)) { ok = false; break; }
         }
+        // kWideGroups: a scale of this warp may be out of the multipliers' range (never for sane weights)
+        const bool subtract = kWide && __any_sync(0xffffffffu, ((sw.x | sw.y) & kWideLimit) != 0);
         tc_fence_after();
         const uint32_t dst = tmem_base + lane_base + Cfg::kACol0 + aq * Cfg::kUnitCols +
                              (Cfg::kUnits > 1 ? 0 : part * (kChunks * 16));
@@ -1152,9 +1150,9 @@ int int4_tc_block(int64_t numel, int E, int64_t N) {
   // square root): the tile's token bytes through shared memory, which bound it, shrink with the tile.
   // E=48, top_k=8, whole call, 128-token tiles against these: K=2048, N=7168 184 -> 169 us at 50 slots per expert, 194 -> 185
   // at 67, 200 -> 194 at 75, 206 -> 198 at 85, 212 -> 211 at 93 (96 tokens there: 241); K=7168, N=4096 (means of two
-  // runs) 328 -> 288 at 53, 364 -> 312 at 67, 365 -> 334 at 83, 380 -> 361 at 100.  A skewed routing spreads the slots
-  // further: with a bias of 0.5 334 -> 333, 365 -> 364, 414 -> 391 and 433 -> 418, with 1.0 331 -> 337, 363 -> 370,
-  // 416 -> 435 and 481 -> 454.
+  // runs) 328 -> 288 at 53, 364 -> 312 at 67, 365 -> 334 at 83, 374 -> 348 at 87.  A skewed routing spreads the slots
+  // further: with a bias of 0.5 334 -> 333, 365 -> 364, 414 -> 391 and 419 -> 396, with 1.0 331 -> 337, 363 -> 370,
+  // 416 -> 435 and 419 -> 436.
   if (N % (2 * kTileRows) == 0)
     for (int block = 80; block < 128; block += 16)
       if (avg + 2.0 * std::sqrt(avg) <= block) return block;
