@@ -204,13 +204,13 @@ def moe_align_block_size(topk_ids, block_size, num_experts, truncate=True, works
             num_post = torch.empty(1, dtype=torch.int32, device=dev)
             if max_blocks == 0:
                 expert_ids.zero_()
-            # one block sorts up to 1024 slots without scratch memory
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev) if numel > 1024 else None
+            # one block sorts up to 1024 slots without scratch memory (new_empty: half the host time)
+            ws = ids.new_empty(-(-ws_bytes // 4)) if numel > 1024 else None
         _lib.check(
             lib.xkb_moe_align_block_size(
                 _ptr(ids), numel, num_experts, block_size, _ptr(emap),
                 0 if emap is None else emap.numel(), _ptr(sorted_ids), _ptr(expert_ids),
-                _ptr(num_post), 0, _ptr(ws), 0 if ws is None else ws.numel(), _stream(dev)),
+                _ptr(num_post), 0, _ptr(ws), 0 if ws is None else ws.numel() * ws.element_size(), _stream(dev)),
             "xkb_moe_align_block_size")
     sorted_ids = sorted_ids[:max_pad]
     if truncate:
