@@ -212,7 +212,8 @@ def moe_align_block_size(topk_ids, block_size, num_experts, truncate=True, works
                 0 if emap is None else emap.numel(), _ptr(sorted_ids), _ptr(expert_ids),
                 _ptr(num_post), 0, _ptr(ws), 0 if ws is None else ws.numel() * ws.element_size(), _stream(dev)),
             "xkb_moe_align_block_size")
-    sorted_ids = sorted_ids[:max_pad]
+    if sorted_ids.numel() != max_pad:
+        sorted_ids = sorted_ids[:max_pad]
     if truncate:
         used = int(num_post.item()) // block_size
         expert_ids = expert_ids[: max(used, 1)]
