@@ -54,7 +54,7 @@ namespace {
 struct RoutingBuffers {
   int* status;
   int32_t* counters;        // directly behind the status header: cleared as one span
-  int64_t counters_each;
+  int64_t num_counters;
   int32_t* sorted_ids;
   int32_t* expert_ids;
   int32_t* num_post;
@@ -77,8 +77,8 @@ int64_t routing_max_pad(int64_t numel, int E, int block) {
 RoutingBuffers carve_routing(Carver& c, int64_t numel, int E) {
   RoutingBuffers r;
   r.status = c.take<int>(64);  // workspace header: word 0 = device status of the last call
-  r.counters_each = numel / kMinBlock + E + 2;     // >= token blocks at the smallest token tile
-  r.counters = c.take<int32_t>(2 * r.counters_each);
+  r.num_counters = numel / kMinBlock + E + 2;     // >= token blocks at the smallest token tile
+  r.counters = c.take<int32_t>(r.num_counters);
   r.sorted_ids = c.take<int32_t>(routing_max_pad(numel, E, kMaxBlock));
   r.expert_ids = c.take<int32_t>(ceil_div(routing_max_pad(numel, E, kMinBlock), kMinBlock) + 1);
   r.num_post = c.take<int32_t>(1);
@@ -90,7 +90,7 @@ RoutingBuffers carve_routing(Carver& c, int64_t numel, int E) {
 }
 
 // status header and the block counters behind it, as one span
-int64_t header_ints(const RoutingBuffers& r) { return r.counters + 2 * r.counters_each - r.status; }
+int64_t header_ints(const RoutingBuffers& r) { return r.counters + r.num_counters - r.status; }
 
 int64_t routing_bytes(int64_t numel, int E) {
   Carver c(nullptr);
@@ -110,7 +110,6 @@ Routing make_routing(const RoutingBuffers& b, int64_t numel, int E, int block) {
   r.max_pad = routing_max_pad(numel, E, block);
   r.max_blocks = ceil_div(r.max_pad, block);
   r.block_counters = b.counters;
-  r.counters_each = b.counters_each;
   r.job = nullptr;
   return r;
 }

@@ -687,7 +687,7 @@ int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   if (rc == XKB_OK) rc = token_maps(down + 2, buf.act, r.max_pad, ispp, r.block);
   if (rc != XKB_OK) return rc;
 
-  int32_t* done = r.block_counters != nullptr ? r.block_counters + r.counters_each : nullptr;
+  int32_t* done = r.block_counters;
   MxParams prm;
   prm.sorted_ids = r.sorted_ids;
   prm.expert_ids = r.expert_ids;

@@ -1275,7 +1275,7 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
                        int64_t inter, int E, int top_k, int group, float limit, void* tc_ws, int* status,
                        cudaStream_t stream) {
   Carver carve(tc_ws);
-  int32_t* done = r.block_counters != nullptr ? r.block_counters + r.counters_each : nullptr;   // block hand-over counters
+  int32_t* done = r.block_counters;   // block hand-over counters
   __nv_bfloat16* Ag = carve.take<__nv_bfloat16>(r.max_pad * hidden);
   int rc = launch_gather(A, r, Ag, hidden, top_k, 1, status, stream);
   if (rc != XKB_OK) return rc;
@@ -1371,7 +1371,7 @@ int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   XKB_REQUIRE(reinterpret_cast<uintptr_t>(w13_scale) % 16 == 0 && reinterpret_cast<uintptr_t>(w2_scale) % 16 == 0,
               "mxfp4 tcgen05 path: scale tensors must be 16-byte aligned");
   Carver carve(tc_ws);
-  int32_t* done = r.block_counters != nullptr ? r.block_counters + r.counters_each : nullptr;   // block hand-over counters
+  int32_t* done = r.block_counters;   // block hand-over counters
   __nv_bfloat16* Ag = carve.take<__nv_bfloat16>(r.max_pad * hidden);
   int rc = launch_gather(A, r, Ag, hidden, top_k, r.block == 16 ? 0 : 1, status, stream);   // 16-token tiles convert through the table: natural K order
   if (rc != XKB_OK) return rc;
