@@ -451,12 +451,16 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
     return launch_combine_bf16(rows, mul_routed_weight ? topk_w : nullptr, topk_ids, expert_map, num_map, E, out,
                                a_dtype, M, top_k, hidden, stream);
   }
-  if (use_tc)
-    rc = launch_mxfp4_tc(A, w13, w13_scale, w2, w2_scale, b13, b2, r, topk_w, act, scratch, hidden,
-                         ispp, E, top_k, swiglu_limit, mul_routed_weight, tc_ws, rb.status, stream);
-  else
-    rc = launch_mxfp4_simt(A, a_dtype, w13, w13_scale, w2, w2_scale, b13, b2, r, topk_w, act, scratch,
-                           hidden, ispp, top_k, swiglu_limit, mul_routed_weight, stream);
+  if (use_tc) {
+    __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(scratch);
+    rc = launch_mxfp4_tc(A, w13, w13_scale, w2, w2_scale, b13, b2, r, act, rows, hidden, ispp, E, top_k, swiglu_limit, tc_ws,
+                         rb.status, stream);
+    if (rc != XKB_OK) return rc;
+    return launch_combine_bf16(rows, mul_routed_weight ? topk_w : nullptr, topk_ids, expert_map, num_map, E, out,
+                               a_dtype, M, top_k, hidden, stream);
+  }
+  rc = launch_mxfp4_simt(A, a_dtype, w13, w13_scale, w2, w2_scale, b13, b2, r, topk_w, act, scratch,
+                         hidden, ispp, top_k, swiglu_limit, mul_routed_weight, stream);
   if (rc != XKB_OK) return rc;
   return launch_combine(scratch, topk_ids, expert_map, num_map, E, out, a_dtype, M, top_k, hidden, stream);
 }

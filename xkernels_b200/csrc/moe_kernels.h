@@ -71,8 +71,7 @@ int mxfp4_tc_block(int64_t numel, int E);
 int64_t mxfp4_tc_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, int E);
 int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale, const uint8_t* w2,
                     const uint8_t* w2_scale, const void* b13, const void* b2, const Routing& r,
-                    const float* topk_w, __nv_bfloat16* act, float* scratch, int64_t hidden,
-                    int64_t ispp, int E, int top_k, float limit, int mul_w, void* tc_ws, int* status,
-                    cudaStream_t stream);
+                    __nv_bfloat16* act, __nv_bfloat16* rows16, int64_t hidden, int64_t ispp, int E, int top_k,
+                    float limit, void* tc_ws, int* status, cudaStream_t stream);   // rows before the routing weight, in bf16
 
 }  // namespace xkb

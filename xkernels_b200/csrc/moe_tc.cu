@@ -195,7 +195,7 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
 constexpr int kModeInt4 = 0;      // INT4 W4A16: rows = N, bf16 group scales by TMA, fp32 slot rows out
 constexpr int kModeMxGateUp = 1;  // MXFP4 w13: a tile is 128 gate rows + the 128 matching up rows, the
                                   // two matrices alternate 256-K stages and accumulators; SwiGLU epilogue
-constexpr int kModeMxDown = 2;    // MXFP4 w2: rows = hidden, bf16-rounded result x routing weight out; two 128-row
+constexpr int kModeMxDown = 2;    // MXFP4 w2: rows = hidden, bf16 slot rows out, before the routing weight; two 128-row
                                   // weight tiles per token tile like kModeInt4Pair: with K = ispp of a few
                                   // hundred a single-tile pass would be two stages long, and the per-tile work
                                   // (read-out, loop bookkeeping) would weigh as much as the stages themselves
@@ -221,13 +221,13 @@ struct TcParams {
   const int32_t* expert_ids;
   const int32_t* num_post;
   const float* topk_w;
-  float* scratch;               // [M*top_k, N] fp32 slot rows (INT4, MX down)
+  float* scratch;               // [M*top_k, N] fp32 slot rows (INT4)
   int* status;
   int64_t numel;
   int N, K;                     // tile rows are taken from N rows per expert; K = contraction length
   int mul_w;
   int group_shift;              // kWideGroups: log2 of the scale group (6 .. 8)
-  __nv_bfloat16* rows16;        // kRows16
+  __nv_bfloat16* rows16;        // bf16 slot rows (kRows16, MX down)
   // MXFP4 only
   const __nv_bfloat16* bias;    // b13 [E, 2*ispp] or b2 [E, hidden] or nullptr
   __nv_bfloat16* act;           // gate_up mode output: [positions, N] bf16 in the K-permuted order
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__((TcCfg<BT, mode_mats(MODE), mode_is_int4(MODE)
 moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_constant__ CUtensorMap tm_scale,
                const __grid_constant__ CUtensorMap tm_tokens, const TcParams p) {
   using Cfg = TcCfg<BT, mode_mats(MODE), mode_is_int4(MODE)>;
-  constexpr bool kWide = (VAR & kWideGroups) != 0, kNarrowRows = (VAR & kRows16) != 0;
+  constexpr bool kWide = (VAR & kWideGroups) != 0, kNarrowRows = (VAR & kRows16) != 0 || MODE == kModeMxDown;
   static_assert(VAR == 0 || mode_is_int4(MODE), "variants of the INT4 modes");
   constexpr int kWStages = Cfg::kWStages;
   constexpr int kMatsC = mode_mats(MODE);
@@ -616,7 +616,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     auto load_cols = [&](int b, int c0, int32_t& slot, float& w) {
       slot = (lane < 16 && c0 < BT) ? __ldcg(p.sorted_ids + (int64_t)b * BT + c0 + lane) : -1;   // written by a kernel this one overlaps: no .nc load
       const bool live = slot >= 0 && slot < p.numel;
-      w = (!mode_is_gate_up(MODE) && p.mul_w && live) ? __ldg(p.topk_w + slot) : 1.f;
+      w = (mode_is_int4(MODE) && !mode_is_gate_up(MODE) && p.mul_w && live) ? __ldg(p.topk_w + slot) : 1.f;
     };
     auto run_epilogue = [&](int b, int nt, uint32_t dbuf, uint32_t duse, uint32_t tile_g0, int cg, int32_t my_slot,
                             float my_w) -> bool {
@@ -694,12 +694,11 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
             if (!((live >> j) & 1u)) continue;          // warp-uniform
             const int32_t slot = __shfl_sync(0xffffffffu, cur_slot, j);
             constexpr bool kLateWeight = kWide;   // (170 against 177 us at group 128, 168 against 166 at group 32: M=64)
-            float v = __uint_as_float(acc[j]), w = kLateWeight ? 1.f : __shfl_sync(0xffffffffu, cur_w, j);
+            float v = __uint_as_float(acc[j]), w = kLateWeight || MODE == kModeMxDown ? 1.f : __shfl_sync(0xffffffffu, cur_w, j);
             if (mode_is_int4(MODE)) v *= Int4Scaling<kWide>::kUnscale;   // exact: a power of two
-            if (MODE == kModeMxDown) {  // reference rounds `down` to bf16, adds the bf16 bias, then x w
+            if (MODE == kModeMxDown) {  // reference rounds `down` to bf16, adds the bf16 bias, then x w: the combine does that
               v = round_to_bf16(Cfg::kLut ? v : v * kMxUnscale);
               if (p.bias != nullptr) v = round_to_bf16(v + bias0);
-              if (p.mul_w) v = v * w;
             } else {
               if (p.mul_w) {
                 if (kLateWeight) w = __shfl_sync(0xffffffffu, cur_w, j);
@@ -716,7 +715,6 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
               } else {
                 v2 = round_to_bf16(Cfg::kLut ? v2 : v2 * kMxUnscale);
                 if (p.bias != nullptr) v2 = round_to_bf16(v2 + bias1);
-                if (p.mul_w) v2 = v2 * w;
               }
               if (kNarrowRows) p.rows16[(int64_t)slot * p.N + n_glob + kTileRows] = __float2bfloat16_rn(v2);
               else p.scratch[(int64_t)slot * p.N + n_glob + kTileRows] = v2;
@@ -1365,8 +1363,8 @@ int64_t mxfp4_tc_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, in
 
 int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale, const uint8_t* w2,
                     const uint8_t* w2_scale, const void* b13, const void* b2, const Routing& r,
-                    const float* topk_w, __nv_bfloat16* act, float* scratch, int64_t hidden, int64_t ispp,
-                    int E, int top_k, float limit, int mul_w, void* tc_ws, int* status, cudaStream_t stream) {
+                    __nv_bfloat16* act, __nv_bfloat16* rows16, int64_t hidden, int64_t ispp, int E, int top_k,
+                    float limit, void* tc_ws, int* status, cudaStream_t stream) {
   XKB_REQUIRE(r.block == 16 || r.block == 128, "mxfp4 tcgen05 path: unsupported token tile %d", r.block);
   XKB_REQUIRE(reinterpret_cast<uintptr_t>(w13_scale) % 16 == 0 && reinterpret_cast<uintptr_t>(w2_scale) % 16 == 0,
               "mxfp4 tcgen05 path: scale tensors must be 16-byte aligned");
@@ -1400,12 +1398,12 @@ int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   prm.sorted_ids = r.sorted_ids;
   prm.expert_ids = r.expert_ids;
   prm.num_post = r.num_post;
-  prm.topk_w = topk_w;
+  prm.topk_w = nullptr;   // the combine multiplies
   prm.status = status;
   prm.numel = r.numel;
   prm.max_blocks = (int)r.max_blocks;
   prm.num_experts = E;
-  prm.mul_w = mul_w;
+  prm.mul_w = 0;
   prm.group_shift = 5;
   prm.rows16 = nullptr;
   prm.limit = limit;
@@ -1424,8 +1422,11 @@ int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   rc = r.block == 16 ? launch_bt<16, kModeMxGateUp>(tm_w13, tm_s13, tm_tok0, prm, max_tiles, stream)
                      : launch_bt<128, kModeMxGateUp>(tm_w13, tm_s13, tm_tok0, prm, max_tiles, stream);
   if (rc != XKB_OK) return rc;
-  // stage 1: down -> fp32 slot rows
-  prm.scratch = scratch;
+  // stage 1: down -> slot rows in bf16, which they are rounded to.  (Kept as fp32 products with the routing weight they
+  // were twice the bytes to write and to read again: the same values, since the combine rounds that product to fp32
+  // before it adds it.  E=256, hidden 4096, ispp 512, top 6: M=4096 691 -> 643 us, M=8000 1257 -> 1179.)
+  prm.scratch = nullptr;
+  prm.rows16 = rows16;
   prm.act = nullptr;
   prm.N = (int)hidden;
   prm.K = (int)ispp;
