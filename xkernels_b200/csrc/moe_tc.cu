@@ -82,11 +82,6 @@ constexpr int kEpiDelay = 2;
 // from shared memory into registers, before they convert it (one arrival per warp of the group):
 // the turn-round of a ring slot (TMA latency + wait for the readers + their wake-up) then does not
 // contain the conversion time.
-// MMA issuer warps run their loop with all 32 lanes (waits included) and only the tcgen05.mma /
-// commit / arrive instructions themselves are predicated on lane 0: the loop is then warp-uniform
-// and descriptors and tensor-memory addresses are computed in uniform registers, instead of being
-// moved there one by one for every MMA as in a loop that only lane 0 executes.
-constexpr bool kUniformIssuer = false;
 constexpr int kTmemCols = 512;     // one CTA per SM owns all of tensor memory
 constexpr int kPackedStageBytes = kTileRows * (kStageK / 2);  // 16 KiB
 constexpr int kScaleStageBytes = kTileRows * (kStageK / 32) * 2;  // 2 KiB
@@ -524,10 +519,13 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     // sixteen M=128 N=BT K=16 MMAs into its own accumulator of the stage's matrix and commits.
     constexpr int kIssuers = Cfg::kIssuers;
     const uint32_t me = warp - 1;
-    if ((kUniformIssuer || lane == 0) && me < (uint32_t)kIssuers) {
-      const uint32_t leader = (lane == 0) ? 1u : 0u;
-      // in the warp-uniform form every wait result is made uniform with a vote
-      auto uni = [&](bool v) -> bool { return kUniformIssuer ? (__all_sync(0xffffffffu, v) != 0) : v; };
+    if (me < (uint32_t)kIssuers) {
+      // All 32 lanes run the loop, and one elected lane issues a unit's MMAs and commits: descriptors and
+      // tensor-memory addresses then live in uniform registers.  In a loop of lane 0 alone they are moved there one by
+      // one for every MMA, and an MMA takes its issuer 112 cycles beside busy dequantiser warps where the tensor pipe
+      // needs 64.  Whole calls in a loop: M=256 302 -> 281 us (K=7168), M=64 123 -> 115 and M=509 223 -> 213 (K=2048).
+      // Every wait result is made uniform with a vote.
+      auto uni = [&](bool v) -> bool { return __all_sync(0xffffffffu, v) != 0; };
       constexpr uint32_t idesc = umma_idesc_bf16(kTileRows, BT);
       // This issuer's stages are g = me, me + kIssuers, ...; its ring positions advance with them
       // (no division in the loop: the issuing thread is on the critical path of every hand-off).
@@ -562,19 +560,22 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
             }
             tc_fence_after();
             const uint32_t a_tmem = tmem_base + Cfg::kACol0 + (aq0 + h) * Cfg::kUnitCols;
+            if (elect_one()) {
 #pragma unroll
-            for (int us = 0; us < Cfg::kUnitSubs; ++us) {
-              const int sub = h * Cfg::kUnitSubs + us;
+              for (int us = 0; us < Cfg::kUnitSubs; ++us) {
+                const int sub = h * Cfg::kUnitSubs + us;
 #pragma unroll
-              for (int kk = 0; kk < kSubK / 16; ++kk)
-                umma_ts_bf16_if(d_tmem, a_tmem + us * kSubCols + kk * 8,
-                                b_desc + (uint64_t)((sub * Cfg::kBSubBytes) >> 4) + (uint64_t)(kk * 2), idesc,
-                                (fresh && sub == 0 && kk == 0) ? 0u : 1u, leader);
+                for (int kk = 0; kk < kSubK / 16; ++kk)
+                  umma_ts_bf16(d_tmem, a_tmem + us * kSubCols + kk * 8,
+                               b_desc + (uint64_t)((sub * Cfg::kBSubBytes) >> 4) + (uint64_t)(kk * 2), idesc,
+                               (fresh && sub == 0 && kk == 0) ? 0u : 1u);
+              }
+              tc_commit(&a_empty[ab0 + h]);
+              if (h == Cfg::kUnits - 1) tc_commit(&b_empty[bbar]);   // kMats arrivals release the token stage
             }
-            tc_commit_if(&a_empty[ab0 + h], leader);
+            __syncwarp();
           }
           if (!ok) break;
-          tc_commit_if(&b_empty[bbar], leader);   // kMats arrivals release the token stage
           // on to this issuer's next stage
           aq0 += kDU; if (aq0 >= (uint32_t)Cfg::kASlots) aq0 -= Cfg::kASlots;
           if (kDU >= (uint32_t)Cfg::kASlots && aq0 >= (uint32_t)Cfg::kASlots) aq0 -= Cfg::kASlots;
@@ -585,7 +586,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           bbar += kDTB; if (bbar >= (uint32_t)Cfg::kBBars) { bbar -= Cfg::kBBars; bcyc ^= 1u; }
         }
         if (!ok) break;
-        tc_commit_if(&d_full[dbuf], leader);
+        if (elect_one()) tc_commit(&d_full[dbuf]);
+        __syncwarp();
         g0mod += vsmod; if (g0mod >= (uint32_t)kIssuers) g0mod -= kIssuers;
       }
     }

@@ -98,6 +98,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, Guard&
   return mbar_wait_slow(bar, parity, g, where, sleep_ns, budget_ns);
 }
 
+// True in one lane of a converged warp: the one that issues tcgen05.mma and commits.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // Variants for warp-uniform code: every lane of the warp executes the call with the same operands
 // and `leader` (non-zero in exactly one lane) selects the lane whose instruction takes effect.
 __device__ __forceinline__ void mbar_arrive_if(uint64_t* bar, uint32_t leader) {
@@ -162,13 +169,6 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
                : "memory");
 }
 
-__device__ __forceinline__ void tc_commit_if(uint64_t* bar, uint32_t leader) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(smem_u32(bar)), "r"(leader) : "memory");
-}
-
 // 32 lanes x 8 columns store (registers r[0..7] of each thread).
 __device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3,
                                              uint32_t r4, uint32_t r5, uint32_t r6, uint32_t r7) {
@@ -215,18 +215,6 @@ __device__ __forceinline__ void umma_ts_bf16(uint32_t d_tmem, uint32_t a_tmem, u
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same, executed by a whole warp with identical operands; only the lane with `leader` != 0 issues.
-__device__ __forceinline__ void umma_ts_bf16_if(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                                uint32_t accumulate, uint32_t leader) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 
