@@ -38,10 +38,10 @@ align_small_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int E, i
                    int32_t* __restrict__ sorted_ids, int64_t max_pad,
                    int32_t* __restrict__ expert_ids, int64_t max_blocks,
                    int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out,
-                   int32_t* __restrict__ slot_pos, int32_t* __restrict__ zero, int64_t zero_n) {
+                   int32_t* __restrict__ slot_pos, int32_t* __restrict__ block_live, int32_t* __restrict__ zero, int64_t zero_n) {
   chain_trigger();   // a kernel chained behind this one may be launched; it waits for completion itself
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const Job j{topk_ids, expert_map, sorted_ids, expert_ids, num_post, expert_off_out, zero, zero_n, numel, max_pad,
+  const Job j{topk_ids, expert_map, sorted_ids, expert_ids, num_post, expert_off_out, block_live, zero, zero_n, numel, max_pad,
               max_blocks, num_map, E, block};
   const int pos = align_in_block(j, smem_raw, true);
   if (threadIdx.x < numel && slot_pos != nullptr) slot_pos[threadIdx.x] = pos;
@@ -81,7 +81,7 @@ align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t 
                    const int32_t* chunk_cnt /*[C][E+1]: written by the kernel this one overlaps; nullptr: one chunk*/,
                    int32_t* sorted_ids, int64_t max_pad, int32_t* __restrict__ expert_ids, int64_t max_blocks,
                    int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out,
-                   int32_t* __restrict__ slot_pos) {
+                   int32_t* __restrict__ slot_pos, int32_t* __restrict__ block_live) {
   chain_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int EP = E + 1, tid = threadIdx.x, C = (int)gridDim.x;
@@ -128,7 +128,7 @@ align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t 
     if (expert_off_out != nullptr)
       for (int i = tid; i < EP; i += kThreads) expert_off_out[i] = off[i];
   }
-  write_expert_ids(off, E, block, expert_ids, max_blocks, (int)blockIdx.x * kThreads + tid, C * kThreads);
+  write_expert_ids(off, tot, E, block, expert_ids, block_live, max_blocks, (int)blockIdx.x * kThreads + tid, C * kThreads);
   __syncthreads();
   for (int64_t s0 = first; s0 < last; s0 += kThreads) {
     if (s0 != first) {
@@ -170,7 +170,7 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
                  const int32_t* expert_map, int num_map, int32_t* sorted_ids,
                  int32_t* expert_ids, int32_t* num_post, int32_t* expert_off,
                  void* workspace, int64_t workspace_bytes, cudaStream_t stream, int32_t* zero, int64_t zero_n,
-                 int32_t* slot_pos) {
+                 int32_t* slot_pos, int32_t* block_live) {
   XKB_REQUIRE(numel >= 0 && numel < (1ll << 30), "moe_align: numel=%lld out of range", (long long)numel);
   XKB_REQUIRE(block > 0, "moe_align: block_size must be > 0 (got %d)", block);
   XKB_REQUIRE(E >= 0 && E <= kMaxExperts, "moe_align: num_experts=%d outside [0,%d]", E, kMaxExperts);
@@ -183,7 +183,7 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
     XKB_CHECK_CUDA(allow_smem(align_small_kernel, smem));
     align_small_kernel<<<1, kThreads, smem, stream>>>(topk_ids, numel, E, block, expert_map, num_map,
                                                       sorted_ids, max_pad, expert_ids, max_blocks,
-                                                      num_post, expert_off, slot_pos, zero, zero_n);
+                                                      num_post, expert_off, slot_pos, block_live, zero, zero_n);
     XKB_CHECK_LAUNCH("align_small_kernel");
     return XKB_OK;
   }
@@ -192,7 +192,7 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
     const size_t smem = place_smem(E);
     XKB_CHECK_CUDA(allow_smem(align_place_kernel, smem));
     align_place_kernel<<<1, kThreads, smem, stream>>>(topk_ids, numel, numel, E, block, expert_map, num_map, nullptr, sorted_ids,
-                                                      max_pad, expert_ids, max_blocks, num_post, expert_off, slot_pos);
+                                                      max_pad, expert_ids, max_blocks, num_post, expert_off, slot_pos, block_live);
     XKB_CHECK_LAUNCH("align_place_kernel");
     return XKB_OK;
   }
@@ -210,7 +210,7 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
   XKB_CHECK_LAUNCH("align_count_kernel");
   XKB_CHECK_CUDA(launch_chained(align_place_kernel, dim3((unsigned)C), dim3(kThreads), smem2, stream, topk_ids, numel,
                                 span, E, block, expert_map, num_map, chunk_cnt, sorted_ids, max_pad, expert_ids, max_blocks,
-                                num_post, expert_off, slot_pos));
+                                num_post, expert_off, slot_pos, block_live));
   XKB_CHECK_LAUNCH("align_place_kernel");
   return XKB_OK;
 }

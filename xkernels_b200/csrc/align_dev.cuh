@@ -54,13 +54,13 @@ __device__ inline void padded_offsets(const int* hist, int* off, int* warp_tot, 
 }
 
 // expert_ids[b] for every block b < max_blocks: the expert whose padded run
-// holds position b*block, 0 past the used blocks.
-__device__ inline void write_expert_ids(const int* off, int E, int block, int32_t* expert_ids,
-                                 int64_t max_blocks, int tid0, int stride) {
+// holds position b*block, 0 past the used blocks.  block_live (may be nullptr): the block's slots that are not padding.
+__device__ inline void write_expert_ids(const int* off, const int* count, int E, int block, int32_t* expert_ids,
+                                 int32_t* block_live, int64_t max_blocks, int tid0, int stride) {
   const int total = off[E];
   for (int64_t b = tid0; b < max_blocks; b += stride) {
     const int64_t pos = b * block;
-    int e = 0;
+    int e = 0, live = 0;
     if (pos < total) {
       // largest e with off[e] <= pos and off[e+1] > pos (runs of zero length skipped)
       int lo = 0, hi = E;  // invariant: off[lo] <= pos < off[hi]
@@ -69,8 +69,11 @@ __device__ inline void write_expert_ids(const int* off, int E, int block, int32_
         if (off[mid] <= pos) lo = mid; else hi = mid;
       }
       e = lo;
+      const int left = off[e] + count[e] - (int)pos;   // a run's padding is at its end
+      live = left < block ? left : block;
     }
     expert_ids[b] = e;
+    if (block_live != nullptr) block_live[b] = live;
   }
 }
 
@@ -104,7 +107,7 @@ __device__ inline int round_rank(int my_e, bool active, int E, uint16_t* wcnt, i
   return active ? (int)wcnt[warp * EP + my_e] + rank : 0;
 }
 
-// What one sort reads and writes.  zero / zero_n: ints the caller wants cleared; expert_off may be nullptr.
+// What one sort reads and writes.  zero / zero_n: ints the caller wants cleared; expert_off and block_live may be nullptr.
 struct Job {
   const int32_t* topk_ids;
   const int32_t* expert_map;
@@ -112,6 +115,7 @@ struct Job {
   int32_t* expert_ids;
   int32_t* num_post;
   int32_t* expert_off;
+  int32_t* block_live;
   int32_t* zero;
   int64_t zero_n, numel, max_pad, max_blocks;
   int num_map, E, block;
@@ -156,7 +160,7 @@ __device__ __forceinline__ int align_in_block(const Job& j, unsigned char* smem,
     if (tid == 0) j.num_post[0] = off[E];
     if (j.expert_off != nullptr)
       for (int i = tid; i < EP; i += kThreads) j.expert_off[i] = off[i];
-    write_expert_ids(off, E, j.block, j.expert_ids, j.max_blocks, tid, kThreads);
+    write_expert_ids(off, tot, E, j.block, j.expert_ids, j.block_live, j.max_blocks, tid, kThreads);
   }
   __syncthreads();
   return pos;

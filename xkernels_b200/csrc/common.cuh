@@ -63,6 +63,7 @@ namespace align { struct Job; }
 // sorted_ids[p]  slot id (token*top_k + j) at sorted position p, or `numel`
 //                for a padding position.
 // expert_ids[b]  expert of block b (block = `block_size` consecutive positions).
+// block_live[b]  how many positions of block b hold a slot (its first ones), 0 past the used blocks.
 // slot_pos[s]    sorted position of slot s, -1 for a slot that was dropped.
 // expert_off[e]  first position of expert e's padded run; [E] = num_post_pad.
 struct Routing {
@@ -71,6 +72,7 @@ struct Routing {
   const int32_t* num_post;
   const int32_t* expert_off;
   const int32_t* slot_pos;
+  const int32_t* block_live;
   int64_t numel;     // M * top_k
   int64_t max_pad;   // length of sorted_ids
   int64_t max_blocks;
@@ -89,7 +91,8 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int num_experts, int bl
                  int32_t* expert_ids, int32_t* num_post, int32_t* expert_off,
                  void* workspace, int64_t workspace_bytes, cudaStream_t stream,
                  int32_t* zero = nullptr, int64_t zero_n = 0,   // zero_n ints at `zero` are cleared on the way
-                 int32_t* slot_pos = nullptr);                  // [numel] position of every slot, -1 = dropped
+                 int32_t* slot_pos = nullptr,                   // [numel] position of every slot, -1 = dropped
+                 int32_t* block_live = nullptr);                // [blocks] slots of a block that are not padding
 int64_t align_workspace_bytes(int64_t numel, int num_experts);
 
 // out[m,n] = sum_j scratch[m*top_k+j, n] over the slots whose (mapped) expert id lies in [0, E)

@@ -60,6 +60,7 @@ struct RoutingBuffers {
   int32_t* num_post;
   int32_t* expert_off;
   int32_t* slot_pos;
+  int32_t* block_live;
   void* align_ws;
   int64_t align_ws_bytes;
 };
@@ -84,6 +85,7 @@ RoutingBuffers carve_routing(Carver& c, int64_t numel, int E) {
   r.num_post = c.take<int32_t>(1);
   r.expert_off = c.take<int32_t>(E + 1);
   r.slot_pos = c.take<int32_t>(numel);
+  r.block_live = c.take<int32_t>(ceil_div(routing_max_pad(numel, E, kMinBlock), kMinBlock) + 1);
   r.align_ws_bytes = align_workspace_bytes(numel, E);
   r.align_ws = c.take<char>(r.align_ws_bytes);
   return r;
@@ -105,6 +107,7 @@ Routing make_routing(const RoutingBuffers& b, int64_t numel, int E, int block) {
   r.num_post = b.num_post;
   r.expert_off = b.expert_off;
   r.slot_pos = b.slot_pos;
+  r.block_live = b.block_live;
   r.numel = numel;
   r.block = block;
   r.max_pad = routing_max_pad(numel, E, block);
@@ -140,13 +143,13 @@ int route(const RoutingBuffers& rb, const int32_t* topk_ids, const int32_t* expe
                    gather_grid(r->numel / top_k, gather_units, false, &g) == XKB_OK && g.blocks > kPositionsMinBlocks;
   if (gather_units > 0 && r->numel >= 1 && r->numel <= kSortInGatherMax && top_k <= 32 && E >= 1 && E <= align::kMaxExperts &&
       gather_grid(r->numel / top_k, gather_units, true, &g) == XKB_OK && g.blocks <= kSortInGatherBlocks) {
-    *job = align::Job{topk_ids, expert_map, rb.sorted_ids, rb.expert_ids, rb.num_post, rb.expert_off, rb.status,
+    *job = align::Job{topk_ids, expert_map, rb.sorted_ids, rb.expert_ids, rb.num_post, rb.expert_off, rb.block_live, rb.status,
                       header_ints(rb), r->numel, r->max_pad, r->max_blocks, num_map, E, r->block};
     r->job = job;
     return XKB_OK;
   }
   return launch_align(topk_ids, r->numel, E, r->block, expert_map, num_map, rb.sorted_ids, rb.expert_ids, rb.num_post,
-                      rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb), rb.slot_pos);
+                      rb.expert_off, rb.align_ws, rb.align_ws_bytes, stream, rb.status, header_ints(rb), rb.slot_pos, rb.block_live);
 }
 
 bool tma_base_ok(const void* a, const void* b) {

@@ -11,12 +11,12 @@
 //            row per thread reads conflict-free) + scale tile per stage: bf16 [128 x 8] for INT4,
 //            e8m0 bytes [128 x 16] for MXFP4 (sixteen bytes are the smallest TMA row, so a tile
 //            carries the scales of two stages and each stage uses its half).
-//   then     two or three MMA issuer warps (lane 0 each; warp 1 also allocates and frees tensor
+//   then     two to four MMA issuer warps (one elected lane each; warp 1 also allocates and frees tensor
 //            memory): tcgen05.mma kind::f16, A from tensor memory, B from shared
 //            memory, fp32 accumulators in tensor memory.  They take whole stages in
 //            turn, each into its own accumulator.
-//   then     TMA producer, tokens: four [BT x 64] bf16 sub-tiles per stage (128B swizzle =
-//            the UMMA K-major canonical layout) from the gathered activation buffer.  (In a
+//   then     TMA producer, tokens: the block's slots in groups of eight, [8 x 256] bf16 per stage (128B
+//            swizzle = the UMMA K-major canonical layout) from the gathered activation buffer.  (In a
 //            warp of its own: two polling threads in one warp slow each other down.)
 //   then     sixteen dequantiser warps: thread = weight row; nibbles -> exact bf16 integers
 //            by the 0x4300|nib trick, minus 136, times the group scale in one
@@ -83,6 +83,14 @@ constexpr int kEpiDelay = 2;
 // the turn-round of a ring slot (TMA latency + wait for the readers + their wake-up) then does not
 // contain the conversion time.
 constexpr int kTmemCols = 512;     // one CTA per SM owns all of tensor memory
+// Token stages are made of groups of eight tokens, [8 x 256] bf16 as four swizzle atoms [8 x 64].  One TMA request
+// loads kTokBox tokens, and only as many are made as the block's slots need.
+constexpr int kTokGroup = 8;
+constexpr int kTokAtomBytes = kTokGroup * kSubK * 2;       // 1 KiB
+constexpr int kTokGroupBytes = kSubs * kTokAtomBytes;      // 4 KiB
+// (Requests of 4 KiB throughout cost the token producer's thread more than they save: R=6144 rows of an expert-parallel
+// rank 373 us with them, 356 with 16 KiB ones, which the 128-token tiles take.)
+constexpr int tok_box(int bt) { return bt == 16 ? 8 : bt % 32 == 0 && bt > 64 ? 32 : 16; }
 constexpr int kPackedStageBytes = kTileRows * (kStageK / 2);  // 16 KiB
 constexpr int kScaleStageBytes = kTileRows * (kStageK / 32) * 2;  // 2 KiB
 
@@ -130,8 +138,7 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   // TMA from L2 about a microsecond later; narrow tiles are small, so their ring is made deep
   // enough that the issuers never wait for tokens.
   static constexpr int kBStages = (BT <= 16) ? kBStages16 : (BT <= 32) ? 6 : (BT <= 64) ? (kGroups == 3 ? 3 : 4) : (BT <= 96) ? 3 : 2;
-  static constexpr int kBSubBytes = BT * kSubK * 2;
-  static constexpr int kBStageBytes = kSubs * kBSubBytes;   // [4][BT x 64] bf16
+  static constexpr int kBStageBytes = BT * kStageK * 2;     // [BT / 8][4][8 x 64] bf16
   static constexpr int kWStages = (BT <= 16) ? kWStagesNarrow : (BT <= 32 || kGroups == 3) ? 6 : 4;
   static_assert(kWStages % kGroups == 0, "a weight stage must always be converted by the same group");
   // MMA issuers.  One thread sustains one tcgen05.mma per ~45 cycles (65-100 beside busy
@@ -215,6 +222,7 @@ struct TcParams {
   const int32_t* sorted_ids;
   const int32_t* expert_ids;
   const int32_t* num_post;
+  const int32_t* block_live;
   const float* topk_w;
   float* scratch;               // [M*top_k, N] fp32 slot rows (INT4)
   int* status;
@@ -357,7 +365,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                          ~uintptr_t(1023));
   unsigned char* s_packed = smem;                                         // kWStages x 16 KiB
-  unsigned char* s_tokens = s_packed + kWStages * kPackedStageBytes;      // kBStages x 4 x [BT x 64] bf16
+  unsigned char* s_tokens = s_packed + kWStages * kPackedStageBytes;      // kBStages x [BT / 8] x 4 x [8 x 64] bf16
   unsigned char* s_scale = s_tokens + Cfg::kBStages * Cfg::kBStageBytes;  // kWStages x 2 KiB
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_scale + kWStages * kScaleStageBytes);
   uint64_t* w_full = bars;                       // [kWStages]
@@ -429,6 +437,13 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
   const int n_blocks = routing_ok ? n_post / BT : 0;
   const int total_tiles = n_blocks * n_tiles;   // the host checks that the worst case fits 31 bits
   const int k_stages = p.K / kStageK;   // 256-K stages per tile
+  // Slots of tile t's block, rounded up to whole groups of `unit` positions.  Only these positions' activations are loaded
+  // and multiplied: the tensor pipe's time and energy and the token bytes through L2 and shared memory follow the slots
+  // and not the tile.  E=48, top 8, whole calls: K=7168, N=4096 M=256 285 -> 265 us, M=400 342 -> 317, M=4000 2036 -> 1925;
+  // K=2048, N=7168 M=509 217 -> 204; two-GEMM layer M=600 728 -> 623.
+  // (Read a tile ahead.  A value that no sort wrote only costs time: it is brought into range.)
+  auto block_live = [&](int t) -> int { return t < total_tiles ? __ldcg(p.block_live + t / n_tiles) : 0; };
+  auto rounded = [&](int live, int unit) -> int { return ((live < 1 ? 1 : live > BT ? BT : live) + unit - 1) / unit * unit; };
   // "virtual" weight stages of a tile: two-matrix modes alternate the matrices stage by stage
   constexpr int kMats = mode_mats(MODE);
   const int v_stages = kMats * k_stages;
@@ -473,9 +488,12 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     {
       uint32_t st = 0, tb = 0;   // token stage slot and running number of the token stage
       int ready_b = -1;          // block hand-over: last block whose activations are known to be complete
+      int next_live = block_live((int)blockIdx.x);
       for (int t = (int)blockIdx.x; t < total_tiles && !guard.aborted(); t += (int)gridDim.x) {
         const int b = t / n_tiles;
         const int pos0 = b * BT;
+        const int rows = rounded(next_live, tok_box(BT));
+        next_live = block_live(t + (int)gridDim.x);
         if (hand_over_second && b != ready_b) {   // block hand-over: the first GEMM's read-outs of block b
           uint64_t t0 = 0;
           bool ready = false;
@@ -502,11 +520,10 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
             if (!mbar_wait(&b_empty[tp % Cfg::kBBars], (tp / Cfg::kBBars) & 1u, guard, 2, kProdSleepNs)) break;
           }
           const uint32_t bar = tb % Cfg::kBBars;
-          mbar_expect_tx(&b_full[bar], Cfg::kBStageBytes);
-#pragma unroll
-          for (int j = 0; j < kSubs; ++j)
-            tma_load_2d(s_tokens + st * Cfg::kBStageBytes + j * Cfg::kBSubBytes, &tm_tokens, &b_full[bar],
-                        (ks * kSubs + j) * kSubK, pos0);
+          mbar_expect_tx(&b_full[bar], rows * (kStageK * 2));
+          for (int i = 0; i < rows; i += tok_box(BT))
+            tma_load_4d(s_tokens + st * Cfg::kBStageBytes + i * (kStageK * 2), &tm_tokens, &b_full[bar], 0, 0, ks * kSubs,
+                        (pos0 + i) / kTokGroup);
           if (++st == Cfg::kBStages) st = 0;
           ++tb;
         }
@@ -526,7 +543,6 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
       // needs 64.  Whole calls in a loop: M=256 302 -> 281 us (K=7168), M=64 123 -> 115 and M=509 223 -> 213 (K=2048).
       // Every wait result is made uniform with a vote.
       auto uni = [&](bool v) -> bool { return __all_sync(0xffffffffu, v) != 0; };
-      constexpr uint32_t idesc = umma_idesc_bf16(kTileRows, BT);
       // This issuer's stages are g = me, me + kIssuers, ...; its ring positions advance with them
       // (no division in the loop: the issuing thread is on the critical path of every hand-off).
       constexpr uint32_t kDU = (uint32_t)(kIssuers * Cfg::kUnits);       // units per own-stage step
@@ -537,7 +553,10 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
       uint32_t bbar = (me / kMats) % Cfg::kBBars, bcyc = 0;              // token barrier and lap parity
       uint32_t it = 0, g0mod = 0;                                        // g0mod = (first stage of the tile) % kIssuers
       const uint32_t vsmod = (uint32_t)v_stages % kIssuers;
+      int next_live = block_live((int)blockIdx.x);
       for (int t = (int)blockIdx.x; t < total_tiles && uni(!guard.aborted()); t += (int)gridDim.x, ++it) {
+        const uint32_t idesc = umma_idesc_bf16(kTileRows, rounded(next_live, 16));   // N is a multiple of 16
+        next_live = block_live(t + (int)gridDim.x);
         // accumulator set of this tile; its previous user must have been read out by every epilogue warp
         const uint32_t dbuf = it % Cfg::kDBuf, duse = it / Cfg::kDBuf;
         bool ok = uni(mbar_wait(&d_empty[dbuf], (duse & 1u) ^ 1u, guard, 8, 100));
@@ -547,7 +566,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           const int mat = vs % kMats;                       // which matrix this stage belongs to
           const int acc = (int)me;
           const uint32_t d_tmem = tmem_base + (uint32_t)(((int)dbuf * Cfg::kAccs + acc) * BT);
-          const uint64_t b_desc = umma_desc_k_sw128(smem_u32(s_tokens + bst * Cfg::kBStageBytes));
+          const uint64_t b_desc = umma_desc_k_sw128<kTokGroupBytes>(smem_u32(s_tokens + bst * Cfg::kBStageBytes));
           const bool fresh = ((started >> mat) & 1u) == 0;
           started |= 1u << mat;
 #pragma unroll
@@ -567,7 +586,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
 #pragma unroll
                 for (int kk = 0; kk < kSubK / 16; ++kk)
                   umma_ts_bf16(d_tmem, a_tmem + us * kSubCols + kk * 8,
-                               b_desc + (uint64_t)((sub * Cfg::kBSubBytes) >> 4) + (uint64_t)(kk * 2), idesc,
+                               b_desc + (uint64_t)((sub * kTokAtomBytes) >> 4) + (uint64_t)(kk * 2), idesc,
                                (fresh && sub == 0 && kk == 0) ? 0u : 1u);
               }
               tc_commit(&a_empty[ab0 + h]);
@@ -1011,10 +1030,11 @@ EncodeTiledFn get_encode_fn() {
 // A map holds no device state, so a stale entry (memory freed and reused with another layout) is
 // harmless: the key is everything the encoding depends on.
 struct MapKey {
-  const void* base; uint64_t rows, cols; uint32_t box_rows, box_cols; int dt, elem_bits, swz;
+  const void* base; uint64_t dims[4], strides[3]; uint32_t box[4]; int dt, swz;   // unused dimensions: 1, strides 0
   bool operator==(const MapKey& o) const {
-    return base == o.base && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols &&
-           dt == o.dt && elem_bits == o.elem_bits && swz == o.swz;
+    for (int i = 0; i < 4; ++i)
+      if (dims[i] != o.dims[i] || box[i] != o.box[i] || (i < 3 && strides[i] != o.strides[i])) return false;
+    return base == o.base && dt == o.dt && swz == o.swz;
   }
 };
 constexpr int kMapCacheSize = 64;
@@ -1028,9 +1048,12 @@ MapCache g_map_cache;
 
 }  // namespace
 
-int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bits, const void* base, uint64_t rows,
-                uint64_t cols, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swz, const char* what) {
-  const MapKey key{base, rows, cols, box_rows, box_cols, (int)dt, elem_bits, (int)swz};
+// dims, box: innermost first; strides: bytes of the outer dimensions
+static int make_map(CUtensorMap* map, CUtensorMapDataType dt, int rank, const void* base, const uint64_t* dims,
+                    const uint64_t* strides, const uint32_t* box, CUtensorMapSwizzle swz, const char* what) {
+  MapKey key{base, {1, 1, 1, 1}, {0, 0, 0}, {1, 1, 1, 1}, (int)dt, (int)swz};
+  for (int i = 0; i < rank; ++i) { key.dims[i] = dims[i]; key.box[i] = box[i]; }
+  for (int i = 0; i + 1 < rank; ++i) key.strides[i] = strides[i];
   {
     std::lock_guard<std::mutex> lock(g_map_cache.mu);
     for (int i = 0; i < g_map_cache.used; ++i)
@@ -1039,14 +1062,9 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bits, const v
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return fail(XKB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   XKB_REQUIRE(reinterpret_cast<uintptr_t>(base) % 16 == 0, "%s: base pointer must be 16-byte aligned", what);
-  XKB_REQUIRE((cols * elem_bits) % 128 == 0, "%s: row pitch %llu B is not a multiple of 16", what,
-              (unsigned long long)(cols * elem_bits / 8));
-  XKB_REQUIRE(box_rows <= 256 && box_cols <= 256 && (box_cols * elem_bits) % 128 == 0, "%s: bad box", what);
-  const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * (uint64_t)elem_bits / 8};
-  const cuuint32_t box[2] = {box_cols, box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  const cuuint64_t d[4] = {key.dims[0], key.dims[1], key.dims[2], key.dims[3]}, st[3] = {key.strides[0], key.strides[1], key.strides[2]};
+  CUresult r = fn(map, dt, (cuuint32_t)rank, const_cast<void*>(base), d, st, key.box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(XKB_ERR_CUDA, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", what, (int)r);
   {
@@ -1058,7 +1076,26 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bits, const v
   return XKB_OK;
 }
 
+int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bits, const void* base, uint64_t rows,
+                uint64_t cols, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swz, const char* what) {
+  XKB_REQUIRE((cols * elem_bits) % 128 == 0, "%s: row pitch %llu B is not a multiple of 16", what,
+              (unsigned long long)(cols * elem_bits / 8));
+  XKB_REQUIRE(box_rows <= 256 && box_cols <= 256 && (box_cols * elem_bits) % 128 == 0, "%s: bad box", what);
+  const uint64_t dims[2] = {cols, rows}, strides[1] = {cols * (uint64_t)elem_bits / 8};
+  const uint32_t box[2] = {box_cols, box_rows};
+  return make_map(map, dt, 2, base, dims, strides, box, swz, what);
+}
+
 namespace {
+
+// Activations [rows, K] as (64 K, eight rows, K / 64, groups of eight rows); a box is some groups of one 256-K stage.
+// (Blocks are whole groups, so rows % 8 rows at the end belong to none.)
+int make_token_map(CUtensorMap* map, const __nv_bfloat16* base, int64_t rows, int64_t K, int block, const char* what) {
+  const uint64_t dims[4] = {(uint64_t)kSubK, (uint64_t)kTokGroup, (uint64_t)(K / kSubK), (uint64_t)(rows / kTokGroup)};
+  const uint64_t strides[3] = {(uint64_t)K * 2, (uint64_t)kSubK * 2, (uint64_t)K * 2 * kTokGroup};
+  const uint32_t box[4] = {(uint32_t)kSubK, (uint32_t)kTokGroup, (uint32_t)kSubs, (uint32_t)(tok_box(block) / kTokGroup)};
+  return make_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, what);
+}
 
 int launch_gather(const void* A, const Routing& r, __nv_bfloat16* Ag, int64_t K, int top_k, int permute, int* status,
                   cudaStream_t stream) {
@@ -1229,14 +1266,14 @@ int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, cons
   rc = make_map_2d(&tm_scale, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, scale, (uint64_t)E * N, (uint64_t)(K / group),
                    kTileRows, kStageK / 32, CU_TENSOR_MAP_SWIZZLE_NONE, "group scales");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tokens, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, Ag, (uint64_t)r.max_pad, (uint64_t)K,
-                   (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "gathered activations");
+  rc = make_token_map(&tm_tokens, Ag, r.max_pad, K, r.block, "gathered activations");
   if (rc != XKB_OK) return rc;
 
   TcParams prm;
   prm.sorted_ids = r.sorted_ids;
   prm.expert_ids = r.expert_ids;
   prm.num_post = r.num_post;
+  prm.block_live = r.block_live;
   prm.topk_w = topk_w;
   prm.scratch = scratch;
   prm.status = status;
@@ -1292,17 +1329,16 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
   rc = make_map_2d(&tm_s2, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, s2, (uint64_t)E * hidden, (uint64_t)(inter / group),
                    kTileRows, kStageK / 32, CU_TENSOR_MAP_SWIZZLE_NONE, "w2 group scales");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tok0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, Ag, (uint64_t)r.max_pad, (uint64_t)hidden,
-                   (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "gathered activations");
+  rc = make_token_map(&tm_tok0, Ag, r.max_pad, hidden, r.block, "gathered activations");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tok1, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, act, (uint64_t)r.max_pad, (uint64_t)inter,
-                   (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "SwiGLU activations");
+  rc = make_token_map(&tm_tok1, act, r.max_pad, inter, r.block, "SwiGLU activations");
   if (rc != XKB_OK) return rc;
 
   TcParams prm;
   prm.sorted_ids = r.sorted_ids;
   prm.expert_ids = r.expert_ids;
   prm.num_post = r.num_post;
+  prm.block_live = r.block_live;
   prm.topk_w = topk_w;
   prm.status = status;
   prm.numel = r.numel;
@@ -1389,17 +1425,16 @@ int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   rc = make_map_2d(&tm_s2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 8, w2_scale, (uint64_t)E * hidden, (uint64_t)ispp / 32,
                    kTileRows, 16, CU_TENSOR_MAP_SWIZZLE_NONE, "w2 scales");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tok0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, Ag, (uint64_t)r.max_pad, (uint64_t)hidden,
-                   (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "gathered activations");
+  rc = make_token_map(&tm_tok0, Ag, r.max_pad, hidden, r.block, "gathered activations");
   if (rc != XKB_OK) return rc;
-  rc = make_map_2d(&tm_tok1, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 16, act, (uint64_t)r.max_pad, (uint64_t)ispp,
-                   (uint32_t)r.block, kSubK, CU_TENSOR_MAP_SWIZZLE_128B, "SwiGLU activations");
+  rc = make_token_map(&tm_tok1, act, r.max_pad, ispp, r.block, "SwiGLU activations");
   if (rc != XKB_OK) return rc;
 
   TcParams prm;
   prm.sorted_ids = r.sorted_ids;
   prm.expert_ids = r.expert_ids;
   prm.num_post = r.num_post;
+  prm.block_live = r.block_live;
   prm.topk_w = nullptr;   // the combine multiplies
   prm.status = status;
   prm.numel = r.numel;

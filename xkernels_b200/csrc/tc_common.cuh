@@ -142,6 +142,13 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x,
+                                            int y, int z, int w) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+      : "memory");
+}
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -199,12 +206,14 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes
-// (64 bf16) in the 128-byte swizzle: 8-row groups 1024 bytes apart.
-// start>>4 [0,14), LBO>>4 [16,30) (unused with swizzle: 1), SBO>>4 [32,46) = 64,
+// (64 bf16) in the 128-byte swizzle: 8-row groups of 1024 bytes, GROUP_STRIDE apart.
+// start>>4 [0,14), LBO>>4 [16,30) (unused with swizzle: 1), SBO>>4 [32,46),
 // version [46,48) = 1, layout [61,64) = 2 (SWIZZLE_128B).  The tile base must be
 // 1024-byte aligned; advancing K by 16 elements adds 32 bytes to the start.
+template <int GROUP_STRIDE = 1024>   // bytes from one 8-row group to the next
 __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+  return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(GROUP_STRIDE >> 4) << 32) | (1ull << 46) |
+         (2ull << 61);
 }
 
 // D[tmem] (+)= A[tmem] * B[smem]^T ; one thread issues.
