@@ -106,10 +106,12 @@ constexpr int gcd_c(int a, int b) { return b == 0 ? a : gcd_c(b, a % b); }
 constexpr int lcm_c(int a, int b) { return a / gcd_c(a, b) * b; }
 
 template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
-  // Dequantiser groups that take alternate stages.  Narrow tiles: two groups of eight warps, so
-  // that one group's waits and store drains overlap the other's arithmetic.  Wide tiles are bound by
-  // the tensor pipe and have only two A slots; there all sixteen warps fill one slot together,
-  // which halves the fill latency in the slot's round trip.
+  // Dequantiser groups that take alternate stages: two groups of eight warps, so that one group's waits and store
+  // drains overlap the other's arithmetic.  In the two-matrix modes the matrices alternate too, so a group stays with
+  // one of them.  A stage of wide tiles is four hand-off units of 64 K, and a warpgroup converts two of them in turn: the
+  // units of both matrices come in the order their issuers take them, two by two.  (Sixteen warps on one stage published
+  // its four units together, and the last waited in its slot for the MMAs of three: MXFP4 M=4096 630 -> 609 us, M=8000
+  // 1144 -> 1100; the INT4 modes, whose conversion is shorter, run the same.)
   // dequantiser warpgroups (the four warps of one cover the four tensor-memory lane quarters)
   static constexpr int kWGs = (BT <= 64) ? kNarrowWGs : 4;
   static constexpr int kDequantWarps = 4 * kWGs;
@@ -125,12 +127,14 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   static constexpr int kCtrlWarps = (BT > 32) ? 4 : (MATS == 1) ? (INT4 ? 5 : 4)
                                                 : 2 + (INT4 ? kInt4TwoMatIssuers : kMxIssuers);
   static constexpr int kThreads = 32 * (kCtrlWarps + kDequantWarps);
-  static constexpr int kGroups = (BT <= 64) ? kWGs / 2 : 1;
+  static constexpr int kGroups = kWGs / 2;
   static constexpr int kGroupWarps = kDequantWarps / kGroups;
   static constexpr int kPartsPerStage = kWGs / kGroups;      // warpgroups that share one stage
   static constexpr int kChunks = 8 / kPartsPerStage;         // 16-byte chunks (32 weights, one scale group) per thread and stage
   static constexpr int kUnits = (BT <= 64) ? kUnitsNarrow : kUnitsWide;   // hand-off units per stage
-  static_assert(kUnits == 1 || kUnits == kPartsPerStage, "a unit is a whole stage or one warpgroup's share of it");
+  static constexpr int kPartUnits = kUnits / kPartsPerStage;   // units of a stage that one warpgroup converts, every kPartsPerStage-th
+  static constexpr int kUnitChunks = 8 / kUnits;
+  static_assert(kUnits % kPartsPerStage == 0 && kUnitChunks >= 2, "a unit is one warpgroup's work, whole 64-K sub-tiles");
   static constexpr int kUnitCols = kSlotCols / kUnits;       // tensor-memory columns of one unit
   static constexpr int kUnitSubs = kSubs / kUnits;           // 64-K token sub-tiles one unit spans
   static_assert(kSubs % kUnits == 0, "a unit must span whole 64-K sub-tiles");
@@ -388,7 +392,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
   if (threadIdx.x == 0) {
     for (int i = 0; i < kWStages; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], Cfg::kGroupWarps); }
     for (int i = 0; i < Cfg::kBBars; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], kMatsC); }
-    for (int i = 0; i < Cfg::kABars; ++i) { mbar_init(&a_full[i], Cfg::kGroupWarps / Cfg::kUnits); mbar_init(&a_empty[i], 1); }
+    for (int i = 0; i < Cfg::kABars; ++i) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
     for (int i = 0; i < Cfg::kDBuf; ++i) { mbar_init(&d_full[i], Cfg::kIssuers); mbar_init(&d_empty[i], 4 * Cfg::kEpiWGs); }
     *abort_word = 0;
     mbar_fence_init();
@@ -614,10 +618,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     // ---------------- dequantisers + epilogue ----------------
     // Thread = weight row (the four warps of a warpgroup cover the four tensor-memory lane
     // quarters).  The sixteen warps form two groups of two warpgroups; stages (numbered g across
-    // the tiles of the CTA) alternate between the groups, so that one group's barrier waits,
-    // shared-memory loads and tensor-memory store drains overlap the other group's arithmetic.
-    // Inside a group, warpgroup h converts the K slices 2h and 2h+1 (128 of the stage's 256 K) into
-    // columns [64 h, 64 h + 64) of the stage's A slot, eight columns per tcgen05.st.
+    // the tiles of the CTA) alternate between the groups.  Inside a group, warpgroup `part` converts every other
+    // hand-off unit of a stage, eight columns of its slot per tcgen05.st.
     const int wg = (warp - kCtrlWarps) >> 2;
     constexpr int kGroups = Cfg::kGroups, kChunks = Cfg::kChunks;
     const uint32_t grp = (uint32_t)wg / Cfg::kPartsPerStage;
@@ -626,6 +628,10 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     const int row = quarter * 32 + lane;       // weight row inside the tile
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const uint32_t s_packed_u32 = smem_u32(s_packed), s_scale_u32 = smem_u32(s_scale);
+    // chunk c of this warpgroup's share of a stage: unit (c / kUnitChunks) * kPartsPerStage + part of it, chunk by chunk
+    auto chunk_of = [&](int c) -> int {
+      return ((c / Cfg::kUnitChunks) * Cfg::kPartsPerStage + part) * Cfg::kUnitChunks + c % Cfg::kUnitChunks;
+    };
     const uint32_t lut_lane = smem_u32(lut) + (uint32_t)lane * 4u;   // this lane's column of the table
     // Epilogue of tile (b, nt) whose accumulators sit in set `dbuf` (use number `duse` of that
     // set).  It runs one weight stage into the NEXT tile (or after the last tile), so that the MMAs
@@ -771,7 +777,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     // This group's stages are g = grp, grp + kGroups, ... whatever the tile boundaries, so its ring
     // positions advance by a fixed step per converted stage (no division in the loop).
     constexpr uint32_t kDU = (uint32_t)(kGroups * Cfg::kUnits);           // units per own-stage step
-    const uint32_t u_first = grp * Cfg::kUnits + (Cfg::kUnits > 1 ? (uint32_t)part : 0u);
+    const uint32_t u_first = grp * Cfg::kUnits + (uint32_t)part;
     uint32_t wst = grp % kWStages, wph = 0;                               // weight slot and its lap parity
     uint32_t aq = u_first % Cfg::kASlots;                                 // A slot of this warpgroup's unit
     uint32_t abar = u_first % Cfg::kABars, acyc = 0;                      // its barrier and the barrier ring's lap parity
@@ -792,105 +798,110 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         if (mode_is_int4(MODE)) {
           const uint32_t sa = s_scale_u32 + wst * kScaleStageBytes + row * 16;
           if (!kWide) {
-            if (kChunks == 4) sw = lds64(sa + part * 8);
-            else sw.x = lds32(sa + part * 4);
+            if (Cfg::kPartUnits == 1) sw = lds64(sa + part * 8);
+            else sw = make_uint2(lds32(sa + part * 4), lds32(sa + 8 + part * 4));
           } else {  // two chunks or more share a scale: the first and the third chunk's, each twice
-            const uint32_t k0 = (uint32_t)(vs / kMats) * kStageK + (uint32_t)(part * kChunks) * 32u;
+            const uint32_t k0 = (uint32_t)(vs / kMats) * kStageK + (uint32_t)chunk_of(0) * 32u, k2 = k0 + (uint32_t)(chunk_of(2) - chunk_of(0)) * 32u;
             sw.x = lds16(sa + ((k0 >> p.group_shift) & 7u) * 2u) * 0x00010001u;
-            if (kChunks == 4) sw.y = lds16(sa + (((k0 + 64u) >> p.group_shift) & 7u) * 2u) * 0x00010001u;
+            sw.y = lds16(sa + ((k2 >> p.group_shift) & 7u) * 2u) * 0x00010001u;
           }
-        } else {  // the kChunks e8m0 bytes of this share: this stage's half of the row's sixteen
-          const uint32_t sa = s_scale_u32 + wst * kScaleStageBytes + row * 16 + (((vs / kMats) & 1) << 3) + part * kChunks;
-          if (kChunks == 4) sw.x = lds32(sa);
-          else sw.x = lds16(sa);
+        } else {  // the e8m0 bytes of this share: this stage's half of the row's sixteen
+          const uint32_t sa = s_scale_u32 + wst * kScaleStageBytes + row * 16 + (((vs / kMats) & 1) << 3);
+          if (Cfg::kPartUnits == 1) sw.x = lds32(sa + part * 4);
+          else sw.x = lds16(sa + part * 2) | (lds16(sa + 4 + part * 2) << 16);
         }
-        // 16-byte chunk = 32 weights = one scale group; this share is chunks kChunks * part ...
+        // 16-byte chunk = 32 weights = one scale group
         uint4 w4[kChunks];
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) w4[c] = lds128(pk + (((part * kChunks + c) ^ (row & 7)) << 4));
+        for (int c = 0; c < kChunks; ++c) w4[c] = lds128(pk + ((chunk_of(c) ^ (row & 7)) << 4));
         // This warp's share of the stage is in registers (the shared-memory unit executes a warp's
         // loads and the arrive in order, and the arrive has release semantics): one arrival per warp
         // of the group hands the stage back to the producer.
         __syncwarp();
         mbar_arrive_if(&w_empty[wst], lead);
-        // the slot's previous user was the unit kASlots before this one: wait until its MMAs have completed
-        if (n_own * kDU + u_first >= (uint32_t)Cfg::kASlots) {
-          const bool same_lap = abar >= (uint32_t)Cfg::kASlots;
-          const uint32_t eb = same_lap ? abar - Cfg::kASlots : abar + Cfg::kABars - Cfg::kASlots;
-          if (!mbar_wait(&a_empty[eb], same_lap ? acyc : (acyc ^ 1u), guard, 6)) { ok = false; break; }
-        }
         // kWideGroups: a scale of this warp may be out of the multipliers' range (never for sane weights)
         const bool subtract = kWide && __any_sync(0xffffffffu, ((sw.x | sw.y) & kWideLimit) != 0);
-        tc_fence_after();
-        const uint32_t dst = tmem_base + lane_base + Cfg::kACol0 + aq * Cfg::kUnitCols +
-                             (Cfg::kUnits > 1 ? 0 : part * (kChunks * 16));
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-          const uint32_t words[4] = {w4[c].x, w4[c].y, w4[c].z, w4[c].w};
-          if (mode_is_int4(MODE)) {
-            const uint32_t s01 = (c < 2) ? sw.x : sw.y;
-            const uint32_t s2 = (c & 1) ? __byte_perm(s01, s01, 0x3232) : __byte_perm(s01, s01, 0x1010);
-            if (!kWide || !subtract) {
-              using S = Int4Scaling<kWide>;
-              const uint32_t m_lo = bf2_mul(s2, S::kMulLo), m_hi = bf2_mul(s2, S::kMulHi), add = bf2_mul(s2, S::kMulAdd);
+        for (int pu = 0; pu < Cfg::kPartUnits; ++pu) {
+          const uint32_t uo = (uint32_t)(pu * Cfg::kPartsPerStage);   // this unit of the stage, counted from the warpgroup's first
+          // the slot's previous user was the unit kASlots before this one: wait until its MMAs have completed
+          if (n_own * kDU + u_first + uo >= (uint32_t)Cfg::kASlots) {
+            const bool same_lap = abar + uo >= (uint32_t)Cfg::kASlots;
+            const uint32_t eb = same_lap ? abar + uo - Cfg::kASlots : abar + uo + Cfg::kABars - Cfg::kASlots;
+            if (!mbar_wait(&a_empty[eb], same_lap ? acyc : (acyc ^ 1u), guard, 6)) { ok = false; break; }
+          }
+          tc_fence_after();
+          const uint32_t dst = tmem_base + lane_base + Cfg::kACol0 + (aq + uo) * Cfg::kUnitCols;
 #pragma unroll
-              for (int wp = 0; wp < 2; ++wp) {  // two words = 16 weights = 8 columns
-                const uint32_t x0 = words[2 * wp], x1 = words[2 * wp + 1];
-                const uint32_t y0 = x0 >> 8, y1 = x1 >> 8;
-                tmem_st_32x8(dst + c * 16 + wp * 8,
-                             bf2_fma(x0 & 0x000F000Fu, m_lo, add), bf2_fma(x0 & 0x00F000F0u, m_hi, add),
-                             bf2_fma(y0 & 0x000F000Fu, m_lo, add), bf2_fma(y0 & 0x00F000F0u, m_hi, add),
-                             bf2_fma(x1 & 0x000F000Fu, m_lo, add), bf2_fma(x1 & 0x00F000F0u, m_hi, add),
-                             bf2_fma(y1 & 0x000F000Fu, m_lo, add), bf2_fma(y1 & 0x00F000F0u, m_hi, add));
+          for (int uc = 0; uc < Cfg::kUnitChunks; ++uc) {
+            const int c = pu * Cfg::kUnitChunks + uc;
+            const uint32_t words[4] = {w4[c].x, w4[c].y, w4[c].z, w4[c].w};
+            if (mode_is_int4(MODE)) {
+              const uint32_t s01 = (c < 2) ? sw.x : sw.y;
+              const uint32_t s2 = (c & 1) ? __byte_perm(s01, s01, 0x3232) : __byte_perm(s01, s01, 0x1010);
+              if (!kWide || !subtract) {
+                using S = Int4Scaling<kWide>;
+                const uint32_t m_lo = bf2_mul(s2, S::kMulLo), m_hi = bf2_mul(s2, S::kMulHi), add = bf2_mul(s2, S::kMulAdd);
+#pragma unroll
+                for (int wp = 0; wp < 2; ++wp) {  // two words = 16 weights = 8 columns
+                  const uint32_t x0 = words[2 * wp], x1 = words[2 * wp + 1];
+                  const uint32_t y0 = x0 >> 8, y1 = x1 >> 8;
+                  tmem_st_32x8(dst + uc * 16 + wp * 8,
+                               bf2_fma(x0 & 0x000F000Fu, m_lo, add), bf2_fma(x0 & 0x00F000F0u, m_hi, add),
+                               bf2_fma(y0 & 0x000F000Fu, m_lo, add), bf2_fma(y0 & 0x00F000F0u, m_hi, add),
+                               bf2_fma(x1 & 0x000F000Fu, m_lo, add), bf2_fma(x1 & 0x00F000F0u, m_hi, add),
+                               bf2_fma(y1 & 0x000F000Fu, m_lo, add), bf2_fma(y1 & 0x00F000F0u, m_hi, add));
+                }
+              } else {
+#pragma unroll
+                for (int wp = 0; wp < 2; ++wp) {  // two words = 16 weights = 8 columns
+                  const uint32_t x0 = words[2 * wp], x1 = words[2 * wp + 1];
+                  tmem_st_32x8(dst + uc * 16 + wp * 8,
+                               wide_pair(x0, s2), wide_pair(x0 >> 4, s2), wide_pair(x0 >> 8, s2), wide_pair(x0 >> 12, s2),
+                               wide_pair(x1, s2), wide_pair(x1 >> 4, s2), wide_pair(x1 >> 8, s2), wide_pair(x1 >> 12, s2));
+                }
               }
             } else {
+              const uint32_t sb = (sw.x >> (8 * c)) & 0xFFu;
+              if (Cfg::kLut) {
+                // 2^(sb - 127) as a bf16 pair: exponent field sb; byte 0 is the subnormal 2^-127, 0xFF decodes to 0
+                uint32_t f = sb << 7;
+                if (sb == 0u) f = 0x40u;
+                if (sb == 0xFFu) f = 0u;
+                const uint32_t cf = f * 0x00010001u;
 #pragma unroll
-              for (int wp = 0; wp < 2; ++wp) {  // two words = 16 weights = 8 columns
-                const uint32_t x0 = words[2 * wp], x1 = words[2 * wp + 1];
-                tmem_st_32x8(dst + c * 16 + wp * 8,
-                             wide_pair(x0, s2), wide_pair(x0 >> 4, s2), wide_pair(x0 >> 8, s2), wide_pair(x0 >> 12, s2),
-                             wide_pair(x1, s2), wide_pair(x1 >> 4, s2), wide_pair(x1 >> 8, s2), wide_pair(x1 >> 12, s2));
+                for (int wp = 0; wp < 2; ++wp) {
+                  uint32_t r[8];
+#pragma unroll
+                  for (int h = 0; h < 2; ++h) {
+                    const uint32_t x = words[2 * wp + h];
+                    // entry of byte k of x for this lane: lut_lane + byte * 128 (bytes): one byte
+                    // permute and one multiply-add each
+                    r[4 * h + 0] = bf2_mul(lds32(__byte_perm(x, 0u, 0x4440u) * 128u + lut_lane), cf);
+                    r[4 * h + 1] = bf2_mul(lds32(__byte_perm(x, 0u, 0x4441u) * 128u + lut_lane), cf);
+                    r[4 * h + 2] = bf2_mul(lds32(__byte_perm(x, 0u, 0x4442u) * 128u + lut_lane), cf);
+                    r[4 * h + 3] = bf2_mul(lds32(__byte_perm(x, 0u, 0x4443u) * 128u + lut_lane), cf);
+                  }
+                  tmem_st_32x8(dst + uc * 16 + wp * 8, r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7]);
+                }
+                continue;
               }
-            }
-          } else {
-            const uint32_t sb = (sw.x >> (8 * c)) & 0xFFu;
-            if (Cfg::kLut) {
-              // 2^(sb - 127) as a bf16 pair: exponent field sb; byte 0 is the subnormal 2^-127, 0xFF decodes to 0
-              uint32_t f = sb << 7;
-              if (sb == 0u) f = 0x40u;
-              if (sb == 0xFFu) f = 0u;
-              const uint32_t cf = f * 0x00010001u;
+              if (sb > kMxMaxScale && sb != 0xFFu) atomicCAS(p.status, 0, kErrMxScaleRange);   // never taken for sane weights
+              const uint32_t cf = mx_scale_factor(sb);
 #pragma unroll
               for (int wp = 0; wp < 2; ++wp) {
                 uint32_t r[8];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                  const uint32_t x = words[2 * wp + h];
-                  // entry of byte k of x for this lane: lut_lane + byte * 128 (bytes): one byte
-                  // permute and one multiply-add each
-                  r[4 * h + 0] = bf2_mul(lds32(__byte_perm(x, 0u, 0x4440u) * 128u + lut_lane), cf);
-                  r[4 * h + 1] = bf2_mul(lds32(__byte_perm(x, 0u, 0x4441u) * 128u + lut_lane), cf);
-                  r[4 * h + 2] = bf2_mul(lds32(__byte_perm(x, 0u, 0x4442u) * 128u + lut_lane), cf);
-                  r[4 * h + 3] = bf2_mul(lds32(__byte_perm(x, 0u, 0x4443u) * 128u + lut_lane), cf);
-                }
-                tmem_st_32x8(dst + c * 16 + wp * 8, r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7]);
+                mx_word(words[2 * wp], cf, r[0], r[1], r[2], r[3]);
+                mx_word(words[2 * wp + 1], cf, r[4], r[5], r[6], r[7]);
+                tmem_st_32x8(dst + uc * 16 + wp * 8, r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7]);
               }
-              continue;
-            }
-            if (sb > kMxMaxScale && sb != 0xFFu) atomicCAS(p.status, 0, kErrMxScaleRange);   // never taken for sane weights
-            const uint32_t cf = mx_scale_factor(sb);
-#pragma unroll
-            for (int wp = 0; wp < 2; ++wp) {
-              uint32_t r[8];
-              mx_word(words[2 * wp], cf, r[0], r[1], r[2], r[3]);
-              mx_word(words[2 * wp + 1], cf, r[4], r[5], r[6], r[7]);
-              tmem_st_32x8(dst + c * 16 + wp * 8, r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7]);
             }
           }
+          tmem_wait_st();          // warp-wide: every lane's stores have landed
+          tc_fence_before();
+          mbar_arrive_if(&a_full[abar + uo], lead);
         }
-        tmem_wait_st();          // warp-wide: every lane's stores have landed
-        tc_fence_before();
-        mbar_arrive_if(&a_full[abar], lead);
+        if (!ok) break;
         // on to this group's next stage
         ++n_own;
         wst += kGroups; if (wst >= (uint32_t)kWStages) { wst -= kWStages; wph ^= 1u; }
