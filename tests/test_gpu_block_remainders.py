@@ -14,11 +14,15 @@ from xkernels_b200 import ops, synth
 pytestmark = pytest.mark.gpu
 
 COUNTS = [
-    (1, 7, 8, 9, 16, 17, 0, 2),             # token tiles of 16
-    (15, 16, 17, 31, 32, 33, 1, 23),        # 32
+    (1, 7, 8, 9, 0, 2, 0, 1),               # token tiles of 16
+    (1, 7, 8, 0, 0, 0, 0, 0),               # the fewest tokens that take them whatever the average
+    (16, 17, 0, 1, 0, 0, 0, 0),             # experts of more slots than a tile
+    (15, 16, 17, 31, 32, 33, 1, 23),        # 64 (32: MXFP4)
+    (5, 16, 17, 31, 32, 33, 1, 0),          # 64
+    (8, 9, 31, 32, 33, 7, 1, 0),            # 32, the most slots per expert
     (33, 47, 48, 49, 64, 65, 8, 1),         # 64
-    (81, 80, 1, 66, 63, 65, 17, 97),        # 80 (INT4)
-    (128, 129, 96, 97, 255, 1, 150, 127),   # 128
+    (81, 80, 1, 66, 63, 65, 17, 97),        # 128 (MXFP4 too)
+    (128, 129, 96, 97, 255, 1, 150, 127),
 ]
 
 

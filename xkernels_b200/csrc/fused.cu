@@ -219,7 +219,7 @@ static int int4_impl(const void* A, int a_dtype, const int32_t* packed, const vo
                 "fused_moe_int4_w4a16: shape not supported by the tcgen05 path (needs bf16 A, "
                 "N %% 128 == 0, K %% 256 == 0, group_size 32)");
   const bool use_tc = (path == XKB_PATH_TC) || (path == XKB_PATH_AUTO && tc_fit);
-  const int block = use_tc ? int4_tc_block(numel, E, N) : kSimtBlock;
+  const int block = use_tc ? int4_tc_block(numel, E, top_k) : kSimtBlock;
 
   Routing r = make_routing(rb, numel, E, block);
   align::Job job;
@@ -364,7 +364,7 @@ extern "C" int xkb_fused_moe_int4_ffn(const void* A, int a_dtype, const int32_t*
     return fail(XKB_ERR_ARG, "fused_moe_int4_ffn: shape not supported by the tcgen05 path (needs bf16 A, "
                              "hidden %% 256 == 0, inter %% 256 == 0, group_size 32)");
   const bool use_tc = (path == XKB_PATH_TC) || (path == XKB_PATH_AUTO && tc_fit);
-  const int block = use_tc ? int4_tc_block(numel, E, hidden) : kSimtBlock;
+  const int block = use_tc ? int4_tc_block(numel, E, top_k) : kSimtBlock;
   Routing r = make_routing(rb, numel, E, block);
   align::Job job;
   int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? hidden / 8 : 0, &r, &job, stream);

@@ -38,7 +38,7 @@ constexpr int kErrBadRouting = 3;   // status code: a routing value read by a ke
 
 // ---- tcgen05 path (moe_tc.cu) ----------------------------------------------
 bool int4_tc_supported(int a_dtype, int64_t M, int64_t N, int64_t K, int E, int top_k, int group);
-int int4_tc_block(int64_t numel, int E, int64_t N);
+int int4_tc_block(int64_t numel, int E, int top_k);
 int64_t int4_tc_workspace_bytes(int64_t numel, int64_t N, int64_t K, int E);
 int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, const Routing& r,
                    const float* topk_w, float* scratch, int64_t N, int64_t K, int E, int top_k, int group,

@@ -42,7 +42,6 @@
 // a status code, all roles leave their loops, and tensor memory is released.
 
 #include <atomic>
-#include <cmath>
 #include <mutex>
 #include "align_dev.cuh"
 #include "moe_kernels.h"
@@ -61,10 +60,7 @@ constexpr int kSubK = 64;        // K per 128-byte swizzled token sub-tile / per
 constexpr int kSubs = kStageK / kSubK;  // 4
 constexpr int kSlotCols = kStageK / 2;                 // 128 columns of bf16 pairs per A slot
 constexpr int kSubCols = kSubK / 2;                    // 32 of them per warpgroup
-constexpr int kMaxIssuers = 4;
-constexpr int kMxIssuers = 2;          // MMA issuer warps of the two-matrix modes at token tiles <= 32 (2 or 4)
-constexpr int kInt4TwoMatIssuers = 4;   // measured on the two-GEMM layer at decode: 290 us with four, 307 with two
-constexpr int kWStagesNarrow = 6;      // weight ring depth for token tiles of 16
+constexpr int kWStagesNarrow = 6;      // weight ring depth for token tiles of 16 and 32
 constexpr int kBStages16 = 9;          // token ring depth for token tiles of 16
 constexpr uint32_t kProdSleepNs = 400; // back-off of the TMA producers, which run a whole ring ahead
 constexpr uint32_t kIssSleepNs = 32;   // back-off of the MMA issuers (on the critical path: short)
@@ -90,7 +86,7 @@ constexpr int kTokAtomBytes = kTokGroup * kSubK * 2;       // 1 KiB
 constexpr int kTokGroupBytes = kSubs * kTokAtomBytes;      // 4 KiB
 // (Requests of 4 KiB throughout cost the token producer's thread more than they save: R=6144 rows of an expert-parallel
 // rank 373 us with them, 356 with 16 KiB ones, which the 128-token tiles take.)
-constexpr int tok_box(int bt) { return bt == 16 ? 8 : bt % 32 == 0 && bt > 64 ? 32 : 16; }
+constexpr int tok_box(int bt) { return bt == 16 ? 8 : bt <= 64 ? 16 : 32; }
 constexpr int kPackedStageBytes = kTileRows * (kStageK / 2);  // 16 KiB
 constexpr int kScaleStageBytes = kTileRows * (kStageK / 32) * 2;  // 2 KiB
 
@@ -121,11 +117,9 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   // its share of the conversion.
   static constexpr int kColGroups = BT / 16;
   static constexpr int kEpiWGs = kColGroups < kWGs ? kColGroups : kWGs;
-  // Control warps: weight producer, the issuers, token producer.  Narrow INT4 tiles run three
-  // issuers (five control warps; 21 warps get 80 registers each, enough for the INT4 dequantiser);
-  // the others two issuers (four control warps, 96 registers, which the E2M1 dequantiser needs).
-  static constexpr int kCtrlWarps = (BT > 32) ? 4 : (MATS == 1) ? (INT4 ? 5 : 4)
-                                                : 2 + (INT4 ? kInt4TwoMatIssuers : kMxIssuers);
+  // Control warps: weight producer, the issuers, token producer.  (Twenty warps get 96 registers each, 21 and more 80.)
+  static constexpr int kIssuers = 2;
+  static constexpr int kCtrlWarps = 2 + kIssuers;
   static constexpr int kThreads = 32 * (kCtrlWarps + kDequantWarps);
   static constexpr int kGroups = kWGs / 2;
   static constexpr int kGroupWarps = kDequantWarps / kGroups;
@@ -141,24 +135,20 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   // Token ring.  A token stage is released by the commit of the MMAs that read it and re-filled by
   // TMA from L2 about a microsecond later; narrow tiles are small, so their ring is made deep
   // enough that the issuers never wait for tokens.
-  static constexpr int kBStages = (BT <= 16) ? kBStages16 : (BT <= 32) ? 6 : (BT <= 64) ? (kGroups == 3 ? 3 : 4) : (BT <= 96) ? 3 : 2;
+  static constexpr int kBStages = (BT <= 16) ? kBStages16 : (BT <= 32) ? 6 : (BT <= 64) ? 4 : 2;
   static constexpr int kBStageBytes = BT * kStageK * 2;     // [BT / 8][4][8 x 64] bf16
-  static constexpr int kWStages = (BT <= 16) ? kWStagesNarrow : (BT <= 32 || kGroups == 3) ? 6 : 4;
+  static constexpr int kWStages = (BT <= 32) ? kWStagesNarrow : 4;
   static_assert(kWStages % kGroups == 0, "a weight stage must always be converted by the same group");
-  // MMA issuers.  One thread sustains one tcgen05.mma per ~45 cycles (65-100 beside busy
-  // dequantiser warps) whatever the shape, and that is an issue limit of the thread, not of the
-  // tensor pipe: measured aggregate rates for N = 16 are 45 / 27 / 13 cycles per MMA with 1 / 2 / 4
-  // issuing warps, while N = 128 is pipe-bound at 64 cycles.  Besides the MMAs a visit to a stage
-  // costs the issuing thread several hundred cycles of waits, fences and commits, so the issuers
-  // take whole stages in turn: stage g (numbered across the tiles of the CTA) belongs to issuer
-  // g % kIssuers, which puts it into its own accumulator (per matrix); the epilogue adds them.
-  // (Measured at decode: two issuers + token producer in its own warp 222 us, three issuers with
-  // both producers in one warp 238 us, three issuers + five control warps 210 us.)
-  static constexpr int kIssuers = kCtrlWarps - 2;
-  static_assert(kIssuers <= kMaxIssuers, "not enough issuer warps");
-  // One accumulator per issuer.  A tile has a multiple of MATS stages and kIssuers is a multiple of
-  // MATS, so the matrix of stage g is g % MATS = (g % kIssuers) % MATS: issuer j only ever sees matrix
-  // j % MATS, and accumulator a belongs to matrix a % MATS.  (kIssuers == MATS: one per matrix.)
+  // MMA issuers.  One thread sustains one tcgen05.mma per ~45 cycles up to 64 tokens, and that is an issue limit of the
+  // thread, not of the tensor pipe: measured aggregate rates for N = 16 are 45 / 27 / 13 cycles per MMA with 1 / 2 / 4
+  // issuing warps, while N = 128 is pipe-bound at 64 cycles.  The waits, fences and commits of a stage come on top, so
+  // two issuers take whole stages in turn: stage g (numbered across the tiles of the CTA) belongs to issuer g % 2, which
+  // puts it into its own accumulator; the epilogue adds them.  A third and a fourth cost more issue slots, registers and
+  // accumulator sets than they give.  Whole calls with one / two / three issuers, K=7168, N=4096: M=1 47.2 / 41.9 / 42.9 us,
+  // M=12 189 / 173 / 177, M=64 (32-token tiles) 217 / 200 / 206; with one / two / four per pair of matrices, the two-GEMM
+  // layer at M=1: - / 61.5 / 65.7, M=37 - / 307 / 311.
+  // One accumulator per issuer.  A tile has a multiple of MATS stages, so with two matrices an issuer only ever sees
+  // one of them (kLocked) and its accumulator belongs to that.
   static constexpr bool kLocked = (kIssuers == MATS);
   static constexpr int kAccs = kIssuers;
   // Two or three accumulator sets when tensor memory has room beside three stages of A slots: the
@@ -214,9 +204,7 @@ constexpr bool mode_is_gate_up(int mode) { return mode == kModeMxGateUp || mode 
 constexpr int mode_mats(int mode) { return (mode_is_gate_up(mode) || mode_is_pair(mode)) ? 2 : 1; }
 constexpr bool mode_is_int4(int mode) { return mode == kModeInt4 || mode == kModeInt4Pair || mode == kModeInt4GateUp; }
 
-// Variants of the INT4 modes.  Instances of their own and not run-time switches: the narrow tiles run at their
-// register cap of 80, and with the switches inside <16, kModeInt4> spilled 16 bytes and <32, kModeInt4GateUp> 60 (8 and
-// 52 now; a form without any was timed at M=64 and takes the same time).
+// Variants of the INT4 modes: instances of their own and not run-time switches, which cost registers.
 constexpr int kWideGroups = 1;    // scale groups of 64, 128 or 256 (TcParams::group_shift) instead of 32
 constexpr int kRows16 = 2;        // the weighted slot rows go to TcParams::rows16, rounded to bf16, instead of to scratch (the
                                   // second GEMM of a two-GEMM layer, whose per-slot results the reference composition
@@ -1189,22 +1177,21 @@ bool int4_tc_supported(int a_dtype, int64_t M, int64_t N, int64_t K, int E, int 
          M > 0 && E > 0 && top_k > 0 && (int64_t)E * N < (1ll << 31) && K < (1 << 30);
 }
 
-int int4_tc_block(int64_t numel, int E, int64_t N) {
+// A tile multiplies and loads its block's slots only, so a tile wider than they are costs little (shallower rings, one
+// accumulator set from 64 on), and one that an expert's slots do not fit streams that expert's weights twice.  Lines a
+// little below the crossing at uniform routing, since skewed routing spreads the slots (bias 0.4 to 0.8 below).  E=48, top 8,
+// whole calls in a loop, us at 16 / 32 / 64 / 128 tokens; K=7168, N=4096: 2 slots per expert on average 173 / 176 / 182 / -,
+// 5 196 / 198 / 205 / -, 5 skewed 160 / 153 / 157 / -, 11 203 / 202 / 207 / 232, 11 skewed 225 / 200 / 198 / 202,
+// 20 312 / 221 / 226 / -, 25 343 / 239 / 234 / 251, 33 skewed 428 / 324 / 276 / 268, 35 443 / 326 / 249 / 270, 42 507 / 375 / 266 / 279,
+// 50 582 / 417 / 286 / 288, 50 skewed 562 / 403 / 322 / 301; K=2048, N=7168: 11 110 / 113 / 121 / 126, 33 237 / 173 / 148 / 149, 47 309 / 242 / 163 / 162;
+// two-GEMM layer: 18 463 / 341 / 348 / 360, 42 821 / 600 / 412 / 408.  (Tiles of 80, 96 and 112 tokens are within 2 % of the
+// 128-token one wherever a block holds nearly every expert.)  Sixteen tokens or fewer fit a 16-token tile however they
+// are routed (an expert takes a token once).
+int int4_tc_block(int64_t numel, int E, int top_k) {
   const double avg = (double)numel / (E > 0 ? E : 1);
-  if (avg <= 12) return 16;
-  if (avg <= 24) return 32;
-  if (avg <= 48) return 64;
-  // 80, 96 or 112 tokens x two row tiles, while nearly every expert fits one block (its slots spread by about their
-  // square root): the tile's token bytes through shared memory, which bound it, shrink with the tile.
-  // E=48, top_k=8, whole call, 128-token tiles against these: K=2048, N=7168 184 -> 169 us at 50 slots per expert, 194 -> 185
-  // at 67, 200 -> 194 at 75, 206 -> 198 at 85, 212 -> 211 at 93 (96 tokens there: 241); K=7168, N=4096 (means of two
-  // runs) 328 -> 288 at 53, 364 -> 312 at 67, 365 -> 334 at 83, 374 -> 348 at 87.  A skewed routing spreads the slots
-  // further: with a bias of 0.5 334 -> 333, 365 -> 364, 414 -> 391 and 419 -> 396, with 1.0 331 -> 337, 363 -> 370,
-  // 416 -> 435 and 419 -> 436.
-  if (N % (2 * kTileRows) == 0)
-    for (int block = 80; block < 128; block += 16)
-      if (avg + 2.0 * std::sqrt(avg) <= block) return block;
-  return 128;  // wide: 128 tokens x two 128-row weight tiles per CTA (one tile if N % 256 != 0)
+  if (avg <= 4 || numel <= 16 * (int64_t)top_k) return 16;
+  if (avg <= 16) return 32;
+  return avg <= 40 ? 64 : 128;   // 128: x two 128-row weight tiles per CTA (one tile if N % 256 != 0)
 }
 
 // read-out warps that count per tile of the first GEMM: four per warpgroup on duty
@@ -1225,9 +1212,6 @@ static int launch_int4_variant(const CUtensorMap& tm_packed, const CUtensorMap& 
     case 16: return launch_bt<16, kModeInt4, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
     case 32: return launch_bt<32, kModeInt4, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
     case 64: return launch_bt<64, kModeInt4, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles, stream);
-    case 80: return launch_bt<80, kModeInt4Pair, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
-    case 96: return launch_bt<96, kModeInt4Pair, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
-    case 112: return launch_bt<112, kModeInt4Pair, VAR>(tm_packed, tm_scale, tm_tokens, prm, max_tiles / 2, stream);
     case 128:
       if constexpr ((VAR & kRows16) == 0) {   // (a two-GEMM layer's N is a multiple of 256)
         if (N % (2 * kTileRows) != 0)
@@ -1253,9 +1237,6 @@ static int launch_int4_gate_up(const CUtensorMap& tm_packed, const CUtensorMap& 
     case 16: return launch_bt<16, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
     case 32: return launch_bt<32, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
     case 64: return launch_bt<64, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
-    case 80: return launch_bt<80, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
-    case 96: return launch_bt<96, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
-    case 112: return launch_bt<112, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
     case 128: return launch_bt<128, kModeInt4GateUp, VAR>(tm_packed, tm_scale, tm_tokens, prm, tiles, stream);
     default: return fail(XKB_ERR_ARG, "int4 tcgen05 path: unsupported token tile %d", r.block);
   }
