@@ -148,8 +148,7 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   // M=12 189 / 173 / 177, M=64 (32-token tiles) 217 / 200 / 206; with one / two / four per pair of matrices, the two-GEMM
   // layer at M=1: - / 61.5 / 65.7, M=37 - / 307 / 311.
   // One accumulator per issuer.  A tile has a multiple of MATS stages, so with two matrices an issuer only ever sees
-  // one of them (kLocked) and its accumulator belongs to that.
-  static constexpr bool kLocked = (kIssuers == MATS);
+  // one of them and its accumulator belongs to that.
   static constexpr int kAccs = kIssuers;
   // Two or three accumulator sets when tensor memory has room beside three stages of A slots: the
   // MMAs of the next tiles start while an earlier tile's accumulators still wait to be read out.
@@ -633,17 +632,18 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
       const bool live = slot >= 0 && slot < p.numel;
       w = (mode_is_int4(MODE) && !mode_is_gate_up(MODE) && p.mul_w && live) ? __ldg(p.topk_w + slot) : 1.f;
     };
-    auto run_epilogue = [&](int b, int nt, uint32_t dbuf, uint32_t duse, uint32_t tile_g0, int cg, int32_t my_slot,
-                            float my_w) -> bool {
+    // the first 16-column group of tile number `it` that this warpgroup reads out (kColGroups and more: none)
+    auto first_group = [&](uint32_t it) -> int {
+      if (Cfg::kEpiWGs == Cfg::kWGs) return wg;
+      return (int)(((uint32_t)wg + (uint32_t)Cfg::kWGs - (it * (uint32_t)Cfg::kColGroups) % (uint32_t)Cfg::kWGs) % (uint32_t)Cfg::kWGs);
+    };
+    auto run_epilogue = [&](int b, int nt, uint32_t it, int32_t my_slot, float my_w) -> bool {
+      const uint32_t dbuf = it % Cfg::kDBuf, duse = it / Cfg::kDBuf;
+      const int cg = first_group(it);
       const uint32_t d_base = tmem_base + lane_base + dbuf * (uint32_t)(Cfg::kAccs * BT);
-      // which accumulators the tile's stages went to: stage vs -> issuer (g0 + vs) % kIssuers
-      uint32_t valid = 0;
-      if (Cfg::kLocked) {
-        valid = (1u << kMats) - 1u;
-      } else {
-        for (int vs = 0; vs < v_stages && vs < Cfg::kIssuers; ++vs)
-          valid |= 1u << ((tile_g0 + (uint32_t)vs) % Cfg::kIssuers);
-      }
+      // One matrix: the issuers' accumulators are added, those that the tile's stages went to (issuer
+      // g % 2 of the running stage number g; a tile of one stage wrote only one).
+      const uint32_t first_acc = it % Cfg::kIssuers;
       if (!mbar_wait(&d_full[dbuf], duse & 1u, guard, 7)) return false;
       tc_fence_after();
       const int64_t n_glob = (int64_t)nt * (mode_is_pair(MODE) ? 2 * kTileRows : kTileRows) + row;
@@ -662,29 +662,31 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         // Everything below is skipped for padding positions, and a block of padding only costs the load.
         const int32_t cur_slot = my_slot;
         const float cur_w = my_w;
-        if (c0 + 16 * Cfg::kWGs < BT) load_cols(b, c0 + 16 * Cfg::kWGs, my_slot, my_w);   // the next group's, in flight meanwhile
+        const bool last = c0 + 16 * Cfg::kWGs >= BT;
+        if (!last) load_cols(b, c0 + 16 * Cfg::kWGs, my_slot, my_w);   // the next group's, in flight meanwhile
         const uint32_t live = __ballot_sync(0xffffffffu, cur_slot >= 0 && cur_slot < p.numel) & 0xFFFFu;
-        if (live == 0u) continue;
-        // acc = matrix 0 (INT4 / down: the only one; gate_up: gate; pair: first row tile), more = matrix 1,
-        // each the sum of the accumulators that were written in this tile
+        // acc = matrix 0 (INT4 / down: the only one; gate_up: gate; pair: first row tile), more = matrix 1
         uint32_t acc[16], more[16];
+        if (live != 0u) {
+          tmem_ld_32x16(d_base + c0, acc);
+          tmem_ld_32x16(d_base + BT + c0, more);
+          tmem_wait_ld();
+          if (kMats == 1) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) { acc[q] = 0u; more[q] = 0u; }
-#pragma unroll
-        for (int a = 0; a < Cfg::kAccs; ++a) {
-          if ((valid >> a) & 1u) {
-            uint32_t part[16];
-            tmem_ld_32x16(d_base + a * BT + c0, part);
-            tmem_wait_ld();
-            if (kMats == 2 && (a & 1)) {
-#pragma unroll
-              for (int q = 0; q < 16; ++q) more[q] = __float_as_uint(__uint_as_float(more[q]) + __uint_as_float(part[q]));
-            } else {
-#pragma unroll
-              for (int q = 0; q < 16; ++q) acc[q] = __float_as_uint(__uint_as_float(acc[q]) + __uint_as_float(part[q]));
-            }
+            for (int q = 0; q < 16; ++q)
+              acc[q] = v_stages > 1 ? __float_as_uint(__uint_as_float(acc[q]) + __uint_as_float(more[q])) : first_acc == 0 ? acc[q] : more[q];
           }
         }
+        // The accumulators are in registers: the MMAs of the tile that needs them next run beside the arithmetic and the
+        // stores below.
+        if (last) {
+          tc_fence_before();
+          __syncwarp();
+          mbar_arrive_if(&d_empty[dbuf], (lane == 0) ? 1u : 0u);
+        }
+        if (live == 0u) continue;
+        // The sixteen columns are computed side by side whether they are live or padding, and only the stores look: a
+        // branch per column kept their chains from overlapping.
         if (mode_is_gate_up(MODE)) {
           // acc = gate, more = up.  Rounding points of the reference
           // (src/xkernels/ops/moe/mxfp4_reference.py:92-100): gate_up to bf16, (+ bf16 bias, rounded),
@@ -692,54 +694,53 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           // down GEMM's dequantiser produces: element j of a group of 8 at ((j & 3) << 1) | (j >> 2).
           const int64_t col = Cfg::kLut ? n_glob   // the table path of the next GEMM reads natural K order
                                         : ((n_glob & ~int64_t(7)) | (((n_glob & 3) << 1) | ((n_glob >> 2) & 1)));
+          constexpr float kUnscale = (MODE == kModeInt4GateUp) ? Int4Scaling<kWide>::kUnscale : (Cfg::kLut ? 1.f : kMxUnscale);
+          __nv_bfloat16* out = p.act + ((int64_t)b * BT + c0) * p.N + col;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            if (!((live >> j) & 1u)) continue;          // warp-uniform
-            constexpr float kUnscale = (MODE == kModeInt4GateUp) ? Int4Scaling<kWide>::kUnscale : (Cfg::kLut ? 1.f : kMxUnscale);
             float g = round_to_bf16(__uint_as_float(acc[j]) * kUnscale);   // exact: a power of two
             float u = round_to_bf16(__uint_as_float(more[j]) * kUnscale);
             if (p.bias != nullptr) { g = round_to_bf16(g + bias0); u = round_to_bf16(u + bias1); }
             if (p.limit > 0.f) { g = fminf(g, p.limit); u = fminf(fmaxf(u, -p.limit), p.limit); }
             const float silu = g / (1.f + expf(-g));
-            p.act[((int64_t)b * BT + c0 + j) * p.N + col] = __float2bfloat16_rn(silu * u);
+            acc[j] = __float_as_uint(silu * u);
           }
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if ((live >> j) & 1u) out[(int64_t)j * p.N] = __float2bfloat16_rn(__uint_as_float(acc[j]));   // warp-uniform
         } else {
+          // INT4: x routing weight here.  MXFP4: the reference rounds `down` to bf16 and adds the bf16 bias; the combine multiplies.
+          constexpr float kUnscale = mode_is_int4(MODE) ? Int4Scaling<kWide>::kUnscale : Cfg::kLut ? 1.f : kMxUnscale;
+          auto value = [&](uint32_t a, float w, float bias) -> float {
+            float v = __uint_as_float(a) * kUnscale;   // exact: a power of two
+            if (MODE == kModeMxDown) {
+              v = round_to_bf16(v);
+              if (p.bias != nullptr) v = round_to_bf16(v + bias);
+            } else if (p.mul_w) {
+              v = w * v;
+            }
+            return v;
+          };
+          char* const base = kNarrowRows ? reinterpret_cast<char*>(p.rows16 + n_glob) : reinterpret_cast<char*>(p.scratch + n_glob);
+          const uint32_t pitch = (uint32_t)p.N * (kNarrowRows ? 2u : 4u);
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
+            const uint32_t slot = __shfl_sync(0xffffffffu, (uint32_t)cur_slot, j);
+            const float w = MODE == kModeMxDown ? 1.f : __shfl_sync(0xffffffffu, cur_w, j);
+            const float v = value(acc[j], w, bias0), v2 = mode_is_pair(MODE) ? value(more[j], w, bias1) : 0.f;
             if (!((live >> j) & 1u)) continue;          // warp-uniform
-            const int32_t slot = __shfl_sync(0xffffffffu, cur_slot, j);
-            constexpr bool kLateWeight = kWide;   // (170 against 177 us at group 128, 168 against 166 at group 32: M=64)
-            float v = __uint_as_float(acc[j]), w = kLateWeight || MODE == kModeMxDown ? 1.f : __shfl_sync(0xffffffffu, cur_w, j);
-            if (mode_is_int4(MODE)) v *= Int4Scaling<kWide>::kUnscale;   // exact: a power of two
-            if (MODE == kModeMxDown) {  // reference rounds `down` to bf16, adds the bf16 bias, then x w: the combine does that
-              v = round_to_bf16(Cfg::kLut ? v : v * kMxUnscale);
-              if (p.bias != nullptr) v = round_to_bf16(v + bias0);
+            char* out = base + (uint64_t)slot * pitch;
+            if (kNarrowRows) {
+              reinterpret_cast<__nv_bfloat16*>(out)[0] = __float2bfloat16_rn(v);
+              if (mode_is_pair(MODE)) reinterpret_cast<__nv_bfloat16*>(out)[kTileRows] = __float2bfloat16_rn(v2);   // 128 rows further down
             } else {
-              if (p.mul_w) {
-                if (kLateWeight) w = __shfl_sync(0xffffffffu, cur_w, j);
-                v = w * v;
-              }
-            }
-            if (kNarrowRows) p.rows16[(int64_t)slot * p.N + n_glob] = __float2bfloat16_rn(v);
-            else p.scratch[(int64_t)slot * p.N + n_glob] = v;
-            if (mode_is_pair(MODE)) {  // the second weight tile: rows 128 further down
-              float v2 = __uint_as_float(more[j]);
-              if (MODE == kModeInt4Pair) {
-                v2 *= Int4Scaling<kWide>::kUnscale;
-                if (p.mul_w) v2 = w * v2;
-              } else {
-                v2 = round_to_bf16(Cfg::kLut ? v2 : v2 * kMxUnscale);
-                if (p.bias != nullptr) v2 = round_to_bf16(v2 + bias1);
-              }
-              if (kNarrowRows) p.rows16[(int64_t)slot * p.N + n_glob + kTileRows] = __float2bfloat16_rn(v2);
-              else p.scratch[(int64_t)slot * p.N + n_glob + kTileRows] = v2;
+              reinterpret_cast<float*>(out)[0] = v;
+              if (mode_is_pair(MODE)) reinterpret_cast<float*>(out)[kTileRows] = v2;
             }
           }
         }
       }
-      tc_fence_before();
       __syncwarp();
-      mbar_arrive_if(&d_empty[dbuf], (lane == 0) ? 1u : 0u);
       if (mode_is_gate_up(MODE) && p.done_signal != nullptr) {
         // this warp's part of block b is written (the __syncwarp above orders the other lanes' stores
         // before lane 0's release): one count per warp and tile, 4 * kEpiWGs per tile
@@ -750,18 +751,11 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
       }
       return true;
     };
-    // Read-outs that are still due, oldest first (at most two wait at any time: a tile is read out
-    // before its accumulator set is needed again, see below).
-    struct Pending { int b, nt; uint32_t it, g0; int wait, cg; int32_t slot; float w; };
-    Pending pq0{0, 0, 0, 0, 0, 0, -1, 1.f}, pq1{0, 0, 0, 0, 0, 0, -1, 1.f};
+    // Read-outs that are still due, oldest first (at most two wait at any time, one if there is one accumulator set: a
+    // tile is read out before its set is needed again, see below).
+    struct Pending { int b, nt; uint32_t it; int wait; int32_t slot; float w; };
+    Pending pq0{0, 0, 0, 0, -1, 1.f}, pq1{0, 0, 0, 0, -1, 1.f};
     int n_pend = 0;
-    auto run_oldest = [&]() -> bool {
-      const Pending e = pq0;
-      pq0 = pq1;
-      --n_pend;
-      return run_epilogue(e.b, e.nt, e.it % Cfg::kDBuf, e.it / Cfg::kDBuf, e.g0, e.cg, e.slot, e.w);
-    };
-    uint32_t it = 0, g0 = 0;      // g0 = number of the tile's first stage
     // This group's stages are g = grp, grp + kGroups, ... whatever the tile boundaries, so its ring
     // positions advance by a fixed step per converted stage (no division in the loop).
     constexpr uint32_t kDU = (uint32_t)(kGroups * Cfg::kUnits);           // units per own-stage step
@@ -771,16 +765,47 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     uint32_t abar = u_first % Cfg::kABars, acyc = 0;                      // its barrier and the barrier ring's lap parity
     uint32_t n_own = 0;                                                   // own stages converted so far
     const uint32_t lead = (lane == 0) ? 1u : 0u;
-    uint32_t g0mod = 0;                                                   // g0 % kGroups
-    const uint32_t vsmod = (uint32_t)v_stages % kGroups;
     // (b, nt) of the tile advance with it: no division in the loop
     const int step_b = (int)gridDim.x / n_tiles, step_nt = (int)gridDim.x - step_b * n_tiles;
     int b = (int)blockIdx.x / n_tiles, nt = (int)blockIdx.x - b * n_tiles;
-    for (int t = (int)blockIdx.x; t < total_tiles; t += (int)gridDim.x, ++it, g0 += (uint32_t)v_stages,
-             b += step_b, nt += step_nt, b += (nt >= n_tiles ? 1 : 0), nt -= (nt >= n_tiles ? n_tiles : 0)) {
-      bool ok = true;
-      for (int vs = (int)(grp >= g0mod ? grp - g0mod : grp + kGroups - g0mod); vs < v_stages && ok; vs += kGroups) {
-        if (!mbar_wait(&w_full[wst], wph, guard, 5)) { ok = false; break; }
+    // One step a pass: read out the oldest tile that is due, convert the next own stage, or go on to the next tile.  (Steps
+    // of one loop, so that the code of a read-out is there once.)
+    uint32_t it = 0;
+    int t = (int)blockIdx.x, vs = (int)grp;
+    for (;;) {
+      const bool tiles_left = t < total_tiles, tile_done = vs >= v_stages;
+      // At the end of a tile, before it joins the queue: a tile must have been read out before the MMAs of the tile
+      // kDBuf further on, which re-use its accumulator set, can start.  Reading it out no later than
+      // here (before any stage of tile it + 1 is converted) keeps every converted stage consumable,
+      // so the A slots can never fill up with stages that wait for a read-out.
+      if (n_pend > 0 && (pq0.wait <= 0 || !tiles_left || (tile_done && (pq0.it + (uint32_t)Cfg::kDBuf <= it + 1u || n_pend == 2)))) {
+        const Pending e = pq0;
+        if (Cfg::kDBuf > 1) pq0 = pq1;
+        --n_pend;
+        if (guard.aborted() || !run_epilogue(e.b, e.nt, e.it, e.slot, e.w)) break;
+        continue;
+      }
+      if (!tiles_left) break;
+      if (tile_done) {
+        // is this warpgroup on read-out duty for this tile?
+        const int cg = first_group(it);
+        if (cg < Cfg::kColGroups) {
+          Pending e{b, nt, it, Cfg::kDBuf >= 2 ? kEpiDelay : 1, -1, 1.f};   // one set: the next tile's MMAs wait for it
+          load_cols(b, cg * 16, e.slot, e.w);
+          if (Cfg::kDBuf == 1 || n_pend == 0) pq0 = e; else pq1 = e;
+          ++n_pend;
+        }
+        vs -= v_stages;
+        t += (int)gridDim.x;
+        ++it;
+        b += step_b;
+        nt += step_nt;
+        if (nt >= n_tiles) { ++b; nt -= n_tiles; }
+        continue;
+      }
+      {
+        bool ok = true;
+        if (!mbar_wait(&w_full[wst], wph, guard, 5)) break;
         const uint32_t pk = s_packed_u32 + wst * kPackedStageBytes + row * 128;
         uint2 sw = make_uint2(0, 0);  // INT4: the kChunks bf16 group scales of this share; MXFP4: .x = its e8m0 bytes
         if (mode_is_int4(MODE)) {
@@ -895,30 +920,10 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         wst += kGroups; if (wst >= (uint32_t)kWStages) { wst -= kWStages; wph ^= 1u; }
         aq += kDU; if (aq >= (uint32_t)Cfg::kASlots) aq -= Cfg::kASlots;
         abar += kDU; if (abar >= (uint32_t)Cfg::kABars) { abar -= Cfg::kABars; acyc ^= 1u; }
-        // read-outs whose delay has run out
-        --pq0.wait; --pq1.wait;
-        while (n_pend > 0 && pq0.wait <= 0 && ok) ok = run_oldest();
+        vs += kGroups;
+        --pq0.wait;
+        if (Cfg::kDBuf > 1) --pq1.wait;
       }
-      if (!ok) break;
-      // Before this tile joins the queue: a tile must have been read out before the MMAs of the tile
-      // kDBuf further on, which re-use its accumulator set, can start.  Reading it out no later than
-      // here (before any stage of tile it + 1 is converted) keeps every converted stage consumable,
-      // so the A slots can never fill up with stages that wait for a read-out.
-      while (n_pend > 0 && (pq0.it + (uint32_t)Cfg::kDBuf <= it + 1u || n_pend == 2) && ok) ok = run_oldest();
-      if (!ok) break;
-      // is this warpgroup on read-out duty for this tile, and for which column group?
-      const int cg = (Cfg::kEpiWGs == Cfg::kWGs) ? wg
-                                                 : (int)(((uint32_t)wg + (uint32_t)Cfg::kWGs - (it * (uint32_t)Cfg::kColGroups) % (uint32_t)Cfg::kWGs) % (uint32_t)Cfg::kWGs);
-      if (cg < Cfg::kColGroups || Cfg::kEpiWGs == Cfg::kWGs) {
-        Pending e{b, nt, it, g0, Cfg::kDBuf >= 2 ? kEpiDelay : 1, cg, -1, 1.f};   // one set: the next tile's MMAs wait for it
-        load_cols(b, cg * 16, e.slot, e.w);
-        if (n_pend == 0) pq0 = e; else pq1 = e;
-        ++n_pend;
-      }
-      g0mod += vsmod; if (g0mod >= (uint32_t)kGroups) g0mod -= kGroups;
-    }
-    while (n_pend > 0 && !guard.aborted()) {
-      if (!run_oldest()) break;
     }
   }
 
