@@ -418,11 +418,18 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
             uint32_t top[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              float v0 = round_to_bf16(__uint_as_float(a0[j])), v1 = round_to_bf16(__uint_as_float(a1[j]));
-              if (p.bias != nullptr) { v0 = round_to_bf16(v0 + bias0); v1 = round_to_bf16(v1 + bias1); }
+              float v0 = __uint_as_float(a0[j]), v1 = __uint_as_float(a1[j]);
+              round_pair_to_bf16(v0, v1);
+              if (p.bias != nullptr) { v0 += bias0; v1 += bias1; round_pair_to_bf16(v0, v1); }
               if (p.limit > 0.f) { v0 = fminf(v0, p.limit); v1 = fminf(fmaxf(v1, -p.limit), p.limit); }
               const float silu = v0 / (1.f + expf(-v0));
-              a0[j] = __float_as_uint(round_to_bf16(silu * v1));
+              a0[j] = __float_as_uint(silu * v1);
+              if (j & 1) {
+                float x0 = __uint_as_float(a0[j - 1]), x1 = silu * v1;
+                round_pair_to_bf16(x0, x1);
+                a0[j - 1] = __float_as_uint(x0);
+                a0[j] = __float_as_uint(x1);
+              }
             }
             // this warp's 32 rows are one scale block of the next contraction
 #pragma unroll
@@ -450,13 +457,14 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           } else {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              float v0 = round_to_bf16(__uint_as_float(a0[j])), v1 = round_to_bf16(__uint_as_float(a1[j]));
-              if (p.bias != nullptr) { v0 = round_to_bf16(v0 + bias0); v1 = round_to_bf16(v1 + bias1); }
+              float v0 = __uint_as_float(a0[j]), v1 = __uint_as_float(a1[j]);
+              if (p.bias != nullptr) { round_pair_to_bf16(v0, v1); v0 += bias0; v1 += bias1; }
+              const uint32_t two = pack_bf16(v0, v1);
               const int32_t slot = __shfl_sync(0xffffffffu, my_slot, j);
               if (!((live >> j) & 1u)) continue;        // warp-uniform
               __nv_bfloat16* out = p.rows + (int64_t)slot * p.N + n_glob;
-              out[0] = __float2bfloat16_rn(v0);         // exact: rounded above
-              out[kRows] = __float2bfloat16_rn(v1);
+              out[0] = low_bf16(two);
+              out[kRows] = high_bf16(two);
             }
           }
         }

@@ -698,44 +698,59 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           __nv_bfloat16* out = p.act + ((int64_t)b * BT + c0) * p.N + col;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            float g = round_to_bf16(__uint_as_float(acc[j]) * kUnscale);   // exact: a power of two
-            float u = round_to_bf16(__uint_as_float(more[j]) * kUnscale);
-            if (p.bias != nullptr) { g = round_to_bf16(g + bias0); u = round_to_bf16(u + bias1); }
+            float g = __uint_as_float(acc[j]) * kUnscale, u = __uint_as_float(more[j]) * kUnscale;   // exact: a power of two
+            round_pair_to_bf16(g, u);
+            if (p.bias != nullptr) { g += bias0; u += bias1; round_pair_to_bf16(g, u); }
             if (p.limit > 0.f) { g = fminf(g, p.limit); u = fminf(fmaxf(u, -p.limit), p.limit); }
             const float silu = g / (1.f + expf(-g));
             acc[j] = __float_as_uint(silu * u);
           }
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if ((live >> j) & 1u) out[(int64_t)j * p.N] = __float2bfloat16_rn(__uint_as_float(acc[j]));   // warp-uniform
+          for (int j = 0; j < 16; j += 2) {
+            const uint32_t two = pack_bf16(__uint_as_float(acc[j]), __uint_as_float(acc[j + 1]));
+            if ((live >> j) & 1u) out[(int64_t)j * p.N] = low_bf16(two);   // warp-uniform
+            if ((live >> (j + 1)) & 1u) out[(int64_t)(j + 1) * p.N] = high_bf16(two);
+          }
         } else {
-          // INT4: x routing weight here.  MXFP4: the reference rounds `down` to bf16 and adds the bf16 bias; the combine multiplies.
           constexpr float kUnscale = mode_is_int4(MODE) ? Int4Scaling<kWide>::kUnscale : Cfg::kLut ? 1.f : kMxUnscale;
-          auto value = [&](uint32_t a, float w, float bias) -> float {
-            float v = __uint_as_float(a) * kUnscale;   // exact: a power of two
-            if (MODE == kModeMxDown) {
-              v = round_to_bf16(v);
-              if (p.bias != nullptr) v = round_to_bf16(v + bias);
-            } else if (p.mul_w) {
-              v = w * v;
-            }
-            return v;
-          };
+          // INT4: x routing weight here.  MXFP4: the reference rounds `down` to bf16 and adds the bf16 bias; the combine multiplies.
           char* const base = kNarrowRows ? reinterpret_cast<char*>(p.rows16 + n_glob) : reinterpret_cast<char*>(p.scratch + n_glob);
           const uint32_t pitch = (uint32_t)p.N * (kNarrowRows ? 2u : 4u);
+          auto row = [&](uint32_t slot) -> char* { return base + (uint64_t)slot * pitch; };
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const uint32_t slot = __shfl_sync(0xffffffffu, (uint32_t)cur_slot, j);
-            const float w = MODE == kModeMxDown ? 1.f : __shfl_sync(0xffffffffu, cur_w, j);
-            const float v = value(acc[j], w, bias0), v2 = mode_is_pair(MODE) ? value(more[j], w, bias1) : 0.f;
-            if (!((live >> j) & 1u)) continue;          // warp-uniform
-            char* out = base + (uint64_t)slot * pitch;
-            if (kNarrowRows) {
-              reinterpret_cast<__nv_bfloat16*>(out)[0] = __float2bfloat16_rn(v);
-              if (mode_is_pair(MODE)) reinterpret_cast<__nv_bfloat16*>(out)[kTileRows] = __float2bfloat16_rn(v2);   // 128 rows further down
-            } else {
-              reinterpret_cast<float*>(out)[0] = v;
-              if (mode_is_pair(MODE)) reinterpret_cast<float*>(out)[kTileRows] = v2;
+          for (int j = 0; j < 16; j += 2) {
+            float v[2] = {__uint_as_float(acc[j]) * kUnscale, __uint_as_float(acc[j + 1]) * kUnscale};   // exact: a power of two
+            float v2[2] = {0.f, 0.f};
+            if (mode_is_pair(MODE)) { v2[0] = __uint_as_float(more[j]) * kUnscale; v2[1] = __uint_as_float(more[j + 1]) * kUnscale; }
+            if (mode_is_int4(MODE) && p.mul_w) {
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                const float w = __shfl_sync(0xffffffffu, cur_w, j + q);
+                v[q] *= w;
+                v2[q] *= w;
+              }
+            }
+            if (MODE == kModeMxDown && p.bias != nullptr) {
+              round_pair_to_bf16(v[0], v[1]);
+              round_pair_to_bf16(v2[0], v2[1]);
+              v[0] += bias0; v[1] += bias0;
+              v2[0] += bias1; v2[1] += bias1;
+            }
+            const uint32_t two = kNarrowRows ? pack_bf16(v[0], v[1]) : 0u, two2 = kNarrowRows ? pack_bf16(v2[0], v2[1]) : 0u;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              const uint32_t slot = __shfl_sync(0xffffffffu, (uint32_t)cur_slot, j + q);
+              if (!((live >> (j + q)) & 1u)) continue;          // warp-uniform
+              // the second row tile's rows are 128 further down
+              if (kNarrowRows) {
+                __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(row(slot));
+                out[0] = q == 0 ? low_bf16(two) : high_bf16(two);
+                if (mode_is_pair(MODE)) out[kTileRows] = q == 0 ? low_bf16(two2) : high_bf16(two2);
+              } else {
+                float* out = reinterpret_cast<float*>(row(slot));
+                out[0] = v[q];
+                if (mode_is_pair(MODE)) out[kTileRows] = v2[q];
+              }
             }
           }
         }
