@@ -447,17 +447,17 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
   if (rc != XKB_OK) return rc;
   if (use_bs) {
     const __nv_bfloat16* rows = nullptr;
-    // batches of more than 48 slots per expert report scale bytes 191..254, as they always have
-    rc = launch_mxfp4_bs(A, w13, w13_scale, w2, w2_scale, b13, b2, r, hidden, ispp, E, top_k, swiglu_limit,
-                         mxfp4_tc_block(numel, E) == 128, bs_ws, rb.status, &rows, stream);
+    rc = launch_mxfp4_bs(A, w13, w13_scale, w2, w2_scale, b13, b2, r, hidden, ispp, E, top_k, swiglu_limit, bs_ws, rb.status,
+                         &rows, stream);
     if (rc != XKB_OK) return rc;
     return launch_combine_bf16(rows, mul_routed_weight ? topk_w : nullptr, topk_ids, expert_map, num_map, E, out,
                                a_dtype, M, top_k, hidden, stream);
   }
   if (use_tc) {
     __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(scratch);
-    rc = launch_mxfp4_tc(A, w13, w13_scale, w2, w2_scale, b13, b2, r, act, rows, hidden, ispp, E, top_k, swiglu_limit, tc_ws,
-                         rb.status, stream);
+    const int check_scale = numel > 48 * (int64_t)E;   // these batches report scale bytes 191..254, as they always have
+    rc = launch_mxfp4_tc(A, w13, w13_scale, w2, w2_scale, b13, b2, r, act, rows, hidden, ispp, E, top_k, swiglu_limit,
+                         check_scale, tc_ws, rb.status, stream);
     if (rc != XKB_OK) return rc;
     return launch_combine_bf16(rows, mul_routed_weight ? topk_w : nullptr, topk_ids, expert_map, num_map, E, out,
                                a_dtype, M, top_k, hidden, stream);

@@ -63,8 +63,8 @@ int mxfp4_bs_block(int64_t numel, int E);
 int64_t mxfp4_bs_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, int E);
 int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale, const uint8_t* w2,
                     const uint8_t* w2_scale, const void* b13, const void* b2, const Routing& r, int64_t hidden,
-                    int64_t ispp, int E, int top_k, float limit, int check_scale, void* ws, int* status,
-                    const __nv_bfloat16** rows, cudaStream_t stream);
+                    int64_t ispp, int E, int top_k, float limit, void* ws, int* status, const __nv_bfloat16** rows,
+                    cudaStream_t stream);
 
 bool mxfp4_tc_supported(int a_dtype, int64_t M, int64_t hidden, int64_t ispp, int E, int top_k);
 int mxfp4_tc_block(int64_t numel, int E);
@@ -72,6 +72,6 @@ int64_t mxfp4_tc_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, in
 int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale, const uint8_t* w2,
                     const uint8_t* w2_scale, const void* b13, const void* b2, const Routing& r,
                     __nv_bfloat16* act, __nv_bfloat16* rows16, int64_t hidden, int64_t ispp, int E, int top_k,
-                    float limit, void* tc_ws, int* status, cudaStream_t stream);   // rows before the routing weight, in bf16
+                    float limit, int check_scale, void* tc_ws, int* status, cudaStream_t stream);   // rows before the routing weight, in bf16
 
 }  // namespace xkb

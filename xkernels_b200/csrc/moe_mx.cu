@@ -4,14 +4,14 @@
 // nibbles into the byte containers the instruction reads, and nothing converts them.  The activations are
 // bf16 and go in as three block-scaled 8-bit terms that hold every element down to 2^-31 of the largest of its
 // 32 exactly (mx_split.cuh).  What bounds the kernel is the weight stream; there is no conversion beside it.
-// Prefill-sized batches stay on the kernel that converts to bf16 (moe_tc.cu): three terms are half as many token
-// bytes again as bf16 activations, and from L2 they bound wide tiles (mxfp4_bs_block has the line).
+// Larger batches stay on the kernel that converts to bf16 (moe_tc.cu): three terms are half as many token
+// bytes again as bf16 activations, and half as many multiplications at twice the rate (mxfp4_bs_block has the line).
 //
 // Swap-AB like the bf16 kernel: a tile is BT tokens of one expert block x two 128-row weight tiles (gate and
 // up rows, or two neighbouring row tiles of the down projection).  One persistent CTA per SM, sixteen warps:
 //   warp 0      weight producer: per 128-K stage two [128 x 128] tiles, per four stages their scales
-//   warps 1, 2  MMA issuers, one per weight matrix.  One thread issues a narrow MMA per 45 cycles at best, so token
-//               tiles up to 32 multiply the three terms in one instruction of 3 BT tokens (four a stage): M=48 below
+//   warps 1, 2  MMA issuers, one per weight matrix.  One thread issues a narrow MMA per 45 cycles at best, so
+//               the three terms are multiplied in one instruction of 3 BT tokens (four a stage): M=48 below
 //               184 us with the terms on two issuers, 168 on three, 144 in one instruction.
 //   warp 3      token producer (the terms of the stage, per four stages their scales)
 //   warps 4-7   scale movers: the scale tiles are row-major, the instruction wants row r of a 128-row tile in
@@ -46,29 +46,25 @@ constexpr int kTerms = 3;             // of an activation: hi, mid, lo
 constexpr int kThreads = 512;
 constexpr int kTmemCols = 512;
 constexpr uint32_t kProdSleepNs = 200;
-constexpr int kErrMxScaleRange = 2;
-constexpr uint32_t kMxMaxScale = 190;
 
 template <int BT> struct MxCfg {
-  static_assert(BT % 16 == 0 && BT <= 64, "token tile");
-  // Narrow tiles multiply all three terms in ONE instruction: the terms' tiles lie behind one another in shared
+  static_assert(BT == 16 || BT == 32, "token tile");
+  // All three terms are multiplied in ONE instruction: the terms' tiles lie behind one another in shared
   // memory, which is a tile of 3 BT tokens, each term with accumulators of its own that the read-out adds up.  An
-  // instruction costs its issuer 45 cycles up to 32 tokens or so, whatever its width.  Wider tiles have no room for the
-  // accumulators and issue three instructions into one.
-  static constexpr bool kMerged = BT <= 32;
-  static constexpr int kMmaTokens = kMerged ? kTerms * BT : BT;       // UMMA N
+  // instruction costs its issuer 45 cycles up to 32 tokens or so, whatever its width.
+  static constexpr int kMmaTokens = kTerms * BT;                      // UMMA N
   static constexpr int kTokRowGroups = (kMmaTokens + 31) / 32;
   static constexpr int kTokBytes = BT * kStageK;                      // one term
   static_assert(kTokBytes % 1024 == 0, "swizzle atoms");
   static constexpr int kStageBytes = 2 * kWBytes + kTerms * kTokBytes;
-  static constexpr int kStages = BT <= 16 ? 5 : BT <= 32 ? 4 : 3;
+  static constexpr int kStages = BT <= 16 ? 5 : 4;
   // Scale tiles are loaded with the first stage of their four and read with all four: a slot is free again
   // when the MMAs kStages before that first stage are done, if kStages <= 4 * slots - 3.
   static constexpr int kScSlots = 2;
   static_assert(kStages <= 4 * kScSlots - 3, "scale slots");
   static constexpr int kScBytes = 2 * kRows * 16 + BT * 16;
-  // columns: accumulator sets of two matrices, then per stage 4 gate + 4 up + 4 scale columns a token operand
-  static constexpr int kScStageCols = 8 + 4 * (kMerged ? 1 : kTerms);
+  // columns: accumulator sets of two matrices, then per stage 4 gate + 4 up + 4 token scale columns
+  static constexpr int kScStageCols = 12;
   static constexpr int kScCols = kScStageCols * kStages;
   static constexpr int kSetCols = 2 * kMmaTokens;                     // accumulators of matrix 1 behind those of matrix 0
   static constexpr int kDFit = (kTmemCols - kScCols) / kSetCols;
@@ -99,7 +95,6 @@ struct MxParams {
   int mat_row;                  // rows between the two matrices of a tile
   int tile_step;                // output rows per tile: 128 gate_up, 256 down
   float limit;                  // SwiGLU clamp, <= 0 disables
-  int check_scale;              // record scale bytes 191..254 (status 2)
   int max_blocks, num_experts;
   int32_t* done_signal;         // gate_up: finished read-outs per token block
   const int32_t* done_wait;     // down: the same, waited for
@@ -265,18 +260,11 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           tc_fence_after();
           const uint32_t s = smem_u32(smem + st * Cfg::kStageBytes);
           const uint64_t a = umma_desc_k_sw128(s + mat * kWBytes);
-          const uint64_t bh = umma_desc_k_sw128(s + 2 * kWBytes), bm = umma_desc_k_sw128(s + 2 * kWBytes + Cfg::kTokBytes),
-                         bl = umma_desc_k_sw128(s + 2 * kWBytes + 2 * Cfg::kTokBytes);
+          const uint64_t bt = umma_desc_k_sw128(s + 2 * kWBytes);
           const uint32_t sc = tmem_base + Cfg::kScCol0 + st * Cfg::kScStageCols, sw = sc + mat * 4;
           // 32 K each: 32 bytes on in the swizzled rows, the next scale byte
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            umma_mx(d, a + k * 2, bh + k * 2, mx_idesc(Cfg::kMmaTokens, k), sw, sc + 8, (ks | k) != 0);
-            if (!Cfg::kMerged) {
-              umma_mx(d, a + k * 2, bm + k * 2, mx_idesc(BT, k), sw, sc + 12, 1u);
-              umma_mx(d, a + k * 2, bl + k * 2, mx_idesc(BT, k), sw, sc + 16, 1u);
-            }
-          }
+          for (int k = 0; k < 4; ++k) umma_mx(d, a + k * 2, bt + k * 2, mx_idesc(Cfg::kMmaTokens, k), sw, sc + 8, (ks | k) != 0);
           tc_commit(&empty[st]);
           if (++st == kStages) { st = 0; ph ^= 1; }
         }
@@ -334,11 +322,6 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
               }
               asm volatile("fence.proxy.async;" ::: "memory");   // the MMAs read the cleared weights
             }
-            if (p.check_scale) {
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-                if (c == quarter && __vcmpgtu4(v[c], kMxMaxScale * 0x01010101u) != 0) atomicCAS(p.status, 0, kErrMxScaleRange);
-            }
             tmem_st_32x4(dst + m * 4, v[0], v[1], v[2], v[3]);
           }
           uint32_t v[4] = {0, 0, 0, 0};
@@ -346,18 +329,12 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           for (int c = 0; c < Cfg::kTokRowGroups; ++c) v[c] = word_of(x[c], j);
           // hi's bytes are kLoShift at least (padding positions hold anything: their columns are never read)
           constexpr uint32_t kMid4 = mx::kMidShift * 0x01010101u, kLo4 = mx::kLoShift * 0x01010101u;
-          if (Cfg::kMerged) {
 #pragma unroll
-            for (int c = 0; c < Cfg::kTokRowGroups; ++c) {
-              const int term = (c * 32 + lane) / BT;
-              v[c] = __vsub4(v[c], term == 0 ? 0u : term == 1 ? kMid4 : kLo4);
-            }
-            tmem_st_32x4(dst + 8, v[0], v[1], v[2], v[3]);
-          } else {
-            tmem_st_32x4(dst + 8, v[0], v[1], v[2], v[3]);
-            tmem_st_32x4(dst + 12, __vsub4(v[0], kMid4), __vsub4(v[1], kMid4), __vsub4(v[2], kMid4), __vsub4(v[3], kMid4));
-            tmem_st_32x4(dst + 16, __vsub4(v[0], kLo4), __vsub4(v[1], kLo4), __vsub4(v[2], kLo4), __vsub4(v[3], kLo4));
+          for (int c = 0; c < Cfg::kTokRowGroups; ++c) {
+            const int term = (c * 32 + lane) / BT;
+            v[c] = __vsub4(v[c], term == 0 ? 0u : term == 1 ? kMid4 : kLo4);
           }
+          tmem_st_32x4(dst + 8, v[0], v[1], v[2], v[3]);
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
@@ -400,7 +377,7 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           tmem_ld_32x16(d + Cfg::kMmaTokens, a1);
           tmem_wait_ld();
 #pragma unroll
-          for (int i = 1; i < (Cfg::kMerged ? kTerms : 1); ++i) {
+          for (int i = 1; i < kTerms; ++i) {
             uint32_t b0[16], b1[16];
             tmem_ld_32x16(d + i * BT, b0);
             tmem_ld_32x16(d + Cfg::kMmaTokens + i * BT, b1);
@@ -596,7 +573,6 @@ int launch_mx_by_block(int block, const CUtensorMap (&tm)[6], const MxParams& pr
   switch (block) {
     case 16: return launch_mx<16, GATE_UP>(tm, prm, max_tiles, stream);
     case 32: return launch_mx<32, GATE_UP>(tm, prm, max_tiles, stream);
-    case 64: return launch_mx<64, GATE_UP>(tm, prm, max_tiles, stream);
     default: return fail(XKB_ERR_ARG, "mxfp4 block-scaled path: unsupported token tile %d", block);
   }
 }
@@ -642,15 +618,14 @@ bool mxfp4_bs_supported(const void* w13, const void* w2, const void* s13, const 
 }
 
 // A narrower tile is taken while a block still holds nearly every expert's slots (an expert that needs a second block
-// streams its weights twice); 0 = the bf16 kernel's 128-token tiles, whose tokens are 2 bytes and not 3.  Whole
-// calls in a graph, E=256, hidden 4096, ispp 512 / E=128, 4096, 1024 / E=64, 2048, 1024:
-//   16 against 32 tokens  241 / 241 us at 11 slots per expert, 259 / 247 at 14; 222 / 227 at 12; 73 / 80 at 12
-//   32 against 64         323 / 362 at 30, 398 / 374 at 36; 282 / 348 at 28, 403 / 355 at 40; 95 / 111 at 28, 123 / 115 at 40
-//   64 against bf16       484 / 500 at 54, 525 / 526 at 60; 422 / 451 at 56, 527 / 459 at 64; 126 / 133 at 56, 158 / 138 at 64
-// (96-token tiles, the widest that fit: 537 / 565 at 66, but 495 / 459 and 138 / 138 at 64; left out.)
+// streams its weights twice); 0 = the bf16 kernel's 128-token tiles, whose tokens are 2 bytes and not 3 and which multiply
+// a block's slots only.  Whole calls in a loop, us at 16 / 32 / bf16; E=256, hidden 4096, ispp 512: 232 / 261 / 331 at 7
+// slots per expert, 261 / 276 / 333 at 12, 370 / 294 / 352 at 19, 447 / 334 / 370 at 26, 513 / 424 / 391 at 33; E=128, 4096,
+// 1024: 389 / 302 / 346 at 25, 514 / 444 / 373 at 38; E=64, 2048, 1024: 82 / 84 / 104 at 14, 120 / 99 / 109 at 28.  (64-token
+// tiles of this kernel took 10 to 20 % longer than the bf16 kernel from 26 slots on: 417 us at 26, 430 at 33, 449 / 411 at 40.)
 int mxfp4_bs_block(int64_t numel, int E) {
   const double avg = (double)numel / (E > 0 ? E : 1);
-  return avg <= 12 ? 16 : avg <= 32 ? 32 : avg <= 56 ? 64 : 0;
+  return avg <= 12 ? 16 : avg <= 28 ? 32 : 0;
 }
 
 int64_t mxfp4_bs_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, int E) {
@@ -663,8 +638,8 @@ int64_t mxfp4_bs_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, in
 
 int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale, const uint8_t* w2,
                     const uint8_t* w2_scale, const void* b13, const void* b2, const Routing& r, int64_t hidden,
-                    int64_t ispp, int E, int top_k, float limit, int check_scale, void* ws, int* status,
-                    const __nv_bfloat16** rows_out, cudaStream_t stream) {
+                    int64_t ispp, int E, int top_k, float limit, void* ws, int* status, const __nv_bfloat16** rows_out,
+                    cudaStream_t stream) {
   Carver carve(ws);
   const MxBuffers buf = carve_mx(carve, r.numel, r.max_pad, hidden, ispp);
   *rows_out = buf.rows;
@@ -702,7 +677,6 @@ int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   prm.num_post = r.num_post;
   prm.status = status;
   prm.numel = r.numel;
-  prm.check_scale = check_scale;
   prm.max_blocks = (int)r.max_blocks;
   prm.num_experts = E;
   prm.bias = static_cast<const __nv_bfloat16*>(b13);

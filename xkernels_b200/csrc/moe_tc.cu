@@ -226,6 +226,7 @@ struct TcParams {
   const __nv_bfloat16* bias;    // b13 [E, 2*ispp] or b2 [E, hidden] or nullptr
   __nv_bfloat16* act;           // gate_up mode output: [positions, N] bf16 in the K-permuted order
   int rows_per_expert;          // 2*ispp (gate_up) or hidden (down)
+  int check_scale;              // report scale bytes 191..254
   float limit;                  // SwiGLU clamp, <= 0 disables
   // Two GEMMs of one expert layer that overlap (see "block hand-over" at the kernel): the first
   // counts the finished read-outs of every token block in done_signal, the second waits until the
@@ -298,21 +299,24 @@ __device__ __forceinline__ uint32_t wide_pair(uint32_t x, uint32_t scale2) { ret
 // The three magnitude bits (e1 e0 m) placed at bf16 bits 8..6 read as  e2m1 * 2^-126  (the code
 // 0b001 = 0.5 lands on the bf16 subnormal 2^-127), the sign bit goes to bit 15.  One bf16 multiply
 // by a power of two then gives the weight exactly.  The true factor 2^126 * 2^(s-127) does not fit
-// bf16 for s > 128, so all weights are kept 2^-62 smaller than they are: the factor is 2^(s-63),
-// a bf16 number for every e8m0 byte up to 190, and the epilogue multiplies the fp32 accumulators
-// by 2^62, which is exact.  s = 0xFF decodes to 0 like in the reference
-// (src/xkernels/ops/gather/mxfp4.py:60-66).  Exact for 57 <= s <= 190 (weights of magnitude
-// 2^-70 ... 2^63 and above 2^-134 after scaling); smaller scales land on bf16 subnormals and lose
-// bits far below anything an output can show; a scale byte in 191..254 (weights of 2^64 and
-// more) is reported through the status word instead of being converted.
-constexpr int kMxShift = 62;
-constexpr float kMxUnscale = 4611686018427387904.f;   // 2^62
+// bf16 for s > 128, so all weights are kept 2^-5 smaller than they are, which still holds the smallest one (0.5 * 2^-127)
+// exactly, and the epilogue multiplies the fp32 accumulators by 2^5.  One multiplication takes every byte up to 133
+// (weights of 2^6 and more); a warp that meets a larger one converts that stage with two, e2m1 first and
+// 2^(s - 132) then.  s = 0xFF decodes to 0 like in the reference
+// (src/xkernels/ops/gather/mxfp4.py:60-66).  Batches of more than 48 slots per expert report bytes of 191..254 (weights
+// of 2^64 and more) through the status word, as they did when their conversion did not take them.
+constexpr int kMxShift = 5;
+constexpr float kMxUnscale = 32.f;                   // 2^5
+constexpr uint32_t kMxOneMul = 128 + kMxShift;       // the largest byte that one multiplication takes
 constexpr uint32_t kMxMaxScale = 190;
 constexpr int kErrMxScaleRange = 2;                  // status code: an e8m0 scale byte in 191..254
-__device__ __forceinline__ uint32_t mx_scale_factor(uint32_t s) {
-  // exponent field of 2^(s - 1 - kMxShift), twice; 0 for the NaN code
-  const uint32_t f = (s + (uint32_t)(126 - kMxShift)) * 0x00800080u;
-  return s == 0xFFu ? 0u : f;
+__device__ __forceinline__ uint32_t mx_scale_factor(uint32_t s) {   // 2^(s - 1 - kMxShift), twice; s <= kMxOneMul
+  return (s + (uint32_t)(126 - kMxShift)) * 0x00800080u;
+}
+constexpr uint32_t kMxE2m1 = 0x7E807E80u;            // 2^126, twice: makes the e2m1 value of the bits
+__device__ __forceinline__ uint32_t mx_far_factor(uint32_t s) {     // 2^(s - 127 - kMxShift), twice, for any s; 0 for the NaN code
+  const uint32_t f = s > kMxShift ? (s - kMxShift) << 7 : 1u << (s + 6 - kMxShift);   // subnormal: multiples of 2^-133
+  return s == 0xFFu ? 0u : f * 0x00010001u;
 }
 __device__ __forceinline__ uint32_t mx_pair(uint32_t mag_shifted, uint32_t sign_shifted, uint32_t c) {
   uint32_t t;
@@ -848,6 +852,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         __syncwarp();
         mbar_arrive_if(&w_empty[wst], lead);
         // kWideGroups: a scale of this warp may be out of the multipliers' range (never for sane weights)
+        const bool far = !mode_is_int4(MODE) && !Cfg::kLut && __any_sync(0xffffffffu, __vcmpgtu4(sw.x, kMxOneMul * 0x01010101u) != 0);   // MXFP4: likewise
         const bool subtract = kWide && __any_sync(0xffffffffu, ((sw.x | sw.y) & kWideLimit) != 0);
 #pragma unroll
         for (int pu = 0; pu < Cfg::kPartUnits; ++pu) {
@@ -914,14 +919,26 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
                 }
                 continue;
               }
-              if (sb > kMxMaxScale && sb != 0xFFu) atomicCAS(p.status, 0, kErrMxScaleRange);   // never taken for sane weights
-              const uint32_t cf = mx_scale_factor(sb);
+              if (!far) {
+                const uint32_t cf = mx_scale_factor(sb);
 #pragma unroll
-              for (int wp = 0; wp < 2; ++wp) {
-                uint32_t r[8];
-                mx_word(words[2 * wp], cf, r[0], r[1], r[2], r[3]);
-                mx_word(words[2 * wp + 1], cf, r[4], r[5], r[6], r[7]);
-                tmem_st_32x8(dst + uc * 16 + wp * 8, r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7]);
+                for (int wp = 0; wp < 2; ++wp) {
+                  uint32_t r[8];
+                  mx_word(words[2 * wp], cf, r[0], r[1], r[2], r[3]);
+                  mx_word(words[2 * wp + 1], cf, r[4], r[5], r[6], r[7]);
+                  tmem_st_32x8(dst + uc * 16 + wp * 8, r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7]);
+                }
+              } else {
+                if (p.check_scale && sb > kMxMaxScale && sb != 0xFFu) atomicCAS(p.status, 0, kErrMxScaleRange);
+                const uint32_t c2 = mx_far_factor(sb);
+#pragma unroll
+                for (int wp = 0; wp < 2; ++wp) {
+                  uint32_t r[8];
+                  mx_word(words[2 * wp], kMxE2m1, r[0], r[1], r[2], r[3]);
+                  mx_word(words[2 * wp + 1], kMxE2m1, r[4], r[5], r[6], r[7]);
+                  tmem_st_32x8(dst + uc * 16 + wp * 8, bf2_mul(r[0], c2), bf2_mul(r[1], c2), bf2_mul(r[2], c2), bf2_mul(r[3], c2),
+                               bf2_mul(r[4], c2), bf2_mul(r[5], c2), bf2_mul(r[6], c2), bf2_mul(r[7], c2));
+                }
               }
             }
           }
@@ -1300,6 +1317,7 @@ int launch_int4_tc(const void* A, const int32_t* packed, const void* scale, cons
   prm.bias = nullptr;
   prm.act = nullptr;
   prm.rows_per_expert = (int)N;
+  prm.check_scale = 0;
   prm.limit = 0.f;
   prm.done_signal = nullptr;
   prm.done_wait = nullptr;
@@ -1357,6 +1375,7 @@ int launch_int4_ffn_tc(const void* A, const int32_t* w13, const void* s13, const
   prm.max_blocks = (int)r.max_blocks;
   prm.num_experts = E;
   prm.bias = nullptr;
+  prm.check_scale = 0;
   prm.group_shift = log2_of(group);
   prm.limit = limit;
   // gate_up + SwiGLU -> act
@@ -1400,10 +1419,9 @@ bool mxfp4_tc_supported(int a_dtype, int64_t M, int64_t hidden, int64_t ispp, in
 }
 
 int mxfp4_tc_block(int64_t numel, int E) {
-  // decode-sized batches: token tiles of 16; prefill-sized ones: 128 (gate and up then get one
-  // MMA issuer each, like the row-tile pairs of the INT4 wide mode)
+  // decode-sized batches whose weights the block-scaled kernel cannot read: token tiles of 16; the line as at mxfp4_bs_block
   const double avg = (double)numel / (E > 0 ? E : 1);
-  return avg <= 48 ? 16 : 128;
+  return avg <= 28 ? 16 : 128;
 }
 
 int64_t mxfp4_tc_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, int E) {
@@ -1414,7 +1432,7 @@ int64_t mxfp4_tc_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, in
 int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale, const uint8_t* w2,
                     const uint8_t* w2_scale, const void* b13, const void* b2, const Routing& r,
                     __nv_bfloat16* act, __nv_bfloat16* rows16, int64_t hidden, int64_t ispp, int E, int top_k,
-                    float limit, void* tc_ws, int* status, cudaStream_t stream) {
+                    float limit, int check_scale, void* tc_ws, int* status, cudaStream_t stream) {
   XKB_REQUIRE(r.block == 16 || r.block == 128, "mxfp4 tcgen05 path: unsupported token tile %d", r.block);
   XKB_REQUIRE(reinterpret_cast<uintptr_t>(w13_scale) % 16 == 0 && reinterpret_cast<uintptr_t>(w2_scale) % 16 == 0,
               "mxfp4 tcgen05 path: scale tensors must be 16-byte aligned");
@@ -1453,6 +1471,7 @@ int launch_mxfp4_tc(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   prm.max_blocks = (int)r.max_blocks;
   prm.num_experts = E;
   prm.mul_w = 0;
+  prm.check_scale = check_scale;
   prm.group_shift = 5;
   prm.rows16 = nullptr;
   prm.limit = limit;
