@@ -784,6 +784,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     uint32_t abar = u_first % Cfg::kABars, acyc = 0;                      // its barrier and the barrier ring's lap parity
     uint32_t n_own = 0;                                                   // own stages converted so far
     const uint32_t lead = (lane == 0) ? 1u : 0u;
+    const uint32_t zero = gridDim.z - 1u;                                 // 0, which the compiler does not know
     // (b, nt) of the tile advance with it: no division in the loop
     const int step_b = (int)gridDim.x / n_tiles, step_nt = (int)gridDim.x - step_b * n_tiles;
     int b = (int)blockIdx.x / n_tiles, nt = (int)blockIdx.x - b * n_tiles;
@@ -846,11 +847,14 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         uint4 w4[kChunks];
 #pragma unroll
         for (int c = 0; c < kChunks; ++c) w4[c] = lds128(pk + ((chunk_of(c) ^ (row & 7)) << 4));
-        // This warp's share of the stage is in registers (the shared-memory unit executes a warp's
-        // loads and the arrive in order, and the arrive has release semantics): one arrival per warp
-        // of the group hands the stage back to the producer.
+        // One arrival per warp of the group hands the stage back to the producer, once this warp's share of it is in
+        // registers: the arrive takes a value computed from every load, so that it is not issued while a load is still
+        // queued behind the tensor cores' reads of shared memory.
+        uint32_t landed = sw.x | sw.y;
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) landed |= w4[c].x;
         __syncwarp();
-        mbar_arrive_if(&w_empty[wst], lead);
+        mbar_arrive_if(&w_empty[wst], lead | (landed & zero));
         // kWideGroups: a scale of this warp may be out of the multipliers' range (never for sane weights)
         const bool far = !mode_is_int4(MODE) && !Cfg::kLut && __any_sync(0xffffffffu, __vcmpgtu4(sw.x, kMxOneMul * 0x01010101u) != 0);   // MXFP4: likewise
         const bool subtract = kWide && __any_sync(0xffffffffu, ((sw.x | sw.y) & kWideLimit) != 0);
