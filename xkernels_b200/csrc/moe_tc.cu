@@ -847,14 +847,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         uint4 w4[kChunks];
 #pragma unroll
         for (int c = 0; c < kChunks; ++c) w4[c] = lds128(pk + ((chunk_of(c) ^ (row & 7)) << 4));
-        // One arrival per warp of the group hands the stage back to the producer, once this warp's share of it is in
-        // registers: the arrive takes a value computed from every load, so that it is not issued while a load is still
-        // queued behind the tensor cores' reads of shared memory.
         uint32_t landed = sw.x | sw.y;
 #pragma unroll
         for (int c = 0; c < kChunks; ++c) landed |= w4[c].x;
-        __syncwarp();
-        mbar_arrive_if(&w_empty[wst], lead | (landed & zero));
         // kWideGroups: a scale of this warp may be out of the multipliers' range (never for sane weights)
         const bool far = !mode_is_int4(MODE) && !Cfg::kLut && __any_sync(0xffffffffu, __vcmpgtu4(sw.x, kMxOneMul * 0x01010101u) != 0);   // MXFP4: likewise
         const bool subtract = kWide && __any_sync(0xffffffffu, ((sw.x | sw.y) & kWideLimit) != 0);
@@ -866,6 +861,14 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
             const bool same_lap = abar + uo >= (uint32_t)Cfg::kASlots;
             const uint32_t eb = same_lap ? abar + uo - Cfg::kASlots : abar + uo + Cfg::kABars - Cfg::kASlots;
             if (!mbar_wait(&a_empty[eb], same_lap ? acyc : (acyc ^ 1u), guard, 6)) { ok = false; break; }
+          }
+          if (pu == 0) {
+            // One arrival per warp of the group hands the stage back to the producer, once this warp's share of it is in
+            // registers: the arrive takes a value computed from every load, so that it is not issued while a load is still
+            // queued behind the tensor cores' reads of shared memory.  (Behind the wait for the slot, during which the
+            // loads land: in front of it the loads' latency was in the way, M=1 42.5 -> 41.5 us.)
+            __syncwarp();
+            mbar_arrive_if(&w_empty[wst], lead | (landed & zero));
           }
           tc_fence_after();
           const uint32_t dst = tmem_base + lane_base + Cfg::kACol0 + (aq + uo) * Cfg::kUnitCols;
