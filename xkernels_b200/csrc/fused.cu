@@ -69,7 +69,7 @@ struct RoutingBuffers {
 // may pick: the longest sorted_ids (largest block) and the most blocks
 // (smallest block).
 constexpr int kMaxBlock = 256;
-constexpr int kMinBlock = 16;
+constexpr int kMinBlock = 8;
 
 int64_t routing_max_pad(int64_t numel, int E, int block) {
   return numel + (int64_t)(E + 1) * (block - 1);

@@ -12,7 +12,7 @@
 //   warp 0      weight producer: per 128-K stage two [128 x 128] tiles, per four stages their scales
 //   warps 1, 2  MMA issuers, one per weight matrix.  One thread issues a narrow MMA per 45 cycles at best, so
 //               the three terms are multiplied in one instruction of 3 BT tokens (four a stage): M=48 below
-//               184 us with the terms on two issuers, 168 on three, 144 in one instruction.
+//               184 us with the terms on two issuers, 168 on three, 144 in one instruction (16-token tiles).
 //   warp 3      token producer (the terms of the stage, per four stages their scales)
 //   warps 4-7   scale movers: the scale tiles are row-major, the instruction wants row r of a 128-row tile in
 //               lane r % 32, column r / 32 of tensor memory, the same in all four lane quarters.  Sixteen
@@ -21,7 +21,7 @@
 //   warps 8-15  read-out, a tile behind the MMAs (two to four accumulator sets)
 //
 // Measured at E=256, hidden 4096, ispp 512, top_k 6, whole call in a graph, against the kernel that converts to
-// bf16: M=48 189 -> 144 us (0.58 GB of weights: 89 us at the copy rate), M=768 466 -> 259, M=2048 955 -> 425.
+// bf16: M=48 189 -> 139 us (0.58 GB of weights: 89 us at the copy rate), M=768 466 -> 259.
 //
 // Scale byte 0xFF means weight 0 here (it is NaN to the instruction): a mover that meets one clears the
 // group's weights in shared memory and puts byte 0 in its place.
@@ -48,21 +48,24 @@ constexpr int kTmemCols = 512;
 constexpr uint32_t kProdSleepNs = 200;
 
 template <int BT> struct MxCfg {
-  static_assert(BT == 16 || BT == 32, "token tile");
+  static_assert(BT == 8 || BT == 16 || BT == 32, "token tile");
   // All three terms are multiplied in ONE instruction: the terms' tiles lie behind one another in shared
   // memory, which is a tile of 3 BT tokens, each term with accumulators of its own that the read-out adds up.  An
   // instruction costs its issuer 45 cycles up to 32 tokens or so, whatever its width.
-  static constexpr int kMmaTokens = kTerms * BT;                      // UMMA N
+  static constexpr int kTermRows = kTerms * BT;
+  // UMMA N, a multiple of 16: 8-token tiles read eight rows more (of what lies behind the stage; columns that nobody reads)
+  static constexpr int kMmaTokens = (kTermRows + 15) / 16 * 16;
   static constexpr int kTokRowGroups = (kMmaTokens + 31) / 32;
   static constexpr int kTokBytes = BT * kStageK;                      // one term
   static_assert(kTokBytes % 1024 == 0, "swizzle atoms");
   static constexpr int kStageBytes = 2 * kWBytes + kTerms * kTokBytes;
-  static constexpr int kStages = BT <= 16 ? 5 : 4;
+  static constexpr int kStages = BT == 8 ? 6 : BT == 16 ? 5 : 4;
   // Scale tiles are loaded with the first stage of their four and read with all four: a slot is free again
   // when the MMAs kStages before that first stage are done, if kStages <= 4 * slots - 3.
-  static constexpr int kScSlots = 2;
+  static constexpr int kScSlots = kStages > 5 ? 3 : 2;
   static_assert(kStages <= 4 * kScSlots - 3, "scale slots");
   static constexpr int kScBytes = 2 * kRows * 16 + BT * 16;
+  static_assert(kTokBytes >= (kMmaTokens - kTermRows) * kStageK, "the rows read behind the last stage lie in the scale tiles");
   // columns: accumulator sets of two matrices, then per stage 4 gate + 4 up + 4 token scale columns
   static constexpr int kScStageCols = 12;
   static constexpr int kScCols = kScStageCols * kStages;
@@ -73,7 +76,8 @@ template <int BT> struct MxCfg {
   // (with one column group the two warpgroups take alternate tiles: each must meet every use of its accumulator sets)
   static_assert(BT > 16 || kDBuf % 2 == 0, "accumulator sets alternate with the warpgroups");
   static constexpr int kScCol0 = kDBuf * kSetCols;
-  static constexpr int kColGroups = BT / 16;
+  static constexpr int kCols = BT < 16 ? BT : 16;                     // columns of a read-out step
+  static constexpr int kColGroups = BT / kCols;
   static constexpr int kEpiWGs = kColGroups < 2 ? 1 : 2;              // read-out warpgroups per tile
   static constexpr int kNumBars = 3 * kStages + 2 * kDBuf;
   static constexpr size_t kSmemBytes = 1024 + (size_t)kStages * kStageBytes + (size_t)kScSlots * kScBytes + kNumBars * 8 + 64;
@@ -131,7 +135,7 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
               const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_mid,
               const __grid_constant__ CUtensorMap tm_lo, const __grid_constant__ CUtensorMap tm_xs, const MxParams p) {
   using Cfg = MxCfg<BT>;
-  constexpr int kStages = Cfg::kStages, kDBuf = Cfg::kDBuf;
+  constexpr int kStages = Cfg::kStages, kDBuf = Cfg::kDBuf, kCols = Cfg::kCols;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* s_sc = smem + kStages * Cfg::kStageBytes;     // kScSlots x { gate, up [128 x 16], tokens [BT x 16] }
@@ -293,7 +297,7 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
               for (int c = 0; c < 4; ++c) w[m][c] = lds128(sc + (uint32_t)((m * kRows + c * 32 + lane) * 16));
 #pragma unroll
             for (int c = 0; c < Cfg::kTokRowGroups; ++c)
-              x[c] = (c * 32 + lane < Cfg::kMmaTokens) ? lds128(sc + 2 * kRows * 16 + (uint32_t)((c * 32 + lane) % BT * 16))
+              x[c] = (c * 32 + lane < Cfg::kTermRows) ? lds128(sc + 2 * kRows * 16 + (uint32_t)((c * 32 + lane) % BT * 16))
                                                        : make_uint4(0, 0, 0, 0);
           }
           const uint32_t dst = tmem_base + lane_base + Cfg::kScCol0 + st * Cfg::kScStageCols;
@@ -361,40 +365,40 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
           bias0 = __bfloat162float(eb[0]);
           bias1 = __bfloat162float(eb[p.mat_row]);
         }
-        int32_t next = lane < 16 ? __ldcg(p.sorted_ids + (int64_t)b * BT + cg0 * 16 + lane) : -1;
+        int32_t next = lane < kCols ? __ldcg(p.sorted_ids + (int64_t)b * BT + cg0 * kCols + lane) : -1;
         if (!mbar_wait(&d_full[dbuf], dph, guard, 7, 100)) break;
         tc_fence_after();
 #pragma unroll 1
         for (int cg = cg0; cg < Cfg::kColGroups; cg += Cfg::kEpiWGs) {
           const int32_t my_slot = next;
           if (cg + Cfg::kEpiWGs < Cfg::kColGroups)
-            next = lane < 16 ? __ldcg(p.sorted_ids + (int64_t)b * BT + (cg + Cfg::kEpiWGs) * 16 + lane) : -1;
-          const uint32_t live = __ballot_sync(0xffffffffu, my_slot >= 0 && my_slot < p.numel) & 0xFFFFu;
+            next = lane < kCols ? __ldcg(p.sorted_ids + (int64_t)b * BT + (cg + Cfg::kEpiWGs) * kCols + lane) : -1;
+          const uint32_t live = __ballot_sync(0xffffffffu, my_slot >= 0 && my_slot < p.numel) & ((1u << kCols) - 1u);
           if (live == 0u) continue;
-          uint32_t a0[16], a1[16];
-          const uint32_t d = tmem_base + lane_base + dbuf * Cfg::kSetCols + cg * 16;
-          tmem_ld_32x16(d, a0);
-          tmem_ld_32x16(d + Cfg::kMmaTokens, a1);
+          uint32_t a0[kCols], a1[kCols];
+          const uint32_t d = tmem_base + lane_base + dbuf * Cfg::kSetCols + cg * kCols;
+          tmem_ld(d, a0);
+          tmem_ld(d + Cfg::kMmaTokens, a1);
           tmem_wait_ld();
 #pragma unroll
           for (int i = 1; i < kTerms; ++i) {
-            uint32_t b0[16], b1[16];
-            tmem_ld_32x16(d + i * BT, b0);
-            tmem_ld_32x16(d + Cfg::kMmaTokens + i * BT, b1);
+            uint32_t b0[kCols], b1[kCols];
+            tmem_ld(d + i * BT, b0);
+            tmem_ld(d + Cfg::kMmaTokens + i * BT, b1);
             tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < kCols; ++j) {
               a0[j] = __float_as_uint(__uint_as_float(a0[j]) + __uint_as_float(b0[j]));
               a1[j] = __float_as_uint(__uint_as_float(a1[j]) + __uint_as_float(b1[j]));
             }
           }
-          // The sixteen columns are computed side by side whether they are live or padding (whose values are
+          // The columns are computed side by side whether they are live or padding (whose values are
           // never stored): their chains overlap, which branches between them would not allow.
           if (GATE_UP) {
             // rounding points of the reference (src/xkernels/ops/moe/mxfp4_reference.py:92-100)
-            uint32_t top[16];
+            uint32_t top[kCols];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < kCols; ++j) {
               float v0 = __uint_as_float(a0[j]), v1 = __uint_as_float(a1[j]);
               round_pair_to_bf16(v0, v1);
               if (p.bias != nullptr) { v0 += bias0; v1 += bias1; round_pair_to_bf16(v0, v1); }
@@ -410,11 +414,11 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
             }
             // this warp's 32 rows are one scale block of the next contraction
 #pragma unroll
-            for (int j = 0; j < 16; ++j) top[j] = __reduce_max_sync(0xffffffffu, mx::finite_abs_bits(a0[j] >> 16));
-            const int64_t pos = (int64_t)b * BT + cg * 16;
+            for (int j = 0; j < kCols; ++j) top[j] = __reduce_max_sync(0xffffffffu, mx::finite_abs_bits(a0[j] >> 16));
+            const int64_t pos = (int64_t)b * BT + cg * kCols;
             const int64_t at = pos * p.N + n_glob;
 #pragma unroll
-            for (int j = 0; j < 16; j += 2) {
+            for (int j = 0; j < kCols; j += 2) {
               const float x0 = __uint_as_float(a0[j]), x1 = __uint_as_float(a0[j + 1]);
               const uint32_t s0 = mx::hi_scale(top[j]), s1 = mx::hi_scale(top[j + 1]);
               uint32_t term[kTerms];
@@ -428,12 +432,12 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
             // lane j stores the scale byte of position j
             uint32_t sh = 0;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) sh = lane == j ? mx::hi_scale(top[j]) : sh;
-            if ((live >> lane) & 1u)   // (live has sixteen bits)
+            for (int j = 0; j < kCols; ++j) sh = lane == j ? mx::hi_scale(top[j]) : sh;
+            if ((live >> lane) & 1u)   // (live has kCols bits)
               p.act_scale[(pos + lane) * (p.N / 32) + (n_glob >> 5)] = (uint8_t)sh;
           } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < kCols; ++j) {
               float v0 = __uint_as_float(a0[j]), v1 = __uint_as_float(a1[j]);
               if (p.bias != nullptr) { round_pair_to_bf16(v0, v1); v0 += bias0; v1 += bias1; }
               const uint32_t two = pack_bf16(v0, v1);
@@ -571,6 +575,7 @@ int launch_mx(const CUtensorMap (&tm)[6], const MxParams& prm, int64_t max_tiles
 template <bool GATE_UP>
 int launch_mx_by_block(int block, const CUtensorMap (&tm)[6], const MxParams& prm, int64_t max_tiles, cudaStream_t stream) {
   switch (block) {
+    case 8: return launch_mx<8, GATE_UP>(tm, prm, max_tiles, stream);
     case 16: return launch_mx<16, GATE_UP>(tm, prm, max_tiles, stream);
     case 32: return launch_mx<32, GATE_UP>(tm, prm, max_tiles, stream);
     default: return fail(XKB_ERR_ARG, "mxfp4 block-scaled path: unsupported token tile %d", block);
@@ -623,9 +628,11 @@ bool mxfp4_bs_supported(const void* w13, const void* w2, const void* s13, const 
 // slots per expert, 261 / 276 / 333 at 12, 370 / 294 / 352 at 19, 447 / 334 / 370 at 26, 513 / 424 / 391 at 33; E=128, 4096,
 // 1024: 389 / 302 / 346 at 25, 514 / 444 / 373 at 38; E=64, 2048, 1024: 82 / 84 / 104 at 14, 120 / 99 / 109 at 28.  (64-token
 // tiles of this kernel took 10 to 20 % longer than the bf16 kernel from 26 slots on: 417 us at 26, 430 at 33, 449 / 411 at 40.)
+// 8 against 16 tokens (half the token bytes, one more stage of weights in flight): 32.9 / 36.9 us at M=1, 81 / 87 at M=16,
+// 139 / 145 at one slot per expert (M=48), 199 / 212 at 3.5, 212 / 220 at 4.7, 240 / 239 at 9.4; E=128: 167 / 182 at 1.9.
 int mxfp4_bs_block(int64_t numel, int E) {
   const double avg = (double)numel / (E > 0 ? E : 1);
-  return avg <= 12 ? 16 : avg <= 28 ? 32 : 0;
+  return avg <= 5 ? 8 : avg <= 12 ? 16 : avg <= 28 ? 32 : 0;
 }
 
 int64_t mxfp4_bs_workspace_bytes(int64_t numel, int64_t hidden, int64_t ispp, int E) {
@@ -691,7 +698,7 @@ int launch_mxfp4_bs(const void* A, const uint8_t* w13, const uint8_t* w13_scale,
   prm.limit = limit;
   prm.done_signal = done;
   prm.done_wait = nullptr;
-  prm.done_target = (int)(ispp / kRows) * 4 * (r.block == 16 ? 1 : 2);
+  prm.done_target = (int)(ispp / kRows) * 4 * (r.block <= 16 ? 1 : 2);
   GemmTimerScope timed(stream);   // both GEMMs in one scope: they overlap
   rc = launch_mx_by_block<true>(r.block, up, prm, r.max_blocks * (ispp / kRows), stream);
   if (rc != XKB_OK) return rc;
