@@ -1,4 +1,5 @@
-"""ctypes binding of ``libxkb200.so`` — the only route from Python to the kernels.
+"""Binding of ``libxkb200.so`` — the only route from Python to the kernels: ctypes, and a native call path for plain
+calls of the small ops.
 
 The library is built in-tree by :mod:`xkernels_b200.build`.  There is no CPU or
 eager fallback: if the shared object is missing or fails to load, importing any
@@ -8,10 +9,13 @@ op raises, and every op raises on non-CUDA tensors.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 from ctypes import c_char_p, c_float, c_int, c_int64, c_void_p
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libxkb200.so"
+CALLS_PATH = Path(__file__).resolve().parent / "_torch_calls.so"
 
 XKB_BF16 = 0
 XKB_F32 = 1
@@ -109,6 +113,26 @@ def load() -> ctypes.CDLL:
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+_calls = None
+
+
+def load_calls():
+    """The native call path of the small ops (``csrc/torch_calls.cpp``), bound to the library's functions."""
+    global _calls
+    if _calls is not None:
+        return _calls
+    if not CALLS_PATH.exists():
+        raise RuntimeError(f"{CALLS_PATH} is missing: build it with `python -m xkernels_b200.build` (there is no fallback path)")
+    loader = importlib.machinery.ExtensionFileLoader("_torch_calls", str(CALLS_PATH))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_torch_calls", loader))
+    loader.exec_module(module)
+    lib = load()
+    module.bind(*(ctypes.cast(fn, c_void_p).value for fn in (
+        lib.xkb_topk_softmax, lib.xkb_moe_align_block_size, lib.xkb_moe_align_workspace_bytes, lib.xkb_moe_sum_reduce)))
+    _calls = module
+    return module
 
 
 def check(status: int, what: str) -> None:

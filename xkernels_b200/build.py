@@ -1,4 +1,5 @@
-"""Builds ``libxkb200.so`` (the C-ABI library of sm_100a kernels) in-tree with nvcc.
+"""Builds ``libxkb200.so`` (the C-ABI library of sm_100a kernels) in-tree with nvcc, and ``_torch_calls.so`` (the native
+call path of the small ops) with the host compiler.
 
 Run ``python -m xkernels_b200.build`` or call :func:`build`.  The objects are
 compiled in parallel, one nvcc process per ``.cu`` file, and linked into
@@ -12,12 +13,16 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
+
+import torch
 
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libxkb200.so"
+CALLS_PATH = PKG_DIR / "_torch_calls.so"
 OBJ_DIR = PKG_DIR / "build"
 
 NVCC_FLAGS = [
@@ -45,17 +50,32 @@ def _fingerprint() -> str:
                     + [PKG_DIR.parent / "include" / "xkb200.h"]):
         h.update(p.name.encode())
         h.update(p.read_bytes())
+    h.update((CSRC / "torch_calls.cpp").read_bytes())
+    h.update(f"{torch.__version__} {sys.version}".encode())
     h.update(" ".join(NVCC_FLAGS).encode())
     return h.hexdigest()
 
 
 def is_current() -> bool:
     stamp = OBJ_DIR / "fingerprint"
-    return LIB_PATH.exists() and stamp.exists() and stamp.read_text() == _fingerprint()
+    return LIB_PATH.exists() and CALLS_PATH.exists() and stamp.exists() and stamp.read_text() == _fingerprint()
+
+
+def _build_calls() -> None:
+    from torch.utils import cpp_extension as ext
+
+    cxx = os.environ.get("CXX") or shutil.which("g++") or "c++"
+    dirs = [*ext.include_paths(), sysconfig.get_paths()["include"], str(Path(_nvcc()).resolve().parents[1] / "include")]
+    cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *(f"-I{d}" for d in dirs), str(CSRC / "torch_calls.cpp"), "-o", str(CALLS_PATH),
+           *(f"-L{d}" for d in ext.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"build of _torch_calls.so failed:\n{res.stdout}\n{res.stderr}")
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every ``csrc/*.cu`` for sm_100a and link the shared library."""
+    """Compile every ``csrc/*.cu`` for sm_100a and link the shared library; compile the call path beside it."""
     if not force and is_current():
         return LIB_PATH
     nvcc = _nvcc()
@@ -73,7 +93,9 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         return obj
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        calls = pool.submit(_build_calls)
         objs = list(pool.map(compile_one, _sources()))
+        calls.result()
     cmd = [nvcc, "-shared", "-o", str(LIB_PATH), *map(str, objs)]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:

@@ -166,6 +166,15 @@ def moe_align_block_size(topk_ids, block_size, num_experts, truncate=True, works
     ``moe_align_block_size_ep`` (w4a16.py:104-155): ``num_experts`` is then the
     local expert count and non-local slots are dropped.
     """
+    if workspace is None and expert_map is None:
+        got = (_lib._calls or _lib.load_calls()).moe_align_block_size(topk_ids, block_size, num_experts)
+        if got is not None:
+            if type(got) is int:
+                _lib.check(got, "xkb_moe_align_block_size")
+            if not truncate:
+                return got
+            sorted_ids, expert_ids, num_post = got
+            return sorted_ids, expert_ids[: max(int(num_post.item()) // block_size, 1)], num_post
     lib = _lib.load()
     dev = _require_cuda("moe_align_block_size", topk_ids, expert_map)
     block_size, num_experts = int(block_size), int(num_experts)
@@ -233,6 +242,11 @@ def topk_softmax(gating_output, topk, renormalize=True):
 
     Reference: ``topk_softmax_ref`` (src/xkernels/ops/moe/topk_softmax.py:33-95).
     """
+    got = (_lib._calls or _lib.load_calls()).topk_softmax(gating_output, topk, renormalize)
+    if got is not None:
+        if type(got) is int:
+            _lib.check(got, "xkb_topk_softmax")
+        return got
     lib = _lib.load()
     dev = _require_cuda("topk_softmax", gating_output)
     if gating_output.dim() != 2:
@@ -261,6 +275,11 @@ def moe_sum_reduce(y, w=None, routed_scaling_factor=1.0):
     ``y`` is ``[M, top_k, H]`` bf16/fp32, ``w`` ``[M, top_k]`` fp32/bf16 or None;
     the result has ``y.dtype``.
     """
+    got = (_lib._calls or _lib.load_calls()).moe_sum_reduce(y, w, routed_scaling_factor)
+    if got is not None:
+        if type(got) is int:
+            _lib.check(got, "xkb_moe_sum_reduce")
+        return got
     lib = _lib.load()
     dev = _require_cuda("moe_sum_reduce", y, w)
     if y.dim() != 3:
