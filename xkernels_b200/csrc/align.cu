@@ -3,21 +3,19 @@
 // stable order inside an expert, every run padded to a multiple of block_size,
 // unused entries of sorted_ids = numel, unused entries of expert_ids = 0.
 //
-// Stability without sorting: a slot's rank inside its expert is
-//   (# same-expert slots in earlier 1024-slot chunks)      -> chunk x expert matrix
-// + (# same-expert slots in earlier warps of its chunk)    -> warp x expert matrix (smem)
-// + (# same-expert lanes below it in its warp)             -> __match_any_sync ballot
+// Stability without sorting: a slot's rank inside its expert is the number of same-expert slots before it, which is
+// counted in pieces (earlier chunks or blocks, earlier warps, lower lanes by a __match_any_sync ballot).
 // Counters only ever count, so atomics never decide an output position.
 //
 // Latency-bound: a call moves about a megabyte at most, so what counts is the number of dependent steps.
-// numel <= kSmallMax (a decode batch) runs as ONE single-CTA kernel with one pass over the ids: the ranks
-// of the slots and the expert counts come out of the same warp x expert matrix.  Larger inputs use two
-// launches over at most kMaxChunks chunks of whole 1024-slot rounds: count, then place.  Every CTA of the
-// second adds up the chunk x expert matrix for itself (a few hundred KB from L2 at most) instead of waiting
-// for a single-CTA scan between the two, and is launched while the first still runs.
-// M=16384, top_k=8, E=48, block 16: 10.5 us on the device for the two launches (7.5 of it the second), a call 29.4 ->
-// 24.7 us, 18.0 with the shorter host path (which still bounds it); the fused calls lose a memset launch besides,
-// 49.1 -> 45.7 us at M=1.
+//   numel <= kSmallMax (a decode batch): ONE single-CTA kernel with one pass over the ids; the ranks
+//     of the slots and the expert counts come out of the same warp x expert matrix.
+//   numel <= kClusterMax: one cluster of eight CTAs.  Every warp counts a contiguous segment of 32 or 64 slots, the CTAs
+//     read one another's expert counts through distributed shared memory, and every warp then walks its segment
+//     again with running positions: two cluster barriers and no launch between counting and placing.
+//   larger inputs: two launches over at most kMaxChunks chunks of whole 1024-slot rounds, count, then place.  Every CTA of
+//     the second adds up the chunk x expert matrix for itself and is launched while the first still runs.
+// A call: 1040 to 6000 slots 9.6 -> 8.2 us with the cluster; M=16384, top_k=8, E=48, block 16 (two launches) 10.4.
 #include "align_dev.cuh"
 #include "common.cuh"
 
@@ -28,6 +26,11 @@ using namespace align;
 
 constexpr int kMaxChunks = 148;        // CTAs of the two-launch path: one wave
 constexpr int64_t kNoWorkspaceMax = 8192;   // slots that need no workspace (callers may pass none)
+constexpr int kCluster = 8;            // CTAs of the cluster path: the portable cluster size
+constexpr int kRounds = 2;             // rounds of 32 slots a warp of the cluster takes at most
+// Walking longer segments takes longer than the second launch: 8.2 us a call against 9.6 at 6000 slots and E=64, 12.3 / 12.3 at
+// 24000 and 256, 22.6 / 11.3 at 131072 and 48.
+constexpr int64_t kClusterMax = (int64_t)kCluster * kWarps * 32 * kRounds;   // 16384
 
 // ---------------------------------------------------------------------------
 // Single-CTA path: numel <= 1024.  zero / zero_n: ints the caller wants cleared (nullptr, 0: none).
@@ -45,6 +48,113 @@ align_small_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int E, i
               max_blocks, num_map, E, block};
   const int pos = align_in_block(j, smem_raw, true);
   if (threadIdx.x < numel && slot_pos != nullptr) slot_pos[threadIdx.x] = pos;
+}
+
+// ---------------------------------------------------------------------------
+// Cluster path: warp g of the cluster (kCluster * kWarps of them) takes the slots [g * segment, (g + 1) * segment)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// the int at the same shared-memory address in CTA `rank` of the cluster
+__device__ __forceinline__ int load_remote(const int* p, int rank) {
+  uint32_t at;
+  int v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+  return v;
+}
+
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads)
+align_cluster_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t segment, int E, int block,
+                     const int32_t* __restrict__ expert_map, int num_map,
+                     int32_t* __restrict__ sorted_ids, int64_t max_pad, int32_t* __restrict__ expert_ids, int64_t max_blocks,
+                     int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out, int32_t* __restrict__ slot_pos,
+                     int32_t* __restrict__ block_live, int32_t* __restrict__ zero, int64_t zero_n) {
+  chain_trigger();   // a kernel chained behind this one may be launched; it waits for completion itself
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int EP = E + 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)blockIdx.x;   // (one cluster)
+  int* wcnt = reinterpret_cast<int*>(smem_raw);   // [kWarps][EP] a warp's slots per expert, then their next place in the CTA
+  int* own = wcnt + kWarps * EP;                  // [EP] this CTA's slots per expert
+  int* tot = own + EP;                            // [EP] all slots per expert
+  int* off = tot + EP;                            // [EP] off[E] = total
+  int* base = off + EP;                           // [EP] first position of this CTA's slots
+  int* warp_tot = base + EP;                      // [kWarps]
+  const int64_t first = ((int64_t)rank * kWarps + warp) * segment;
+  const int64_t last = first + segment < numel ? first + segment : numel;
+  int e[kRounds];   // the slots' experts (E: dropped); no slot: a number of the lane's own, which matches nobody
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const int64_t slot = first + r * 32 + lane;
+    e[r] = slot < last ? map_expert(topk_ids[slot], E, expert_map, num_map) : EP + lane;
+  }
+  for (int i = tid; i < kWarps * EP; i += kThreads) wcnt[i] = 0;
+  for (int64_t i = (int64_t)rank * kThreads + tid; i < zero_n; i += (int64_t)kCluster * kThreads) zero[i] = 0;
+  __syncthreads();
+  int* mine = wcnt + warp * EP;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r)
+    if (e[r] < EP) atomicAdd(&mine[e[r]], 1);
+  __syncthreads();
+  // exclusive scan over the warps, one expert per scanning warp per step
+  for (int x = warp; x < EP; x += kWarps) {
+    const int v = wcnt[lane * EP + x];
+    int incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += u;
+    }
+    wcnt[lane * EP + x] = incl - v;
+    if (lane == 31) own[x] = incl;
+  }
+  __syncthreads();
+  cluster_arrive();
+  cluster_wait();
+  int before = 0;
+  if (tid < E) {   // E <= kThreads
+    int all = 0;
+#pragma unroll
+    for (int r = 0; r < kCluster; ++r) {
+      const int v = load_remote(own + tid, r);
+      all += v;
+      before += r < rank ? v : 0;
+    }
+    tot[tid] = all;
+  }
+  __syncthreads();
+  cluster_arrive();   // this CTA has read the others' counts; the wait for theirs is at the end
+  padded_offsets(tot, off, warp_tot, E, block);
+  if (tid < E) base[tid] = off[tid] + before;
+  if (rank == 0) {
+    if (tid == 0) num_post[0] = off[E];
+    if (expert_off_out != nullptr)
+      for (int i = tid; i < EP; i += kThreads) expert_off_out[i] = off[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const int x = e[r];
+    const int64_t slot = first + r * 32 + lane;
+    const unsigned peers = __match_any_sync(0xffffffffu, x);
+    const int below = __popc(peers & ((1u << lane) - 1u));
+    const int at = x < EP ? mine[x] : 0;
+    __syncwarp();
+    if (x < EP && below == 0) mine[x] = at + __popc(peers);
+    __syncwarp();
+    if (x < E) sorted_ids[base[x] + at + below] = (int32_t)slot;
+    if (x < EP && slot_pos != nullptr) slot_pos[slot] = x < E ? base[x] + at + below : -1;
+  }
+  // the positions that hold no slot: the ends of the experts' runs, and what lies behind the last
+  for (int x = rank * kWarps + warp; x < E; x += kCluster * kWarps)
+    for (int i = off[x] + tot[x] + lane; i < off[x + 1]; i += 32) sorted_ids[i] = (int32_t)numel;
+  for (int64_t i = off[E] + (int64_t)rank * kThreads + tid; i < max_pad; i += (int64_t)kCluster * kThreads) sorted_ids[i] = (int32_t)numel;
+  write_expert_ids(off, tot, E, block, expert_ids, block_live, max_blocks, rank * kThreads + tid, kCluster * kThreads);
+  cluster_wait();     // no CTA leaves while another may read its counts
+}
+
+size_t cluster_smem(int E) {
+  const size_t EP = E + 1;
+  return (kWarps * EP + 4 * EP + kWarps) * sizeof(int);
 }
 
 // ---------------------------------------------------------------------------
@@ -78,7 +188,7 @@ align_count_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t 
 __global__ void __launch_bounds__(kThreads)
 align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t span, int E, int block,
                    const int32_t* __restrict__ expert_map, int num_map,
-                   const int32_t* chunk_cnt /*[C][E+1]: written by the kernel this one overlaps; nullptr: one chunk*/,
+                   const int32_t* chunk_cnt /*[C][E+1]: written by the kernel this one overlaps*/,
                    int32_t* sorted_ids, int64_t max_pad, int32_t* __restrict__ expert_ids, int64_t max_blocks,
                    int32_t* __restrict__ num_post, int32_t* __restrict__ expert_off_out,
                    int32_t* __restrict__ slot_pos, int32_t* __restrict__ block_live) {
@@ -98,16 +208,11 @@ align_place_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_t 
   bool active = slot < last;
   int e = active ? map_expert(topk_ids[slot], E, expert_map, num_map) : E;   // an input of the call, not of the kernel before
   chain_wait();
-  if (chunk_cnt == nullptr) {   // one CTA without a workspace: counts and fills for itself
-    for (int64_t s = tid; s < numel; s += kThreads)
-      atomicAdd(&tot[map_expert(topk_ids[s], E, expert_map, num_map)], 1);
-    for (int64_t i = tid; i < max_pad; i += kThreads) sorted_ids[i] = (int32_t)numel;
-  }
   // slots per expert in all chunks (tot) and in the chunks before this one (base): threads side by side
   // take neighbouring experts, the groups of threads share the chunks out
   const int width = E < kThreads ? (E > 0 ? E : 1) : kThreads;
   const int groups = kThreads / width, grp = tid / width;
-  if (chunk_cnt != nullptr && grp < groups) {
+  if (grp < groups) {
     for (int x = tid - grp * width; x < E; x += width) {
       int all = 0, before = 0;
 #pragma unroll 8
@@ -188,17 +293,19 @@ int launch_align(const int32_t* topk_ids, int64_t numel, int E, int block,
     return XKB_OK;
   }
   const int64_t need = align_workspace_bytes(numel, E);
-  if ((workspace == nullptr || workspace_bytes < need) && numel <= kNoWorkspaceMax && zero_n == 0) {
-    const size_t smem = place_smem(E);
-    XKB_CHECK_CUDA(allow_smem(align_place_kernel, smem));
-    align_place_kernel<<<1, kThreads, smem, stream>>>(topk_ids, numel, numel, E, block, expert_map, num_map, nullptr, sorted_ids,
-                                                      max_pad, expert_ids, max_blocks, num_post, expert_off, slot_pos, block_live);
-    XKB_CHECK_LAUNCH("align_place_kernel");
-    return XKB_OK;
-  }
-  if (workspace == nullptr || workspace_bytes < need)
+  if ((workspace == nullptr || workspace_bytes < need) && (numel > kNoWorkspaceMax || zero_n != 0))
     return fail(XKB_ERR_WORKSPACE, "moe_align: workspace of %lld bytes needed, %lld given",
                 (long long)need, (long long)workspace_bytes);
+  if (numel <= kClusterMax) {
+    const int64_t segment = align_up(ceil_div(numel, (int64_t)kCluster * kWarps), 32);
+    const size_t smem = cluster_smem(E);
+    XKB_CHECK_CUDA(allow_smem(align_cluster_kernel, smem));
+    align_cluster_kernel<<<kCluster, kThreads, smem, stream>>>(topk_ids, numel, segment, E, block, expert_map, num_map, sorted_ids,
+                                                               max_pad, expert_ids, max_blocks, num_post, expert_off, slot_pos,
+                                                               block_live, zero, zero_n);
+    XKB_CHECK_LAUNCH("align_cluster_kernel");
+    return XKB_OK;
+  }
   const int64_t span = ceil_div(numel, (int64_t)kMaxChunks * kChunk) * kChunk;
   const int C = (int)ceil_div(numel, span);
   int32_t* chunk_cnt = static_cast<int32_t*>(workspace);
