@@ -385,7 +385,7 @@ def run_single_gpu(args):
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
                 "traffic_source": "estimated: ncu dram bytes of a 16-expert capture scaled by experts touched",
-                "kernel": "moe_tc_kernel<16, int4>", "kernel_us": gemm_avg_ms * 1e3,
+                "kernel": "moe_tc_kernel<32, int4>", "kernel_us": gemm_avg_ms * 1e3,
                 "algorithmic_bytes": alg_bytes, "peak_source": peaks["source"],
                 "whole_call_frac": (alg_bytes / (ms_per_step * 1e-3) / 1e9) / peaks["hbm_gbs"]}
 
