@@ -31,7 +31,7 @@ constexpr int kMaxPerLane = 32;               // experts per lane -> at most 102
 constexpr int kWarpsPerBlock = 8;
 // Up to this top-k the candidates of rows of independent logits fit 32 lanes (74-100 % of the rows at 20, E = 48 to
 // 1024; 31-99 % at 22; 5-85 % at 24); above, looking for them mostly comes on top of the rounds (top 32 of 1024
-// experts, M=16384: 227 us without, 231 with).  Up to 32 experts they fit in any case.
+// experts, M=16384: 227 us without, 231 with, in the form with strided logits).  Up to 32 experts they fit in any case.
 constexpr int kShortTopk = 20;
 
 template <typename T> __device__ __forceinline__ float load_logit(const T* p);
