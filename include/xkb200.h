@@ -134,6 +134,11 @@ int xkb_moe_sum_reduce(const void* y, int y_dtype, const void* w, int w_dtype,
                        void* out, int out_dtype, int64_t M, int top_k,
                        int64_t H, float routed_scaling_factor, void* stream);
 
+/* Token blocks that a fused call's workspace has room for, whatever block size
+ * the call picks (a block is a token tile: some positions of one expert).
+ * -1 for a negative argument.  No reference counterpart. */
+int64_t xkb_routing_blocks(int64_t numel, int num_experts);
+
 /* ------------------------------------------------------------------------
  * fused_moe_int4_w4a16: out[m] = sum_j w[m,j] * (A[m] @ dequant(W[e_mj])^T)
  * Replaces: src/xkernels/ops/moe/reference.py:22-70 (moe_w4a16_ref) and

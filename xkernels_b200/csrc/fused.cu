@@ -53,8 +53,9 @@ namespace {
 
 struct RoutingBuffers {
   int* status;
-  int32_t* counters;        // directly behind the status header: cleared as one span
-  int64_t num_counters;
+  int64_t num_blocks;       // token blocks that the arrays with one entry per block hold
+  int64_t num_positions;    // length of sorted_ids
+  int32_t* counters;        // one per block, directly behind the status header: cleared as one span
   int32_t* sorted_ids;
   int32_t* expert_ids;
   int32_t* num_post;
@@ -65,34 +66,38 @@ struct RoutingBuffers {
   int64_t align_ws_bytes;
 };
 
-// Routing buffers are sized for the worst case over the block sizes any path
-// may pick: the longest sorted_ids (largest block) and the most blocks
-// (smallest block).
+// Routing buffers are sized for the worst case over the block sizes any path may pick: the longest
+// sorted_ids (largest block) and the most blocks.  The sort writes ceil((numel + (E + 1) (B - 1)) / B) entries
+// per block array at block size B, which is below numel / B + E + 2 - (E + 1) / B, so numel / kMinBlock + E + 2 holds them
+// at every B >= kMinBlock.  (The count at the smallest block is no such bound: with fewer slots than experts wider
+// blocks have more entries, 257 at B = 16 and 240 at B = 8 for 8 slots and 272 experts.)
 constexpr int kMaxBlock = 256;
 constexpr int kMinBlock = 8;
 
 int64_t routing_max_pad(int64_t numel, int E, int block) {
   return numel + (int64_t)(E + 1) * (block - 1);
 }
+int64_t routing_max_blocks(int64_t numel, int E) { return numel / kMinBlock + E + 2; }
 
 RoutingBuffers carve_routing(Carver& c, int64_t numel, int E) {
   RoutingBuffers r;
   r.status = c.take<int>(64);  // workspace header: word 0 = device status of the last call
-  r.num_counters = numel / kMinBlock + E + 2;     // >= token blocks at the smallest token tile
-  r.counters = c.take<int32_t>(r.num_counters);
-  r.sorted_ids = c.take<int32_t>(routing_max_pad(numel, E, kMaxBlock));
-  r.expert_ids = c.take<int32_t>(ceil_div(routing_max_pad(numel, E, kMinBlock), kMinBlock) + 1);
+  r.num_blocks = routing_max_blocks(numel, E);
+  r.num_positions = routing_max_pad(numel, E, kMaxBlock);
+  r.counters = c.take<int32_t>(r.num_blocks);
+  r.sorted_ids = c.take<int32_t>(r.num_positions);
+  r.expert_ids = c.take<int32_t>(r.num_blocks);
   r.num_post = c.take<int32_t>(1);
   r.expert_off = c.take<int32_t>(E + 1);
   r.slot_pos = c.take<int32_t>(numel);
-  r.block_live = c.take<int32_t>(ceil_div(routing_max_pad(numel, E, kMinBlock), kMinBlock) + 1);
+  r.block_live = c.take<int32_t>(r.num_blocks);
   r.align_ws_bytes = align_workspace_bytes(numel, E);
   r.align_ws = c.take<char>(r.align_ws_bytes);
   return r;
 }
 
 // status header and the block counters behind it, as one span
-int64_t header_ints(const RoutingBuffers& r) { return r.counters + r.num_counters - r.status; }
+int64_t header_ints(const RoutingBuffers& r) { return r.counters + r.num_blocks - r.status; }
 
 int64_t routing_bytes(int64_t numel, int E) {
   Carver c(nullptr);
@@ -100,7 +105,7 @@ int64_t routing_bytes(int64_t numel, int E) {
   return c.off;
 }
 
-Routing make_routing(const RoutingBuffers& b, int64_t numel, int E, int block) {
+int make_routing(const RoutingBuffers& b, int64_t numel, int E, int block, Routing* out) {
   Routing r;
   r.sorted_ids = b.sorted_ids;
   r.expert_ids = b.expert_ids;
@@ -114,7 +119,11 @@ Routing make_routing(const RoutingBuffers& b, int64_t numel, int E, int block) {
   r.max_blocks = ceil_div(r.max_pad, block);
   r.block_counters = b.counters;
   r.job = nullptr;
-  return r;
+  XKB_REQUIRE(r.max_pad <= b.num_positions && r.max_blocks <= b.num_blocks,
+              "routing: blocks of %d do not fit the routing buffers (%lld of %lld positions, %lld of %lld blocks)", block,
+              (long long)r.max_pad, (long long)b.num_positions, (long long)r.max_blocks, (long long)b.num_blocks);
+  *out = r;
+  return XKB_OK;
 }
 
 // The align stage of a fused call: clears the status word and the block counters on its way.  A decode batch on
@@ -164,6 +173,8 @@ using namespace xkb;
 extern "C" const char* xkb_version(void) { return "xkb200 0.1 (sm_100a)"; }
 extern "C" const char* xkb_last_error(void) { return last_error_buf(); }
 extern "C" int64_t xkb_launch_count(void) { return g_launches.load(); }
+
+extern "C" int64_t xkb_routing_blocks(int64_t numel, int E) { return numel < 0 || E < 0 ? -1 : routing_max_blocks(numel, E); }
 
 // ---------------------------------------------------------------------------
 // INT4 W4A16
@@ -221,9 +232,11 @@ static int int4_impl(const void* A, int a_dtype, const int32_t* packed, const vo
   const bool use_tc = (path == XKB_PATH_TC) || (path == XKB_PATH_AUTO && tc_fit);
   const int block = use_tc ? int4_tc_block(numel, E, top_k) : kSimtBlock;
 
-  Routing r = make_routing(rb, numel, E, block);
+  Routing r;
   align::Job job;
-  int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? K / 8 : 0, &r, &job, stream);
+  int rc = make_routing(rb, numel, E, block, &r);
+  if (rc != XKB_OK) return rc;
+  rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? K / 8 : 0, &r, &job, stream);
   if (rc != XKB_OK) return rc;
   if (use_tc)
     rc = launch_int4_tc(A, packed, scale, r, topk_w, scratch, N, K, E, top_k, group_size,
@@ -365,9 +378,11 @@ extern "C" int xkb_fused_moe_int4_ffn(const void* A, int a_dtype, const int32_t*
                              "hidden %% 256 == 0, inter %% 256 == 0, group_size 32)");
   const bool use_tc = (path == XKB_PATH_TC) || (path == XKB_PATH_AUTO && tc_fit);
   const int block = use_tc ? int4_tc_block(numel, E, top_k) : kSimtBlock;
-  Routing r = make_routing(rb, numel, E, block);
+  Routing r;
   align::Job job;
-  int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? hidden / 8 : 0, &r, &job, stream);
+  int rc = make_routing(rb, numel, E, block, &r);
+  if (rc != XKB_OK) return rc;
+  rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? hidden / 8 : 0, &r, &job, stream);
   if (rc != XKB_OK) return rc;
   if (use_tc) {
     __nv_bfloat16* rows16 = reinterpret_cast<__nv_bfloat16*>(scratch);
@@ -441,9 +456,11 @@ extern "C" int xkb_fused_moe_mxfp4(const void* A, int a_dtype, const uint8_t* w1
   const bool use_bs = bs_block > 0;
   const int block = use_bs ? bs_block : use_tc ? mxfp4_tc_block(numel, E) : kSimtBlock;
 
-  Routing r = make_routing(rb, numel, E, block);
+  Routing r;
   align::Job job;
-  int rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? hidden / 8 : 0, &r, &job, stream);
+  int rc = make_routing(rb, numel, E, block, &r);
+  if (rc != XKB_OK) return rc;
+  rc = route(rb, topk_ids, expert_map, num_map, E, top_k, use_tc ? hidden / 8 : 0, &r, &job, stream);
   if (rc != XKB_OK) return rc;
   if (use_bs) {
     const __nv_bfloat16* rows = nullptr;
