@@ -150,11 +150,15 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   // One accumulator per issuer.  A tile has a multiple of MATS stages, so with two matrices an issuer only ever sees
   // one of them and its accumulator belongs to that.
   static constexpr int kAccs = kIssuers;
-  // Two or three accumulator sets when tensor memory has room beside three stages of A slots: the
+  // Two or four accumulator sets when tensor memory has room beside three stages of A slots: the
   // MMAs of the next tiles start while an earlier tile's accumulators still wait to be read out.
-  // (Three sets let the read-out trail two tiles behind, which short tiles need: see kEpiDelay.)
-  static constexpr int kDBuf = (3 * kAccs * BT + 3 * kSlotCols <= kTmemCols) ? 3
+  // (Short tiles need the four: see kEpiDelay.)  Tile `it` takes set it % kDBuf, and the warpgroups on read-out duty rotate
+  // by kColGroups a tile: the number of sets is such that a set always meets the same warpgroups, so that each of
+  // them waits for every phase of the barriers of its sets.  (Three sets and four warpgroups in turn would wait for one
+  // phase in four, and with one stage a tile nothing else says that the use in between is over.)
+  static constexpr int kDBuf = (4 * kAccs * BT + 3 * kSlotCols <= kTmemCols) ? 4
                                : (2 * kAccs * BT + 3 * kSlotCols <= kTmemCols) ? 2 : 1;
+  static_assert(kEpiWGs == kWGs || (kDBuf * kColGroups) % kWGs == 0, "a set is always read out by the same warpgroups");
   static constexpr int kDCols = kDBuf * kAccs * BT;         // accumulator a of set d at (d * kAccs + a) * BT
   static constexpr int kACol0 = kDCols;                     // the A slots follow the accumulators
   // A slots, counted in units (three stages' worth at most)
@@ -636,7 +640,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
       const bool live = slot >= 0 && slot < p.numel;
       w = (mode_is_int4(MODE) && !mode_is_gate_up(MODE) && p.mul_w && live) ? __ldg(p.topk_w + slot) : 1.f;
     };
-    // the first 16-column group of tile number `it` that this warpgroup reads out (kColGroups and more: none)
+    // the first 16-column group of tile number `it` that this warpgroup reads out (kColGroups and more: none); the same
+    // for all tiles of a set (kDBuf)
     auto first_group = [&](uint32_t it) -> int {
       if (Cfg::kEpiWGs == Cfg::kWGs) return wg;
       return (int)(((uint32_t)wg + (uint32_t)Cfg::kWGs - (it * (uint32_t)Cfg::kColGroups) % (uint32_t)Cfg::kWGs) % (uint32_t)Cfg::kWGs);
