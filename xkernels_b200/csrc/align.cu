@@ -53,6 +53,7 @@ align_small_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int E, i
 // ---------------------------------------------------------------------------
 // Cluster path: warp g of the cluster (kCluster * kWarps of them) takes the slots [g * segment, (g + 1) * segment)
 // ---------------------------------------------------------------------------
+// (.aligned: every lane of the warp executes it together)
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // the int at the same shared-memory address in CTA `rank` of the cluster
@@ -149,6 +150,7 @@ align_cluster_kernel(const int32_t* __restrict__ topk_ids, int64_t numel, int64_
     for (int i = off[x] + tot[x] + lane; i < off[x + 1]; i += 32) sorted_ids[i] = (int32_t)numel;
   for (int64_t i = off[E] + (int64_t)rank * kThreads + tid; i < max_pad; i += (int64_t)kCluster * kThreads) sorted_ids[i] = (int32_t)numel;
   write_expert_ids(off, tot, E, block, expert_ids, block_live, max_blocks, rank * kThreads + tid, kCluster * kThreads);
+  __syncwarp();       // the loops above end lane by lane, and the barrier takes whole warps
   cluster_wait();     // no CTA leaves while another may read its counts
 }
 
