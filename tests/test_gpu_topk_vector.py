@@ -1,6 +1,6 @@
-"""The router's loads: a lane's neighbouring logits in one load of 4, 8 or 16 bytes or several where E and the base address
-allow it, one by one elsewhere; expert counts around those that fill the lanes.  Ids exact (few distinct logits, so that
-ties cross lanes), weights within fp32 round-off of the oracle."""
+"""The router's loads: pieces of two or four neighbouring logits where E and the base address allow them, one by one
+elsewhere; expert counts around those that fill the lanes.  Ids exact (few distinct logits, so that ties cross pieces and
+lanes), weights within fp32 round-off of the oracle."""
 
 import pytest
 import torch

@@ -6,20 +6,24 @@
 // selected weights are optionally divided by their sum.  Equal logits give equal probabilities
 // here as there, so the tie rule decides the same way.
 //
-// One warp per token row: lane l holds the PER_LANE experts from l * PER_LANE on, read with as few loads as their
-// alignment allows; row maximum by one warp reduction, sum by shuffles.
+// One warp per token row.  A row is dealt to the lanes in pieces of P neighbouring experts, piece i to lane i % 32, one
+// load a piece; row maximum by one warp reduction, sum by shuffles.
 //
 // Bound by the warp's instructions, not by memory (a row of 256 bf16 logits is 512 bytes).  k rounds of
 // "best of my lane, then best of the warp" over all experts cost about 900 instructions per row, so the
 // selection first cuts the row down to a handful of candidates: the k-th largest of the 32 lane maxima
 // bounds the k-th largest element from below, usually 8 to 16 of the experts reach it, and only those
 // are divided by the sum (one per lane), ranked against each other and written.  They are collected by ascending id
-// (a lane's experts are neighbours), so a rank is a count of larger probabilities and of equal ones in lower lanes.
+// (piece by piece), so a rank is a count of larger probabilities and of equal ones in lower lanes.
 // Rows that leave more than 32 candidates (long runs of equal logits, a k-th probability near the subnormals), a top-k
 // above 32 or a sum that is not finite take the rounds (select_by_rounds), which order every probability of the row.
 // They pay for the candidates first, and make that good with two warp reductions a round instead of ten shuffles.
-// M=16384, E=256, bf16, top 8, renormalised: 28.7 us with the rounds, 10.8 with strided loads of one
-// logit, branches around the candidates' stores and a loop over all of them, 9.2 now (460 instructions a row).
+// Why small pieces in turn: rows whose live logits are neighbours (routers that mask all groups of experts but a few) have
+// to spread them over the lanes, or few lanes carry maxima, the bound gets loose and the row takes the rounds.
+// M=16384, E=256, bf16, top 8, renormalised, on the device: 28.7 us with the rounds; 10.9 with single logits dealt to the lanes
+// and a loop over all candidates; 9.3 with eight neighbours a lane, but 28.3, 17.1 and 9.6 where one, two and four groups of 32
+// are live, 22.1 for sorted rows; 9.2 with pieces of two, and 9.3, 9.4, 9.5 and 9.5 for those rows.  (E=1024, where the
+// rounds are common: top 8 34.4 / 21.0 / 20.5, top 20 158 / 105 / 114, top 32 227 / 165 / 181.)
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -41,8 +45,11 @@ template <> __device__ __forceinline__ float load_logit<__nv_bfloat16>(const __n
 }
 template <> __device__ __forceinline__ float load_logit<__half>(const __half* p) { return __half2float(*p); }
 
-// k rounds over the whole row: p[t] = probability of expert lane * PER_LANE + t, or -1 where there is none.
-template <int PER_LANE>
+// The id of a lane's t-th expert is lane * P plus this; a lane's ids ascend with t.
+template <int P> struct Deal { static __device__ __forceinline__ constexpr int at(int t) { return t / P * 32 * P + t % P; } };
+
+// k rounds over the whole row: p[t] = probability of the lane's t-th expert, or -1 where there is none.
+template <int PER_LANE, int P>
 __device__ __forceinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t row, int lane, int topk, int renormalize,
                                               float* __restrict__ topk_w, int32_t* __restrict__ topk_ids) {
   float wsum = 0.f;
@@ -52,17 +59,17 @@ __device__ __forceinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t r
     int bt = 0;
 #pragma unroll
     for (int t = 0; t < PER_LANE; ++t)   // a lane's ids ascend: the first of equal ones stays
-      if (p[t] > bp) { bp = p[t]; bt = t; }
-    int bi = bp >= 0.f ? lane * PER_LANE + bt : 0x7fffffff;
+      if (p[t] > bp) { bp = p[t]; bt = Deal<P>::at(t); }
+    const int mine = bp >= 0.f ? lane * P + bt : 0x7fffffff;
     // best of the warp: bp is -1 or >= 0 and never NaN (no comparison with one holds), so its bits order as signed integers
     const int top = __reduce_max_sync(0xffffffffu, __float_as_int(bp));
-    bi = __reduce_min_sync(0xffffffffu, __float_as_int(bp) == top ? bi : 0x7fffffff);
+    const int bi = __reduce_min_sync(0xffffffffu, __float_as_int(bp) == top ? mine : 0x7fffffff);
     bp = __int_as_float(top);
     // every lane now holds the same winner; its owner retires it
     // (bi of no expert: every remaining probability is NaN, and nothing is retired)
 #pragma unroll
     for (int t = 0; t < PER_LANE; ++t)
-      if (t == bi - lane * PER_LANE) p[t] = -1.f;
+      if (Deal<P>::at(t) == bi - lane * P) p[t] = -1.f;
     wsum += bp;
     if (lane == 0) topk_ids[row * topk + j] = bi;
     if (renormalize) {
@@ -91,27 +98,20 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// PER_LANE neighbouring logits.  VEC: E is a multiple of PER_LANE and every lane's first one lies on a VEC-byte boundary.
-template <typename T, int PER_LANE, int VEC>
-__device__ __forceinline__ void load_lane(const T* row, int lane, int E, float (&v)[PER_LANE]) {
-  if constexpr (VEC == 0) {
-#pragma unroll
-    for (int t = 0; t < PER_LANE; ++t) v[t] = lane * PER_LANE + t < E ? load_logit<T>(row + lane * PER_LANE + t) : -INFINITY;
-  } else {
-    constexpr int kPer = VEC / (int)sizeof(T);
-    struct alignas(VEC) Chunk { T x[kPer]; };
-#pragma unroll
-    for (int c = 0; c < PER_LANE / kPer; ++c) {
-      Chunk q;
-      if (lane * PER_LANE < E) q = reinterpret_cast<const Chunk*>(row + lane * PER_LANE)[c];
-#pragma unroll
-      for (int i = 0; i < kPer; ++i) v[c * kPer + i] = lane * PER_LANE < E ? load_logit<T>(&q.x[i]) : -INFINITY;
-    }
-  }
+// Counts of up to four or eight pieces, eight bits each.
+template <bool WIDE> struct FieldsOf { using type = uint32_t; };
+template <> struct FieldsOf<true> { using type = unsigned long long; };
+__device__ __forceinline__ int sum_of_fields(uint32_t v) { return (int)__dp4a(v, 0x01010101u, 0u); }
+__device__ __forceinline__ int sum_of_fields(unsigned long long v) {
+  return (int)__dp4a((uint32_t)(v >> 32), 0x01010101u, __dp4a((uint32_t)v, 0x01010101u, 0u));
 }
 
-template <typename T, int PER_LANE, int VEC>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+// Experts per lane, in the order of the instances: an instance takes the rows that the one before it does not hold.
+template <int PER_LANE> constexpr int kPerLaneBefore = PER_LANE == 16 ? 12 : PER_LANE == 12 ? 8 : PER_LANE / 2;
+
+// P > 1: E is a multiple of P and every row lies on a boundary of P logits, so that a piece is in the row or not.
+template <typename T, int PER_LANE, int P>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, PER_LANE == 32 ? 0 : 1)   // (1 against 0, which leaves it open: E=256 9.2 / 9.4 us, E=1024 23.7 / 20.4)
 topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, int32_t* __restrict__ topk_ids,
                     int64_t M, int E, int topk, int renormalize) {
   __shared__ uint2 s_cand[kWarpsPerBlock][32];   // candidates by ascending id: exponential, id
@@ -119,26 +119,37 @@ topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, in
   const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
   if (row >= M) return;
 
+  constexpr int kPieces = PER_LANE / P;
+  constexpr int kSure = kPerLaneBefore<PER_LANE>;   // the lane's first experts are in every row of this instance
+  auto valid = [&](int t) -> bool { return t < kSure || (t / P * 32 + lane) * P < E; };
+  struct alignas(P * sizeof(T)) Piece { T x[P]; };
+  const Piece* x = reinterpret_cast<const Piece*>(gating + row * E);
   float p[PER_LANE];
-  load_lane<T, PER_LANE, VEC>(gating + row * E, lane, E, p);
-  // a lane's experts are all in the row or none is (VEC), or one by one
-  const bool in_row = VEC == 0 || lane * PER_LANE < E;
-  auto valid = [&](int t) -> bool { return VEC != 0 || lane * PER_LANE + t < E; };
+#pragma unroll
+  for (int c = 0; c < kPieces; ++c) {
+    Piece q;
+#pragma unroll
+    for (int i = 0; i < P; ++i) q.x[i] = T(-INFINITY);
+    if (valid(c * P)) q = x[c * 32 + lane];
+#pragma unroll
+    for (int i = 0; i < P; ++i) p[c * P + i] = load_logit<T>(&q.x[i]);
+  }
   float mx = p[0];
 #pragma unroll
   for (int t = 1; t < PER_LANE; ++t) mx = fmaxf(mx, p[t]);
   mx = warp_max(mx);
-  float sum = 0.f, lane_max = -1.f;
+  // (experts behind the row: -inf, which is 0 here unless the whole row is -inf or NaN, and then the sum is NaN)
+  float sum = 0.f, lane_max = 0.f;
 #pragma unroll
   for (int t = 0; t < PER_LANE; ++t) {
-    p[t] = valid(t) ? expf(p[t] - mx) : -1.f;    // -1 marks "not a candidate" (exponentials are >= 0)
-    sum += valid(t) ? p[t] : 0.f;
+    p[t] = expf(p[t] - mx);
+    sum += p[t];
     lane_max = fmaxf(lane_max, p[t]);
   }
-  sum = warp_sum(in_row ? sum : 0.f);
+  sum = warp_sum(sum);
 
   // The k-th largest lane maximum (equal ones leave together, so it may be a smaller one: still a bound).
-  float tau = -1.f, lm = in_row ? lane_max : -1.f;
+  float tau = -1.f, lm = lane_max;
   const bool short_way = topk <= (PER_LANE == 1 ? 32 : kShortTopk) && sum < INFINITY;   // (a NaN sum fails the comparison)
   if (short_way) {
     int j = topk;
@@ -162,30 +173,59 @@ topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, in
   float bound = 0.f;
   if (short_way && tau >= 0.f && tau >= sum * 7.8886090522101181e-31f)   // 2^-100
     bound = tau * (1.f - 9.5367431640625e-7f);
-  int mine = 0;
+  // an exponential is a candidate from here on; experts behind the row never are (none is infinite on the short way)
+  auto low = [&](int t) -> float { return valid(t) ? bound : INFINITY; };
+  // Candidates are counted piece by piece.  P > 1: a lane's counts are fields of eight bits (a piece has at most 128
+  // candidates in the warp), so that one sum over the lanes serves all pieces.
+  using Fields = typename FieldsOf<(kPieces > 4)>::type;
+  Fields mine = 0, upto = 0, all = 0;   // this lane's, the lanes' up to it, the warp's
+  int n = 0;
+  if constexpr (P > 1) {
 #pragma unroll
-  for (int t = 0; t < PER_LANE; ++t) mine += p[t] >= bound ? 1 : 0;
-  if (!in_row) mine = 0;
-  int at = mine;   // inclusive sum over the lanes
+    for (int t = 0; t < PER_LANE; ++t) mine += p[t] >= low(t) ? Fields(1) << (8 * (t / P)) : Fields(0);
+    upto = mine;
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const int below = __shfl_up_sync(0xffffffffu, at, d);
-    if (lane >= d) at += below;
+    for (int d = 1; d < 32; d <<= 1) {
+      const Fields below = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto += below;
+    }
+    all = __shfl_sync(0xffffffffu, upto, 31);
+    n = sum_of_fields(all);
+  } else {
+#pragma unroll
+    for (int t = 0; t < PER_LANE; ++t) n += __popc(__ballot_sync(0xffffffffu, p[t] >= low(t)));
   }
-  const int n = __shfl_sync(0xffffffffu, at, 31);
   if (!short_way || n > 32) {
 #pragma unroll
-    for (int t = 0; t < PER_LANE; ++t) p[t] = in_row && valid(t) ? p[t] / sum : -1.f;
-    select_by_rounds<PER_LANE>(p, row, lane, topk, renormalize, topk_w, topk_ids);
+    for (int t = 0; t < PER_LANE; ++t) p[t] = valid(t) ? p[t] / sum : -1.f;
+    select_by_rounds<PER_LANE, P>(p, row, lane, topk, renormalize, topk_w, topk_ids);
     return;
   }
   uint2* cand = s_cand[warp];
-  uint32_t to = (uint32_t)__cvta_generic_to_shared(cand + (at - mine));
-  const float low = in_row ? bound : INFINITY;
+  const uint32_t cand_u32 = (uint32_t)__cvta_generic_to_shared(cand);
+  if constexpr (P > 1) {
+    const Fields first = upto - mine + all * Fields(0x0101010101010100ull);   // (the fields before it, and the lanes before)
 #pragma unroll
-  for (int t = 0; t < PER_LANE; ++t)   // predicated: a branch each took twice as many instructions
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ge.f32 q, %1, %2;\n\t@q st.shared.v2.b32 [%0], {%3, %4};\n\t@q add.u32 %0, %0, 8;\n\t}"
-                 : "+r"(to) : "f"(p[t]), "f"(low), "r"(__float_as_uint(p[t])), "r"(lane * PER_LANE + t) : "memory");
+    for (int c = 0; c < kPieces; ++c) {
+      uint32_t to = cand_u32 + (uint32_t)(first >> (8 * c) & 0xFFu) * 8u;
+#pragma unroll
+      for (int i = 0; i < P; ++i)   // predicated: a branch each took twice as many instructions
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ge.f32 q, %1, %2;\n\t@q st.shared.v2.b32 [%0], {%3, %4};\n\t@q add.u32 %0, %0, 8;\n\t}"
+                     : "+r"(to) : "f"(p[c * P + i]), "f"(low(c * P)), "r"(__float_as_uint(p[c * P + i])),
+                       "r"(lane * P + Deal<P>::at(c * P + i))
+                     : "memory");
+    }
+  } else {
+    uint32_t to = cand_u32;
+#pragma unroll
+    for (int t = 0; t < PER_LANE; ++t) {
+      const unsigned who = __ballot_sync(0xffffffffu, p[t] >= low(t));
+      asm volatile("{\n\t.reg .pred q;\n\tsetp.ge.f32 q, %1, %2;\n\t@q st.shared.v2.b32 [%0], {%3, %4};\n\t}"
+                   :: "r"(to + (uint32_t)__popc(who & ((1u << lane) - 1u)) * 8u), "f"(p[t]), "f"(low(t)), "r"(__float_as_uint(p[t])),
+                      "r"(t * 32 + lane) : "memory");
+      to += (uint32_t)__popc(who) * 8u;
+    }
+  }
   __syncwarp();
   // one candidate per lane
   float prob = -1.f;
@@ -211,23 +251,23 @@ topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, in
   }
 }
 
-// the widest load of 16 bytes or less that a lane's `bytes` are a multiple of (at least two logits), 0: one by one
-constexpr int lane_vec(int bytes) { return bytes % 16 == 0 ? 16 : bytes % 8 == 0 ? 8 : bytes == 4 ? 4 : 0; }
+// Experts of a piece.  Wider ones take fewer loads and spread less: E=256 with pieces of four 9.1 us for independent logits
+// and 14.3, 12.4 for one and two live groups, of two 9.2 and 9.3, 9.4; E=128 with pieces of two 7.9 and 9.7 for two live
+// groups of sixteen, of one 7.8 and 7.8.  From 257 experts on a live group is rarely that small.
+constexpr int piece_of(int per_lane) { return per_lane <= 4 ? 1 : per_lane == 8 ? 2 : 4; }
 
 template <typename T>
 int launch_for_type(const void* gating, float* w, int32_t* ids, int64_t M, int E, int topk, int renorm,
                     cudaStream_t s) {
   const unsigned blocks = (unsigned)ceil_div(M, (int64_t)kWarpsPerBlock);
   const T* g = static_cast<const T*>(gating);
-  // neighbours per lane: the fewest that cover the row.  Loads of up to 16 bytes where every lane's first logit lies
-  // on them, of one logit otherwise.
+  // the fewest experts per lane that cover the row; single logits where pieces would straddle its ends or their alignment
   const int per_lane = (E + 31) / 32;
-  const uintptr_t odd = reinterpret_cast<uintptr_t>(gating) | (uintptr_t)(E * (int64_t)sizeof(T));
 #define XKB_TS_CASE(PL)                                                                                  \
   if (per_lane <= PL) {                                                                                  \
-    constexpr int kVec = lane_vec(PL * (int)sizeof(T));                                                  \
-    const bool vec = kVec > 0 && E % PL == 0 && odd % (kVec > 0 ? kVec : 1) == 0;                                     \
-    (vec ? topk_softmax_kernel<T, PL, kVec> : topk_softmax_kernel<T, PL, 0>)<<<blocks, 32 * kWarpsPerBlock, 0, s>>>( \
+    constexpr int kP = piece_of(PL);                                                                     \
+    const bool whole = E % kP == 0 && reinterpret_cast<uintptr_t>(gating) % (kP * sizeof(T)) == 0;       \
+    (whole ? topk_softmax_kernel<T, PL, kP> : topk_softmax_kernel<T, PL, 1>)<<<blocks, 32 * kWarpsPerBlock, 0, s>>>( \
         g, w, ids, M, E, topk, renorm);                                                                  \
     XKB_CHECK_LAUNCH("topk_softmax_kernel");                                                             \
     return XKB_OK;                                                                                       \
