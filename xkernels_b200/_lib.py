@@ -1,5 +1,5 @@
-"""Binding of ``libxkb200.so`` — the only route from Python to the kernels: ctypes, and a native call path for plain
-calls of the small ops.
+"""Binding of ``libxkb200.so`` — the only route from Python to the kernels: ctypes, and, where it is built for this torch, a
+native call path for plain calls of the small ops.
 
 The library is built in-tree by :mod:`xkernels_b200.build`.  There is no CPU or
 eager fallback: if the shared object is missing or fails to load, importing any
@@ -11,11 +11,16 @@ from __future__ import annotations
 import ctypes
 import importlib.machinery
 import importlib.util
+import sys
 from ctypes import c_char_p, c_float, c_int, c_int64, c_void_p
 from pathlib import Path
 
+import torch
+
 LIB_PATH = Path(__file__).resolve().parent / "libxkb200.so"
-CALLS_PATH = Path(__file__).resolve().parent / "_torch_calls.so"
+# The call path is compiled against torch's and Python's headers: its name says which, so that a file built for others is
+# never loaded.
+CALLS_PATH = Path(__file__).resolve().parent / f"_torch_calls.{sys.implementation.cache_tag}-torch{torch.__version__}.so"
 
 XKB_BF16 = 0
 XKB_F32 = 1
@@ -119,17 +124,29 @@ def load() -> ctypes.CDLL:
 _calls = None
 
 
+class PythonCalls:
+    """In the place of the native call path where there is none for this torch: every call is the Python form's."""
+
+    @staticmethod
+    def _not_served(*args):
+        return None
+
+    topk_softmax = moe_align_block_size = moe_sum_reduce = _not_served
+
+
 def load_calls():
-    """The native call path of the small ops (``csrc/torch_calls.cpp``), bound to the library's functions."""
+    """The native call path of the small ops (``csrc/torch_calls.cpp``), bound to the library's functions.  It only
+    saves host time: without it (:data:`CALLS_PATH` is missing) the Python form makes the same library calls."""
     global _calls
     if _calls is not None:
         return _calls
+    lib = load()
     if not CALLS_PATH.exists():
-        raise RuntimeError(f"{CALLS_PATH} is missing: build it with `python -m xkernels_b200.build` (there is no fallback path)")
+        _calls = PythonCalls
+        return _calls
     loader = importlib.machinery.ExtensionFileLoader("_torch_calls", str(CALLS_PATH))
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_torch_calls", loader))
     loader.exec_module(module)
-    lib = load()
     module.bind(*(ctypes.cast(fn, c_void_p).value for fn in (
         lib.xkb_topk_softmax, lib.xkb_moe_align_block_size, lib.xkb_moe_align_workspace_bytes, lib.xkb_moe_sum_reduce)))
     _calls = module

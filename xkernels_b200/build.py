@@ -1,5 +1,5 @@
-"""Builds ``libxkb200.so`` (the C-ABI library of sm_100a kernels) in-tree with nvcc, and ``_torch_calls.so`` (the native
-call path of the small ops) with the host compiler.
+"""Builds ``libxkb200.so`` (the C-ABI library of sm_100a kernels) in-tree with nvcc, and the native call path of the small
+ops (``_torch_calls.*.so``, for the torch and Python that run the build) with the host compiler.
 
 Run ``python -m xkernels_b200.build`` or call :func:`build`.  The objects are
 compiled in parallel, one nvcc process per ``.cu`` file, and linked into
@@ -14,15 +14,15 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
-import torch
+from ._lib import CALLS_PATH
 
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libxkb200.so"
-CALLS_PATH = PKG_DIR / "_torch_calls.so"
 OBJ_DIR = PKG_DIR / "build"
 
 NVCC_FLAGS = [
@@ -50,18 +50,28 @@ def _fingerprint() -> str:
                     + [PKG_DIR.parent / "include" / "xkb200.h"]):
         h.update(p.name.encode())
         h.update(p.read_bytes())
-    h.update((CSRC / "torch_calls.cpp").read_bytes())
-    h.update(f"{torch.__version__} {sys.version}".encode())
     h.update(" ".join(NVCC_FLAGS).encode())
     return h.hexdigest()
 
 
 def is_current() -> bool:
     stamp = OBJ_DIR / "fingerprint"
-    return LIB_PATH.exists() and CALLS_PATH.exists() and stamp.exists() and stamp.read_text() == _fingerprint()
+    return LIB_PATH.exists() and stamp.exists() and stamp.read_text() == _fingerprint()
 
 
-def _build_calls() -> None:
+def _calls_fingerprint() -> str:
+    h = hashlib.sha256((CSRC / "torch_calls.cpp").read_bytes())
+    h.update((PKG_DIR.parent / "include" / "xkb200.h").read_bytes())
+    return f"{CALLS_PATH.name} {sys.version} {h.hexdigest()}"
+
+
+def calls_are_current() -> bool:
+    stamp = OBJ_DIR / "calls_fingerprint"
+    return CALLS_PATH.exists() and stamp.exists() and stamp.read_text() == _calls_fingerprint()
+
+
+def _compile_calls() -> None:
+    import torch
     from torch.utils import cpp_extension as ext
 
     cxx = os.environ.get("CXX") or shutil.which("g++") or "c++"
@@ -71,13 +81,29 @@ def _build_calls() -> None:
            *(f"-L{d}" for d in ext.library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
-        raise RuntimeError(f"build of _torch_calls.so failed:\n{res.stdout}\n{res.stderr}")
+        raise RuntimeError(f"build of {CALLS_PATH.name} failed:\n{res.stdout}\n{res.stderr}")
 
 
-def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every ``csrc/*.cu`` for sm_100a and link the shared library; compile the call path beside it."""
+def build_calls(force: bool = False) -> bool:
+    """Compile the native call path for this torch and Python.  Returns whether it is there: it needs a host compiler and
+    both's headers, and without them the ops take their Python form, so a failure is a warning."""
+    if not force and calls_are_current():
+        return True
+    OBJ_DIR.mkdir(exist_ok=True)
+    CALLS_PATH.unlink(missing_ok=True)   # never the path of another source
+    try:
+        _compile_calls()
+    except (ImportError, OSError, RuntimeError) as e:
+        warnings.warn(f"the small ops take their Python form, 5 to 8 us more of host time a call: {e}", stacklevel=2)
+        return False
+    (OBJ_DIR / "calls_fingerprint").write_text(_calls_fingerprint())
+    return True
+
+
+def build_library(force: bool = False, verbose: bool = False) -> None:
+    """Compile every ``csrc/*.cu`` for sm_100a and link the shared library."""
     if not force and is_current():
-        return LIB_PATH
+        return
     nvcc = _nvcc()
     OBJ_DIR.mkdir(exist_ok=True)
     extra = ["-Xptxas", "-v"] if verbose else []
@@ -93,14 +119,20 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         return obj
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
-        calls = pool.submit(_build_calls)
         objs = list(pool.map(compile_one, _sources()))
-        calls.result()
     cmd = [nvcc, "-shared", "-o", str(LIB_PATH), *map(str, objs)]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link of libxkb200.so failed:\n{res.stdout}\n{res.stderr}")
     (OBJ_DIR / "fingerprint").write_text(_fingerprint())
+
+
+def build(force: bool = False, verbose: bool = False) -> Path:
+    """Build what is not current: the library, and the call path beside it."""
+    with ThreadPoolExecutor(max_workers=1) as pool:
+        calls = pool.submit(build_calls, force)
+        build_library(force, verbose)
+        calls.result()
     return LIB_PATH
 
 
