@@ -134,6 +134,14 @@ int xkb_moe_sum_reduce(const void* y, int y_dtype, const void* w, int w_dtype,
                        void* out, int out_dtype, int64_t M, int top_k,
                        int64_t H, float routed_scaling_factor, void* stream);
 
+/* The token tile (positions of a token block) that a fused call picks on the
+ * tensor cores, from its number of slots; no GPU is needed to ask.  INT4: 16,
+ * 32, 64 or 128.  MXFP4, with weights on 32 bytes: 8, 16 or 32 of the
+ * block-scaled kernel, 128 of the kernel that converts weights to bf16.  No
+ * reference counterpart. */
+int xkb_int4_token_tile(int64_t numel, int num_experts, int top_k);
+int xkb_mxfp4_token_tile(int64_t numel, int num_experts);
+
 /* Token blocks that a fused call's workspace has room for, whatever block size
  * the call picks (a block is a token tile: some positions of one expert).
  * -1 for a negative argument.  No reference counterpart. */

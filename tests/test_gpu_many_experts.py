@@ -7,14 +7,10 @@ import torch
 
 import xkernels_b200 as xkb
 from oracle import moe_oracle as oracle
-from tests.gpu_util import assert_within
-from xkernels_b200 import _lib, ops, synth
+from tests.gpu_util import assert_within, poisoned_workspace
+from xkernels_b200 import ops, synth
 
 pytestmark = pytest.mark.gpu
-
-
-def _workspace(nbytes, dev):
-    return torch.full((nbytes,), 0xFF, dtype=torch.uint8, device=dev)   # NaN as bf16 and as fp32
 
 
 @pytest.mark.parametrize("path", ["tc", "simt"])
@@ -27,7 +23,7 @@ def test_int4(E, M, top_k, path, cuda_device):
     ids, w = synth.routing(M, E, top_k, seed=7)
     want = oracle.moe_w4a16(A, packed, scale, ids, w, 32)
     args = [t.to(cuda_device) for t in (A, packed, scale, ids, w)]
-    ws = _workspace(_lib.load().xkb_fused_moe_int4_w4a16_workspace_bytes(M, N, K, E, top_k, 0), cuda_device)
+    ws = poisoned_workspace("xkb_fused_moe_int4_w4a16_workspace_bytes", M, N, K, E, top_k, 0, device=cuda_device)
     for _ in range(3):
         ws.fill_(0xFF)
         got = xkb.fused_moe_int4_w4a16(*args, workspace=ws, path=path)
@@ -43,7 +39,7 @@ def test_mxfp4_generic_path(E, M, top_k, cuda_device):
     ids, w = synth.routing(M, E, top_k, seed=7)
     want = oracle.moe_mxfp4(A, t["w13"], t["w13_scale"], t["w2"], t["w2_scale"], ids, w)
     dev = [x.to(cuda_device) for x in (A, t["w13"], t["w13_scale"], t["w2"], t["w2_scale"], ids, w)]
-    ws = _workspace(_lib.load().xkb_fused_moe_mxfp4_workspace_bytes(M, hidden, ispp, E, top_k), cuda_device)
+    ws = poisoned_workspace("xkb_fused_moe_mxfp4_workspace_bytes", M, hidden, ispp, E, top_k, device=cuda_device)
     got = xkb.fused_moe_mxfp4(*dev, workspace=ws)
     ops.check_workspace_status(ws)
     assert_within(got, want, 2e-2, 1e-2, what=f"E={E} M={M}", allowed=max(1, want.numel() // 2000))

@@ -7,7 +7,7 @@ import torch
 
 import xkernels_b200 as xkb
 from oracle import moe_oracle as oracle
-from tests.gpu_util import assert_within
+from tests.gpu_util import assert_within, int4_tile
 from xkernels_b200 import ops, synth
 
 pytestmark = pytest.mark.gpu
@@ -17,6 +17,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("M,E,N,group", [(8, 16, 16384, 32), (1, 8, 16384, 32), (3, 8, 8192 + 128, 32)])
 def test_int4(M, E, N, group, K, cuda_device):
     top_k = 8
+    assert int4_tile(M, E, top_k) == 16
     A = synth.activations(M, K, seed=M)
     packed, scale = synth.int4_weights(E, N, K, group, seed=E)
     ids, w = synth.routing(M, E, top_k, seed=7)

@@ -71,6 +71,8 @@ SIGNATURES = {
         [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_int, c_int,
          c_int, c_void_p, c_int64, c_void_p],
     ),
+    "xkb_int4_token_tile": (c_int, [c_int64, c_int, c_int]),
+    "xkb_mxfp4_token_tile": (c_int, [c_int64, c_int]),
     "xkb_routing_blocks": (c_int64, [c_int64, c_int]),
     "xkb_set_sm_margin": (c_int, [c_int]),
     "xkb_ep_plan_workspace_bytes": (c_int64, [c_int64, c_int, c_int, c_int]),

@@ -174,6 +174,11 @@ extern "C" const char* xkb_version(void) { return "xkb200 0.1 (sm_100a)"; }
 extern "C" const char* xkb_last_error(void) { return last_error_buf(); }
 extern "C" int64_t xkb_launch_count(void) { return g_launches.load(); }
 
+extern "C" int xkb_int4_token_tile(int64_t numel, int E, int top_k) { return int4_tc_block(numel, E, top_k); }
+extern "C" int xkb_mxfp4_token_tile(int64_t numel, int E) {
+  const int block = mxfp4_bs_block(numel, E);
+  return block > 0 ? block : mxfp4_tc_block(numel, E);
+}
 extern "C" int64_t xkb_routing_blocks(int64_t numel, int E) { return numel < 0 || E < 0 ? -1 : routing_max_blocks(numel, E); }
 
 // ---------------------------------------------------------------------------
