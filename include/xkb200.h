@@ -62,8 +62,9 @@ int64_t xkb_launch_count(void);
  * expert_offsets NULL or [num_experts+1] int32: start of each expert's padded
  *               run in sorted_ids (entry num_experts = num_post_pad).
  * workspace     xkb_moe_align_workspace_bytes(numel, num_experts) bytes.  Calls of up
- *               to 8192 slots may pass less or none (NULL, 0): one thread block
- *               then does the whole sort, from 1025 slots on in more time.
+ *               to 8192 slots may pass less or none (NULL, 0): they are sorted in one
+ *               launch without it (so are those of up to 16384, whose
+ *               workspace is required all the same).
  * ---------------------------------------------------------------------- */
 int64_t xkb_moe_align_workspace_bytes(int64_t numel, int num_experts);
 int xkb_moe_align_block_size(const int32_t* topk_ids, int64_t numel,

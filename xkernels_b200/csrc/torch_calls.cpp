@@ -109,7 +109,7 @@ PyObject* moe_align_block_size(PyObject*, PyObject* const* args, Py_ssize_t n) {
   at::Tensor sorted = at::empty({max_pad}, opt), experts = at::empty({max_blocks}, opt), post = at::empty({1}, opt), ws;
   void* ws_ptr = nullptr;
   int64_t ws_bytes = 0;
-  if (numel > 1024) {   // one block sorts up to 1024 slots without scratch memory
+  if (numel > 8192) {   // up to there the sort takes no scratch memory
     ws_bytes = (g_align_bytes(numel, (int)E) + 3) / 4 * 4;
     ws = at::empty({ws_bytes / 4}, opt);
     ws_ptr = ws.mutable_data_ptr();
