@@ -65,7 +65,7 @@ template <int BT> struct MxCfg {
   static constexpr int kScSlots = kStages > 5 ? 3 : 2;
   static_assert(kStages <= 4 * kScSlots - 3, "scale slots");
   static constexpr int kScBytes = 2 * kRows * 16 + BT * 16;
-  static_assert(kTokBytes >= (kMmaTokens - kTermRows) * kStageK, "the rows read behind the last stage lie in the scale tiles");
+  static_assert(kScSlots * kScBytes >= (kMmaTokens - kTermRows) * kStageK, "the rows read behind the last stage lie in the scale tiles");
   // columns: accumulator sets of two matrices, then per stage 4 gate + 4 up + 4 token scale columns
   static constexpr int kScStageCols = 12;
   static constexpr int kScCols = kScStageCols * kStages;

@@ -5,13 +5,13 @@
 // tokens of one expert block), so a decode batch with a handful of tokens per
 // expert still fills the 128-row datapath and the kernel's cost is the weight
 // stream.  One persistent CTA per SM (it owns all 512 tensor-memory columns),
-// twenty or twenty-one warps, everything handed over in whole 256-K stages:
+// twenty warps, everything handed over in whole 256-K stages:
 //
 //   warp 0   TMA producer, weights: packed tile [128 rows x 128 B] (128B swizzle, so that one
 //            row per thread reads conflict-free) + scale tile per stage: bf16 [128 x 8] for INT4,
 //            e8m0 bytes [128 x 16] for MXFP4 (sixteen bytes are the smallest TMA row, so a tile
 //            carries the scales of two stages and each stage uses its half).
-//   then     two to four MMA issuer warps (one elected lane each; warp 1 also allocates and frees tensor
+//   then     two MMA issuer warps (one elected lane each; warp 1 also allocates and frees tensor
 //            memory): tcgen05.mma kind::f16, A from tensor memory, B from shared
 //            memory, fp32 accumulators in tensor memory.  They take whole stages in
 //            turn, each into its own accumulator.
@@ -64,7 +64,6 @@ constexpr int kWStagesNarrow = 6;      // weight ring depth for token tiles of 1
 constexpr int kBStages16 = 9;          // token ring depth for token tiles of 16
 constexpr uint32_t kProdSleepNs = 400; // back-off of the TMA producers, which run a whole ring ahead
 constexpr uint32_t kIssSleepNs = 32;   // back-off of the MMA issuers (on the critical path: short)
-constexpr int kNarrowWGs = 4;          // dequantiser warpgroups for token tiles <= 64
 // Hand-off units per 256-K stage (1 = the whole stage, or one unit per warpgroup that shares the
 // stage): every unit has its own tensor-memory slot and its own full/empty barriers, so its MMAs
 // start as soon as its warpgroup has published it and its slot is free again as soon as they end.
@@ -74,10 +73,10 @@ constexpr int kUnitsWide = 4;          // token tiles of 128: four warpgroups sh
 // further stages of their own: the last MMAs of the tile (about one conversion time of issue and
 // commit latency behind the conversion) have then long completed and the read-out never waits.
 constexpr int kEpiDelay = 2;
-// The dequantiser warps hand a weight stage back to the TMA producer as soon as they have read it
-// from shared memory into registers, before they convert it (one arrival per warp of the group):
-// the turn-round of a ring slot (TMA latency + wait for the readers + their wake-up) then does not
-// contain the conversion time.
+// The dequantiser warps hand a weight stage back to the TMA producer when they have read it
+// from shared memory into registers and the slot for it is free, before they convert it (one arrival per warp
+// of the group): the turn-round of a ring slot (TMA latency + wait for the readers + their wake-up) then does
+// not contain the conversion time.
 constexpr int kTmemCols = 512;     // one CTA per SM owns all of tensor memory
 // Token stages are made of groups of eight tokens, [8 x 256] bf16 as four swizzle atoms [8 x 64].  One TMA request
 // loads kTokBox tokens, and only as many are made as the block's slots need.
@@ -109,7 +108,7 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   // its four units together, and the last waited in its slot for the MMAs of three: MXFP4 M=4096 630 -> 609 us, M=8000
   // 1144 -> 1100; the INT4 modes, whose conversion is shorter, run the same.)
   // dequantiser warpgroups (the four warps of one cover the four tensor-memory lane quarters)
-  static constexpr int kWGs = (BT <= 64) ? kNarrowWGs : 4;
+  static constexpr int kWGs = 4;
   static constexpr int kDequantWarps = 4 * kWGs;
   // Read-out of a tile's accumulators: one task per 16 token columns.  A tile with fewer tasks than
   // warpgroups (token tiles of 16 and 32) is read out by kEpiWGs warpgroups only, and the duty
@@ -117,7 +116,7 @@ template <int BT, int MATS = 1, bool INT4 = true> struct TcCfg {
   // its share of the conversion.
   static constexpr int kColGroups = BT / 16;
   static constexpr int kEpiWGs = kColGroups < kWGs ? kColGroups : kWGs;
-  // Control warps: weight producer, the issuers, token producer.  (Twenty warps get 96 registers each, 21 and more 80.)
+  // Control warps: weight producer, the issuers, token producer.  (Twenty warps get 96 registers each, more would get 80.)
   static constexpr int kIssuers = 2;
   static constexpr int kCtrlWarps = 2 + kIssuers;
   static constexpr int kThreads = 32 * (kCtrlWarps + kDequantWarps);
@@ -392,10 +391,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     *abort_word = 0;
     mbar_fence_init();
   }
-  // the token producer gets a warp of its own when the issuers leave one free (two threads of one warp
-  // that both poll with back-off slow each other down); otherwise it shares the weight producer's
   constexpr int kCtrlWarps = Cfg::kCtrlWarps;
-  constexpr int kTokWarp = kCtrlWarps - 1, kTokLane = 0;   // a warp of its own: two polling threads in one warp slow each other down
+  constexpr int kTokWarp = kCtrlWarps - 1;   // a warp of its own: two threads of one warp that both poll slow each other down
   if (Cfg::kLut) {   // byte -> (bf16 of the low code, bf16 of the high code), one copy per lane/bank
     for (int i = threadIdx.x; i < 256 * 32; i += Cfg::kThreads) {
       const uint32_t b = (uint32_t)i >> 5;
@@ -404,7 +401,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
   }
   if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
   if (warp == 0 && lane == 0) { prefetch_tensormap(&tm_packed); prefetch_tensormap(&tm_scale); }
-  if (warp == kTokWarp && lane == kTokLane) prefetch_tensormap(&tm_tokens);
+  if (warp == kTokWarp && lane == 0) prefetch_tensormap(&tm_tokens);
   // Block hand-over between the two GEMMs of an expert layer.  The second GEMM is launched as a
   // programmatic dependent of the first and does NOT wait for the first grid to complete: its CTAs
   // become resident as CTAs of the first exit (a CTA owns its SM), stream their weights at once and
@@ -482,8 +479,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         }
       }
     }
-  } else if (warp == kTokWarp && lane == kTokLane) {
-    // ---------------- token producer (diverged from lane 0; both make progress independently) ----------------
+  } else if (warp == kTokWarp && lane == 0) {
+    // ---------------- token producer ----------------
     {
       uint32_t st = 0, tb = 0;   // token stage slot and running number of the token stage
       int ready_b = -1;          // block hand-over: last block whose activations are known to be complete
@@ -531,8 +528,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
   } else if (warp >= 1 && warp < kCtrlWarps) {
     // ---------------- MMA issuers ----------------
     // Stage g (numbered across the tiles of this CTA) belongs to issuer g % kIssuers: it waits for
-    // the A slot and the token stage, hands the weight stage back to the producer, issues the
-    // sixteen M=128 N=BT K=16 MMAs into its own accumulator of the stage's matrix and commits.
+    // the A slot and the token stage, issues the sixteen M=128 K=16 MMAs of the block's slots (N of them, rounded up)
+    // into its own accumulator of the stage's matrix and commits.
     constexpr int kIssuers = Cfg::kIssuers;
     const uint32_t me = warp - 1;
     if (me < (uint32_t)kIssuers) {
@@ -596,7 +593,6 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
           if (!ok) break;
           // on to this issuer's next stage
           aq0 += kDU; if (aq0 >= (uint32_t)Cfg::kASlots) aq0 -= Cfg::kASlots;
-          if (kDU >= (uint32_t)Cfg::kASlots && aq0 >= (uint32_t)Cfg::kASlots) aq0 -= Cfg::kASlots;
           ab0 += kDU; if (ab0 >= (uint32_t)Cfg::kABars) { ab0 -= Cfg::kABars; acyc ^= 1u; }
           // a two-matrix tile shares a token stage between the matrices: with kIssuers == kMats every
           // own stage is a new token stage; otherwise the step is kIssuers / kMats token stages
@@ -775,11 +771,11 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
       }
       return true;
     };
-    // Read-outs that are still due, oldest first (at most two wait at any time, one if there is one accumulator set: a
-    // tile is read out before its set is needed again, see below).
+    // The read-out that is still due: one at most, since a warpgroup's next tile on duty is kDBuf tiles on (all on every
+    // tile where there is one set) and a tile is read out before its set is needed again, see below.
     struct Pending { int b, nt; uint32_t it; int wait; int32_t slot; float w; };
-    Pending pq0{0, 0, 0, 0, -1, 1.f}, pq1{0, 0, 0, 0, -1, 1.f};
-    int n_pend = 0;
+    Pending due{0, 0, 0, 0, -1, 1.f};
+    bool is_due = false;
     // This group's stages are g = grp, grp + kGroups, ... whatever the tile boundaries, so its ring
     // positions advance by a fixed step per converted stage (no division in the loop).
     constexpr uint32_t kDU = (uint32_t)(kGroups * Cfg::kUnits);           // units per own-stage step
@@ -793,7 +789,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     // (b, nt) of the tile advance with it: no division in the loop
     const int step_b = (int)gridDim.x / n_tiles, step_nt = (int)gridDim.x - step_b * n_tiles;
     int b = (int)blockIdx.x / n_tiles, nt = (int)blockIdx.x - b * n_tiles;
-    // One step a pass: read out the oldest tile that is due, convert the next own stage, or go on to the next tile.  (Steps
+    // One step a pass: read out the tile that is due, convert the next own stage, or go on to the next tile.  (Steps
     // of one loop, so that the code of a read-out is there once.)
     uint32_t it = 0;
     int t = (int)blockIdx.x, vs = (int)grp;
@@ -803,11 +799,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
       // kDBuf further on, which re-use its accumulator set, can start.  Reading it out no later than
       // here (before any stage of tile it + 1 is converted) keeps every converted stage consumable,
       // so the A slots can never fill up with stages that wait for a read-out.
-      if (n_pend > 0 && (pq0.wait <= 0 || !tiles_left || (tile_done && (pq0.it + (uint32_t)Cfg::kDBuf <= it + 1u || n_pend == 2)))) {
-        const Pending e = pq0;
-        if (Cfg::kDBuf > 1) pq0 = pq1;
-        --n_pend;
-        if (guard.aborted() || !run_epilogue(e.b, e.nt, e.it, e.slot, e.w)) break;
+      if (is_due && (due.wait <= 0 || !tiles_left || (tile_done && due.it + (uint32_t)Cfg::kDBuf <= it + 1u))) {
+        is_due = false;
+        if (guard.aborted() || !run_epilogue(due.b, due.nt, due.it, due.slot, due.w)) break;
         continue;
       }
       if (!tiles_left) break;
@@ -815,10 +809,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         // is this warpgroup on read-out duty for this tile?
         const int cg = first_group(it);
         if (cg < Cfg::kColGroups) {
-          Pending e{b, nt, it, Cfg::kDBuf >= 2 ? kEpiDelay : 1, -1, 1.f};   // one set: the next tile's MMAs wait for it
-          load_cols(b, cg * 16, e.slot, e.w);
-          if (Cfg::kDBuf == 1 || n_pend == 0) pq0 = e; else pq1 = e;
-          ++n_pend;
+          due = Pending{b, nt, it, Cfg::kDBuf >= 2 ? kEpiDelay : 1, -1, 1.f};   // one set: the next tile's MMAs wait for it
+          load_cols(b, cg * 16, due.slot, due.w);
+          is_due = true;
         }
         vs -= v_stages;
         t += (int)gridDim.x;
@@ -965,8 +958,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         aq += kDU; if (aq >= (uint32_t)Cfg::kASlots) aq -= Cfg::kASlots;
         abar += kDU; if (abar >= (uint32_t)Cfg::kABars) { abar -= Cfg::kABars; acyc ^= 1u; }
         vs += kGroups;
-        --pq0.wait;
-        if (Cfg::kDBuf > 1) --pq1.wait;
+        --due.wait;
       }
     }
   }
