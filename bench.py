@@ -379,9 +379,9 @@ def run_single_gpu(args):
     gemm_avg_ms = sum(gemm_ms) / max(len(gemm_ms), 1)
     achieved = alg_bytes / (gemm_avg_ms * 1e-3) / 1e9
     # DRAM traffic per launch from the ncu capture of the 16-expert relative of this workload
-    # (--case int4_decode_small: 273.9 MB read+write for 264.2 MB of weights and scales); traffic
-    # grows with the experts touched, so it is scaled by n_active / 16.
-    traffic = 273.9e6 * n_active / 16.0
+    # (--case int4_decode_small: 268.1 MB read and 5.3 MB written for 264.2 MB of weights and scales, by the same
+    # 32-token instance); traffic grows with the experts touched, so it is scaled by n_active / 16.
+    traffic = 273.4e6 * n_active / 16.0
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
                 "traffic_source": "estimated: ncu dram bytes of a 16-expert capture scaled by experts touched",
