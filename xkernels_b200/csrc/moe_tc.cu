@@ -774,8 +774,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
     // The read-out that is still due: one at most, since a warpgroup's next tile on duty is kDBuf tiles on (all on every
     // tile where there is one set) and a tile is read out before its set is needed again, see below.
     struct Pending { int b, nt; uint32_t it; int wait; int32_t slot; float w; };
-    Pending due{0, 0, 0, 0, -1, 1.f};
-    bool is_due = false;
+    Pending due{-1, 0, 0, 0, -1, 1.f};   // b < 0: none
     // This group's stages are g = grp, grp + kGroups, ... whatever the tile boundaries, so its ring
     // positions advance by a fixed step per converted stage (no division in the loop).
     constexpr uint32_t kDU = (uint32_t)(kGroups * Cfg::kUnits);           // units per own-stage step
@@ -799,9 +798,10 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
       // kDBuf further on, which re-use its accumulator set, can start.  Reading it out no later than
       // here (before any stage of tile it + 1 is converted) keeps every converted stage consumable,
       // so the A slots can never fill up with stages that wait for a read-out.
-      if (is_due && (due.wait <= 0 || !tiles_left || (tile_done && due.it + (uint32_t)Cfg::kDBuf <= it + 1u))) {
-        is_due = false;
-        if (guard.aborted() || !run_epilogue(due.b, due.nt, due.it, due.slot, due.w)) break;
+      if (due.b >= 0 && (due.wait <= 0 || !tiles_left || (tile_done && due.it + (uint32_t)Cfg::kDBuf <= it + 1u))) {
+        const Pending e = due;
+        due.b = -1;
+        if (guard.aborted() || !run_epilogue(e.b, e.nt, e.it, e.slot, e.w)) break;
         continue;
       }
       if (!tiles_left) break;
@@ -811,7 +811,6 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_consta
         if (cg < Cfg::kColGroups) {
           due = Pending{b, nt, it, Cfg::kDBuf >= 2 ? kEpiDelay : 1, -1, 1.f};   // one set: the next tile's MMAs wait for it
           load_cols(b, cg * 16, due.slot, due.w);
-          is_due = true;
         }
         vs -= v_stages;
         t += (int)gridDim.x;
