@@ -21,11 +21,3 @@ def test_sizes(numel, E, block, kind, cuda_device):
     if kind == "dropped":
         ids = torch.where(torch.rand(numel, 1, generator=g) < 0.5, torch.full_like(ids, E), ids)
     check(ids, block, E, False, cuda_device)
-
-
-@pytest.mark.parametrize("numel,E,block", [(1025, 5, 1000), (3001, 37, 100), (16381, 1000, 77)])
-def test_fills_that_end_lane_by_lane(numel, E, block, cuda_device):
-    """Paddings and tails whose lengths are no multiples of a warp, right before the cluster's last barrier."""
-    ids = torch.randint(0, E, (numel, 1), generator=torch.Generator().manual_seed(E), dtype=torch.int32)
-    for _ in range(5):
-        check(ids, block, E, False, cuda_device)

@@ -1,13 +1,12 @@
 """Decode batches, whose routing the activation gather sorts itself (up to 512 slots, 148 blocks and a top-k of 32):
 both sides of those limits, few and many experts, dropped slots, an expert map.  The generic path, which
-takes the sort's own kernels, is the check: same bf16 weights, fp32 sums in another order.  Each path has a workspace of its
-own full of NaN, so that neither returns rows the other left there."""
+takes the sort's own kernels, is the check: same bf16 weights, fp32 sums in another order."""
 
 import pytest
 import torch
 
 import xkernels_b200 as xkb
-from tests.gpu_util import assert_within, poisoned_workspace
+from tests.gpu_util import assert_within
 from xkernels_b200 import ops, synth
 
 pytestmark = pytest.mark.gpu
@@ -30,15 +29,9 @@ def test_int4(M, top_k, E, dropped, cuda_device):
         emap = torch.arange(E, dtype=torch.int32, device=cuda_device).flip(0).contiguous()
         emap[::5] = -1
     args = (A, packed, scale, ids, w)
-
-    def own_workspace(path):
-        ws = poisoned_workspace("xkb_fused_moe_int4_w4a16_workspace_bytes", M, N, K, E, top_k, 0, device=cuda_device)
-        out = xkb.fused_moe_int4_w4a16(*args, expert_map=emap, path=path, workspace=ws)
-        ops.check_workspace_status(ws)
-        return out
-
-    got = own_workspace("tc")
-    assert_within(got, own_workspace("simt"), 1e-2, 1e-2, what="tc vs simt")
+    got = xkb.fused_moe_int4_w4a16(*args, expert_map=emap, path="tc")
+    ops.check_status(cuda_device)
+    assert_within(got, xkb.fused_moe_int4_w4a16(*args, expert_map=emap, path="simt"), 1e-2, 1e-2, what="tc vs simt")
     assert torch.equal(got, xkb.fused_moe_int4_w4a16(*args, expert_map=emap, path="tc"))
 
 

@@ -16,9 +16,9 @@ KEYS = ("A", "packed", "scale", "topk_ids", "topk_w")
 @pytest.mark.parametrize("M,K,N,E,top_k,group", [
     (1, 1024, 128, 8, 2, 128),     # one tile row, one lap of a scale tile
     (16, 2048, 256, 8, 2, 128),    # 16-token tiles, two laps
-    (17, 1024, 384, 8, 3, 64),     # 32-token tiles
+    (17, 1024, 384, 8, 3, 64),
     (64, 1024, 128, 8, 3, 64),     # 64-token tiles
-    (33, 2048, 256, 2, 2, 256),    # the same, one scale per stage
+    (33, 2048, 256, 2, 2, 256),    # 64-token tiles, one scale per stage
     (96, 1024, 256, 6, 4, 128),    # 128-token tiles, two row tiles per token tile
     (300, 2048, 128, 3, 2, 256),   # 128-token tiles, one row tile
     (5, 1280, 128, 4, 2, 128),     # K is not a multiple of eight groups: the generic path
