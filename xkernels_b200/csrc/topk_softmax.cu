@@ -45,6 +45,18 @@ template <> __device__ __forceinline__ float load_logit<__nv_bfloat16>(const __n
 }
 template <> __device__ __forceinline__ float load_logit<__half>(const __half* p) { return __half2float(*p); }
 
+// The largest of the warp's values that are not NaN (-inf if all are).
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // The id of a lane's t-th expert is lane * P plus this; a lane's ids ascend with t.
 template <int P> struct Deal { static __device__ __forceinline__ constexpr int at(int t) { return t / P * 32 * P + t % P; } };
 
@@ -52,7 +64,7 @@ template <int P> struct Deal { static __device__ __forceinline__ constexpr int a
 template <int PER_LANE, int P>
 __device__ __forceinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t row, int lane, int topk, int renormalize,
                                               float* __restrict__ topk_w, int32_t* __restrict__ topk_ids) {
-  float wsum = 0.f;
+  float rest = 0.f;     // every lane's share of the sum of further ones (600 weights added one by one were off by 2.2e-6 of it)
   float my_w = 0.f;     // lane j keeps the j-th selected weight (j < 32), further ones go out directly
   for (int j = 0; j < topk; ++j) {
     float bp = -1.f;
@@ -70,32 +82,24 @@ __device__ __forceinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t r
 #pragma unroll
     for (int t = 0; t < PER_LANE; ++t)
       if (Deal<P>::at(t) == bi - lane * P) p[t] = -1.f;
-    wsum += bp;
     if (lane == 0) topk_ids[row * topk + j] = bi;
     if (renormalize) {
-      if (j < 32) { if (lane == j) my_w = bp; }
-      else if (lane == 0) topk_w[row * topk + j] = bp;   // divided below
+      if (j < 32) {
+        if (lane == j) my_w = bp;
+      } else {
+        if (lane == (j & 31)) rest += bp;
+        if (lane == 0) topk_w[row * topk + j] = bp;   // divided below
+      }
     } else if (lane == 0) {
       topk_w[row * topk + j] = bp;
     }
   }
   if (renormalize) {
+    const float wsum = warp_sum(my_w + rest);
     if (lane < topk) topk_w[row * topk + lane] = my_w / wsum;
     if (lane == 0)
       for (int j = 32; j < topk; ++j) topk_w[row * topk + j] = topk_w[row * topk + j] / wsum;
   }
-}
-
-// The largest of the warp's values that are not NaN (-inf if all are).
-__device__ __forceinline__ float warp_max(float v) {
-  float r;
-  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
 }
 
 // Counts of up to four or eight pieces, eight bits each.
