@@ -23,7 +23,8 @@
 // M=16384, E=256, bf16, top 8, renormalised, on the device: 28.7 us with the rounds; 10.9 with single logits dealt to the lanes
 // and a loop over all candidates; 9.3 with eight neighbours a lane, but 28.3, 17.1 and 9.6 where one, two and four groups of 32
 // are live, 22.1 for sorted rows; 9.2 with pieces of two, and 9.3, 9.4, 9.5 and 9.5 for those rows.  (E=1024, where the
-// rounds are common: top 8 34.4 / 21.0 / 20.5, top 20 158 / 105 / 114, top 32 227 / 165 / 181.)
+// rounds are common, a call in a loop: top 8 34.4 / 22.9 / 20.8, top 20 158 / 106 / 109, top 32 227 / 166 / 168; all logits
+// equal, top 8 - / 55.4 / 57.5.)
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -60,7 +61,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // The id of a lane's t-th expert is lane * P plus this; a lane's ids ascend with t.
 template <int P> struct Deal { static __device__ __forceinline__ constexpr int at(int t) { return t / P * 32 * P + t % P; } };
 
-// k rounds over the whole row: p[t] = probability of the lane's t-th expert, or -1 where there is none.
+// k rounds over the whole row: p[t] = probability of the lane's t-th expert, 0 behind the row.
 template <int PER_LANE, int P>
 __device__ __forceinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t row, int lane, int topk, int renormalize,
                                               float* __restrict__ topk_w, int32_t* __restrict__ topk_ids) {
@@ -69,9 +70,19 @@ __device__ __forceinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t r
   for (int j = 0; j < topk; ++j) {
     float bp = -1.f;
     int bt = 0;
+    // a lane's ids ascend: the first of equal ones stays.  (Many experts: the maximum first, which takes half the instructions of
+    // carrying the id along.  M=16384, top 32 of 1024: 178 -> 168 us; top 24 of 128: 35 -> 40, so not there.)
+    if constexpr (PER_LANE >= 8) {
 #pragma unroll
-    for (int t = 0; t < PER_LANE; ++t)   // a lane's ids ascend: the first of equal ones stays
-      if (p[t] > bp) { bp = p[t]; bt = Deal<P>::at(t); }
+      for (int t = 0; t < PER_LANE; ++t) bp = fmaxf(bp, p[t]);
+#pragma unroll
+      for (int t = PER_LANE - 1; t >= 0; --t)
+        if (p[t] == bp) bt = Deal<P>::at(t);
+    } else {
+#pragma unroll
+      for (int t = 0; t < PER_LANE; ++t)
+        if (p[t] > bp) { bp = p[t]; bt = Deal<P>::at(t); }
+    }
     const int mine = bp >= 0.f ? lane * P + bt : 0x7fffffff;
     // best of the warp: bp is -1 or >= 0 and never NaN (no comparison with one holds), so its bits order as signed integers
     const int top = __reduce_max_sync(0xffffffffu, __float_as_int(bp));
@@ -102,20 +113,12 @@ __device__ __forceinline__ void select_by_rounds(float (&p)[PER_LANE], int64_t r
   }
 }
 
-// Counts of up to four or eight pieces, eight bits each.
-template <bool WIDE> struct FieldsOf { using type = uint32_t; };
-template <> struct FieldsOf<true> { using type = unsigned long long; };
-__device__ __forceinline__ int sum_of_fields(uint32_t v) { return (int)__dp4a(v, 0x01010101u, 0u); }
-__device__ __forceinline__ int sum_of_fields(unsigned long long v) {
-  return (int)__dp4a((uint32_t)(v >> 32), 0x01010101u, __dp4a((uint32_t)v, 0x01010101u, 0u));
-}
-
 // Experts per lane, in the order of the instances: an instance takes the rows that the one before it does not hold.
 template <int PER_LANE> constexpr int kPerLaneBefore = PER_LANE == 16 ? 12 : PER_LANE == 12 ? 8 : PER_LANE / 2;
 
 // P > 1: E is a multiple of P and every row lies on a boundary of P logits, so that a piece is in the row or not.
 template <typename T, int PER_LANE, int P>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, PER_LANE == 32 ? 0 : 1)   // (1 against 0, which leaves it open: E=256 9.2 / 9.4 us, E=1024 23.7 / 20.4)
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, PER_LANE == 32 ? 0 : 1)   // (1 against 0, which leaves it open: E=256 9.2 / 9.4 us; E=1024, all logits equal, 58.6 / 57.5)
 topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, int32_t* __restrict__ topk_ids,
                     int64_t M, int E, int topk, int renormalize) {
   __shared__ uint2 s_cand[kWarpsPerBlock][32];   // candidates by ascending id: exponential, id
@@ -177,41 +180,57 @@ topk_softmax_kernel(const T* __restrict__ gating, float* __restrict__ topk_w, in
   float bound = 0.f;
   if (short_way && tau >= 0.f && tau >= sum * 7.8886090522101181e-31f)   // 2^-100
     bound = tau * (1.f - 9.5367431640625e-7f);
-  // an exponential is a candidate from here on; experts behind the row never are (none is infinite on the short way)
-  auto low = [&](int t) -> float { return valid(t) ? bound : INFINITY; };
+  // An exponential is a candidate from here on.  Places behind the row hold 0: with a bound of 0 the row's own experts,
+  // more than 32 from two a lane on, are candidates too, and the row takes the rounds.
+  auto low = [&](int t) -> float { return PER_LANE > 1 || valid(t) ? bound : INFINITY; };
   // Candidates are counted piece by piece.  P > 1: a lane's counts are fields of eight bits (a piece has at most 128
-  // candidates in the warp), so that one sum over the lanes serves all pieces.
-  using Fields = typename FieldsOf<(kPieces > 4)>::type;
-  Fields mine = 0, upto = 0, all = 0;   // this lane's, the lanes' up to it, the warp's
-  int n = 0;
-  if constexpr (P > 1) {
+  // candidates in the warp), so that one sum over the lanes serves four pieces.
+  constexpr int kWords = (kPieces + 3) / 4;
+  uint32_t mine[kWords] = {}, upto[kWords] = {}, all[kWords] = {};   // this lane's, the lanes' up to it, the warp's
+  int n = 33;
+  if (PER_LANE > 8 && !short_way) {   // (a branch for up to eight costs the short way more than it gives: E=256 10.4 / 10.9 us)
+  } else if constexpr (P > 1) {
+    n = 0;
 #pragma unroll
-    for (int t = 0; t < PER_LANE; ++t) mine += p[t] >= low(t) ? Fields(1) << (8 * (t / P)) : Fields(0);
-    upto = mine;
+    for (int t = 0; t < PER_LANE; ++t) mine[t / P / 4] += p[t] >= low(t) ? 1u << (8 * (t / P % 4)) : 0u;
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) upto[i] = mine[i];
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      const Fields below = __shfl_up_sync(0xffffffffu, upto, d);
-      if (lane >= d) upto += below;
+#pragma unroll
+      for (int i = 0; i < kWords; ++i) {
+        const uint32_t below = __shfl_up_sync(0xffffffffu, upto[i], d);
+        if (lane >= d) upto[i] += below;
+      }
     }
-    all = __shfl_sync(0xffffffffu, upto, 31);
-    n = sum_of_fields(all);
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
+      all[i] = __shfl_sync(0xffffffffu, upto[i], 31);
+      n = (int)__dp4a(all[i], 0x01010101u, (uint32_t)n);
+    }
   } else {
+    n = 0;
 #pragma unroll
     for (int t = 0; t < PER_LANE; ++t) n += __popc(__ballot_sync(0xffffffffu, p[t] >= low(t)));
   }
   if (!short_way || n > 32) {
 #pragma unroll
-    for (int t = 0; t < PER_LANE; ++t) p[t] = valid(t) ? p[t] / sum : -1.f;
+    for (int t = 0; t < PER_LANE; ++t) p[t] = p[t] / sum;   // (behind the row: 0, or NaN if all are, and higher ids than topk needs)
     select_by_rounds<PER_LANE, P>(p, row, lane, topk, renormalize, topk_w, topk_ids);
     return;
   }
   uint2* cand = s_cand[warp];
   const uint32_t cand_u32 = (uint32_t)__cvta_generic_to_shared(cand);
   if constexpr (P > 1) {
-    const Fields first = upto - mine + all * Fields(0x0101010101010100ull);   // (the fields before it, and the lanes before)
+    uint32_t first[kWords], before = 0;   // the fields before it, and the lanes before
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
+      first[i] = upto[i] - mine[i] + all[i] * 0x01010100u + before * 0x01010101u;
+      before = __dp4a(all[i], 0x01010101u, before);
+    }
 #pragma unroll
     for (int c = 0; c < kPieces; ++c) {
-      uint32_t to = cand_u32 + (uint32_t)(first >> (8 * c) & 0xFFu) * 8u;
+      uint32_t to = cand_u32 + (first[c / 4] >> (8 * (c % 4)) & 0xFFu) * 8u;
 #pragma unroll
       for (int i = 0; i < P; ++i)   // predicated: a branch each took twice as many instructions
         asm volatile("{\n\t.reg .pred q;\n\tsetp.ge.f32 q, %1, %2;\n\t@q st.shared.v2.b32 [%0], {%3, %4};\n\t@q add.u32 %0, %0, 8;\n\t}"
